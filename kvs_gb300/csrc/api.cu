@@ -308,7 +308,9 @@ void gather_setup(kvsmc_context* ctx, Plan& pl)
         pl.f = kvsmc_host::make_fast(j.ip.iso, j.ip.vmin, j.ip.vmax, dt);
         j.node_tiles = steps;   // node units, for the counts and their scan
         // the triangles too: the streaming count and the streaming connection
-        // pass when the volume takes the streaming layout with one row per task
+        // pass, with one row per task at every width (a 385-node row leaves a
+        // quarter of the lanes idle and still takes 1/3 of the gather
+        // kernels' time)
         if (pl.sb) {
             pl.sconn = true;
             j.cell_tiles = 0;
@@ -316,17 +318,15 @@ void gather_setup(kvsmc_context* ctx, Plan& pl)
             pl.batch.reset(new StreamBatch());
             pl.batch->ctx = ctx;
             pl.batch->items = {pl.item};
+            pl.batch->want_nodes = true;
+            pl.batch->one_row = true;
             pl.batch->plan_tables();
-            pl.sconn = pl.batch->groups.size() == 1 && pl.batch->launches.size() == 1 && pl.batch->groups[0].rows == 1;
-            if (pl.sconn) {
-                j.cell_tiles = 0;
-                pl.sb = pl.batch.get();
-                pl.sb_group = 0;
-                pl.sb_iso = 0;
-                pl.sb_tasks = pl.batch->launches[0].ntasks;
-            } else {
-                pl.batch.reset();
-            }
+            pl.sconn = true;
+            j.cell_tiles = 0;
+            pl.sb = pl.batch.get();
+            pl.sb_group = 0;
+            pl.sb_iso = 0;
+            pl.sb_tasks = pl.batch->launches[0].ntasks;
         }
     }
 }
@@ -342,6 +342,12 @@ size_t gather_own_bytes(const Plan& pl)
            align_up(rank_words * 16, 256) + align_up(scan_scratch_bytes(ct), 256) + align_up(scan_scratch_bytes(nt), 256);
 }
 
+// Bytes a request of a grouped pass keeps to itself: its rank words.
+size_t grouped_own_bytes(const Plan& pl)
+{
+    return (size_t)pl.job.vol.nz * pl.job.vol.ny * pl.job.words_per_row * 16;
+}
+
 // Count pass of one set-up request with its arrays carved from `base`
 // (gather_own_bytes, then its own streaming count): fills pl.ntri / pl.nvert
 // and leaves the per-tile offsets there for gather_emit.
@@ -352,7 +358,11 @@ kvsmc_status gather_count_at(kvsmc_context* ctx, Plan& pl, char* base)
     const uint64_t rank_words = pl.shared ? (uint64_t)j.vol.nz * j.vol.ny * j.words_per_row : 0;
     const size_t own = gather_own_bytes(pl);
     Carve cv{base};
+    // totals (triangles, vertices), the status word and the task counters, in
+    // one piece: one memset, one read-back
     uint64_t* d_totals = cv.take<uint64_t>(256);
+    pl.d_status = reinterpret_cast<int*>(d_totals + 2);
+    pl.d_next = reinterpret_cast<unsigned long long*>(d_totals + 3);
     j.tile_counts = cv.take<uint32_t>(ct * 4);
     j.tile_offsets = cv.take<uint64_t>(ct * 8);
     j.vtile_counts = cv.take<uint32_t>(nt * 4);
@@ -360,36 +370,37 @@ kvsmc_status gather_count_at(kvsmc_context* ctx, Plan& pl, char* base)
     j.rank = cv.take<uint4>(rank_words * 16);
     void* scan_a = cv.take<char>(scan_scratch_bytes(ct));
     void* scan_b = cv.take<char>(scan_scratch_bytes(nt));
-    pl.d_status = cv.take<int>(256);
-    pl.d_next = cv.take<unsigned long long>(256);
     const kvsmc::Launch L = launch_of(ctx);
-    KVSMC_CUDA(ctx, cudaMemsetAsync(d_totals, 0, 3 * sizeof(uint64_t), ctx->stream));
+    KVSMC_CUDA(ctx, cudaMemsetAsync(d_totals, 0, 256, ctx->stream));
     if (pl.sconn && pl.batch) {
         // unit counts, unit scan, plane scan: the streaming count of one request
         pl.batch->carve(base + own);
         kvsmc_status bst = pl.batch->upload_tables();
-        if (!bst) bst = pl.batch->count();
+        // (the tables' host copies may be overwritten by the read-back below
+        // only once they have left: both are copies on this stream, in order)
+        if (!bst) bst = pl.batch->count_enqueue();
         if (bst) return bst;
+        const kvsmc::StreamGroup& G = pl.batch->groups[0];
+        if (G.node_units) pl.sb_nodes = pl.batch->d_node_counts + G.node_base;
     }
     if (ct) {
         KVSMC_CUDA(ctx, launch_cell_count(j, L));
         KVSMC_CUDA(ctx, launch_scan(j.tile_counts, j.tile_offsets, ct, scan_a, d_totals, L));
     }
     if (nt && pl.snode) {
-        KVSMC_CUDA(ctx, cudaMemsetAsync(pl.d_status, 0, sizeof(int), ctx->stream));
-        KVSMC_CUDA(ctx, cudaMemsetAsync(pl.d_next, 0, 3 * sizeof(unsigned long long), ctx->stream));
         if (!pl.sb_nodes)
             KVSMC_CUDA(ctx, kvsmc::launch_snode(false, j, pl.f, pl.wprn, pl.zchunk, pl.ntasks, j.vtile_counts,
                                                 nullptr, pl.d_status, pl.d_next, L));
         KVSMC_CUDA(ctx, launch_scan(pl.sb_nodes ? pl.sb_nodes : j.vtile_counts, j.vtile_offsets, nt, scan_b,
                                     d_totals + 1, L));
-        KVSMC_CUDA(ctx, cudaMemcpyAsync(d_totals + 2, pl.d_status, sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
     } else if (nt) {
         KVSMC_CUDA(ctx, launch_node_count(j, L));
         KVSMC_CUDA(ctx, launch_scan(j.vtile_counts, j.vtile_offsets, nt, scan_b, d_totals + 1, L));
     }
     KVSMC_CUDA(ctx, cudaMemcpyAsync(ctx->h_small, d_totals, 3 * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->stream));
     KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (pl.sconn && pl.batch)
+        if (kvsmc_status bst = pl.batch->count_finish()) return bst;
     if (ctx->h_small[2]) return fail(ctx, KVSMC_ERR_TIMEOUT, "shared-vertex count: a shared-memory load did not complete");
     pl.ntri = pl.sconn ? pl.item->sizes.ntriangles : ctx->h_small[0];
     pl.nvert = pl.shared ? ctx->h_small[1] : 3 * pl.ntri;
@@ -464,24 +475,17 @@ kvsmc_status gather_emit(kvsmc_context* ctx, Plan& pl, float* coords, float* nor
     } else {
         j.tri_normals = nullptr;
     }
-    // A pass whose bounded waits gave up leaves its outputs unwritten: the next
-    // pass would read those as vertex ids, so the status is checked before it.
-    auto check_status = [&](const char* what) -> kvsmc_status {
-        int* h = reinterpret_cast<int*>(ctx->h_small);
-        KVSMC_CUDA(ctx, cudaMemcpyAsync(h, pl.d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-        KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        if (*h == 1) return fail(ctx, KVSMC_ERR_TIMEOUT, "%s: a shared-memory load did not complete", what);
-        if (*h) return fail(ctx, KVSMC_ERR_CUDA, "%s: a vertex id out of range", what);
-        return KVSMC_OK;
-    };
-    kvsmc_status st = KVSMC_OK;
+    // A pass whose bounded waits gave up leaves its outputs unwritten.  The
+    // connection pass then writes nothing (it reads the node emit's status
+    // word), the vertex normals check every id they follow, and the status is
+    // read once behind them all.
+    const bool own_passes = pl.snode && !pl.nodes_done && pl.nvert;
     if (pl.nodes_done) {
         // written already
     } else if (pl.nvert && pl.snode) {
         uint32_t* counts = const_cast<uint32_t*>(pl.sb_nodes ? pl.sb_nodes : j.vtile_counts);
         KVSMC_CUDA(ctx, kvsmc::launch_snode(true, j, pl.f, pl.wprn, pl.zchunk, pl.ntasks, counts, j.vtile_offsets,
                                             pl.d_status, pl.d_next + 1, L));
-        if ((st = check_status("shared-vertex node emit"))) return st;
     } else if (pl.nvert) {
         KVSMC_CUDA(ctx, launch_node_emit(j, L));
     }
@@ -492,7 +496,6 @@ kvsmc_status gather_emit(kvsmc_context* ctx, Plan& pl, float* coords, float* nor
         KVSMC_CUDA(ctx, kvsmc::launch_sconnect(j, b.d_groups + pl.sb_group, b.d_isos, b.d_unit_counts,
                                                b.d_unit_offsets, b.d_plane_base, pl.sb_iso, pl.sb_tasks, pl.nvert,
                                                pl.ntri, pl.d_status, pl.d_next + 2, L));
-        if ((st = check_status("shared-vertex connections"))) return st;
     } else if (pl.ntri) {
         KVSMC_CUDA(ctx, launch_connect(j, L));
     }
@@ -503,6 +506,13 @@ kvsmc_status gather_emit(kvsmc_context* ctx, Plan& pl, float* coords, float* nor
         // (calculate_normals_on_vertex adds nothing to its zeroed array)
         KVSMC_CUDA(ctx, cudaMemsetAsync(j.normals, 0, 12 * pl.nvert, ctx->stream));
     }
+    if (own_passes) {
+        int* h = reinterpret_cast<int*>(ctx->h_small);
+        KVSMC_CUDA(ctx, cudaMemcpyAsync(h, pl.d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        if (*h == 1) return fail(ctx, KVSMC_ERR_TIMEOUT, "shared-vertex passes: a shared-memory load did not complete");
+        if (*h) return fail(ctx, KVSMC_ERR_CUDA, "shared-vertex connections: a vertex id out of range");
+    }
     return KVSMC_OK;
 }
 
@@ -511,9 +521,8 @@ kvsmc_status gather_emit(kvsmc_context* ctx, Plan& pl, float* coords, float* nor
 // isolevels per group), and each request's connection pass takes its
 // isolevel's unit offsets from it.  The same pass counts each request's
 // vertices per node unit (groups whose node segments are their cell
-// segments), so the requests skip their node count passes.  Requests whose
-// group does not take one row per task, and a batch with a single such
-// request, keep their own counts.
+// segments), so the requests skip their node count passes.  A batch with a
+// single such request keeps its own count.
 struct SharedCount {
     std::unique_ptr<StreamBatch> sb;
     std::vector<Item*> cand;   // the requests counted here
@@ -550,8 +559,8 @@ kvsmc_status shared_count(kvsmc_context* ctx, const std::vector<Item*>& items, S
         const int m = it->params.mode, dt = it->vol->view.dtype;
         if ((m == KVSMC_SHARED_POLYGON_NORMAL || m == KVSMC_SHARED_VERTEX_NORMAL) && ctx->path == 0 &&
             (dt == KVSMC_I8 || dt == KVSMC_I16 || dt == KVSMC_U8 || dt == KVSMC_U16 || dt == KVSMC_F32) &&
-            stream_volume_eligible(ctx, *it) && stream_shape(ctx, it->vol->view).rows == 1)
-            sc.cand.push_back(it);   // (the connection pass takes one-row tasks only)
+            stream_volume_eligible(ctx, *it))
+            sc.cand.push_back(it);
     }
     if (sc.cand.size() < 2) {
         sc.cand.clear();
@@ -562,6 +571,7 @@ kvsmc_status shared_count(kvsmc_context* ctx, const std::vector<Item*>& items, S
     b.ctx = ctx;
     b.items = sc.cand;
     b.want_nodes = true;
+    b.one_row = true;
     b.plan_tables();
     const size_t need = b.scratch_bytes();
     if (need > ctx->arena3_bytes) {
@@ -587,7 +597,6 @@ kvsmc_status shared_count(kvsmc_context* ctx, const std::vector<Item*>& items, S
     for (const StreamBatch::Launch1& l : b.launches) {
         for (int g = l.g0; g < l.g0 + l.ng; ++g) {
             const kvsmc::StreamGroup& G = b.groups[g];
-            if (G.rows != 1) continue;
             const uint64_t end = g + 1 < l.g0 + l.ng ? b.groups[g + 1].task_begin : l.ntasks;
             for (int k = 0; k < G.niso; ++k) {
                 const uint32_t* nodes = G.node_units ? b.d_node_counts + G.node_base + (uint64_t)k * G.node_units
@@ -617,15 +626,36 @@ kvsmc_status grouped_shared(kvsmc_context* ctx, const SharedCount& sc, std::vect
                             const std::function<kvsmc_status(Item*, int)>& ready = {})
 {
     std::vector<Plan> plans(items.size());
+    std::map<const Item*, Plan*> plan_of;
     size_t total = 0;
     std::vector<size_t> off(items.size());
     for (size_t i = 0; i < items.size(); ++i) {
         gather_plan(*items[i], plans[i]);
         sc.attach(items[i], plans[i]);
         gather_setup(ctx, plans[i]);
+        plan_of[items[i]] = &plans[i];
         off[i] = total;
-        total += align_up(gather_own_bytes(plans[i]), 256);
+        total += align_up(grouped_own_bytes(plans[i]), 256);
     }
+    // per group: one scan of all its requests' vertex counts (request k's node
+    // units follow request k - 1's), so a request's first vertex ids are its
+    // entries less its first one
+    const StreamBatch& b = *sc.sb;
+    std::vector<char> used(b.groups.size(), 0);
+    for (size_t g = 0; g < b.groups.size(); ++g)
+        for (int k = 0; k < b.groups[g].niso; ++k)
+            if (b.groups[g].node_units && plan_of.count(b.iso_item[b.groups[g].iso_begin + k])) used[g] = 1;
+    std::vector<size_t> goff(b.groups.size());
+    for (size_t g = 0; g < b.groups.size(); ++g) {
+        goff[g] = total;
+        if (!used[g]) continue;
+        const uint64_t n = (uint64_t)b.groups[g].niso * b.groups[g].node_units;
+        total += align_up(n * 8, 256) + align_up(scan_scratch_bytes(n), 256);
+    }
+    const size_t totals_off = total;
+    total += align_up((b.isos.size() + b.groups.size()) * 8, 256);
+    const size_t status_off = total;
+    total += align_up(b.groups.size() * 64, 256);   // per group: status word, two task counters
     const size_t tables = align_up((size_t)kvsmc::kStreamMaxIso * sizeof(kvsmc::NodeIso), 256) +
                           align_up((size_t)kvsmc::kStreamMaxIso * sizeof(kvsmc::ConnIso), 256);
     const size_t need = total + tables;
@@ -643,13 +673,48 @@ kvsmc_status grouped_shared(kvsmc_context* ctx, const SharedCount& sc, std::vect
         ctx->arena4_bytes = want;
     }
     char* base = static_cast<char*>(ctx->arena4);
+    const kvsmc::Launch L = launch_of(ctx);
+    uint64_t* d_vtot = reinterpret_cast<uint64_t*>(base + totals_off);   // per isolevel, then per group the grand total
+    char* d_status_all = base + status_off;
+    KVSMC_CUDA(ctx, cudaMemsetAsync(d_status_all, 0, b.groups.size() * 64, ctx->stream));
+    for (size_t g = 0; g < b.groups.size(); ++g) {
+        if (!used[g]) continue;
+        const kvsmc::StreamGroup& G = b.groups[g];
+        const uint64_t n = (uint64_t)G.niso * G.node_units;
+        uint64_t* d_off = reinterpret_cast<uint64_t*>(base + goff[g]);
+        uint64_t* d_grand = d_vtot + b.isos.size() + g;
+        KVSMC_CUDA(ctx, launch_scan(b.d_node_counts + G.node_base, d_off, n, base + goff[g] + align_up(n * 8, 256),
+                                    d_grand, L));
+        KVSMC_CUDA(ctx, kvsmc::launch_slice_totals(d_off, G.node_units, G.niso, d_grand, d_vtot + G.iso_begin, L));
+        for (int k = 0; k < G.niso; ++k) {
+            const auto f = plan_of.find(b.iso_item[G.iso_begin + k]);
+            if (f != plan_of.end()) f->second->job.vtile_offsets = d_off + (uint64_t)k * G.node_units;
+        }
+    }
+    kvsmc_status tst = ensure_stage(ctx, b.isos.size() * 8 + b.groups.size() * 64);
+    if (tst) return tst;
+    KVSMC_CUDA(ctx, cudaMemcpyAsync(ctx->h_stage, d_vtot, b.isos.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     std::vector<Item*> ok;
+    {
+        const uint64_t* h = static_cast<const uint64_t*>(ctx->h_stage);
+        for (size_t k = 0; k < b.isos.size(); ++k) {
+            const auto f = plan_of.find(b.iso_item[k]);
+            if (f != plan_of.end()) f->second->nvert = h[k];
+        }
+    }
     for (size_t i = 0; i < items.size(); ++i) {
         Item* it = items[i];
-        kvsmc_status st = gather_count_at(ctx, plans[i], base + off[i]);
-        if (!st) gather_sizes(plans[i], *it, &it->sizes);
-        if (st) it->status = st;
-        else ok.push_back(it);
+        Plan& pl = plans[i];
+        pl.ntri = it->sizes.ntriangles;
+        pl.job.rank = reinterpret_cast<uint4*>(base + off[i]);
+        if (pl.nvert > 0xffffffffull) {
+            it->status = fail(ctx, KVSMC_ERR_TOO_LARGE, "%llu shared vertices exceed 32-bit connection ids",
+                              (unsigned long long)pl.nvert);
+            continue;
+        }
+        gather_sizes(pl, *it, &it->sizes);
+        ok.push_back(it);
     }
     if (!emit || ok.empty()) return KVSMC_OK;
     if (kvsmc_status st = outputs(ok)) return st;
@@ -680,14 +745,32 @@ kvsmc_status grouped_shared(kvsmc_context* ctx, const SharedCount& sc, std::vect
                 o += align_up(12 * plans[i].ntri, 256);
             }
     }
-    std::map<const Item*, Plan*> plan_of;
-    for (size_t i = 0; i < items.size(); ++i) plan_of[items[i]] = &plans[i];
-    // one node emit per group: its requests in threshold order
-    const StreamBatch& b = *sc.sb;
+    // one node emit and one connection pass per group: its requests in
+    // threshold order.  Their tables are staged for all groups at once, since a
+    // group's copies may still be in flight when the next one's are written;
+    // the connection pass stops at once when the node emit of its group gave
+    // up, so the status words are read once, at the end (with a caller that
+    // copies finished outputs while later passes run, after each pass).
+    const size_t stage_group = (size_t)kvsmc::kStreamMaxIso * (sizeof(kvsmc::NodeIso) + sizeof(kvsmc::ConnIso));
+    if ((tst = ensure_stage(ctx, b.groups.size() * (stage_group + 64)))) return tst;
+    char* const h_status = static_cast<char*>(ctx->h_stage) + b.groups.size() * stage_group;
+    auto group_status = [&](size_t g) -> kvsmc_status {
+        int h;
+        std::memcpy(&h, h_status + 64 * g, sizeof h);
+        if (h == 1) return fail(ctx, KVSMC_ERR_TIMEOUT, "shared-vertex passes: a shared-memory load did not complete");
+        if (h) return fail(ctx, KVSMC_ERR_CUDA, "shared-vertex connections: a vertex id out of range");
+        return KVSMC_OK;
+    };
+    auto read_status = [&]() -> kvsmc_status {
+        KVSMC_CUDA(ctx, cudaMemcpyAsync(h_status, d_status_all, b.groups.size() * 64, cudaMemcpyDeviceToHost,
+                                        ctx->stream));
+        KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        return KVSMC_OK;
+    };
     kvsmc::NodeIso* d_node = reinterpret_cast<kvsmc::NodeIso*>(base + total);
     kvsmc::ConnIso* d_conn = reinterpret_cast<kvsmc::ConnIso*>(
         base + total + align_up((size_t)kvsmc::kStreamMaxIso * sizeof(kvsmc::NodeIso), 256));
-    const kvsmc::Launch L = launch_of(ctx);
+    std::vector<std::vector<Plan*>> group_plans(b.groups.size());
     for (size_t g = 0; g < b.groups.size(); ++g) {
         const kvsmc::StreamGroup& G = b.groups[g];
         std::vector<Plan*> gp;
@@ -698,72 +781,59 @@ kvsmc_status grouped_shared(kvsmc_context* ctx, const SharedCount& sc, std::vect
             gp.push_back(f->second);
         }
         if (gp.empty()) continue;
-        kvsmc_status st = ensure_stage(ctx, gp.size() * sizeof(kvsmc::NodeIso));
-        if (!st) {
-            kvsmc::NodeIso* h = static_cast<kvsmc::NodeIso*>(ctx->h_stage);
-            for (size_t k = 0; k < gp.size(); ++k) {
-                const Plan& pl = *gp[k];
-                h[k].f = pl.f;
-                h[k].ip = pl.job.ip;
-                h[k].coords = pl.item->d_coords;
-                h[k].rank = pl.job.rank;
-                h[k].offsets = pl.job.vtile_offsets;
-                h[k].counts = pl.sb_nodes;
-            }
-            const Plan& p0 = *gp[0];
-            int* d_status = p0.d_status;
-            unsigned long long* d_next = p0.d_next + 1;
-            KVSMC_CUDA(ctx, cudaMemcpyAsync(d_node, h, gp.size() * sizeof(kvsmc::NodeIso), cudaMemcpyHostToDevice,
-                                            ctx->stream));
-            KVSMC_CUDA(ctx, cudaMemsetAsync(d_status, 0, sizeof(int), ctx->stream));
-            KVSMC_CUDA(ctx, cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), ctx->stream));
-            KVSMC_CUDA(ctx, kvsmc::launch_snode_multi(p0.job.vol, d_node, (int)gp.size(), G.bs, G.bo, p0.wprn,
-                                                      p0.zchunk, p0.ntasks, p0.job.words_per_row, d_status, d_next, L));
-            int* hs = reinterpret_cast<int*>(ctx->h_small);
-            KVSMC_CUDA(ctx, cudaMemcpyAsync(hs, d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-            KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            if (*hs) st = fail(ctx, KVSMC_ERR_TIMEOUT, "shared-vertex node emit: a shared-memory load did not complete");
-            if (!st && ready)   // the vertices leave while the connections are written
-                for (Plan* p : gp)
-                    if ((st = ready(p->item, 0))) break;
-            // then the group's connection pass, every request of the group in its
-            // isolevel order (the ones not written here disabled)
-            if (!st) st = ensure_stage(ctx, (size_t)G.niso * sizeof(kvsmc::ConnIso));
-            if (!st) {
-                kvsmc::ConnIso* hc = static_cast<kvsmc::ConnIso*>(ctx->h_stage);
-                std::memset(hc, 0, (size_t)G.niso * sizeof(kvsmc::ConnIso));
-                uint64_t tasks = 0;
-                for (int k = 0; k < G.niso; ++k) {
-                    Item* it = b.iso_item[G.iso_begin + k];
-                    const auto f = plan_of.find(it);
-                    if (f == plan_of.end()) continue;
-                    const Plan& pl = *f->second;
-                    if (std::find(gp.begin(), gp.end(), f->second) == gp.end() || !pl.ntri) continue;
-                    hc[k].rank = pl.job.rank;
-                    hc[k].coords = it->d_coords;
-                    hc[k].connections = it->d_conn;
-                    hc[k].tri_out = pl.job.mode == KVSMC_SHARED_VERTEX_NORMAL ? pl.tri_normals : it->d_normals;
-                    hc[k].nvert = pl.nvert;
-                    hc[k].ntri = pl.ntri;
-                    hc[k].enabled = 1;
-                    tasks = pl.sb_tasks;
-                }
-                if (tasks) {
-                    KVSMC_CUDA(ctx, cudaMemcpyAsync(d_conn, hc, (size_t)G.niso * sizeof(kvsmc::ConnIso),
-                                                    cudaMemcpyHostToDevice, ctx->stream));
-                    KVSMC_CUDA(ctx, cudaMemsetAsync(d_status, 0, sizeof(int), ctx->stream));
-                    KVSMC_CUDA(ctx, cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), ctx->stream));
-                    KVSMC_CUDA(ctx, kvsmc::launch_sconnect_multi(b.d_groups + g, b.d_isos, d_conn, p0.job.vol.dtype,
-                                                                 b.d_unit_counts, b.d_unit_offsets, b.d_plane_base,
-                                                                 tasks, d_status, d_next, L));
-                    KVSMC_CUDA(ctx, cudaMemcpyAsync(hs, d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-                    KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-                    if (*hs == 1)
-                        st = fail(ctx, KVSMC_ERR_TIMEOUT, "shared-vertex connections: a shared-memory load did not complete");
-                    else if (*hs)
-                        st = fail(ctx, KVSMC_ERR_CUDA, "shared-vertex connections: a vertex id out of range");
-                }
-            }
+        group_plans[g] = gp;
+        char* const h_group = static_cast<char*>(ctx->h_stage) + g * stage_group;
+        kvsmc::NodeIso* h = reinterpret_cast<kvsmc::NodeIso*>(h_group);
+        for (size_t k = 0; k < gp.size(); ++k) {
+            const Plan& pl = *gp[k];
+            h[k].f = pl.f;
+            h[k].ip = pl.job.ip;
+            h[k].coords = pl.item->d_coords;
+            h[k].rank = pl.job.rank;
+            h[k].offsets = pl.job.vtile_offsets;
+            h[k].counts = pl.sb_nodes;
+        }
+        const Plan& p0 = *gp[0];
+        int* d_status = reinterpret_cast<int*>(d_status_all + 64 * g);
+        unsigned long long* d_next = reinterpret_cast<unsigned long long*>(d_status_all + 64 * g + 16);
+        KVSMC_CUDA(ctx, cudaMemcpyAsync(d_node, h, gp.size() * sizeof(kvsmc::NodeIso), cudaMemcpyHostToDevice,
+                                        ctx->stream));
+        KVSMC_CUDA(ctx, kvsmc::launch_snode_multi(p0.job.vol, d_node, (int)gp.size(), G.bs, G.bo, p0.wprn, p0.zchunk,
+                                                  p0.ntasks, p0.job.words_per_row, d_status, d_next, L));
+        kvsmc_status st = KVSMC_OK;
+        if (ready) {   // the vertices leave while the connections are written
+            if (!(st = read_status())) st = group_status(g);
+            for (Plan* p : gp)
+                if (st || (st = ready(p->item, 0))) break;
+        }
+        // then the group's connection pass, every request of the group in its
+        // isolevel order (the ones not written here disabled)
+        kvsmc::ConnIso* hc = reinterpret_cast<kvsmc::ConnIso*>(h_group + (size_t)kvsmc::kStreamMaxIso *
+                                                                             sizeof(kvsmc::NodeIso));
+        std::memset(hc, 0, (size_t)G.niso * sizeof(kvsmc::ConnIso));
+        uint64_t tasks = 0;
+        for (int k = 0; k < G.niso; ++k) {
+            Item* it = b.iso_item[G.iso_begin + k];
+            const auto f = plan_of.find(it);
+            if (f == plan_of.end()) continue;
+            const Plan& pl = *f->second;
+            if (std::find(gp.begin(), gp.end(), f->second) == gp.end() || !pl.ntri) continue;
+            hc[k].rank = pl.job.rank;
+            hc[k].coords = it->d_coords;
+            hc[k].connections = it->d_conn;
+            hc[k].tri_out = pl.job.mode == KVSMC_SHARED_VERTEX_NORMAL ? pl.tri_normals : it->d_normals;
+            hc[k].nvert = pl.nvert;
+            hc[k].ntri = pl.ntri;
+            hc[k].enabled = 1;
+            tasks = pl.sb_tasks;
+        }
+        if (!st && tasks) {
+            KVSMC_CUDA(ctx, cudaMemcpyAsync(d_conn, hc, (size_t)G.niso * sizeof(kvsmc::ConnIso),
+                                            cudaMemcpyHostToDevice, ctx->stream));
+            KVSMC_CUDA(ctx, kvsmc::launch_sconnect_multi(b.d_groups + g, b.d_isos, d_conn, p0.job.vol.dtype,
+                                                         b.d_unit_counts, b.d_unit_offsets, b.d_plane_base, tasks,
+                                                         d_status, d_next + 1, L));
+            if (ready && !(st = read_status())) st = group_status(g);
         }
         for (Plan* pl : gp) {
             if (st) {
@@ -781,10 +851,19 @@ kvsmc_status grouped_shared(kvsmc_context* ctx, const SharedCount& sc, std::vect
         if (it->status || !it->emit) continue;
         kvsmc_status st = gather_emit(ctx, plans[i], it->d_coords, it->d_normals, it->d_conn);
         if (!st && ready) st = ready(it, 2);
-        if (!st && !ready) KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         if (st) it->status = st;
     }
-    if (ready) KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (ready) {
+        KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        return KVSMC_OK;
+    }
+    if (kvsmc_status st = read_status()) return st;
+    for (size_t g = 0; g < b.groups.size(); ++g) {
+        if (group_plans[g].empty()) continue;
+        if (kvsmc_status st = group_status(g))
+            for (Plan* pl : group_plans[g])
+                if (!pl->item->status) pl->item->status = st;
+    }
     return KVSMC_OK;
 }
 

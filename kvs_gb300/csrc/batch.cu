@@ -148,12 +148,13 @@ void StreamBatch::plan_tables()
     std::vector<std::pair<int, int>> kinds;
     std::map<const kvsmc_volume*, kvsmc_tune_choice> shape;
     for (auto& l : lists) shape[l[0]->vol] = stream_shape(ctx, l[0]->vol->view);
+    if (one_row)
+        for (auto& l : lists) shape[l[0]->vol].rows = 1;
     // Under the built-in rules, a value type whose volumes mix one- and two-row
     // tasks takes two rows for all of them: one launch per type instead of two
     // (two-row tasks suit every width; on the uneven 200-volume batch this took
-    // the replay from 10.06 to 9.17 ms).  Not for the shared-vertex count,
-    // whose connection pass takes one-row groups only.
-    if (!want_nodes && !ctx->tune_forced && ctx->tuning.empty()) {
+    // the replay from 10.06 to 9.17 ms).
+    if (!one_row && !ctx->tune_forced && ctx->tuning.empty()) {
         std::map<int, int> rows_seen;   // value type -> bit r set: some volume takes r rows
         for (auto& l : lists) rows_seen[(int)l[0]->vol->view.dtype] |= 1 << shape[l[0]->vol].rows;
         for (auto& l : lists)
@@ -271,17 +272,21 @@ void StreamBatch::carve(char* base)
     Carve cv{base};
     d_groups = cv.take<StreamGroup>(groups.size() * sizeof(StreamGroup));
     d_isos = cv.take<StreamIso>(niso * sizeof(StreamIso));
+    // what a count starts from zero, in one piece (one memset): the status
+    // word, the totals right behind it (one read-back), the task counters and
+    // the unit counts
+    d_status = cv.take<int>(256);
+    d_totals = cv.take<uint64_t>(niso * 8);
+    d_next = cv.take<unsigned long long>(launches.size() * 16);
+    d_next_parts = cv.take<unsigned long long>(kMaxParts * 8);
     d_unit_counts = cv.take<uint16_t>(unit_elems * 2);
+    d_node_counts = node_elems ? cv.take<uint32_t>(node_elems * 4) : nullptr;
+    zero_bytes = (size_t)(base + cv.off - reinterpret_cast<char*>(d_status));
     d_unit_offsets = cv.take<uint32_t>(unit_elems * 4);
     d_plane_totals = cv.take<uint32_t>(iso_planes * 4);
     d_plane_base = cv.take<uint64_t>(iso_planes * 8);
     d_scan = cv.take<char>(kvsmc::scan_scratch_bytes(iso_planes));
-    d_totals = cv.take<uint64_t>(niso * 8);
     d_total = cv.take<uint64_t>(256);
-    d_status = cv.take<int>(256);
-    d_next = cv.take<unsigned long long>(launches.size() * 16);
-    d_next_parts = cv.take<unsigned long long>(kMaxParts * 8);
-    d_node_counts = node_elems ? cv.take<uint32_t>(node_elems * 4) : nullptr;
 }
 
 kvsmc_status StreamBatch::plan()
@@ -308,12 +313,17 @@ kvsmc_status StreamBatch::upload_tables()
 
 kvsmc_status StreamBatch::count()
 {
+    kvsmc_status st = count_enqueue();
+    if (st) return st;
+    KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return count_finish();
+}
+
+kvsmc_status StreamBatch::count_enqueue()
+{
     const kvsmc::Launch L = launch_of(ctx);
-    KVSMC_CUDA(ctx, cudaMemsetAsync(d_status, 0, sizeof(int), ctx->stream));
-    // units the kernels skip as empty space keep these zeros
-    KVSMC_CUDA(ctx, cudaMemsetAsync(d_unit_counts, 0, unit_elems * sizeof(uint16_t), ctx->stream));
-    KVSMC_CUDA(ctx, cudaMemsetAsync(d_next, 0, launches.size() * 16, ctx->stream));
-    if (node_elems) KVSMC_CUDA(ctx, cudaMemsetAsync(d_node_counts, 0, node_elems * 4, ctx->stream));
+    // (units the kernels skip as empty space keep these zeros)
+    KVSMC_CUDA(ctx, cudaMemsetAsync(d_status, 0, zero_bytes, ctx->stream));
     // one count launch per (value type, rows) kind, side by side
     KVSMC_CUDA(ctx, fan_out(ctx, ctx->stream, launches.size(), [&](size_t i, cudaStream_t st) {
         const Launch1& l = launches[i];
@@ -327,20 +337,24 @@ kvsmc_status StreamBatch::count()
                                             d_unit_offsets, d_plane_totals, L, scan_threads));
     KVSMC_CUDA(ctx, kvsmc::launch_scan(d_plane_totals, d_plane_base, iso_planes, d_scan, d_total, L));
     KVSMC_CUDA(ctx, kvsmc::launch_iso_totals(d_isos, (int)isos.size(), d_plane_base, d_total, d_totals, L));
-    // read back: status word, then one total per isolevel
+    // read back: status word, then (256 bytes on) one total per isolevel
     const size_t n = isos.size();
-    kvsmc_status st = ensure_stage(ctx, (n + 2) * 8);
+    kvsmc_status st = ensure_stage(ctx, 256 + n * 8);
     if (st) return st;
-    uint64_t* h = static_cast<uint64_t*>(ctx->h_stage);
-    KVSMC_CUDA(ctx, cudaMemcpyAsync(h, d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    KVSMC_CUDA(ctx, cudaMemcpyAsync(h + 1, d_totals, n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    KVSMC_CUDA(ctx, cudaMemcpyAsync(ctx->h_stage, d_status, 256 + n * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    return KVSMC_OK;
+}
+
+kvsmc_status StreamBatch::count_finish()
+{
+    const size_t n = isos.size();
     int status;
-    std::memcpy(&status, h, sizeof(int));
+    std::memcpy(&status, ctx->h_stage, sizeof(int));
     if (status) return fail(ctx, KVSMC_ERR_TIMEOUT, "streaming count: a shared-memory load did not complete");
+    const uint64_t* h = reinterpret_cast<const uint64_t*>(static_cast<const char*>(ctx->h_stage) + 256);
     for (size_t i = 0; i < n; ++i) {
         Item* it = iso_item[i];
-        const uint64_t t = h[1 + i];
+        const uint64_t t = h[i];
         std::memset(&it->sizes, 0, sizeof it->sizes);
         it->sizes.ntriangles = t;
         it->sizes.nvertices = 3 * t;

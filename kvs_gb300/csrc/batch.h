@@ -70,6 +70,9 @@ struct StreamBatch {
     // (isolevel, node unit) for the groups that take one row per task and
     // whose node segments are its cell segments (set before plan_tables)
     bool want_nodes = false;
+    // every group takes one cell row per task, whatever its width (the
+    // shared-vertex connection passes walk one-row tasks only)
+    bool one_row = false;
     uint64_t node_elems = 0;
     uint32_t* d_node_counts = nullptr;
 
@@ -87,9 +90,15 @@ struct StreamBatch {
 
     unsigned long long* d_next_parts = nullptr;   // task counters of a split emit (kMaxParts)
     static constexpr int kMaxParts = 16;
+    size_t zero_bytes = 0;   // from d_status on: zeroed before a count
 
     kvsmc_status plan();
     kvsmc_status count();
+    // count() in two: everything enqueued on the context's stream, the sizes'
+    // read-back (into h_stage) included; then, once the stream is waited for,
+    // the items' sizes from it.  h_stage is not used in between.
+    kvsmc_status count_enqueue();
+    kvsmc_status count_finish();
     kvsmc_status emit();
     kvsmc_status finish();
 

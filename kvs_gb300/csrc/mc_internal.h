@@ -130,6 +130,11 @@ cudaError_t launch_unit_scan(const StreamGroup* d_groups, int ngroups, uint32_t 
 cudaError_t launch_iso_totals(const StreamIso* d_isos, int n, const uint64_t* d_plane_base, const uint64_t* d_total,
                               uint64_t* d_totals, const Launch& L);
 
+// totals[k] = the entries' sum of slice k of a scan over n slices of `len`
+// entries each (offsets: the exclusive scan, *d_total its grand total).
+cudaError_t launch_slice_totals(const uint64_t* offsets, uint64_t len, int n, const uint64_t* d_total,
+                                uint64_t* totals, const Launch& L);
+
 // ---- shared-vertex node passes on the streaming kernels (mc_snode.cu):
 // node units (plane, row, 256-node segment) numbered in node order; the count
 // pass writes one vertex count per unit, the emit pass (unit_offsets: the
@@ -145,7 +150,7 @@ struct NodeIso {
     Interp ip;
     float* coords;              // the request's vertices
     uint4* rank;                // its rank words (nz * ny * words_per_row)
-    const uint64_t* offsets;    // per node unit: its first vertex id
+    const uint64_t* offsets;    // per node unit: its first vertex id + offsets[0]
     const uint32_t* counts;     // per node unit: its vertices
 };
 size_t snode_multi_shared_bytes(int dtype);

@@ -324,6 +324,7 @@ __global__ void __launch_bounds__(kSnThreads, KVSMC_SNODE_MULTI_CTAS)
     const uint32_t nx = vol.nx, ny = vol.ny, nz = vol.nz;
     const uint64_t pitch = vol.pitch, slice = vol.slice;
     const T* vp = static_cast<const T*>(vol.data);
+    const uint64_t first_id = lane < (unsigned)niso ? C.iso[lane].offsets[0] : 0;
     uint32_t ph = 0;
     for (;;) {
         unsigned long long tk = 0;
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(kSnThreads, KVSMC_SNODE_MULTI_CTAS)
         uint64_t next_base = 0;
         if (lane < (unsigned)niso) {
             next_n = C.iso[lane].counts[unit_of(z0)];
-            next_base = C.iso[lane].offsets[unit_of(z0)];
+            next_base = C.iso[lane].offsets[unit_of(z0)] - first_id;
         }
         const float fyf = __uint2float_rn(y);
         for (uint32_t z = z0; z < z1; ++z) {
@@ -377,7 +378,7 @@ __global__ void __launch_bounds__(kSnThreads, KVSMC_SNODE_MULTI_CTAS)
             const uint64_t base_now = next_base;
             if (z + 1 < z1 && lane < (unsigned)niso) {
                 next_n = C.iso[lane].counts[unit_of(z + 1)];
-                next_base = C.iso[lane].offsets[unit_of(z + 1)];
+                next_base = C.iso[lane].offsets[unit_of(z + 1)] - first_id;
             }
             bool ok = true;
             while (ok && acq <= need) {
@@ -561,6 +562,8 @@ __global__ void __launch_bounds__(kSnThreads)
                uint32_t wait_polls)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    // the node emit gave up: its rank words and vertices are not all there
+    if (__syncthreads_or(*status != 0)) return;
     __shared__ uint64_t s_tri[256];
     __shared__ uint8_t s_ntri[256];
     __shared__ uint8_t s_edge[16];
@@ -822,6 +825,8 @@ __global__ void __launch_bounds__(kSnThreads, 3)
                      uint32_t wait_polls)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    // the node emit gave up: its rank words and vertices are not all there
+    if (__syncthreads_or(*status != 0)) return;
     const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const StreamGroup& G = groups[0];
     const int niso = G.niso;

@@ -1030,6 +1030,12 @@ __global__ void k_iso_totals(const StreamIso* isos, int n, const uint64_t* plane
     totals[i] = next - first;
 }
 
+__global__ void k_slice_totals(const uint64_t* offsets, uint64_t len, int n, const uint64_t* d_total, uint64_t* totals)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) totals[k] = (k + 1 < n ? offsets[(uint64_t)(k + 1) * len] : *d_total) - offsets[(uint64_t)k * len];
+}
+
 }  // namespace
 
 size_t stream_row_elems(int dtype, int rows)
@@ -1155,6 +1161,17 @@ cudaError_t launch_iso_totals(const StreamIso* d_isos, int n, const uint64_t* d_
 {
     prof_begin(L, "iso_totals");
     k_iso_totals<<<(n + 127) / 128, 128, 0, L.stream>>>(d_isos, n, d_plane_base, d_total, d_totals);
+    prof_end(L);
+    *L.counter += 1;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_slice_totals(const uint64_t* offsets, uint64_t len, int n, const uint64_t* d_total,
+                                uint64_t* totals, const Launch& L)
+{
+    if (n <= 0) return cudaSuccess;
+    prof_begin(L, "slice_totals");
+    k_slice_totals<<<(n + 31) / 32, 32, 0, L.stream>>>(offsets, len, n, d_total, totals);
     prof_end(L);
     *L.counter += 1;
     return cudaGetLastError();

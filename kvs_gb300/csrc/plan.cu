@@ -61,9 +61,7 @@ cudaError_t record(kvsmc_host::StreamBatch& b, cudaStream_t s, int num_sms, uint
                                         Li, l.ctas_per_sm);
         });
     };
-    cudaError_t e = cudaMemsetAsync(b.d_status, 0, sizeof(int), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b.d_unit_counts, 0, b.unit_elems * sizeof(uint16_t), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b.d_next, 0, b.launches.size() * 16, s);
+    cudaError_t e = cudaMemsetAsync(b.d_status, 0, b.zero_bytes, s);
     if (e == cudaSuccess) e = per_kind(false);
     if (e == cudaSuccess)
         e = kvsmc::launch_unit_scan(b.d_groups, (int)b.groups.size(), b.scan_blocks, b.d_isos, b.d_unit_counts,

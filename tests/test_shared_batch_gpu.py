@@ -178,3 +178,26 @@ def test_shared_batch_random_shapes_equal_alone(kvsmc_ctx, seed):
         _same(batch[i], alone, f"seed {seed} request {i}")
     for dv in {id(d): d for d in vols}.values():
         dv.free()
+
+
+@pytest.mark.parametrize("nx", [2, 3, 33, 100, 128, 129, 256, 257, 258, 385, 513])
+def test_shared_modes_at_every_width(kvsmc_ctx, oracle_lib, nx):
+    """Rows narrower than a segment, one node past a segment's cells or nodes,
+    a partial last segment: one request alone (its own counts) and three in a
+    batch (one count, one node emit, one connection pass), against the oracle."""
+    f = S.fbm((11, 9, nx), base_freq=1.0 / 8.0, seed=nx, device="cuda")
+    for dtype in (np.float32, np.uint8):
+        v = S.to_numpy(f if dtype == np.float32 else S._cast(f.double() * 255.0, dtype))
+        lo, hi = float(v.min()), float(v.max())
+        vol = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+        reqs = [(lo + q * (hi - lo), m) for q, m in ((0.31, 1), (0.52, 2), (0.64, 2))]
+        params = [_abi.make_params(x, m) for x, m in reqs]
+        batch = extract_batch(kvsmc_ctx, [vol] * 3, params, _abi.PATH_AUTO)
+        for (x, m), p, o in zip(reqs, params, batch):
+            ref = oracle_lib.extract(v, x, m, lo, hi)
+            for got in (o, extract_batch(kvsmc_ctx, [vol], [p], _abi.PATH_AUTO)[0]):
+                assert got["status"] == _abi.OK
+                assert same_bits(got["coords"], ref["coords"]), (nx, dtype, x, m)
+                assert same_bits(got["normals"], ref["normals"]), (nx, dtype, x, m)
+                assert np.array_equal(got["connections"], ref["connections"].view(np.uint32)), (nx, dtype, x, m)
+        vol.free()

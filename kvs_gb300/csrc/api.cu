@@ -379,6 +379,7 @@ kvsmc_status gather_count_at(kvsmc_context* ctx, Plan& pl, char* base)
         // (the tables' host copies may be overwritten by the read-back below
         // only once they have left: both are copies on this stream, in order)
         if (!bst) bst = pl.batch->count_enqueue();
+        if (!bst) bst = pl.batch->read_enqueue();
         if (bst) return bst;
         const kvsmc::StreamGroup& G = pl.batch->groups[0];
         if (G.node_units) pl.sb_nodes = pl.batch->d_node_counts + G.node_base;
@@ -892,18 +893,15 @@ kvsmc_status run_items(kvsmc_context* ctx, std::vector<Item*>& items, bool emit)
         StreamBatch b;
         b.ctx = ctx;
         b.items = stream_items;
-        kvsmc_status st = b.plan();
-        if (!st) st = b.count();
+        kvsmc_status st = b.place();
         if (!st && emit) {
-            for (Item* it : stream_items) {
-                it->emit = true;
-                if (!capacity_ok(*it)) {
+            st = b.extract();
+            for (Item* it : stream_items)
+                if (!st && !capacity_ok(*it))
                     it->status = fail(ctx, KVSMC_ERR_CAPACITY, "output needs %llu coords, %llu normals",
                                       (unsigned long long)it->sizes.ncoords, (unsigned long long)it->sizes.nnormals);
-                }
-            }
-            st = b.emit();
-            if (!st) st = b.finish();
+        } else if (!st) {
+            if (!(st = b.upload_tables())) st = b.count();
         }
         if (st) {
             for (Item* it : stream_items) if (!it->status) it->status = st;

@@ -171,6 +171,15 @@ void StreamBatch::plan_tables()
     scan_threads = largest ? shape[largest].scan_threads : 256;
     for (auto& l : lists)
         if (std::find(kinds.begin(), kinds.end(), kind_of(l)) == kinds.end()) kinds.push_back(kind_of(l));
+    // the kind with the most cells first: the kinds' persistent launches share
+    // the SMs one after the other, and the last one's tail is then the shortest
+    {
+        std::map<std::pair<int, int>, uint64_t> work;
+        for (auto& l : lists) work[kind_of(l)] += cells_of(l[0]->vol->view) * l.size();
+        std::stable_sort(kinds.begin(), kinds.end(), [&](const std::pair<int, int>& a, const std::pair<int, int>& b) {
+            return work[a] > work[b];
+        });
+    }
     groups.clear();
     isos.clear();
     iso_item.clear();
@@ -289,13 +298,19 @@ void StreamBatch::carve(char* base)
     d_total = cv.take<uint64_t>(256);
 }
 
-kvsmc_status StreamBatch::plan()
+kvsmc_status StreamBatch::place()
 {
     plan_tables();
     kvsmc_status st = ensure_scratch(ctx, scratch_bytes());
     if (st) return st;
     carve(static_cast<char*>(ctx->scratch));
-    return upload_tables();
+    return KVSMC_OK;
+}
+
+kvsmc_status StreamBatch::plan()
+{
+    kvsmc_status st = place();
+    return st ? st : upload_tables();
 }
 
 kvsmc_status StreamBatch::upload_tables()
@@ -314,6 +329,7 @@ kvsmc_status StreamBatch::upload_tables()
 kvsmc_status StreamBatch::count()
 {
     kvsmc_status st = count_enqueue();
+    if (!st) st = read_enqueue();
     if (st) return st;
     KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return count_finish();
@@ -333,11 +349,26 @@ kvsmc_status StreamBatch::count_enqueue()
                                     nullptr, nullptr, d_status, d_next + 2 * i, Li, l.ctas_per_sm, 0,
                                     node_elems && l.rows == 1 ? d_node_counts : nullptr);
     }));
-    KVSMC_CUDA(ctx, kvsmc::launch_unit_scan(d_groups, (int)groups.size(), scan_blocks, d_isos, d_unit_counts,
-                                            d_unit_offsets, d_plane_totals, L, scan_threads));
-    KVSMC_CUDA(ctx, kvsmc::launch_scan(d_plane_totals, d_plane_base, iso_planes, d_scan, d_total, L));
-    KVSMC_CUDA(ctx, kvsmc::launch_iso_totals(d_isos, (int)isos.size(), d_plane_base, d_total, d_totals, L));
-    // read back: status word, then (256 bytes on) one total per isolevel
+    KVSMC_CUDA(ctx, scans(L));
+    return KVSMC_OK;
+}
+
+cudaError_t StreamBatch::scans(const kvsmc::Launch& L)
+{
+    if (iso_planes <= kvsmc::kPlaneScanMax)
+        return kvsmc::launch_count_scans(d_groups, (int)groups.size(), scan_blocks, d_isos, (int)isos.size(), iso_planes,
+                                         d_unit_counts, d_unit_offsets, d_plane_totals, d_plane_base, d_totals,
+                                         reinterpret_cast<unsigned int*>(d_status) + 16, L, scan_threads);
+    cudaError_t e = kvsmc::launch_unit_scan(d_groups, (int)groups.size(), scan_blocks, d_isos, d_unit_counts,
+                                            d_unit_offsets, d_plane_totals, L, scan_threads);
+    if (e == cudaSuccess) e = kvsmc::launch_scan(d_plane_totals, d_plane_base, iso_planes, d_scan, d_total, L);
+    if (e == cudaSuccess) e = kvsmc::launch_iso_totals(d_isos, (int)isos.size(), d_plane_base, d_total, d_totals, L);
+    return e;
+}
+
+kvsmc_status StreamBatch::read_enqueue()
+{
+    // status word, then (256 bytes on) one total per isolevel
     const size_t n = isos.size();
     kvsmc_status st = ensure_stage(ctx, 256 + n * 8);
     if (st) return st;
@@ -350,7 +381,7 @@ kvsmc_status StreamBatch::count_finish()
     const size_t n = isos.size();
     int status;
     std::memcpy(&status, ctx->h_stage, sizeof(int));
-    if (status) return fail(ctx, KVSMC_ERR_TIMEOUT, "streaming count: a shared-memory load did not complete");
+    if (status) return fail(ctx, KVSMC_ERR_TIMEOUT, "streaming passes: a shared-memory load did not complete");
     const uint64_t* h = reinterpret_cast<const uint64_t*>(static_cast<const char*>(ctx->h_stage) + 256);
     for (size_t i = 0; i < n; ++i) {
         Item* it = iso_item[i];
@@ -364,6 +395,40 @@ kvsmc_status StreamBatch::count_finish()
         it->sizes.max_value = it->vmax;
         it->sizes.extracted = 1;
     }
+    return KVSMC_OK;
+}
+
+kvsmc_status StreamBatch::extract()
+{
+    bool any = false;
+    for (size_t i = 0; i < isos.size(); ++i) {
+        const Item* it = iso_item[i];
+        const uint64_t cap = cap_triangles(*it);
+        isos[i].coords = cap ? it->d_coords : nullptr;
+        isos[i].normals = cap ? it->d_normals : nullptr;
+        isos[i].cap_tris = cap;
+        any = any || cap;
+    }
+    kvsmc_status st = upload_tables();
+    if (!st) st = count_enqueue();
+    if (!st && any) st = emit_enqueue(d_totals);
+    if (!st) st = read_enqueue();
+    if (st) return st;
+    KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return count_finish();
+}
+
+kvsmc_status StreamBatch::emit_enqueue(const uint64_t* d_fit)
+{
+    const kvsmc::Launch L = launch_of(ctx);
+    KVSMC_CUDA(ctx, fan_out(ctx, ctx->stream, launches.size(), [&](size_t i, cudaStream_t st) {
+        const Launch1& l = launches[i];
+        kvsmc::Launch Li = L;
+        Li.stream = st;
+        return kvsmc::launch_stream(true, l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts,
+                                    d_unit_offsets, d_plane_base, d_status, d_next + 2 * i + 1, Li, l.ctas_per_sm, 0,
+                                    nullptr, d_fit);
+    }));
     return KVSMC_OK;
 }
 
@@ -385,16 +450,7 @@ kvsmc_status StreamBatch::emit()
             if (isos[g.iso_begin + k].coords) g.skip_emit = 0;
     }
     kvsmc_status st = upload_tables();
-    if (st) return st;
-    const kvsmc::Launch L = launch_of(ctx);
-    KVSMC_CUDA(ctx, fan_out(ctx, ctx->stream, launches.size(), [&](size_t i, cudaStream_t st) {
-        const Launch1& l = launches[i];
-        kvsmc::Launch Li = L;
-        Li.stream = st;
-        return kvsmc::launch_stream(true, l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts,
-                                    d_unit_offsets, d_plane_base, d_status, d_next + 2 * i + 1, Li, l.ctas_per_sm);
-    }));
-    return KVSMC_OK;
+    return st ? st : emit_enqueue(nullptr);
 }
 
 kvsmc_status StreamBatch::emit_parts(int parts, const std::function<kvsmc_status(uint32_t, uint32_t, bool)>& after)

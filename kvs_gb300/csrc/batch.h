@@ -94,11 +94,18 @@ struct StreamBatch {
 
     kvsmc_status plan();
     kvsmc_status count();
-    // count() in two: everything enqueued on the context's stream, the sizes'
-    // read-back (into h_stage) included; then, once the stream is waited for,
-    // the items' sizes from it.  h_stage is not used in between.
+    // count() in three: the passes, then the sizes' read-back (into h_stage),
+    // enqueued on the context's stream; once the stream is waited for, the
+    // items' sizes from it.  h_stage is not used between the last two.
     kvsmc_status count_enqueue();
+    kvsmc_status read_enqueue();
     kvsmc_status count_finish();
+    // Count and emit with one wait for the GPU: the emit follows the count
+    // without the host, and on the device writes nothing of a request whose
+    // triangles exceed its outputs.  After place(); fills every item's sizes
+    // (the caller turns the ones that did not fit into statuses).  Two round
+    // trips less than count + emit + finish: 15 us of a 64^3 extraction.
+    kvsmc_status extract();
     kvsmc_status emit();
     kvsmc_status finish();
 
@@ -110,6 +117,13 @@ struct StreamBatch {
     // outputs of cell planes [z_begin, z_end) (every output when whole) are
     // complete once the stream reaches that point.
     kvsmc_status emit_parts(int parts, const std::function<kvsmc_status(uint32_t, uint32_t, bool)>& after);
+
+    // The emit launches; d_fit: see launch_stream's d_totals.
+    kvsmc_status emit_enqueue(const uint64_t* d_fit);
+    // The scans behind a count: unit offsets, plane bases, totals.
+    cudaError_t scans(const kvsmc::Launch& L);
+    // plan() without the upload of the tables.
+    kvsmc_status place();
 
     // The pieces of plan(): host tables, their device footprint, and the
     // device pointers carved from a region of scratch_bytes().

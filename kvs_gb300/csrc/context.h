@@ -47,6 +47,7 @@ struct kvsmc_context {
     // plane-wait poll limits of the streaming count / emit kernels (kvsmc_set_wait_limit)
     uint32_t wait_polls[2] = {kvsmc::kStreamWaitPolls, kvsmc::kStreamWaitPolls};
     kvsmc::Profiler* prof = nullptr;
+    std::vector<kvsmc::KernelFit> fits;   // launch shapes of the kernels launched so far
     std::string last_error;
     // auxiliary streams for launches that may run side by side (created on first use)
     static constexpr int kAux = 6;
@@ -90,6 +91,7 @@ inline kvsmc::Launch launch_of(kvsmc_context* ctx)
     kvsmc::Launch L{ctx->stream, ctx->num_sms, &ctx->launches, ctx->prof};
     L.wait_polls[0] = ctx->wait_polls[0];
     L.wait_polls[1] = ctx->wait_polls[1];
+    L.fits = &ctx->fits;
     return L;
 }
 kvsmc_status ensure_scratch(kvsmc_context* ctx, size_t bytes);

@@ -1,6 +1,8 @@
 // mc_internal.h -- host-side declarations shared by the library's .cu files.
 #pragma once
 #include <cstdint>
+#include <vector>
+
 #include <cuda_runtime.h>
 
 #include "mc_device.cuh"
@@ -14,6 +16,15 @@ struct Profiler;
 // give up (KVSMC_ERR_TIMEOUT); a plane normally lands within a few polls.
 constexpr uint32_t kStreamWaitPolls = 1u << 22;
 
+// A kernel's launch shape on this device, asked for once per context (the
+// attribute calls and the occupancy query cost 3-4 us of host time a launch).
+struct KernelFit {
+    const void* kernel;
+    int threads;
+    size_t smem;
+    int per_sm;
+};
+
 // Launch bookkeeping passed to every launcher.
 struct Launch {
     cudaStream_t stream;
@@ -22,7 +33,13 @@ struct Launch {
     Profiler* prof;      // per-kernel CUDA-event timing when enabled (may be null)
     // plane-wait poll limit of the streaming count [0] and emit [1] kernels
     uint32_t wait_polls[2] = {kStreamWaitPolls, kStreamWaitPolls};
+    std::vector<KernelFit>* fits = nullptr;   // the context's (null: ask each time)
 };
+
+// Let `kernel` use `smem` bytes of dynamic shared memory (all_shared: the
+// SM's shared memory preferred over L1) and return its resident CTAs per SM.
+cudaError_t kernel_fit(const Launch& L, const void* kernel, int threads, size_t smem, int* per_sm,
+                       bool all_shared = false);
 
 // CUDA events on the launching stream around one kernel family's launch.
 void prof_begin(const Launch& L, const char* name);
@@ -117,16 +134,27 @@ size_t stream_row_elems(int dtype, int rows);
 // steps without triangles.  ctas_per_sm: resident CTAs per SM of the
 // persistent grid (0: as many as fit; never more than fit).  The launch runs
 // the warp tasks [task0, ntasks) of its groups (task0 > 0: a later part of a
-// launch split by z-chunks).
+// launch split by z-chunks).  d_totals (emit): per isolevel record its
+// triangles; a request whose total exceeds its cap_tris writes nothing (null:
+// each request writes up to its cap_tris).  The emit writes nothing when the
+// status word says that the count gave up.
 cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
                           const StreamIso* d_isos, uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
                           const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
                           const Launch& L, int ctas_per_sm = 0, uint64_t task0 = 0,
-                          uint32_t* d_node_counts = nullptr);
+                          uint32_t* d_node_counts = nullptr, const uint64_t* d_totals = nullptr);
 // scan_threads: units per CTA pass (64, 128 or 256; 0 = 256).
 cudaError_t launch_unit_scan(const StreamGroup* d_groups, int ngroups, uint32_t nplanes, const StreamIso* d_isos,
                              const uint16_t* d_unit_counts, uint32_t* d_unit_offsets, uint32_t* d_plane_totals,
                              const Launch& L, int scan_threads = 0);
+// The unit scan, the exclusive scan of the plane totals and the isolevels'
+// totals in one launch: the unit scan's last CTA to finish does the rest.
+// d_done: a zeroed word.  At most kPlaneScanMax planes (see there).
+constexpr uint64_t kPlaneScanMax = 1 << 15;
+cudaError_t launch_count_scans(const StreamGroup* d_groups, int ngroups, uint32_t nplanes, const StreamIso* d_isos,
+                               int niso, uint64_t iso_planes, const uint16_t* d_unit_counts, uint32_t* d_unit_offsets,
+                               uint32_t* d_plane_totals, uint64_t* d_plane_base, uint64_t* d_totals,
+                               unsigned int* d_done, const Launch& L, int scan_threads = 0);
 cudaError_t launch_iso_totals(const StreamIso* d_isos, int n, const uint64_t* d_plane_base, const uint64_t* d_total,
                               uint64_t* d_totals, const Launch& L);
 

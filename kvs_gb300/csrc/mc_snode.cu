@@ -1121,9 +1121,8 @@ cudaError_t launch_sconnect(const Job& j, const StreamGroup* d_groups, const Str
     const size_t smem = sconnect_shared_bytes(dt);
     KVSMC_SN_SWITCH(dt, {
         auto kern = k_sconnect<T>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per_sm = 0;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSnThreads, smem);
+        const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), kSnThreads, smem, &per_sm);
         if (e != cudaSuccess) return e;
         const uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)L.num_sms;
         const uint64_t need = (ntasks + kSnWarps - 1) / kSnWarps;
@@ -1153,9 +1152,8 @@ cudaError_t launch_sconnect_multi(const StreamGroup* d_group, const StreamIso* d
     const size_t smem = sconnect_multi_shared_bytes(dtype);
     KVSMC_SN_SWITCH(dtype, {
         auto kern = k_sconnect_multi<T>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per_sm = 0;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSnThreads, smem);
+        const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), kSnThreads, smem, &per_sm);
         if (e != cudaSuccess) return e;
         const uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)L.num_sms;
         const uint64_t need = (ntasks + kSnWarps - 1) / kSnWarps;
@@ -1195,9 +1193,8 @@ cudaError_t launch_snode_multi(const VolumeView& vol, const NodeIso* d_isos, int
     const uint32_t copy_bytes = row_elems * (uint32_t)dtype_size(dt);
     KVSMC_SN_SWITCH(dt, {
         auto kern = k_snode_multi<T>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per_sm = 0;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSnThreads, smem);
+        const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), kSnThreads, smem, &per_sm);
         if (e != cudaSuccess) return e;
         const uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)L.num_sms;
         const uint64_t need = (ntasks + kSnWarps - 1) / kSnWarps;
@@ -1223,9 +1220,8 @@ cudaError_t launch_snode(bool emit, const Job& j, const FastIso& f, uint32_t wpr
     const uint32_t copy_bytes = row_elems * (uint32_t)dtype_size(dt);
     KVSMC_SN_SWITCH(dt, {
         auto kern = emit ? k_snode<T, true> : k_snode<T, false>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per_sm = 0;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSnThreads, smem);
+        const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), kSnThreads, smem, &per_sm);
         if (e != cudaSuccess) return e;
         const uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)L.num_sms;
         const uint64_t need = (ntasks + kSnWarps - 1) / kSnWarps;

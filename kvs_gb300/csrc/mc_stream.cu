@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
              uint16_t* __restrict__ unit_counts, const uint32_t* __restrict__ unit_offsets,
              const uint64_t* __restrict__ plane_base, int* __restrict__ status,
              unsigned long long* __restrict__ next_task, uint32_t wait_polls, uint64_t task0,
-             uint32_t* __restrict__ node_counts)
+             uint32_t* __restrict__ node_counts, const uint64_t* __restrict__ totals)
 {
     static_assert(!NODES || (!EMIT && R == 1), "node counts come from one-row count tasks");
     constexpr int LPR = 32 / R;                 // lanes per cell row
@@ -422,7 +422,9 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
                                              (c0 & 4u) ? 1.0f : 0.0f, (c1 & d) ? 1.0f : 0.0f);
         }
     }
-    __syncthreads();   // the only CTA-wide barrier: tables are read-only from here on
+    // the only CTA-wide barrier: tables are read-only from here on (an emit
+    // whose count gave up has no offsets to write at)
+    if (__syncthreads_or(EMIT && *status != 0)) return;
 
     const size_t wstride = align128(sizeof(WarpState)) + (EMIT ? align128(sizeof(WarpEmit)) : 0) +
                            align128((size_t)3 * plane_elems * sizeof(T));
@@ -440,6 +442,7 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
 
     uint32_t ph = 0;     // per ring buffer: parity of its next completion
     int gcur = -1;       // group whose tables are in W
+    bool live = true;    // emit: some request of the group is written
     for (;;) {
     unsigned long long tk = 0;
     if (lane == 0) tk = atomicAdd(next_task, 1ull);
@@ -484,11 +487,13 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
                 IsoConst& c = WE->ic[lane];
                 c.f = I.f;
                 for (int a = 0; a < 3; ++a) { c.mc[a] = I.ip.min_coord[a]; c.sc[a] = I.ip.scale[a]; }
-                c.coords = I.coords;
+                // a request that does not fit its outputs is not written at all
+                c.coords = totals && totals[iso_begin + lane] > I.cap_tris ? nullptr : I.coords;
                 c.normals = I.normals;
                 c.cap_tris = I.cap_tris;
             }
         }
+        if (EMIT) live = __any_sync(FULL, lane < (unsigned)niso && WE->ic[lane & 15u].coords != nullptr);
         __syncwarp();
         for (unsigned b = lane; b < (unsigned)kLut; b += 32) {
             uint32_t below = 0, in = 0;
@@ -502,6 +507,7 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
         __syncwarp();
         gcur = gi;
     }
+    if (EMIT && !live) continue;
 
     // empty space: a brick whose node min and max have the same mask (no
     // threshold between them) holds no active cell for any isolevel
@@ -942,11 +948,26 @@ __global__ void __launch_bounds__(256)
 // [unit][isolevel]; the plane is walked in tiles of NT units, each staged
 // through shared memory with coalesced loads and stores, one unit per thread
 // and all isolevels scanned at once.
-template <int NT>
+//
+// FUSED: the last CTA to finish (a counter that every CTA raises once its
+// plane's totals are written) then scans the plane totals of all isolevels
+// into plane bases and takes each isolevel's total, so a count's three scans
+// are one launch instead of five.  For a volume of ordinary size the five
+// were launch-bound (64^3: 27 us of events, 11 us fused); one CTA's serial
+// pass over more than kPlaneScanMax planes would cost more than the launches.
+struct PlaneScan {
+    int niso;
+    uint64_t iso_planes;
+    uint64_t* plane_base;
+    uint64_t* totals;
+    unsigned int* done;
+};
+
+template <int NT, bool FUSED>
 __global__ void __launch_bounds__(NT)
     k_unit_scan(const StreamGroup* __restrict__ groups, int ngroups, const StreamIso* __restrict__ isos,
                 const uint16_t* __restrict__ unit_counts, uint32_t* __restrict__ unit_offsets,
-                uint32_t* __restrict__ plane_totals)
+                uint32_t* plane_totals, PlaneScan ps)
 {
     constexpr int NW = NT / 32;
     __shared__ uint16_t sc[NT * kStreamMaxIso];
@@ -981,7 +1002,8 @@ __global__ void __launch_bounds__(NT)
         uint32_t c[kStreamMaxIso], ex[kStreamMaxIso];
 #pragma unroll
         for (int k = 0; k < kStreamMaxIso; ++k) {
-            c[k] = (k < niso && tid < n) ? sc[tid * niso + k] : 0u;
+            if (k >= niso) continue;
+            c[k] = tid < n ? sc[tid * niso + k] : 0u;
             uint32_t v = c[k];
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -1016,6 +1038,53 @@ __global__ void __launch_bounds__(NT)
         for (int k = 0; k < kStreamMaxIso; ++k)
             if (k == (int)tid) plane_totals[isos[G.iso_begin + k].plane_index + z] = carry[k];
     }
+    if (!FUSED) return;
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(ps.done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    constexpr int PER = 8;
+    __shared__ uint64_t psum[NW];
+    uint64_t run = 0;
+    for (uint64_t t0 = 0; t0 < ps.iso_planes; t0 += (uint64_t)NT * PER) {
+        const uint64_t i0 = t0 + (uint64_t)tid * PER;
+        uint32_t v[PER];
+        uint64_t sum = 0;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            v[k] = i0 + k < ps.iso_planes ? __ldcg(plane_totals + i0 + k) : 0u;
+            sum += v[k];
+        }
+        uint64_t inc = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= (unsigned)o) inc += t;
+        }
+        if (lane == 31) psum[warp] = inc;
+        __syncthreads();
+        uint64_t before = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            before += w < (int)warp ? psum[w] : 0;
+            all += psum[w];
+        }
+        uint64_t e = run + before + inc - sum;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            if (i0 + k < ps.iso_planes) ps.plane_base[i0 + k] = e;
+            e += v[k];
+        }
+        run += all;
+        __syncthreads();
+    }
+    for (int i = (int)tid; i < ps.niso; i += NT) {
+        const uint64_t first = ps.plane_base[isos[i].plane_index];
+        ps.totals[i] = (i + 1 < ps.niso ? ps.plane_base[isos[i + 1].plane_index] : run) - first;
+    }
 }
 
 // Triangles of every isolevel: the difference of its first plane's offset and
@@ -1037,6 +1106,23 @@ __global__ void k_slice_totals(const uint64_t* offsets, uint64_t len, int n, con
 }
 
 }  // namespace
+
+cudaError_t kernel_fit(const Launch& L, const void* kernel, int threads, size_t smem, int* per_sm, bool all_shared)
+{
+    if (L.fits)
+        for (const KernelFit& f : *L.fits)
+            if (f.kernel == kernel && f.threads == threads && f.smem == smem) {
+                *per_sm = f.per_sm;
+                return cudaSuccess;
+            }
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && all_shared)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 (int)cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, smem);
+    if (e == cudaSuccess && L.fits) L.fits->push_back(KernelFit{kernel, threads, smem, *per_sm});
+    return e;
+}
 
 size_t stream_row_elems(int dtype, int rows)
 {
@@ -1078,7 +1164,8 @@ uint64_t brick_count(const VolumeView& v)
 cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
                           const StreamIso* d_isos, uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
                           const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
-                          const Launch& L, int ctas_per_sm, uint64_t task0, uint32_t* d_node_counts)
+                          const Launch& L, int ctas_per_sm, uint64_t task0, uint32_t* d_node_counts,
+                          const uint64_t* d_totals)
 {
     if (ntasks <= task0) return cudaSuccess;
     if (rows != 1 && rows != 2) return cudaErrorInvalidValue;
@@ -1089,12 +1176,8 @@ cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_g
         auto kern = emit ? (rows == 1 ? k_stream<T, true, 1> : k_stream<T, true, 2>)
                          : (rows == 1 ? (d_node_counts ? k_stream<T, false, 1, true> : k_stream<T, false, 1>)
                                       : k_stream<T, false, 2>);
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     (int)cudaSharedmemCarveoutMaxShared);
         int per_sm = 0;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+        const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), threads, smem, &per_sm, true);
         if (e != cudaSuccess) return e;
         if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
         // persistent: as many CTAs as are resident at once (never more than the tasks need)
@@ -1104,7 +1187,7 @@ cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_g
         kern<<<(unsigned)nctas, threads, smem, L.stream>>>(d_groups, ngroups, ntasks, d_isos, d_unit_counts,
                                                            d_unit_offsets, d_plane_base, d_status, d_next_task,
                                                            L.wait_polls[emit ? 1 : 0], task0,
-                                                           emit ? nullptr : d_node_counts);
+                                                           emit ? nullptr : d_node_counts, emit ? d_totals : nullptr);
         prof_end(L);
     });
     *L.counter += 1;
@@ -1127,25 +1210,28 @@ cudaError_t launch_bricks(const VolumeView& v, float2* out, const Launch& L)
     return cudaGetLastError();
 }
 
-cudaError_t launch_unit_scan(const StreamGroup* d_groups, int ngroups, uint32_t nplanes, const StreamIso* d_isos,
-                             const uint16_t* d_unit_counts, uint32_t* d_unit_offsets, uint32_t* d_plane_totals,
-                             const Launch& L, int scan_threads)
+namespace {
+
+template <bool FUSED>
+cudaError_t unit_scan(const StreamGroup* d_groups, int ngroups, uint32_t nplanes, const StreamIso* d_isos,
+                      const uint16_t* d_unit_counts, uint32_t* d_unit_offsets, uint32_t* d_plane_totals,
+                      const PlaneScan& ps, const Launch& L, int scan_threads)
 {
     if (nplanes == 0) return cudaSuccess;
     prof_begin(L, "unit_scan");
     switch (scan_threads) {
     case 64:
-        k_unit_scan<64><<<nplanes, 64, 0, L.stream>>>(d_groups, ngroups, d_isos, d_unit_counts, d_unit_offsets,
-                                                      d_plane_totals);
+        k_unit_scan<64, FUSED><<<nplanes, 64, 0, L.stream>>>(d_groups, ngroups, d_isos, d_unit_counts, d_unit_offsets,
+                                                             d_plane_totals, ps);
         break;
     case 128:
-        k_unit_scan<128><<<nplanes, 128, 0, L.stream>>>(d_groups, ngroups, d_isos, d_unit_counts, d_unit_offsets,
-                                                        d_plane_totals);
+        k_unit_scan<128, FUSED><<<nplanes, 128, 0, L.stream>>>(d_groups, ngroups, d_isos, d_unit_counts,
+                                                               d_unit_offsets, d_plane_totals, ps);
         break;
     case 0:
     case 256:
-        k_unit_scan<256><<<nplanes, 256, 0, L.stream>>>(d_groups, ngroups, d_isos, d_unit_counts, d_unit_offsets,
-                                                        d_plane_totals);
+        k_unit_scan<256, FUSED><<<nplanes, 256, 0, L.stream>>>(d_groups, ngroups, d_isos, d_unit_counts,
+                                                               d_unit_offsets, d_plane_totals, ps);
         break;
     default:
         prof_end(L);
@@ -1154,6 +1240,25 @@ cudaError_t launch_unit_scan(const StreamGroup* d_groups, int ngroups, uint32_t 
     prof_end(L);
     *L.counter += 1;
     return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_unit_scan(const StreamGroup* d_groups, int ngroups, uint32_t nplanes, const StreamIso* d_isos,
+                             const uint16_t* d_unit_counts, uint32_t* d_unit_offsets, uint32_t* d_plane_totals,
+                             const Launch& L, int scan_threads)
+{
+    return unit_scan<false>(d_groups, ngroups, nplanes, d_isos, d_unit_counts, d_unit_offsets, d_plane_totals,
+                            PlaneScan{}, L, scan_threads);
+}
+
+cudaError_t launch_count_scans(const StreamGroup* d_groups, int ngroups, uint32_t nplanes, const StreamIso* d_isos,
+                               int niso, uint64_t iso_planes, const uint16_t* d_unit_counts, uint32_t* d_unit_offsets,
+                               uint32_t* d_plane_totals, uint64_t* d_plane_base, uint64_t* d_totals,
+                               unsigned int* d_done, const Launch& L, int scan_threads)
+{
+    return unit_scan<true>(d_groups, ngroups, nplanes, d_isos, d_unit_counts, d_unit_offsets, d_plane_totals,
+                           PlaneScan{niso, iso_planes, d_plane_base, d_totals, d_done}, L, scan_threads);
 }
 
 cudaError_t launch_iso_totals(const StreamIso* d_isos, int n, const uint64_t* d_plane_base, const uint64_t* d_total,

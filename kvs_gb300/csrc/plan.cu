@@ -63,12 +63,7 @@ cudaError_t record(kvsmc_host::StreamBatch& b, cudaStream_t s, int num_sms, uint
     };
     cudaError_t e = cudaMemsetAsync(b.d_status, 0, b.zero_bytes, s);
     if (e == cudaSuccess) e = per_kind(false);
-    if (e == cudaSuccess)
-        e = kvsmc::launch_unit_scan(b.d_groups, (int)b.groups.size(), b.scan_blocks, b.d_isos, b.d_unit_counts,
-                                    b.d_unit_offsets, b.d_plane_totals, L, b.scan_threads);
-    if (e == cudaSuccess) e = kvsmc::launch_scan(b.d_plane_totals, b.d_plane_base, b.iso_planes, b.d_scan, b.d_total, L);
-    if (e == cudaSuccess)
-        e = kvsmc::launch_iso_totals(b.d_isos, (int)b.isos.size(), b.d_plane_base, b.d_total, b.d_totals, L);
+    if (e == cudaSuccess) e = b.scans(L);
     if (e == cudaSuccess) e = per_kind(true);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h_out, b.d_status, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)

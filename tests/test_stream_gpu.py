@@ -181,3 +181,51 @@ def test_clustered_isolevels(kvsmc_ctx):
     b = extract_batch(kvsmc_ctx, [uvol] * len(ps), ps, _abi.PATH_GATHER)
     for i, iso in enumerate(isos):
         compare(a[i], b[i], f"u8 iso={iso}")
+
+
+def test_batch_of_requests_that_do_not_fit(kvsmc_ctx):
+    """Requests without room write nothing, report what they need and leave the
+    others exact, whether some, all or none of a volume's requests fit."""
+    v = S.to_numpy(S.fbm((20, 33, 70), base_freq=1.0 / 16.0, seed=4, device="cuda"))
+    vol = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+    isos = [0.35, 0.45, 0.5, 0.6]
+    params = [_abi.make_params(x, _abi.MODE_DUP_POLYGON_NORMAL) for x in isos]
+    good = extract_batch(kvsmc_ctx, [vol] * 4, params, _abi.PATH_AUTO)
+    for short in ([], [1], [0, 3], [0, 1, 2, 3]):
+        reqs = (_abi.Request * 4)()
+        bufs = []
+        for i in range(4):
+            t = good[i]["ntri"]
+            cap = t - 1 if i in short else t
+            c = torch.full((9 * t,), -7.0, device="cuda")
+            n = torch.full((3 * t,), -7.0, device="cuda")
+            bufs.append((c, n))
+            reqs[i].volume, reqs[i].params = vol.handle, params[i]
+            reqs[i].d_coords, reqs[i].coords_capacity = c.data_ptr(), 9 * t
+            reqs[i].d_normals, reqs[i].normals_capacity = n.data_ptr(), 3 * cap
+        torch.cuda.synchronize()
+        st = kvsmc_ctx.lib.kvsmc_extract_batch(kvsmc_ctx.handle, reqs, 4)
+        assert st == (_abi.ERR_CAPACITY if short else _abi.OK)
+        for i in range(4):
+            assert reqs[i].sizes.ntriangles == good[i]["ntri"]
+            assert reqs[i].status == (_abi.ERR_CAPACITY if i in short else _abi.OK)
+            c, n = (b.cpu().numpy() for b in bufs[i])
+            if i in short:
+                assert (c == -7.0).all() and (n == -7.0).all()
+            else:
+                assert same_bits(c, good[i]["coords"]) and same_bits(n, good[i]["normals"])
+    vol.free()
+
+
+def test_more_planes_than_one_block_scans(kvsmc_ctx, oracle_lib):
+    """16 isolevels of a volume 2100 planes deep: more (isolevel, plane) totals
+    than the unit scan's last block takes, so they are scanned on their own."""
+    v = S.to_numpy(S.fbm((2100, 5, 6), base_freq=1.0 / 16.0, seed=6, device="cuda"))
+    lo, hi = float(v.min()), float(v.max())
+    vol = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+    isos = [lo + (hi - lo) * (k + 1) / 17 for k in range(16)]
+    out = extract_batch(kvsmc_ctx, [vol] * 16, [_abi.make_params(x, 0) for x in isos], _abi.PATH_AUTO)
+    for x, o in zip(isos, out):
+        ref = oracle_lib.extract(v, x, 0, lo, hi)
+        assert same_bits(o["coords"], ref["coords"]) and same_bits(o["normals"], ref["normals"]), x
+    vol.free()

@@ -42,7 +42,7 @@ kvsmc_status ensure_scratch(kvsmc_context* ctx, size_t bytes)
         ctx->scratch_bytes = 0;
     }
     const size_t want = align_up(bytes + bytes / 4, 1 << 20);
-    KVSMC_CUDA(ctx, cudaMalloc(&ctx->scratch, want));
+    KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->scratch, want));
     ctx->scratch_bytes = want;
     return KVSMC_OK;
 }
@@ -59,24 +59,6 @@ kvsmc_status ensure_stage(kvsmc_context* ctx, size_t bytes)
     const size_t want = align_up(bytes + bytes / 4, 1 << 16);
     KVSMC_CUDA(ctx, cudaMallocHost(&ctx->h_stage, want));
     ctx->h_stage_bytes = want;
-    return KVSMC_OK;
-}
-
-kvsmc_status volume_minmax(kvsmc_context* ctx, kvsmc_volume* v)
-{
-    if (v->has_minmax) return KVSMC_OK;
-    const size_t part = align_up(minmax_scratch_bytes(ctx->num_sms), 256);
-    kvsmc_status st = ensure_scratch(ctx, part + 256);
-    if (st) return st;
-    double* d_out = reinterpret_cast<double*>(static_cast<char*>(ctx->scratch) + part);
-    KVSMC_CUDA(ctx, launch_minmax(v->view, ctx->scratch, d_out, launch_of(ctx)));
-    KVSMC_CUDA(ctx, cudaMemcpyAsync(ctx->h_small, d_out, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    double mm[2];
-    std::memcpy(mm, ctx->h_small, sizeof mm);
-    v->vmin = mm[0];
-    v->vmax = mm[1];
-    v->has_minmax = true;
     return KVSMC_OK;
 }
 
@@ -126,26 +108,6 @@ cudaError_t fan_out(kvsmc_context* ctx, cudaStream_t origin, size_t n,
     return e;
 }
 
-kvsmc_status volume_bricks(kvsmc_context* ctx, kvsmc_volume* v)
-{
-    v->bricks_valid = false;
-    const int dt = v->view.dtype;
-    const bool ok = (dt == KVSMC_I8 || dt == KVSMC_I16 || dt == KVSMC_U8 || dt == KVSMC_U16 || dt == KVSMC_F32) &&
-                    v->view.nx - 1 <= (uint32_t)kvsmc::kStreamMaxCells;
-    if (!ok) return KVSMC_OK;
-    const size_t bytes = kvsmc::brick_count(v->view) * sizeof(float2);
-    if (bytes > v->brick_bytes) {
-        if (v->bricks) cudaFree(v->bricks);
-        v->bricks = nullptr;
-        v->brick_bytes = 0;
-        KVSMC_CUDA(ctx, cudaMalloc(&v->bricks, bytes));
-        v->brick_bytes = bytes;
-    }
-    KVSMC_CUDA(ctx, kvsmc::launch_bricks(v->view, v->bricks, launch_of(ctx)));
-    v->bricks_valid = true;
-    return KVSMC_OK;
-}
-
 // Decide min/max (MapperBase::setRange) and the Equal early exit.
 kvsmc_status prepare(kvsmc_context* ctx, Item& it)
 {
@@ -172,44 +134,6 @@ kvsmc_status prepare(kvsmc_context* ctx, Item& it)
 using namespace kvsmc_host;
 
 namespace {
-
-size_t elems_per_16B(int dtype) { return 16 / dtype_size(dtype); }
-
-kvsmc_status volume_alloc(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, uint32_t ny, uint32_t nz,
-                          kvsmc_volume* v)
-{
-    const size_t es = dtype_size(dtype);
-    const uint64_t pitch = align_up(nx, elems_per_16B(dtype));
-    const size_t bytes = (size_t)pitch * ny * nz * es + 256;
-    v->view.nx = nx; v->view.ny = ny; v->view.nz = nz;
-    v->view.dtype = dtype;
-    v->view.pitch = pitch;
-    v->view.slice = pitch * ny;
-    if (bytes > v->bytes) {
-        if (v->dev) cudaFree(v->dev);
-        v->dev = nullptr;
-        v->bytes = 0;
-        KVSMC_CUDA(ctx, cudaMalloc(&v->dev, bytes));
-        v->bytes = bytes;
-    }
-    v->view.data = v->dev;
-    v->has_minmax = false;
-    return KVSMC_OK;
-}
-
-kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src, cudaMemcpyKind kind)
-{
-    const size_t es = dtype_size(v->view.dtype);
-    const size_t row = (size_t)v->view.nx * es;
-    const size_t rows = (size_t)v->view.ny * v->view.nz;
-    if (v->view.pitch == v->view.nx) {
-        KVSMC_CUDA(ctx, cudaMemcpyAsync(v->dev, src, row * rows, kind, ctx->stream));
-    } else {
-        KVSMC_CUDA(ctx, cudaMemcpy2DAsync(v->dev, v->view.pitch * es, src, row, row, rows, kind, ctx->stream));
-    }
-    v->has_minmax = false;
-    return KVSMC_OK;
-}
 
 kvsmc_status check_shape(kvsmc_context* ctx, int dtype, uint32_t nx, uint32_t ny, uint32_t nz)
 {
@@ -468,7 +392,7 @@ kvsmc_status gather_emit(kvsmc_context* ctx, Plan& pl, float* coords, float* nor
             ctx->arena2 = nullptr;
             ctx->arena2_bytes = 0;
             const size_t want = align_up(need + need / 4, 1 << 20);
-            KVSMC_CUDA(ctx, cudaMalloc(&ctx->arena2, want));
+            KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->arena2, want));
             ctx->arena2_bytes = want;
         }
         kvsmc::vertex_normals_carve(j, pl.ntri, pl.nvert, ctx->arena2);
@@ -581,7 +505,7 @@ kvsmc_status shared_count(kvsmc_context* ctx, const std::vector<Item*>& items, S
         ctx->arena3 = nullptr;
         ctx->arena3_bytes = 0;
         const size_t want = align_up(need, 1 << 20);
-        if (cudaMalloc(&ctx->arena3, want) != cudaSuccess) {
+        if (kvsmc_host::device_malloc(ctx, &ctx->arena3, want) != cudaSuccess) {
             // no room for the shared count: each request counts on its own
             cudaGetLastError();
             ctx->arena3 = nullptr;
@@ -666,7 +590,7 @@ kvsmc_status grouped_shared(kvsmc_context* ctx, const SharedCount& sc, std::vect
         ctx->arena4 = nullptr;
         ctx->arena4_bytes = 0;
         const size_t want = align_up(need, 1 << 20);
-        if (cudaMalloc(&ctx->arena4, want) != cudaSuccess) {
+        if (kvsmc_host::device_malloc(ctx, &ctx->arena4, want) != cudaSuccess) {
             cudaGetLastError();
             ctx->arena4 = nullptr;
             return KVSMC_ERR_OUT_OF_MEMORY;   // the caller runs the requests one by one
@@ -731,7 +655,7 @@ kvsmc_status grouped_shared(kvsmc_context* ctx, const SharedCount& sc, std::vect
         ctx->arena5 = nullptr;
         ctx->arena5_bytes = 0;
         const size_t want = align_up(tn_total, 1 << 20);
-        if (cudaMalloc(&ctx->arena5, want) != cudaSuccess) {
+        if (kvsmc_host::device_malloc(ctx, &ctx->arena5, want) != cudaSuccess) {
             cudaGetLastError();
             ctx->arena5 = nullptr;
             return KVSMC_ERR_OUT_OF_MEMORY;   // the caller runs the requests one by one
@@ -1029,6 +953,8 @@ void kvsmc_destroy(kvsmc_context* ctx)
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     if (ctx->host_vol) { cudaFree(ctx->host_vol->dev); delete ctx->host_vol; }
+    block_release(ctx);
+    if (ctx->dense) cudaFree(ctx->dense);
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->d_flag) cudaFree(ctx->d_flag);
     if (ctx->h_flag) cudaFreeHost(ctx->h_flag);
@@ -1100,10 +1026,8 @@ kvsmc_status kvsmc_volume_upload(kvsmc_context* ctx, const void* host, kvsmc_dty
     if (!host || !out) return fail(ctx, KVSMC_ERR_INVALID_ARGUMENT, "null pointer");
     if ((st = check_shape(ctx, dtype, nx, ny, nz))) return st;
     kvsmc_volume* v = new kvsmc_volume();
-    if ((st = volume_alloc(ctx, dtype, nx, ny, nz, v)) || (st = volume_copy_in(ctx, v, host, cudaMemcpyHostToDevice)) ||
-        (st = volume_bricks(ctx, v))) {
-        if (v->dev) cudaFree(v->dev);
-        delete v;
+    if ((st = volume_alloc(ctx, dtype, nx, ny, nz, v)) || (st = volume_copy_in(ctx, v, host, false))) {
+        volume_destroy(ctx, v);
         return st;
     }
     *out = v;
@@ -1118,10 +1042,8 @@ kvsmc_status kvsmc_volume_from_device(kvsmc_context* ctx, const void* dev, kvsmc
     if (!dev || !out) return fail(ctx, KVSMC_ERR_INVALID_ARGUMENT, "null pointer");
     if ((st = check_shape(ctx, dtype, nx, ny, nz))) return st;
     kvsmc_volume* v = new kvsmc_volume();
-    if ((st = volume_alloc(ctx, dtype, nx, ny, nz, v)) || (st = volume_copy_in(ctx, v, dev, cudaMemcpyDeviceToDevice)) ||
-        (st = volume_bricks(ctx, v))) {
-        if (v->dev) cudaFree(v->dev);
-        delete v;
+    if ((st = volume_alloc(ctx, dtype, nx, ny, nz, v)) || (st = volume_copy_in(ctx, v, dev, true))) {
+        volume_destroy(ctx, v);
         return st;
     }
     *out = v;
@@ -1133,8 +1055,7 @@ kvsmc_status kvsmc_volume_update(kvsmc_context* ctx, kvsmc_volume* v, const void
     kvsmc_status st = use_device(ctx);
     if (st) return st;
     if (!v || !host) return fail(ctx, KVSMC_ERR_INVALID_ARGUMENT, "null pointer");
-    if ((st = volume_copy_in(ctx, v, host, cudaMemcpyHostToDevice))) return st;
-    return v->bricks_valid ? volume_bricks(ctx, v) : KVSMC_OK;
+    return volume_copy_in(ctx, v, host, false);
 }
 
 void kvsmc_volume_free(kvsmc_context* ctx, kvsmc_volume* v)
@@ -1144,9 +1065,7 @@ void kvsmc_volume_free(kvsmc_context* ctx, kvsmc_volume* v)
         cudaSetDevice(ctx->device);
         cudaStreamSynchronize(ctx->stream);
     }
-    if (v->dev) cudaFree(v->dev);
-    if (v->bricks) cudaFree(v->bricks);
-    delete v;
+    volume_destroy(ctx, v);
 }
 
 kvsmc_status kvsmc_volume_download(kvsmc_context* ctx, const kvsmc_volume* v, void* host_values)
@@ -1219,7 +1138,7 @@ kvsmc_status kvsmc_marching_cubes_host(kvsmc_context* ctx, const void* host, kvs
     if (!ctx->host_vol) ctx->host_vol = new kvsmc_volume();
     kvsmc_volume* v = ctx->host_vol;
     if ((st = volume_alloc(ctx, dtype, nx, ny, nz, v))) return st;
-    if ((st = volume_copy_in(ctx, v, host, cudaMemcpyHostToDevice))) return st;
+    if ((st = volume_copy_in(ctx, v, host, false))) return st;
     Item it;
     it.vol = v;
     it.params = *p;
@@ -1231,10 +1150,19 @@ kvsmc_status kvsmc_marching_cubes_host(kvsmc_context* ctx, const void* host, kvs
     const bool streaming = stream_eligible(ctx, it);
     StreamBatch b;
     Plan pl;
+    bool written = false;
     if (streaming) {
+        // into the output arena of the earlier calls right behind the count;
+        // only a result that it does not hold is written in a second go
         b.ctx = ctx;
         b.items = items;
-        if ((st = b.plan()) || (st = b.count())) return st;
+        const uint64_t cap = ctx->out_bytes / 48 / 64 * 64;
+        it.d_coords = cap ? static_cast<float*>(ctx->out_arena) : nullptr;
+        it.d_normals = cap ? it.d_coords + 9 * cap : nullptr;
+        it.coords_cap = 9 * cap;
+        it.normals_cap = 3 * cap;
+        if ((st = b.place()) || (st = b.extract())) return st;
+        written = it.sizes.ntriangles <= cap;
     } else {
         gather_plan(it, pl);
         if ((st = gather_count(ctx, pl))) return st;
@@ -1243,24 +1171,29 @@ kvsmc_status kvsmc_marching_cubes_host(kvsmc_context* ctx, const void* host, kvs
     *sizes = it.sizes;
     const size_t bc = align_up(sizes->ncoords * 4, 256), bn = align_up(sizes->nnormals * 4, 256);
     const size_t bk = align_up(sizes->nconnections * 4, 256);
-    if (bc + bn + bk > ctx->out_bytes) {
-        KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        if (ctx->out_arena) cudaFree(ctx->out_arena);
-        ctx->out_arena = nullptr;
-        ctx->out_bytes = 0;
-        const size_t want = align_up(bc + bn + bk, 1 << 20);
-        KVSMC_CUDA(ctx, cudaMalloc(&ctx->out_arena, want));
-        ctx->out_bytes = want;
+    if (!written) {
+        if (bc + bn + bk > ctx->out_bytes) {
+            KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+            if (ctx->out_arena) cudaFree(ctx->out_arena);
+            ctx->out_arena = nullptr;
+            ctx->out_bytes = 0;
+            // (a mebibyte to spare: a streaming result is split by the capacity above)
+            const size_t want = align_up(bc + bn + bk, 1 << 20) + (1 << 20);
+            KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->out_arena, want));
+            ctx->out_bytes = want;
+        }
+        char* base = static_cast<char*>(ctx->out_arena);
+        it.d_coords = reinterpret_cast<float*>(base);
+        it.d_normals = reinterpret_cast<float*>(base + bc);
+        it.d_conn = reinterpret_cast<uint32_t*>(base + bc + bn);
+        it.coords_cap = sizes->ncoords;
+        it.normals_cap = sizes->nnormals;
+        it.conn_cap = sizes->nconnections;
     }
-    char* base = static_cast<char*>(ctx->out_arena);
-    it.d_coords = reinterpret_cast<float*>(base);
-    it.d_normals = reinterpret_cast<float*>(base + bc);
-    it.d_conn = reinterpret_cast<uint32_t*>(base + bc + bn);
-    it.coords_cap = sizes->ncoords;
-    it.normals_cap = sizes->nnormals;
-    it.conn_cap = sizes->nconnections;
     it.emit = true;
-    if (streaming) {
+    if (written) {
+        // done
+    } else if (streaming) {
         if ((st = b.emit()) || (st = b.finish())) return st;
     } else {
         if ((st = gather_emit(ctx, pl, it.d_coords, it.d_normals, it.d_conn))) return st;
@@ -1291,7 +1224,7 @@ static kvsmc_status arena_outputs(kvsmc_context* ctx, std::vector<Item*>& its)
         ctx->out_arena = nullptr;
         ctx->out_bytes = 0;
         const size_t want = align_up(total, 1 << 20);
-        KVSMC_CUDA(ctx, cudaMalloc(&ctx->out_arena, want));
+        KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->out_arena, want));
         ctx->out_bytes = want;
     }
     Carve cv{static_cast<char*>(ctx->out_arena)};
@@ -1423,7 +1356,7 @@ kvsmc_status kvsmc_extract_batch_host(kvsmc_context* ctx, const void* host, kvsm
     {
         const kvsmc::Launch L = launch_of(ctx);
         kvsmc::prof_begin(L, "copy_h2d");
-        st = volume_copy_in(ctx, v, host, cudaMemcpyHostToDevice);
+        st = volume_copy_in(ctx, v, host, false);
         kvsmc::prof_end(L);
         if (st) return st;
     }
@@ -1603,8 +1536,7 @@ kvsmc_status volume_create(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, u
     if (st) return st;
     kvsmc_volume* v = new kvsmc_volume();
     if ((st = volume_alloc(ctx, dtype, nx, ny, nz, v))) {
-        if (v->dev) cudaFree(v->dev);
-        delete v;
+        volume_destroy(ctx, v);
         return st;
     }
     *out = v;

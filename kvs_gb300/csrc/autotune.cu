@@ -131,7 +131,7 @@ kvsmc_status trial_setup(kvsmc_context* ctx, int dt, int cls, int niso, uint64_t
     const size_t es = dt == KVSMC_F32 ? 4 : (dt == KVSMC_I16 || dt == KVSMC_U16) ? 2 : 1;
     const uint64_t n = (uint64_t)s * s * s;
     void* raw = nullptr;
-    KVSMC_CUDA(ctx, cudaMalloc(&raw, n * es));
+    KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &raw, n * es));
     const uint32_t sd = (uint32_t)(seed * 0x9e3779b97f4a7c15ull >> 32) ^ (uint32_t)(dt * 977 + cls * 131);
     const unsigned blocks = (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx->num_sms * 16);
     cudaStream_t stream = static_cast<cudaStream_t>(kvsmc_stream(ctx));
@@ -165,7 +165,7 @@ kvsmc_status trial_setup(kvsmc_context* ctx, int dt, int cls, int niso, uint64_t
     if ((st = kvsmc_count_batch(ctx, tr.reqs.data(), niso))) return st;
     uint64_t total = 0;
     for (auto& r : tr.reqs) total += r.sizes.ntriangles;
-    KVSMC_CUDA(ctx, cudaMalloc(&tr.d_out, std::max<uint64_t>(1, total) * 12 * sizeof(float)));
+    KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &tr.d_out, std::max<uint64_t>(1, total) * 12 * sizeof(float)));
     uint64_t off = 0;
     for (auto& r : tr.reqs) {
         const uint64_t t = r.sizes.ntriangles;

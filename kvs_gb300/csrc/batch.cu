@@ -450,7 +450,11 @@ kvsmc_status StreamBatch::emit()
             if (isos[g.iso_begin + k].coords) g.skip_emit = 0;
     }
     kvsmc_status st = upload_tables();
-    return st ? st : emit_enqueue(nullptr);
+    if (st) return st;
+    // an emit may follow another one of the same count (a server's rounds, a
+    // result that did not fit the first time): its tasks start over
+    KVSMC_CUDA(ctx, cudaMemsetAsync(d_next, 0, launches.size() * 16, ctx->stream));
+    return emit_enqueue(nullptr);
 }
 
 kvsmc_status StreamBatch::emit_parts(int parts, const std::function<kvsmc_status(uint32_t, uint32_t, bool)>& after)

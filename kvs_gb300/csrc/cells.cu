@@ -977,7 +977,7 @@ struct CellsScratch {
 kvsmc_status cells_prepare(kvsmc_context* ctx, kvsmc::CellJob& j, CellsScratch* sc, int niso = 1)
 {
     using namespace kvsmc_host;
-    if (!ctx->d_flag) KVSMC_CUDA(ctx, cudaMalloc(&ctx->d_flag, sizeof(int)));
+    if (!ctx->d_flag) KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->d_flag, sizeof(int)));
     j.bad_index = ctx->d_flag;
     KVSMC_CUDA(ctx, cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream));
     sc->tiles = kvsmc::cells_tiles(j.ncells);
@@ -1154,7 +1154,7 @@ kvsmc_status kvsmc_marching_cells_host(kvsmc_context* ctx, kvsmc_cell_type cell_
         cudaFree(d_out);
         return s;
     };
-    cudaError_t e = cudaMalloc(&d_in, bv + bx + bk);
+    cudaError_t e = kvsmc_host::device_malloc(ctx, &d_in, bv + bx + bk);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_in, values, nnodes * es, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_in + bv, coords, nnodes * 12, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess && ncells)
@@ -1171,7 +1171,7 @@ kvsmc_status kvsmc_marching_cells_host(kvsmc_context* ctx, kvsmc_cell_type cell_
         (st = cells_passes(ctx, j, sc, false, sizes)) || sizes->ntriangles == 0)
         return done(st);
     const uint64_t t = sizes->ntriangles;
-    if ((e = cudaMalloc(&d_out, t * 12 * sizeof(float))) != cudaSuccess)
+    if ((e = kvsmc_host::device_malloc(ctx, &d_out, t * 12 * sizeof(float))) != cudaSuccess)
         return done(fail(ctx, KVSMC_ERR_OUT_OF_MEMORY, "cells: %s", cudaGetErrorString(e)));
     j.out_coords = d_out;
     j.out_normals = d_out + 9 * t;
@@ -1215,7 +1215,7 @@ kvsmc_status kvsmc_slice_cells_host(kvsmc_context* ctx, kvsmc_cell_type cell_typ
         cudaFree(d_out);
         return s;
     };
-    cudaError_t e = cudaMalloc(&d_in, bv + bx + bk + bt);
+    cudaError_t e = kvsmc_host::device_malloc(ctx, &d_in, bv + bx + bk + bt);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_in, values, nnodes * es, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_in + bv, coords, nnodes * 12, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess)
@@ -1247,7 +1247,7 @@ kvsmc_status kvsmc_slice_cells_host(kvsmc_context* ctx, kvsmc_cell_type cell_typ
     *ntriangles = t;
     if (t == 0) return done(KVSMC_OK);
     const size_t oc = align_up(t * 36, 256), on = align_up(t * 12, 256);
-    if ((e = cudaMalloc(&d_out, oc + on + t * 9)) != cudaSuccess)
+    if ((e = kvsmc_host::device_malloc(ctx, &d_out, oc + on + t * 9)) != cudaSuccess)
         return done(fail(ctx, KVSMC_ERR_OUT_OF_MEMORY, "slice cells: %s", cudaGetErrorString(e)));
     j.out_coords = reinterpret_cast<float*>(d_out);
     j.out_normals = reinterpret_cast<float*>(d_out + oc);
@@ -1284,7 +1284,7 @@ kvsmc_status kvsmc_cells_bounds(kvsmc_context* ctx, kvsmc_cell_type cell_type, c
         cudaFree(d_in);
         return st;
     };
-    cudaError_t e = cudaMalloc(&d_in, bx + bk);
+    cudaError_t e = kvsmc_host::device_malloc(ctx, &d_in, bx + bk);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_in, coords, nnodes * 12, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess && ncells)
         e = cudaMemcpyAsync(d_in + bx, connections, ncells * npc * 4, cudaMemcpyHostToDevice, ctx->stream);
@@ -1297,7 +1297,7 @@ kvsmc_status kvsmc_cells_bounds(kvsmc_context* ctx, kvsmc_cell_type cell_type, c
     kvsmc_status st = ensure_scratch(ctx, bs + 256);
     if (st) return done(st);
     if (!ctx->d_flag) {
-        if ((e = cudaMalloc(&ctx->d_flag, sizeof(int))) != cudaSuccess)
+        if ((e = kvsmc_host::device_malloc(ctx, &ctx->d_flag, sizeof(int))) != cudaSuccess)
             return done(fail(ctx, KVSMC_ERR_OUT_OF_MEMORY, "cells bounds: %s", cudaGetErrorString(e)));
     }
     j.bad_index = ctx->d_flag;

@@ -2,6 +2,7 @@
 #pragma once
 #include <cstdint>
 #include <functional>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -12,12 +13,16 @@ struct kvsmc_volume {
     kvsmc::VolumeView view;
     void* dev = nullptr;        // owned device allocation
     size_t bytes = 0;
+    int device = 0;             // the device it lies on
     bool has_minmax = false;
     double vmin = 0.0, vmax = 0.0;
-    // brick min/max table (streaming kernels' empty-space skip), rebuilt after
-    // every copy into a resident volume
+    // parts of the same allocation, written by the pass that every copy into a
+    // resident volume ends with: the values' range (range_ready; read back
+    // when it is first asked for) and the brick min/max table (the streaming
+    // kernels' empty-space skip; null for volumes that they do not take)
+    kvsmc::IngestOut* range = nullptr;
+    bool range_ready = false;
     float2* bricks = nullptr;
-    size_t brick_bytes = 0;
     bool bricks_valid = false;
 };
 
@@ -47,6 +52,15 @@ struct kvsmc_context {
     // plane-wait poll limits of the streaming count / emit kernels (kvsmc_set_wait_limit)
     uint32_t wait_polls[2] = {kvsmc::kStreamWaitPolls, kvsmc::kStreamWaitPolls};
     kvsmc::Profiler* prof = nullptr;
+    // freed volumes' device blocks, kept for the next volumes (cudaMalloc and
+    // cudaFree of a new field's 83 MB a frame cost 350 us): at most
+    // kSpareBlocks blocks of kSpareBytes in all, given back when an
+    // allocation fails and with the context
+    struct Spare { void* p; size_t bytes; };
+    std::vector<Spare> spare;
+    std::mutex spare_mutex;
+    void* dense = nullptr;       // staging of host volumes whose rows are padded (at most kDenseStage)
+    size_t dense_bytes = 0;
     std::vector<kvsmc::KernelFit> fits;   // launch shapes of the kernels launched so far
     std::string last_error;
     // auxiliary streams for launches that may run side by side (created on first use)
@@ -132,13 +146,41 @@ struct Item {
     kvsmc_status status = KVSMC_OK;
 };
 
+// A volume's device block: from the context's spare blocks, or a new one.
+constexpr size_t kSpareBytes = (size_t)1 << 30;
+constexpr size_t kSpareBlocks = 4;
+kvsmc_status block_alloc(kvsmc_context* ctx, size_t bytes, void** p, size_t* got);
+// Give a block back: kept for the next volumes once nothing on the device
+// reads it any more, or freed (ctx null, or too large).
+void block_free(kvsmc_context* ctx, void* p, size_t bytes);
+// Free every spare block.
+void block_release(kvsmc_context* ctx);
+
+// cudaMalloc that frees the spare blocks before it gives up.
+cudaError_t device_malloc_bytes(kvsmc_context* ctx, void** p, size_t bytes);
+template <typename P> cudaError_t device_malloc(kvsmc_context* ctx, P** p, size_t bytes)
+{
+    void* q = nullptr;
+    const cudaError_t e = device_malloc_bytes(ctx, &q, bytes);
+    *p = static_cast<P*>(q);
+    return e;
+}
+
+// Shape a volume and its allocation (kept when large enough).
+kvsmc_status volume_alloc(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, uint32_t ny, uint32_t nz,
+                          kvsmc_volume* v);
+// Dense values into the volume's layout, with its brick table and range.
+constexpr size_t kDenseStage = (size_t)64 << 20;
+kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src, bool on_device);
+void volume_destroy(kvsmc_context* ctx, kvsmc_volume* v);
+
 // A resident volume of the given shape with uninitialised values (row-padded
 // like the uploads); the caller fills it and then calls volume_bricks.
 kvsmc_status volume_create(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, uint32_t ny, uint32_t nz,
                            kvsmc_volume** out);
 
-// (Re)build a resident volume's brick min/max table on the context's stream
-// (no-op for value types or widths the streaming kernels do not take).
+// (Re)build a resident volume's brick min/max table and its range from its
+// values on the context's stream.
 kvsmc_status volume_bricks(kvsmc_context* ctx, kvsmc_volume* v);
 
 // Run fn(i, stream) for i < n side by side on the context's auxiliary streams,

@@ -261,7 +261,7 @@ kvsmc_status kvsmc_stl_records(kvsmc_context* ctx, int32_t mode, const float* d_
     if (!d_out || (reinterpret_cast<uintptr_t>(d_out) & 15u))
         return fail(ctx, KVSMC_ERR_INVALID_ARGUMENT, "stl: output must be 16-byte aligned device memory");
     KVSMC_CUDA(ctx, cudaSetDevice(ctx->device));
-    if (!ctx->d_flag) KVSMC_CUDA(ctx, cudaMalloc(&ctx->d_flag, sizeof(int)));
+    if (!ctx->d_flag) KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->d_flag, sizeof(int)));
     int* bad = ctx->d_flag;
     KVSMC_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(int), ctx->stream));
     KVSMC_CUDA(ctx, kvsmc::launch_stl_records(d_coords, d_normals, d_connections, nvertices, ntriangles, mode,
@@ -301,13 +301,13 @@ kvsmc_status kvsmc_write_stl(kvsmc_context* ctx, const char* path, int32_t mode,
             }
             ctx->stl_buf_bytes = 0;
             for (int b = 0; b < 2; ++b) {
-                KVSMC_CUDA(ctx, cudaMalloc(&ctx->stl_dbuf[b], bytes));
+                KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->stl_dbuf[b], bytes));
                 KVSMC_CUDA(ctx, cudaMallocHost(&ctx->stl_hbuf[b], bytes));
                 if (!ctx->stl_ev[b]) KVSMC_CUDA(ctx, cudaEventCreateWithFlags(&ctx->stl_ev[b], cudaEventDisableTiming));
             }
             ctx->stl_buf_bytes = bytes;
         }
-        if (!ctx->d_flag) KVSMC_CUDA(ctx, cudaMalloc(&ctx->d_flag, sizeof(int)));
+        if (!ctx->d_flag) KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->d_flag, sizeof(int)));
         if (!ctx->h_flag) KVSMC_CUDA(ctx, cudaMallocHost(&ctx->h_flag, sizeof(int)));
         KVSMC_CUDA(ctx, cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream));
     }
@@ -384,9 +384,9 @@ kvsmc_status kvsmc_write_stl_host(kvsmc_context* ctx, const char* path, int32_t 
     uint32_t* d_k = nullptr;
     cudaError_t e = cudaSuccess;
     if (ntri) {
-        e = cudaMalloc(&d_c, ncoords * sizeof(float));
-        if (e == cudaSuccess) e = cudaMalloc(&d_n, need_normals * sizeof(float));
-        if (e == cudaSuccess && !dup) e = cudaMalloc(&d_k, 3 * ntri * sizeof(uint32_t));
+        e = kvsmc_host::device_malloc(ctx, &d_c, ncoords * sizeof(float));
+        if (e == cudaSuccess) e = kvsmc_host::device_malloc(ctx, &d_n, need_normals * sizeof(float));
+        if (e == cudaSuccess && !dup) e = kvsmc_host::device_malloc(ctx, &d_k, 3 * ntri * sizeof(uint32_t));
         if (e == cudaSuccess) e = cudaMemcpyAsync(d_c, coords, ncoords * sizeof(float), cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(d_n, normals, need_normals * sizeof(float), cudaMemcpyHostToDevice, ctx->stream);

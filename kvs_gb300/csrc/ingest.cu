@@ -589,8 +589,8 @@ kvsmc_status kvsmc_volume_load_avs(kvsmc_context* ctx, const char* path, kvsmc_v
     if ((st = kvsmc_host::volume_create(ctx, (kvsmc_dtype)h.info.dtype, h.info.nx, h.info.ny, h.info.nz, &v)))
         return st;
     st = load_binary(ctx, path, v, h.data_offset);
-    if (!st) st = kvsmc_volume_minmax(ctx, v, &v->vmin, &v->vmax);
     if (!st) st = kvsmc_host::volume_bricks(ctx, v);
+    if (!st) st = kvsmc_volume_minmax(ctx, v, &v->vmin, &v->vmax);
     if (st) {
         kvsmc_volume_free(ctx, v);
         return st;
@@ -641,6 +641,7 @@ kvsmc_status kvsmc_volume_load_kvsml(kvsmc_context* ctx, const char* path, kvsmc
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) st = fail(ctx, KVSMC_ERR_CUDA, "kvsml: byte swap: %s", cudaGetErrorString(e));
     }
+    if (!st) st = kvsmc_host::volume_bricks(ctx, v);
     // the volume's min/max (StructuredVolumeObject.cpp:214-226)
     if (!st) {
         if (h.info.has_min_value && h.info.has_max_value) {
@@ -655,7 +656,6 @@ kvsmc_status kvsmc_volume_load_kvsml(kvsmc_context* ctx, const char* path, kvsmc
             }
         }
     }
-    if (!st) st = kvsmc_host::volume_bricks(ctx, v);
     if (st) {
         kvsmc_volume_free(ctx, v);
         return st;

@@ -212,7 +212,7 @@ kvsmc_status kvsmc_write_kvsml_polygon(kvsmc_context* ctx, const char* path, int
                 }
                 ctx->txt_bytes = 0;
                 for (int b = 0; b < 2; ++b) {
-                    if (cudaMalloc(&ctx->txt_dbuf[b], chunk) != cudaSuccess ||
+                    if (kvsmc_host::device_malloc(ctx, &ctx->txt_dbuf[b], chunk) != cudaSuccess ||
                         cudaMallocHost(&ctx->txt_hbuf[b], chunk) != cudaSuccess ||
                         (!ctx->stl_ev[b] && cudaEventCreateWithFlags(&ctx->stl_ev[b], cudaEventDisableTiming) !=
                                                 cudaSuccess)) {

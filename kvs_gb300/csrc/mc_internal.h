@@ -123,7 +123,16 @@ struct StreamGroup {
 constexpr int kBrickPlanes = 8;
 constexpr uint32_t kBrickCells = 128;
 uint64_t brick_count(const VolumeView& v);
-cudaError_t launch_bricks(const VolumeView& v, float2* out, const Launch& L);
+
+// The range of a volume's values as the ingest pass leaves it (volume.cu):
+// order-preserving keys of the lowest and (inverted) the highest value that is
+// no NaN, index << 1 | sign of the first zero, the bits of values[0]; all ones
+// where there is none.
+struct IngestOut {
+    unsigned long long lo, nhi, zero, first;
+};
+// src: the values, dense, copied into v's layout (null: they are in place).
+cudaError_t launch_ingest(const VolumeView& v, const void* src, float2* bricks, IngestOut* d_out, const Launch& L);
 
 size_t stream_shared_bytes(int dtype, bool emit, int rows);
 size_t stream_warp_smem_bytes(int dtype, bool emit, int rows);

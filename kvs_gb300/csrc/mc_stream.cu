@@ -904,44 +904,6 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
     }   // task loop
 }
 
-// Brick min/max: one warp per brick, lanes across its node rows.
-template <typename T>
-__global__ void __launch_bounds__(256)
-    k_bricks(VolumeView v, uint32_t seg_cells, uint32_t wpr, uint32_t nby, uint64_t nbricks, float2* __restrict__ out)
-{
-    const uint64_t b = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned lane = threadIdx.x & 31u;
-    if (b >= nbricks) return;
-    const uint32_t seg = (uint32_t)(b % wpr);
-    const uint32_t by = (uint32_t)((b / wpr) % nby);
-    const uint32_t bz = (uint32_t)(b / ((uint64_t)wpr * nby));
-    const uint32_t cx = v.nx - 1, cy = v.ny - 1, cz = v.nz - 1;
-    const uint32_t x0 = seg * seg_cells, x1 = min(x0 + seg_cells, cx);
-    const uint32_t y0 = 2 * by, y1 = min(y0 + 2, cy);
-    const uint32_t z0 = bz * kBrickPlanes, z1 = min(z0 + kBrickPlanes, cz);
-    const T* d = static_cast<const T*>(v.data);
-    float lo = __int_as_float(0x7f800000), hi = __int_as_float(0xff800000);
-    bool nan = false;
-    for (uint32_t z = z0; z <= z1; ++z)
-        for (uint32_t y = y0; y <= y1; ++y) {
-            const T* row = d + (uint64_t)z * v.slice + (uint64_t)y * v.pitch;
-            for (uint32_t x = x0 + lane; x <= x1; x += 32) {
-                const float f = (float)row[x];
-                nan |= f != f;
-                lo = fminf(lo, f);
-                hi = fmaxf(hi, f);
-            }
-        }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = fminf(lo, __shfl_xor_sync(FULL, lo, o));
-        hi = fmaxf(hi, __shfl_xor_sync(FULL, hi, o));
-    }
-    nan = __any_sync(FULL, nan);
-    if (lane == 0)
-        out[b] = nan ? make_float2(__int_as_float(0xff800000), __int_as_float(0x7f800000)) : make_float2(lo, hi);
-}
-
 // One CTA per (group, z): for every isolevel of the group, the exclusive scan
 // of its unit counts over the plane's units (rows y, segments x) -> u32
 // offsets inside the plane, and the plane's total.  Counts are stored
@@ -1188,22 +1150,6 @@ cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_g
                                                            d_unit_offsets, d_plane_base, d_status, d_next_task,
                                                            L.wait_polls[emit ? 1 : 0], task0,
                                                            emit ? nullptr : d_node_counts, emit ? d_totals : nullptr);
-        prof_end(L);
-    });
-    *L.counter += 1;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_bricks(const VolumeView& v, float2* out, const Launch& L)
-{
-    const uint64_t n = brick_count(v);
-    if (n == 0) return cudaSuccess;
-    const uint32_t seg = kBrickCells;
-    const uint32_t wpr = (v.nx - 1 + seg - 1) / seg, nby = (v.ny - 1 + 1) / 2;
-    const unsigned blocks = (unsigned)((n * 32 + 255) / 256);
-    KVSMC_STREAM_SWITCH(v.dtype, {
-        prof_begin(L, "bricks");
-        k_bricks<T><<<blocks, 256, 0, L.stream>>>(v, seg, wpr, nby, n, out);
         prof_end(L);
     });
     *L.counter += 1;

@@ -125,7 +125,7 @@ kvsmc_status kvsmc_plan_create(kvsmc_context* ctx, const kvsmc_request* reqs, in
         p->cap.push_back(b.isos[k].cap_tris);
     }
     cudaStream_t cs = nullptr;
-    cudaError_t e = cudaMalloc(&p->d_mem, b.scratch_bytes());
+    cudaError_t e = kvsmc_host::device_malloc(ctx, &p->d_mem, b.scratch_bytes());
     if (e == cudaSuccess) e = cudaMallocHost(&p->h_out, (b.isos.size() + 1) * sizeof(uint64_t));
     if (e == cudaSuccess) {
         std::memset(p->h_out, 0, (b.isos.size() + 1) * sizeof(uint64_t));

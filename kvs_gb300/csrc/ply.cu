@@ -185,7 +185,7 @@ kvsmc_status kvsmc_write_ply(kvsmc_context* ctx, const char* path, const float* 
             }
             ctx->stl_buf_bytes = 0;
             for (int b = 0; b < 2; ++b) {
-                KVSMC_CUDA(ctx, cudaMalloc(&ctx->stl_dbuf[b], bytes));
+                KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->stl_dbuf[b], bytes));
                 KVSMC_CUDA(ctx, cudaMallocHost(&ctx->stl_hbuf[b], bytes));
                 if (!ctx->stl_ev[b]) KVSMC_CUDA(ctx, cudaEventCreateWithFlags(&ctx->stl_ev[b], cudaEventDisableTiming));
             }
@@ -239,7 +239,7 @@ kvsmc_status kvsmc_write_ply_host(kvsmc_context* ctx, const char* path, const fl
     cudaError_t e = cudaSuccess;
     if (nvertices) {
         const size_t oc = kvsmc_host::align_up(bc, 256), ok_ = kvsmc_host::align_up(bk, 256);
-        e = cudaMalloc(&d, oc + ok_ + bn + 16);
+        e = kvsmc_host::device_malloc(ctx, &d, oc + ok_ + bn + 16);
         if (e == cudaSuccess) e = cudaMemcpyAsync(d, coords, bc, cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess && bk) e = cudaMemcpyAsync(d + oc, colors, bk, cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess && bn) e = cudaMemcpyAsync(d + oc + ok_, normals, bn, cudaMemcpyHostToDevice, ctx->stream);

@@ -322,7 +322,7 @@ kvsmc_status kvsmc_server_create(kvsmc_context* ctx, const kvsmc_server_config* 
     // the arena: the budget plus room for the 256-byte rounding of every block
     // of a full batch in each worker
     S->arena_bytes = S->cfg.output_budget_bytes + 2 * kArenaAlign * (uint64_t)S->cfg.max_batch * S->cfg.workers;
-    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&S->arena), S->arena_bytes);
+    cudaError_t e = kvsmc_host::device_malloc(ctx, &S->arena, S->arena_bytes);
     S->free_list.reset(e == cudaSuccess ? S->arena_bytes : 0);
     kvsmc_status st = e == cudaSuccess ? KVSMC_OK
                                        : (e == cudaErrorMemoryAllocation ? KVSMC_ERR_OUT_OF_MEMORY : KVSMC_ERR_CUDA);

@@ -402,7 +402,7 @@ kvsmc_status kvsmc_slice_plane(kvsmc_context* ctx, kvsmc_volume* vol, const kvsm
         ctx->out_arena = nullptr;
         ctx->out_bytes = 0;
         const size_t want = align_up(bc + bn + bk, 1 << 20);
-        KVSMC_CUDA(ctx, cudaMalloc(&ctx->out_arena, want));
+        KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->out_arena, want));
         ctx->out_bytes = want;
     }
     char* base = static_cast<char*>(ctx->out_arena);

@@ -310,7 +310,7 @@ kvsmc_status ascii_buffers(kvsmc_context* ctx, size_t bytes)
     ctx->txt_bytes = 0;
     const size_t want = kvsmc_host::align_up(bytes + bytes / 4, 1 << 20);
     for (int b = 0; b < 2; ++b) {
-        KVSMC_CUDA(ctx, cudaMalloc(&ctx->txt_dbuf[b], want));
+        KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->txt_dbuf[b], want));
         KVSMC_CUDA(ctx, cudaMallocHost(&ctx->txt_hbuf[b], want));
         if (!ctx->stl_ev[b]) KVSMC_CUDA(ctx, cudaEventCreateWithFlags(&ctx->stl_ev[b], cudaEventDisableTiming));
     }
@@ -416,9 +416,9 @@ kvsmc_status kvsmc_write_stl_ascii_host(kvsmc_context* ctx, const char* path, in
     uint32_t* d_k = nullptr;
     cudaError_t e = cudaSuccess;
     if (ntri) {
-        e = cudaMalloc(&d_c, ncoords * sizeof(float));
-        if (e == cudaSuccess) e = cudaMalloc(&d_n, need_normals * sizeof(float));
-        if (e == cudaSuccess && !dup) e = cudaMalloc(&d_k, 3 * ntri * sizeof(uint32_t));
+        e = kvsmc_host::device_malloc(ctx, &d_c, ncoords * sizeof(float));
+        if (e == cudaSuccess) e = kvsmc_host::device_malloc(ctx, &d_n, need_normals * sizeof(float));
+        if (e == cudaSuccess && !dup) e = kvsmc_host::device_malloc(ctx, &d_k, 3 * ntri * sizeof(uint32_t));
         if (e == cudaSuccess) e = cudaMemcpyAsync(d_c, coords, ncoords * sizeof(float), cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(d_n, normals, need_normals * sizeof(float), cudaMemcpyHostToDevice, ctx->stream);

@@ -1,0 +1,461 @@
+// volume.cu -- resident volumes: their device blocks, and the one pass that
+// lays a volume out (rows padded to 16 bytes), takes its brick min/max table
+// and its value range (GetMinMaxValues, StructuredVolumeObject.cpp:66-111).
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <limits>
+#include <mutex>
+
+#include "context.h"
+
+namespace kvsmc {
+
+namespace {
+
+// Order-preserving 64-bit keys of the values (a NaN is never given one).
+template <typename T> __device__ __forceinline__ unsigned long long value_key(T v)
+{
+    if constexpr (sizeof(T) == 4 && T(0.5) != T(0)) {   // float
+        const uint32_t b = __float_as_uint(v == 0.0f ? 0.0f : v);
+        return b & 0x80000000u ? ~b : b | 0x80000000u;
+    } else if constexpr (sizeof(T) == 8 && T(0.5) != T(0)) {   // double
+        const unsigned long long b = (unsigned long long)__double_as_longlong(v == 0.0 ? 0.0 : v);
+        return b >> 63 ? ~b : b | (1ull << 63);
+    } else if constexpr (T(-1) < T(0)) {
+        return (unsigned long long)(long long)v ^ (1ull << 63);
+    } else {
+        return (unsigned long long)v;
+    }
+}
+
+template <typename T> __device__ __forceinline__ unsigned long long raw_bits(T v)
+{
+    unsigned long long r = 0;
+    memcpy(&r, &v, sizeof v);
+    return r;
+}
+
+template <typename T> struct Limits;
+#define KVSMC_LIMITS(T, LO, HI)                                  \
+    template <> struct Limits<T> {                               \
+        __device__ static T lowest() { return LO; }              \
+        __device__ static T highest() { return HI; }             \
+    };
+KVSMC_LIMITS(int8_t, -128, 127)
+KVSMC_LIMITS(int16_t, -32768, 32767)
+KVSMC_LIMITS(int32_t, (int32_t)0x80000000, 0x7fffffff)
+KVSMC_LIMITS(long long, (long long)0x8000000000000000ull, 0x7fffffffffffffffll)
+KVSMC_LIMITS(uint8_t, 0, 255)
+KVSMC_LIMITS(uint16_t, 0, 65535)
+KVSMC_LIMITS(uint32_t, 0u, 0xffffffffu)
+KVSMC_LIMITS(unsigned long long, 0ull, ~0ull)
+KVSMC_LIMITS(float, __int_as_float(0xff800000), __int_as_float(0x7f800000))
+KVSMC_LIMITS(double, __longlong_as_double((long long)0xfff0000000000000ull), __longlong_as_double(0x7ff0000000000000ll))
+#undef KVSMC_LIMITS
+
+constexpr int kIngestThreads = 256;
+
+// One warp per brick of 8 cell planes x 2 cell rows x 128 cells (9 x 3 x 129
+// nodes; bricks share their border nodes), persistent over the bricks.  src
+// (may be null): the values, dense; every node is written once into the
+// padded layout by the brick that owns it.  Without src the values are read
+// in place.  Each brick's min and max go to `bricks` (null: no table), the
+// range of all values to `out`.
+//
+// Each value is read once from HBM (a brick's border nodes again from L1/L2,
+// 1.7 loads a node in all) and written once; a warp's 13-15 loads of one plane
+// are in flight together.  83 MB of floats (301 x 256 x 270): 78 us, 2.2 TB/s
+// read and written together, instead of a copy, a brick pass (72 us) and a
+// min/max scan (137 us); 4.3 GB in 2.9 ms.  Bound by the latency of a plane's
+// loads: one brick's planes follow one another in a warp.
+template <typename T, bool BRICKS, bool COPY>
+__global__ void __launch_bounds__(kIngestThreads)
+    k_ingest(VolumeView v, const T* __restrict__ src, uint32_t nbx, uint32_t nby, uint64_t nbricks,
+             float2* __restrict__ bricks, IngestOut* __restrict__ out)
+{
+    constexpr bool kFloat = T(0.5) != T(0);
+    __shared__ unsigned long long s_lo[kIngestThreads / 32], s_nhi[kIngestThreads / 32], s_zero[kIngestThreads / 32];
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    T* const dst = static_cast<T*>(const_cast<void*>(v.data));
+    const uint32_t cx = v.nx - 1, cy = v.ny - 1, cz = v.nz - 1;
+    const uint64_t rp = COPY ? v.nx : v.pitch, sp = COPY ? (uint64_t)v.nx * v.ny : v.slice;
+    const T* const from = COPY ? src : dst;
+    T lo = Limits<T>::highest(), hi = Limits<T>::lowest();   // over this thread's values, NaN apart
+    unsigned long long zero = ~0ull;                          // (index << 1 | sign) of its first zero
+    const uint64_t warps = (uint64_t)gridDim.x * (kIngestThreads / 32);
+    for (uint64_t b = (uint64_t)blockIdx.x * (kIngestThreads / 32) + warp; b < nbricks; b += warps) {
+        const uint32_t q = (uint32_t)(b / nbx), bx = (uint32_t)(b - (uint64_t)q * nbx);   // (below 2^32 brick rows)
+        const uint32_t bz = q / nby, by = q - bz * nby;
+        const uint32_t x0 = bx * kBrickCells, x1 = min(x0 + kBrickCells, cx);
+        const uint32_t y0 = 2 * by, y1 = min(y0 + 2, cy);
+        const uint32_t z0 = bz * kBrickPlanes, z1 = min(z0 + kBrickPlanes, cz);
+        // this lane's nodes of a row: x0 + lane + 32 i, and lane 0 the one past
+        // the brick's 128 cells (its own only at the end of the row)
+        bool have[5];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) have[i] = x0 + lane + 32 * i <= x1;
+        have[4] = lane == 0 && x0 + kBrickCells <= x1;
+        const bool own4 = x0 + kBrickCells == cx;
+        float blo = __int_as_float(0x7f800000), bhi = __int_as_float(0xff800000);
+        bool nan = false;
+        const T* in = from + (uint64_t)z0 * sp + (uint64_t)y0 * rp + x0 + lane;
+        T* to = dst + (uint64_t)z0 * v.slice + (uint64_t)y0 * v.pitch + x0 + lane;
+        for (uint32_t z = z0; z <= z1; ++z, in += sp, to += v.slice) {
+            const bool own_z = COPY && (z < z0 + kBrickPlanes || z == cz);
+            T w[3][5];
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                const T* row = in + (uint64_t)r * rp;
+                const bool there = y0 + r <= y1;
+#pragma unroll
+                for (int i = 0; i < 5; ++i)
+                    if (there && have[i]) w[r][i] = row[32 * i];
+            }
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                T* row = to + (uint64_t)r * v.pitch;
+                const uint32_t y = y0 + r;
+                const bool there = y <= y1, own = own_z && there && (r < 2 || y == cy);
+#pragma unroll
+                for (int i = 0; i < 5; ++i) {
+                    if (!(there && have[i])) continue;
+                    const T val = w[r][i];
+                    if (COPY && own && (i < 4 || own4)) row[32 * i] = val;
+                    if constexpr (BRICKS) {
+                        const float f = (float)val;
+                        blo = fminf(blo, f);
+                        bhi = fmaxf(bhi, f);
+                    } else {
+                        if (val < lo) lo = val;
+                        if (val > hi) hi = val;
+                    }
+                    if constexpr (kFloat) {
+                        nan |= val != val;
+                        // among equal values the scan keeps the first: only zeros' signs show it
+                        if (val == T(0) && zero == ~0ull)
+                            zero = ((((uint64_t)z * v.ny + y) * v.nx + x0 + lane + 32 * i) << 1) |
+                                   (raw_bits(val) != 0 ? 1u : 0u);
+                    }
+                }
+            }
+        }
+        if constexpr (BRICKS) {
+            if (blo <= bhi) {   // (values of these types are floats exactly)
+                const T a = (T)blo, c = (T)bhi;
+                if (a < lo) lo = a;
+                if (c > hi) hi = c;
+            }
+            if (bricks) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    blo = fminf(blo, __shfl_xor_sync(0xffffffffu, blo, o));
+                    bhi = fmaxf(bhi, __shfl_xor_sync(0xffffffffu, bhi, o));
+                }
+                nan = __any_sync(0xffffffffu, nan);
+                // a brick holding a NaN is never skipped
+                if (lane == 0)
+                    bricks[b] = nan ? make_float2(__int_as_float(0xff800000), __int_as_float(0x7f800000))
+                                    : make_float2(blo, bhi);
+            }
+        }
+    }
+    const bool any = lo <= hi;
+    unsigned long long klo = any ? value_key(lo) : ~0ull, knhi = any ? ~value_key(hi) : ~0ull;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        klo = min(klo, __shfl_xor_sync(0xffffffffu, klo, o));
+        knhi = min(knhi, __shfl_xor_sync(0xffffffffu, knhi, o));
+        zero = min(zero, __shfl_xor_sync(0xffffffffu, zero, o));
+    }
+    if (lane == 0) {
+        s_lo[warp] = klo;
+        s_nhi[warp] = knhi;
+        s_zero[warp] = zero;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < kIngestThreads / 32; ++k) {
+            klo = min(klo, s_lo[k]);
+            knhi = min(knhi, s_nhi[k]);
+            zero = min(zero, s_zero[k]);
+        }
+        atomicMin(&out->lo, klo);
+        atomicMin(&out->nhi, knhi);
+        if (kFloat) atomicMin(&out->zero, zero);
+        if (blockIdx.x == 0) out->first = raw_bits(from[0]);
+    }
+}
+
+}  // namespace
+
+#define KVSMC_INGEST_SWITCH(DT, ...)                                                  \
+    switch (DT) {                                                                     \
+    case 0: { using T = int8_t; constexpr bool B = true; __VA_ARGS__; } break;        \
+    case 1: { using T = int16_t; constexpr bool B = true; __VA_ARGS__; } break;       \
+    case 2: { using T = int32_t; constexpr bool B = false; __VA_ARGS__; } break;      \
+    case 3: { using T = long long; constexpr bool B = false; __VA_ARGS__; } break;    \
+    case 4: { using T = uint8_t; constexpr bool B = true; __VA_ARGS__; } break;       \
+    case 5: { using T = uint16_t; constexpr bool B = true; __VA_ARGS__; } break;      \
+    case 6: { using T = uint32_t; constexpr bool B = false; __VA_ARGS__; } break;     \
+    case 7: { using T = unsigned long long; constexpr bool B = false; __VA_ARGS__; } break; \
+    case 8: { using T = float; constexpr bool B = true; __VA_ARGS__; } break;         \
+    case 9: { using T = double; constexpr bool B = false; __VA_ARGS__; } break;       \
+    default: return cudaErrorInvalidValue;                                            \
+    }
+
+cudaError_t launch_ingest(const VolumeView& v, const void* src, float2* bricks, IngestOut* d_out, const Launch& L)
+{
+    const uint32_t nbx = std::max(1u, (v.nx - 1 + kBrickCells - 1) / kBrickCells);
+    const uint32_t nby = std::max(1u, v.ny / 2);
+    const uint64_t nbz = std::max(1u, (v.nz - 1 + kBrickPlanes - 1) / kBrickPlanes);
+    const uint64_t n = (uint64_t)nbx * nby * nbz;
+    cudaError_t e = cudaMemsetAsync(d_out, 0xff, sizeof *d_out, L.stream);
+    if (e != cudaSuccess) return e;
+    const uint64_t need = (n + kIngestThreads / 32 - 1) / (kIngestThreads / 32), cap = (uint64_t)L.num_sms * 8;
+    prof_begin(L, "ingest");
+    KVSMC_INGEST_SWITCH(v.dtype, {
+        const unsigned grid = (unsigned)(need < cap ? need : cap);
+        if (src)
+            k_ingest<T, B, true><<<grid, kIngestThreads, 0, L.stream>>>(v, static_cast<const T*>(src), nbx, nby, n,
+                                                                         bricks, d_out);
+        else
+            k_ingest<T, B, false><<<grid, kIngestThreads, 0, L.stream>>>(v, nullptr, nbx, nby, n, bricks, d_out);
+    });
+    prof_end(L);
+    *L.counter += 1;
+    return cudaGetLastError();
+}
+
+}  // namespace kvsmc
+
+namespace kvsmc_host {
+
+namespace {
+
+// A key of value_key back to its value.
+double key_value(int dtype, unsigned long long k)
+{
+    switch (dtype) {
+    case KVSMC_F32: {
+        const uint32_t b = (uint32_t)k & 0x80000000u ? (uint32_t)k & 0x7fffffffu : ~(uint32_t)k;
+        float f;
+        std::memcpy(&f, &b, sizeof f);
+        return (double)f;
+    }
+    case KVSMC_F64: {
+        const unsigned long long b = k >> 63 ? k & ~(1ull << 63) : ~k;
+        double d;
+        std::memcpy(&d, &b, sizeof d);
+        return d;
+    }
+    case KVSMC_I8: case KVSMC_I16: case KVSMC_I32: case KVSMC_I64: return (double)(long long)(k ^ (1ull << 63));
+    default: return (double)k;
+    }
+}
+
+// GetMinMaxValues (StructuredVolumeObject.cpp:66-85) from the ingest pass's
+// result: the scan starts at values[0], which a NaN there never leaves, and
+// keeps the first of equal values (seen in the sign of a zero).
+void decode_range(int dtype, const kvsmc::IngestOut& o, double& lo, double& hi)
+{
+    if (dtype == KVSMC_F32 || dtype == KVSMC_F64) {
+        double first;
+        if (dtype == KVSMC_F32) {
+            float f;
+            const uint32_t b = (uint32_t)o.first;
+            std::memcpy(&f, &b, sizeof f);
+            first = (double)f;
+        } else {
+            std::memcpy(&first, &o.first, sizeof first);
+        }
+        if (std::isnan(first) || o.lo == ~0ull) {
+            lo = hi = first;
+            return;
+        }
+    }
+    lo = key_value(dtype, o.lo);
+    hi = key_value(dtype, ~o.nhi);
+    if (o.zero != ~0ull) {
+        const double z = o.zero & 1ull ? -0.0 : 0.0;
+        if (lo == 0.0) lo = z;
+        if (hi == 0.0) hi = z;
+    }
+}
+
+size_t table_bytes(const kvsmc::VolumeView& v)
+{
+    const int dt = v.dtype;
+    const bool ok = (dt == KVSMC_I8 || dt == KVSMC_I16 || dt == KVSMC_U8 || dt == KVSMC_U16 || dt == KVSMC_F32) &&
+                    v.nx > 1 && v.ny > 1 && v.nz > 1 && v.nx - 1 <= (uint32_t)kvsmc::kStreamMaxCells;
+    return ok ? kvsmc::brick_count(v) * sizeof(float2) : 0;
+}
+
+}  // namespace
+
+kvsmc_status block_alloc(kvsmc_context* ctx, size_t bytes, void** p, size_t* got)
+{
+    {
+        // a spare block at most a quarter larger than asked for
+        std::lock_guard<std::mutex> lock(ctx->spare_mutex);
+        size_t best = ctx->spare.size();
+        for (size_t i = 0; i < ctx->spare.size(); ++i)
+            if (ctx->spare[i].bytes >= bytes && ctx->spare[i].bytes <= bytes + bytes / 4 + (1 << 20) &&
+                (best == ctx->spare.size() || ctx->spare[i].bytes < ctx->spare[best].bytes))
+                best = i;
+        if (best < ctx->spare.size()) {
+            *p = ctx->spare[best].p;
+            *got = ctx->spare[best].bytes;
+            ctx->spare.erase(ctx->spare.begin() + (long)best);
+            return KVSMC_OK;
+        }
+    }
+    KVSMC_CUDA(ctx, device_malloc(ctx, p, bytes));
+    *got = bytes;
+    return KVSMC_OK;
+}
+
+cudaError_t device_malloc_bytes(kvsmc_context* ctx, void** p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && ctx && !ctx->spare.empty()) {
+        cudaGetLastError();
+        block_release(ctx);
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
+void block_release(kvsmc_context* ctx)
+{
+    std::lock_guard<std::mutex> lock(ctx->spare_mutex);
+    for (const kvsmc_context::Spare& s : ctx->spare) cudaFree(s.p);
+    ctx->spare.clear();
+}
+
+void block_free(kvsmc_context* ctx, void* p, size_t bytes)
+{
+    if (!p) return;
+    // Other streams (a server's workers, a plan's) may still read the block:
+    // cudaFree waits for them, so a block that is kept waits for them here.
+    if (ctx && bytes <= kSpareBytes && cudaDeviceSynchronize() == cudaSuccess) {
+        std::lock_guard<std::mutex> lock(ctx->spare_mutex);
+        size_t held = 0;
+        for (const kvsmc_context::Spare& s : ctx->spare) held += s.bytes;
+        while (!ctx->spare.empty() && (held + bytes > kSpareBytes || ctx->spare.size() >= kSpareBlocks)) {
+            held -= ctx->spare.front().bytes;   // the oldest leaves
+            cudaFree(ctx->spare.front().p);
+            ctx->spare.erase(ctx->spare.begin());
+        }
+        ctx->spare.push_back({p, bytes});
+        return;
+    }
+    cudaFree(p);
+}
+
+kvsmc_status volume_alloc(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, uint32_t ny, uint32_t nz,
+                          kvsmc_volume* v)
+{
+    const size_t es = kvsmc::dtype_size(dtype);
+    const uint64_t pitch = align_up(nx, 16 / es);
+    v->view.nx = nx; v->view.ny = ny; v->view.nz = nz;
+    v->view.dtype = dtype;
+    v->view.pitch = pitch;
+    v->view.slice = pitch * ny;
+    v->has_minmax = false;
+    v->range_ready = false;
+    v->bricks_valid = false;
+    // values and 256 bytes of slack | range record | brick table
+    const size_t values = align_up((size_t)pitch * ny * nz * es + 256, 256);
+    const size_t bytes = values + 256 + table_bytes(v->view);
+    if (bytes > v->bytes) {
+        if (v->dev) block_free(ctx, v->dev, v->bytes);
+        v->dev = nullptr;
+        v->bytes = 0;
+        kvsmc_status st = block_alloc(ctx, bytes, &v->dev, &v->bytes);
+        if (st) return st;
+        v->device = ctx->device;
+    }
+    v->view.data = v->dev;
+    v->range = reinterpret_cast<kvsmc::IngestOut*>(static_cast<char*>(v->dev) + values);
+    v->bricks = table_bytes(v->view) ? reinterpret_cast<float2*>(static_cast<char*>(v->dev) + values + 256) : nullptr;
+    return KVSMC_OK;
+}
+
+kvsmc_status volume_bricks(kvsmc_context* ctx, kvsmc_volume* v)
+{
+    KVSMC_CUDA(ctx, kvsmc::launch_ingest(v->view, nullptr, v->bricks, v->range, launch_of(ctx)));
+    v->bricks_valid = v->bricks != nullptr;
+    v->range_ready = true;
+    return KVSMC_OK;
+}
+
+kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src, bool on_device)
+{
+    const size_t es = kvsmc::dtype_size(v->view.dtype);
+    const size_t row = (size_t)v->view.nx * es;
+    const size_t rows = (size_t)v->view.ny * v->view.nz;
+    const size_t dense = row * rows;
+    v->has_minmax = false;
+    v->range_ready = false;
+    const void* from = nullptr;   // values the ingest pass copies (null: they are in place)
+    if (on_device) {
+        // read in place of a copy where the kernel can: device memory of this
+        // GPU, aligned to the value type (a copy takes any address)
+        cudaPointerAttributes a;
+        if ((reinterpret_cast<uintptr_t>(src) % es) == 0 && cudaPointerGetAttributes(&a, src) == cudaSuccess &&
+            a.type == cudaMemoryTypeDevice && a.device == ctx->device)
+            from = src;
+        else
+            cudaGetLastError();
+    } else if (v->view.pitch != v->view.nx && dense <= kDenseStage) {
+        // rows that are padded on the device: one dense copy into a staging
+        // buffer, padded by the ingest pass (a row-by-row copy of 99-node rows
+        // of 16-bit values ran at 6 GB/s: 2.1 MB in 340 us)
+        if (dense > ctx->dense_bytes) {
+            KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+            if (ctx->dense) cudaFree(ctx->dense);
+            ctx->dense = nullptr;
+            ctx->dense_bytes = 0;
+            const size_t want = align_up(dense, 1 << 20);
+            KVSMC_CUDA(ctx, device_malloc(ctx, &ctx->dense, want));
+            ctx->dense_bytes = want;
+        }
+        KVSMC_CUDA(ctx, cudaMemcpyAsync(ctx->dense, src, dense, cudaMemcpyHostToDevice, ctx->stream));
+        from = ctx->dense;
+    }
+    if (!from) {
+        const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+        if (v->view.pitch == v->view.nx)
+            KVSMC_CUDA(ctx, cudaMemcpyAsync(v->dev, src, dense, kind, ctx->stream));
+        else
+            KVSMC_CUDA(ctx, cudaMemcpy2DAsync(v->dev, v->view.pitch * es, src, row, row, rows, kind, ctx->stream));
+    }
+    KVSMC_CUDA(ctx, kvsmc::launch_ingest(v->view, from, v->bricks, v->range, launch_of(ctx)));
+    v->bricks_valid = v->bricks != nullptr;
+    v->range_ready = true;
+    return KVSMC_OK;
+}
+
+kvsmc_status volume_minmax(kvsmc_context* ctx, kvsmc_volume* v)
+{
+    if (v->has_minmax) return KVSMC_OK;
+    if (!v->range_ready)
+        if (kvsmc_status st = volume_bricks(ctx, v)) return st;
+    KVSMC_CUDA(ctx, cudaMemcpyAsync(ctx->h_small, v->range, sizeof(kvsmc::IngestOut), cudaMemcpyDeviceToHost,
+                                    ctx->stream));
+    KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    kvsmc::IngestOut o;
+    std::memcpy(&o, ctx->h_small, sizeof o);
+    decode_range(v->view.dtype, o, v->vmin, v->vmax);
+    v->has_minmax = true;
+    return KVSMC_OK;
+}
+
+void volume_destroy(kvsmc_context* ctx, kvsmc_volume* v)
+{
+    if (v->dev) block_free(ctx && ctx->device == v->device ? ctx : nullptr, v->dev, v->bytes);
+    delete v;
+}
+
+}  // namespace kvsmc_host

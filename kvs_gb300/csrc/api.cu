@@ -74,7 +74,34 @@ Classifier make_classifier(double iso)
 {
     Classifier c;
     c.iso = iso;
-    c.pad = 0;
+    c.all64 = 0;
+    // 64-bit integers: the conversion to double is monotone, so the values with
+    // (double)v > iso are the ones above the last value without
+    constexpr long long kMin = (-0x7fffffffffffffffLL - 1), kMax = 0x7fffffffffffffffLL;
+    c.l_thr = kMax;
+    if ((double)kMax > iso) {   // (never for a NaN)
+        long long lo = kMin, hi = kMax;
+        while (lo < hi) {   // the smallest such value
+            const long long mid = (lo >> 1) + (hi >> 1) + (lo & hi & 1);   // floor((lo + hi) / 2)
+            if ((double)mid > iso) hi = mid; else lo = mid + 1;
+        }
+        if (lo == kMin) c.all64 |= 1;
+        c.l_thr = lo == kMin ? kMin : lo - 1;
+    }
+    c.u_thr = ~0ull;
+    if ((double)~0ull > iso) {
+        unsigned long long lo = 0, hi = ~0ull;
+        while (lo < hi) {
+            const unsigned long long mid = lo + (hi - lo) / 2;
+            if ((double)mid > iso) hi = mid; else lo = mid + 1;
+        }
+        if (lo == 0) c.all64 |= 2;
+        c.u_thr = lo == 0 ? 0 : lo - 1;
+    }
+    const double z = iso == 0.0 ? 0.0 : iso;
+    long long bits;
+    std::memcpy(&bits, &z, sizeof bits);
+    c.d_key = std::isnan(iso) ? kMax : double_key(bits);
     float f = (float)iso;
     if (!std::isnan(iso) && (double)f > iso) f = std::nextafter(f, -INFINITY);
     c.f_thr = f;
@@ -221,8 +248,7 @@ void gather_setup(kvsmc_context* ctx, Plan& pl)
     pl.ntri = pl.nvert = 0;
     Job& j = pl.job;
     const int dt = j.vol.dtype;
-    pl.snode = pl.shared && ctx->path == 0 &&
-               (dt == KVSMC_I8 || dt == KVSMC_I16 || dt == KVSMC_U8 || dt == KVSMC_U16 || dt == KVSMC_F32);
+    pl.snode = pl.shared && ctx->path == 0;
     if (pl.snode) {
         // node units replace the node tiles: (plane, row, 256-node segment)
         pl.wprn = (j.vol.nx + 255) / 256;
@@ -238,7 +264,7 @@ void gather_setup(kvsmc_context* ctx, Plan& pl)
         if (pl.sb) {
             pl.sconn = true;
             j.cell_tiles = 0;
-        } else if (stream_volume_eligible(ctx, *pl.item)) {
+        } else if (any_stream_eligible(ctx, *pl.item)) {
             pl.batch.reset(new StreamBatch());
             pl.batch->ctx = ctx;
             pl.batch->items = {pl.item};
@@ -810,7 +836,7 @@ kvsmc_status run_items(kvsmc_context* ctx, std::vector<Item*>& items, bool emit)
     for (Item* it : items) {
         if (it->status) continue;
         if (!it->extracted) continue;
-        (stream_eligible(ctx, *it) ? stream_items : gather_items).push_back(it);
+        (dup_stream_eligible(ctx, *it) ? stream_items : gather_items).push_back(it);
     }
     kvsmc_status first = KVSMC_OK;
     if (!stream_items.empty()) {
@@ -1147,7 +1173,7 @@ kvsmc_status kvsmc_marching_cubes_host(kvsmc_context* ctx, const void* host, kvs
     if (!it.extracted) return KVSMC_OK;
     // count, size the device outputs, emit
     std::vector<Item*> items{&it};
-    const bool streaming = stream_eligible(ctx, it);
+    const bool streaming = dup_stream_eligible(ctx, it);
     StreamBatch b;
     Plan pl;
     bool written = false;
@@ -1369,7 +1395,7 @@ kvsmc_status kvsmc_extract_batch_host(kvsmc_context* ctx, const void* host, kvsm
         items[i].status = prepare(ctx, items[i]);
         if (items[i].status) { if (!first) first = items[i].status; continue; }
         if (!items[i].extracted) continue;
-        (stream_eligible(ctx, items[i]) ? s_items : g_items).push_back(&items[i]);
+        (dup_stream_eligible(ctx, items[i]) ? s_items : g_items).push_back(&items[i]);
     }
     if (!s_items.empty()) {
         if ((st = stream_host_pipeline(ctx, s_items, items.data(), alloc, user))) {

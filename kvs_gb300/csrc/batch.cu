@@ -114,6 +114,20 @@ bool stream_eligible(const kvsmc_context* ctx, const Item& it)
     return it.params.mode == KVSMC_DUP_POLYGON_NORMAL && stream_volume_eligible(ctx, it);
 }
 
+bool dup_stream_eligible(const kvsmc_context* ctx, const Item& it)
+{
+    return it.params.mode == KVSMC_DUP_POLYGON_NORMAL && any_stream_eligible(ctx, it);
+}
+
+bool any_stream_eligible(const kvsmc_context* ctx, const Item& it)
+{
+    if (stream_volume_eligible(ctx, it)) return true;
+    if (ctx->path != 0 || !it.vol || stream_dtype(it.vol->view.dtype)) return false;
+    const kvsmc::VolumeView& v = it.vol->view;
+    return v.nx >= 2 && v.ny >= 2 && v.nz >= 2 && v.nx - 1 <= (uint32_t)kvsmc::kStreamMaxCells &&
+           (double)(v.nx - 1) * (double)(v.ny - 1) * 5.0 < 4294967295.0 && std::isfinite(it.params.isolevel);
+}
+
 bool stream_volume_eligible(const kvsmc_context* ctx, const Item& it)
 {
     if (ctx->path != 0 || !it.vol) return false;
@@ -131,12 +145,14 @@ bool stream_volume_eligible(const kvsmc_context* ctx, const Item& it)
 
 void StreamBatch::plan_tables()
 {
-    // group by volume in request order, at most kStreamMaxIso per group
+    // group by volume in request order, at most kStreamMaxIso per group (one
+    // for the value types that are classified per isolevel)
     std::vector<std::vector<Item*>> lists;
     std::map<kvsmc_volume*, size_t> open;
     for (Item* it : items) {
         auto f = open.find(it->vol);
-        if (f == open.end() || lists[f->second].size() == (size_t)kvsmc::kStreamMaxIso) {
+        const size_t most = stream_dtype(it->vol->view.dtype) ? (size_t)kvsmc::kStreamMaxIso : 1;
+        if (f == open.end() || lists[f->second].size() == most) {
             open[it->vol] = lists.size();
             lists.push_back({});
             f = open.find(it->vol);
@@ -148,8 +164,8 @@ void StreamBatch::plan_tables()
     std::vector<std::pair<int, int>> kinds;
     std::map<const kvsmc_volume*, kvsmc_tune_choice> shape;
     for (auto& l : lists) shape[l[0]->vol] = stream_shape(ctx, l[0]->vol->view);
-    if (one_row)
-        for (auto& l : lists) shape[l[0]->vol].rows = 1;
+    for (auto& l : lists)
+        if (one_row || !stream_dtype(l[0]->vol->view.dtype)) shape[l[0]->vol].rows = 1;
     // Under the built-in rules, a value type whose volumes mix one- and two-row
     // tasks takes two rows for all of them: one launch per type instead of two
     // (two-row tasks suit every width; on the uneven 200-volume batch this took
@@ -237,7 +253,7 @@ void StreamBatch::plan_tables()
             bucket_params(sorted.front().first, sorted.back().first, g.bs, g.bo);
             g.unit_base = unit_elems;
             unit_elems += stream_units(v, g.wpr, g.niso);
-            if (want_nodes && rows == 1 && g.wpr == (v.nx + 255) / 256) {
+            if (want_nodes && rows == 1 && stream_dtype(dt) && g.wpr == (v.nx + 255) / 256) {
                 g.node_units = (uint64_t)v.nz * v.ny * g.wpr;
                 g.node_base = node_elems;
                 node_elems += (uint64_t)g.niso * g.node_units;
@@ -249,6 +265,7 @@ void StreamBatch::plan_tables()
                 StreamIso s;
                 std::memset(&s, 0, sizeof s);
                 s.f = make_fast(it->params.isolevel, it->vmin, it->vmax, dt);
+                s.cls = make_classifier(it->params.isolevel);
                 s.ip.iso = it->params.isolevel;
                 s.ip.vmin = it->vmin;
                 s.ip.vmax = it->vmax;

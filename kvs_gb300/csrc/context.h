@@ -202,6 +202,11 @@ bool stream_eligible(const kvsmc_context* ctx, const Item& it);
 // The same volume and isolevel conditions, whatever the mode (the streaming
 // count of a shared-vertex request).
 bool stream_volume_eligible(const kvsmc_context* ctx, const Item& it);
+// The same for all ten value types: the 32/64-bit integer and double volumes
+// take the streaming layout too, one isolevel per pass (mc_wide.cu).  (Plans
+// and the server take the narrow types only.)
+bool any_stream_eligible(const kvsmc_context* ctx, const Item& it);
+bool dup_stream_eligible(const kvsmc_context* ctx, const Item& it);
 // Count (and, for items with emit set, emit) all eligible items together.
 kvsmc_status stream_run(kvsmc_context* ctx, std::vector<Item*>& items);
 

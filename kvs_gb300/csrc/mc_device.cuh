@@ -31,13 +31,25 @@ struct VolumeView {
 // Thresholds that make classification exact without FP64:
 //   float data : v > f_thr   with f_thr = largest float <= isolevel
 //   int data   : v > i_thr   with i_thr = floor(isolevel) (clamped)
-//   64-bit int / double data: (double)v > isolevel
+//   64-bit int data: v > l_thr / u_thr, the largest integer whose nearest
+//                double is at most the isolevel
+//   double data: key(v) > d_key, key = an order-preserving integer of the bits
+//                (FP64 compares run at 1/58 of the integer rate)
 struct Classifier {
     double iso;
     float f_thr;
-    int32_t pad;
+    int32_t all64;              // bit 0 / 1: every int64 / uint64 is above (none is at most the isolevel)
     long long i_thr;
+    long long l_thr;
+    unsigned long long u_thr;
+    long long d_key;            // the isolevel's key (-0 as +0)
 };
+
+// Order-preserving integer key of a double (NaN: beyond the infinities).
+__host__ __device__ __forceinline__ long long double_key(long long bits)
+{
+    return bits < 0 ? (bits ^ 0x7fffffffffffffffll) : bits;
+}
 
 // Constants of the FP64 interpolation sequence of one request.
 struct Interp {
@@ -111,15 +123,19 @@ __device__ __forceinline__ double to_double(double v) { return v; }
 
 // calculate_table_index's test `static_cast<double>(v) > isolevel` (MarchingCubes.cpp:306-313).
 __device__ __forceinline__ bool above(const Classifier& c, float v) { return v > c.f_thr; }
-__device__ __forceinline__ bool above(const Classifier& c, double v) { return v > c.iso; }
+__device__ __forceinline__ bool above(const Classifier& c, double v)
+{
+    const long long k = double_key(__double_as_longlong(v));
+    return k > c.d_key && k <= 0x7ff0000000000000ll;
+}
 __device__ __forceinline__ bool above(const Classifier& c, int8_t v) { return (long long)v > c.i_thr; }
 __device__ __forceinline__ bool above(const Classifier& c, int16_t v) { return (long long)v > c.i_thr; }
 __device__ __forceinline__ bool above(const Classifier& c, int32_t v) { return (long long)v > c.i_thr; }
 __device__ __forceinline__ bool above(const Classifier& c, uint8_t v) { return (long long)v > c.i_thr; }
 __device__ __forceinline__ bool above(const Classifier& c, uint16_t v) { return (long long)v > c.i_thr; }
 __device__ __forceinline__ bool above(const Classifier& c, uint32_t v) { return (long long)v > c.i_thr; }
-__device__ __forceinline__ bool above(const Classifier& c, long long v) { return __ll2double_rn(v) > c.iso; }
-__device__ __forceinline__ bool above(const Classifier& c, unsigned long long v) { return __ull2double_rn(v) > c.iso; }
+__device__ __forceinline__ bool above(const Classifier& c, long long v) { return v > c.l_thr || (c.all64 & 1); }
+__device__ __forceinline__ bool above(const Classifier& c, unsigned long long v) { return v > c.u_thr || (c.all64 & 2); }
 
 template <typename T>
 __device__ __forceinline__ T load(const T* p, uint64_t i) { return __ldg(p + i); }
@@ -177,6 +193,30 @@ __device__ __forceinline__ float3 interpolate_exact(const Interp& j, double va, 
     o.x = __fmul_rn(__fadd_rn(__double2float_rn(px), j.min_coord[0]), j.scale[0]);
     o.y = __fmul_rn(__fadd_rn(__double2float_rn(py), j.min_coord[1]), j.scale[1]);
     o.z = __fmul_rn(__fadd_rn(__double2float_rn(pz), j.min_coord[2]), j.scale[2]);
+    return o;
+}
+
+// interpolate_exact for endpoints that differ along `axis`, where the ratio
+// lies in [0, 1] (always, with finite values on both sides of the isolevel):
+// the two constant coordinates come out as themselves (their FP64 form is
+// within 3 2^-53 of an integer below 2^24), so only the varying one is
+// formed.  Same bits as interpolate_exact.
+__device__ __forceinline__ float3 interpolate_exact_axis(const Interp& j, double va, double vb, float ax, float ay,
+                                                         float az, float bx, float by, float bz, int axis)
+{
+    const double v0 = clamp_ref(va, j.vmin, j.vmax);
+    const double v1 = clamp_ref(vb, j.vmin, j.vmax);
+    const double q = __ddiv_rn(__dsub_rn(j.iso, v0), __dsub_rn(v1, v0));
+    const double r = (q < 0.0) ? -q : q;
+    // by the bits: those of a NaN and of -0 are above those of 1
+    if ((unsigned long long)__double_as_longlong(r) > 0x3ff0000000000000ull)
+        return interpolate_exact(j, va, vb, ax, ay, az, bx, by, bz);
+    const float a = axis == 0 ? ax : (axis == 1 ? ay : az), b = axis == 0 ? bx : (axis == 1 ? by : bz);
+    const float p = __double2float_rn(__dadd_rn(__dmul_rn(__dsub_rn(1.0, r), (double)a), __dmul_rn(r, (double)b)));
+    float3 o;
+    o.x = __fmul_rn(__fadd_rn(axis == 0 ? p : ax, j.min_coord[0]), j.scale[0]);
+    o.y = __fmul_rn(__fadd_rn(axis == 1 ? p : ay, j.min_coord[1]), j.scale[1]);
+    o.z = __fmul_rn(__fadd_rn(axis == 2 ? p : az, j.min_coord[2]), j.scale[2]);
     return o;
 }
 

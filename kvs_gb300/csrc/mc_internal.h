@@ -82,6 +82,7 @@ constexpr int kStreamMaxCells = 4096; // cells per row (width <= 4097 nodes)
 struct StreamIso {
     FastIso f;
     Interp ip;
+    Classifier cls;
     uint64_t plane_index;  // its first (isolevel, z) plane in the plane arrays
     float* coords;         // outputs (null: not written)
     float* normals;
@@ -152,6 +153,12 @@ cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_g
                           const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
                           const Launch& L, int ctas_per_sm = 0, uint64_t task0 = 0,
                           uint32_t* d_node_counts = nullptr, const uint64_t* d_totals = nullptr);
+// The same two passes for the 32/64-bit integer and double volumes (one
+// isolevel per group, one row per task); launch_stream calls it for them.
+cudaError_t launch_wide(bool emit, int dtype, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
+                        const StreamIso* d_isos, uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
+                        const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task, const Launch& L,
+                        uint64_t task0, const uint64_t* d_totals);
 // scan_threads: units per CTA pass (64, 128 or 256; 0 = 256).
 cudaError_t launch_unit_scan(const StreamGroup* d_groups, int ngroups, uint32_t nplanes, const StreamIso* d_isos,
                              const uint16_t* d_unit_counts, uint32_t* d_unit_offsets, uint32_t* d_plane_totals,

@@ -34,7 +34,22 @@ namespace kvsmc {
     default: return cudaErrorInvalidValue;              \
     }
 
+// the passes of one request: every value type
+#define KVSMC_SN_SWITCH_ALL(DT, ...)                              \
+    switch (DT) {                                                 \
+    case 2: { using T = int32_t; __VA_ARGS__; } break;            \
+    case 3: { using T = long long; __VA_ARGS__; } break;          \
+    case 6: { using T = uint32_t; __VA_ARGS__; } break;           \
+    case 7: { using T = unsigned long long; __VA_ARGS__; } break; \
+    case 9: { using T = double; __VA_ARGS__; } break;             \
+    default: KVSMC_SN_SWITCH(DT, __VA_ARGS__)                     \
+    }
+
 namespace {
+
+// Value types that are floats exactly (the FP32 certificate applies).
+template <typename T> constexpr bool kSnFast = sizeof(T) < 4;
+template <> constexpr bool kSnFast<float> = true;
 
 constexpr int kSnThreads = 256;
 constexpr int kSnWarps = kSnThreads / 32;
@@ -226,12 +241,16 @@ __global__ void __launch_bounds__(kSnThreads, EMIT ? KVSMC_SNODE_EMIT_CTAS : 1)
                         }
                     const uint32_t xl = L + 32u * wi;
                     const float ax = __uint2float_rn((uint32_t)xoff + xl);
-                    const float v0 = (float)ra[xl];
-                    const float v1 = (float)(axis == 0 ? ra[xl + 1] : (axis == 1 ? rb[xl] : rz[xl]));
+                    const T v0 = ra[xl], v1 = axis == 0 ? ra[xl + 1] : (axis == 1 ? rb[xl] : rz[xl]);
                     const float bxf = axis == 0 ? __fadd_rn(ax, 1.0f) : ax;
                     const float byf = axis == 1 ? __fadd_rn(fyf, 1.0f) : fyf;
                     const float bzf = axis == 2 ? __fadd_rn(fzf, 1.0f) : fzf;
-                    const float3 p = edge_vertex_fast(j.ip, f, v0, v1, ax, fyf, fzf, bxf, byf, bzf, axis);
+                    float3 p;
+                    if constexpr (kSnFast<T>)
+                        p = edge_vertex_fast(j.ip, f, (float)v0, (float)v1, ax, fyf, fzf, bxf, byf, bzf, axis);
+                    else
+                        p = interpolate_exact_axis(j.ip, to_double(v0), to_double(v1), ax, fyf, fzf, bxf, byf, bzf,
+                                                   axis);
                     float* o = j.coords + 3 * (base + q);
                     o[0] = p.x; o[1] = p.y; o[2] = p.z;
                 }
@@ -1119,7 +1138,7 @@ cudaError_t launch_sconnect(const Job& j, const StreamGroup* d_groups, const Str
     if (ntasks == 0) return cudaSuccess;
     const int dt = j.vol.dtype;
     const size_t smem = sconnect_shared_bytes(dt);
-    KVSMC_SN_SWITCH(dt, {
+    KVSMC_SN_SWITCH_ALL(dt, {
         auto kern = k_sconnect<T>;
         int per_sm = 0;
         const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), kSnThreads, smem, &per_sm);
@@ -1218,7 +1237,7 @@ cudaError_t launch_snode(bool emit, const Job& j, const FastIso& f, uint32_t wpr
     const size_t smem = snode_shared_bytes(dt);
     const uint32_t row_elems = (uint32_t)stream_row_elems(dt, 1);
     const uint32_t copy_bytes = row_elems * (uint32_t)dtype_size(dt);
-    KVSMC_SN_SWITCH(dt, {
+    KVSMC_SN_SWITCH_ALL(dt, {
         auto kern = emit ? k_snode<T, true> : k_snode<T, false>;
         int per_sm = 0;
         const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), kSnThreads, smem, &per_sm);

@@ -843,6 +843,7 @@ kvsmc_status run_items(kvsmc_context* ctx, std::vector<Item*>& items, bool emit)
         StreamBatch b;
         b.ctx = ctx;
         b.items = stream_items;
+        b.want_list = emit;
         kvsmc_status st = b.place();
         if (!st && emit) {
             st = b.extract();
@@ -1182,6 +1183,7 @@ kvsmc_status kvsmc_marching_cubes_host(kvsmc_context* ctx, const void* host, kvs
         // only a result that it does not hold is written in a second go
         b.ctx = ctx;
         b.items = items;
+        b.want_list = true;
         const uint64_t cap = ctx->out_bytes / 48 / 64 * 64;
         it.d_coords = cap ? static_cast<float*>(ctx->out_arena) : nullptr;
         it.d_normals = cap ? it.d_coords + 9 * cap : nullptr;
@@ -1316,6 +1318,7 @@ static kvsmc_status stream_host_pipeline(kvsmc_context* ctx, std::vector<Item*>&
     StreamBatch b;
     b.ctx = ctx;
     b.items = s_items;
+    b.want_list = true;
     kvsmc_status st;
     if ((st = b.plan()) || (st = b.count()) || (st = arena_outputs(ctx, s_items)) ||
         (st = host_alloc(ctx, s_items, first_item, alloc, user)))

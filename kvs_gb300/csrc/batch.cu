@@ -204,6 +204,8 @@ void StreamBatch::plan_tables()
     scan_blocks = 0;
     iso_planes = 0;
     node_elems = 0;
+    pair_units = 0;
+    uint64_t pairs_most = 0;   // (cell, isolevel) pairs of the listed kinds
     for (const auto& kd : kinds) {
         const int dt = kd.first, rows = kd.second;
         Launch1 L;
@@ -211,19 +213,27 @@ void StreamBatch::plan_tables()
         L.rows = rows;
         L.g0 = (int)groups.size();
         L.ntasks = 0;
+        L.netasks = 0;
+        L.listed = want_list && stream_dtype(dt);
+        L.one = true;
         // one z-chunk for the whole launch: sized by all its warp steps, so a
         // batch of small volumes gets long tasks rather than many short ones
-        uint64_t steps = 0;
+        uint64_t steps = 0, units = 0;
         const kvsmc_volume* big = nullptr;
         for (auto& l : lists) {
             if (kind_of(l) != kd) continue;
             const kvsmc::VolumeView& v = l[0]->vol->view;
             steps += (uint64_t)(v.nz - 1) * ((v.ny - 1 + rows - 1) / rows) * segments_per_row(v, rows);
+            units += (uint64_t)(v.nz - 1) * (v.ny - 1) * segments_per_row(v, rows);
             if (!big || cells_of(v) > cells_of(big->view)) big = l[0]->vol;
         }
         const kvsmc_tune_choice& bs_shape = shape[big];
         L.ctas_per_sm = bs_shape.ctas_per_sm;
         const uint32_t zchunk = stream_zchunk(steps, ctx->num_sms, bs_shape.tasks_per_sm);
+        // units per block of the listing emit: enough blocks for every resident
+        // warp to take two, at most a warp's lanes, at least two
+        const uint32_t eblock = (uint32_t)std::min<uint64_t>(
+            32, std::max<uint64_t>(2, units / ((uint64_t)ctx->num_sms * 2 * kvsmc::kPairWarpsPerSm)));
         for (auto& l : lists) {
             if (kind_of(l) != kd) continue;
             const kvsmc::VolumeView v = l[0]->vol->view;
@@ -250,6 +260,7 @@ void StreamBatch::plan_tables()
                              [](const std::pair<float, Item*>& a, const std::pair<float, Item*>& b) { return a.first < b.first; });
             g.iso_begin = (int32_t)isos.size();
             g.niso = (int32_t)sorted.size();
+            L.one = L.one && g.niso == 1;
             bucket_params(sorted.front().first, sorted.back().first, g.bs, g.bo);
             g.unit_base = unit_elems;
             unit_elems += stream_units(v, g.wpr, g.niso);
@@ -257,6 +268,17 @@ void StreamBatch::plan_tables()
                 g.node_units = (uint64_t)v.nz * v.ny * g.wpr;
                 g.node_base = node_elems;
                 node_elems += (uint64_t)g.niso * g.node_units;
+            }
+            g.seg_cells = (uint32_t)(kvsmc::kStreamSegCells / rows);
+            g.eblock = eblock;
+            const uint32_t plane_units = (v.ny - 1) * g.wpr;
+            g.eblocks = (plane_units + eblock - 1) / eblock;
+            g.etask_begin = L.netasks;
+            L.netasks += (uint64_t)cz * g.eblocks;
+            if (L.listed) {
+                g.pair_base = pair_units;
+                pair_units += (uint64_t)cz * plane_units;
+                pairs_most += cells_of(v) * (uint64_t)g.niso;
             }
             g.plane_begin = scan_blocks;
             scan_blocks += cz;
@@ -280,6 +302,19 @@ void StreamBatch::plan_tables()
         L.ng = (int)groups.size() - L.g0;
         launches.push_back(L);
     }
+    // Room for every pair there can be (a warp leaves at most as many entries
+    // of a run unused as it then takes, and a run at its end), up to 2^29
+    // entries (1 GiB); beyond that for one pair in 8 (smooth data has one in
+    // 50, and a foam that exceeds it is classified again), at most 2^31.
+    list_cap = 0;
+    list_sure = false;
+    if (pair_units) {
+        const uint64_t tail = (uint64_t)ctx->num_sms * 32 * kvsmc::kPairRun * launches.size();   // (warps of each count)
+        const uint64_t sure = 2 * pairs_most + tail;
+        list_cap = std::min<uint64_t>(sure, std::max<uint64_t>((uint64_t)1 << 29, pairs_most / 8) + tail);
+        list_cap = std::min<uint64_t>(list_cap, (uint64_t)1 << 31);
+        list_sure = list_cap >= sure;
+    }
 }
 
 size_t StreamBatch::scratch_bytes() const
@@ -289,7 +324,8 @@ size_t StreamBatch::scratch_bytes() const
            align_up(unit_elems * 2, 256) + align_up(unit_elems * 4, 256) + align_up(iso_planes * 4, 256) +
            align_up(iso_planes * 8, 256) + align_up(kvsmc::scan_scratch_bytes(iso_planes), 256) +
            align_up(niso * 8, 256) + align_up(launches.size() * 16, 256) + align_up(kMaxParts * 8, 256) +
-           align_up(node_elems * 4, 256) + 6 * 256;
+           align_up(node_elems * 4, 256) + 6 * 256 +
+           (list_cap ? align_up(pair_units * 2, 256) + align_up(pair_units * 4, 256) + align_up(list_cap * 2, 256) : 0);
 }
 
 void StreamBatch::carve(char* base)
@@ -307,18 +343,32 @@ void StreamBatch::carve(char* base)
     d_next_parts = cv.take<unsigned long long>(kMaxParts * 8);
     d_unit_counts = cv.take<uint16_t>(unit_elems * 2);
     d_node_counts = node_elems ? cv.take<uint32_t>(node_elems * 4) : nullptr;
+    list = kvsmc::PairList{};
+    if (list_cap) list.unit_pairs = cv.take<uint16_t>(pair_units * 2);
     zero_bytes = (size_t)(base + cv.off - reinterpret_cast<char*>(d_status));
     d_unit_offsets = cv.take<uint32_t>(unit_elems * 4);
     d_plane_totals = cv.take<uint32_t>(iso_planes * 4);
     d_plane_base = cv.take<uint64_t>(iso_planes * 8);
     d_scan = cv.take<char>(kvsmc::scan_scratch_bytes(iso_planes));
     d_total = cv.take<uint64_t>(256);
+    if (list_cap) {
+        list.unit_list = cv.take<uint32_t>(pair_units * 4);
+        list.list = cv.take<uint16_t>(list_cap * 2);
+        list.cap = list_cap;
+        list.cursor = reinterpret_cast<unsigned long long*>(d_status) + 16;
+        list.overflow = d_status + 8;
+    }
 }
 
 kvsmc_status StreamBatch::place()
 {
     plan_tables();
     kvsmc_status st = ensure_scratch(ctx, scratch_bytes());
+    if (st == KVSMC_ERR_OUT_OF_MEMORY && list_cap) {   // no room for the list: the emit classifies again
+        cudaGetLastError();
+        list_cap = 0;
+        st = ensure_scratch(ctx, scratch_bytes());
+    }
     if (st) return st;
     carve(static_cast<char*>(ctx->scratch));
     return KVSMC_OK;
@@ -359,15 +409,24 @@ kvsmc_status StreamBatch::count_enqueue()
     KVSMC_CUDA(ctx, cudaMemsetAsync(d_status, 0, zero_bytes, ctx->stream));
     // one count launch per (value type, rows) kind, side by side
     KVSMC_CUDA(ctx, fan_out(ctx, ctx->stream, launches.size(), [&](size_t i, cudaStream_t st) {
-        const Launch1& l = launches[i];
         kvsmc::Launch Li = L;
         Li.stream = st;
-        return kvsmc::launch_stream(false, l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts,
-                                    nullptr, nullptr, d_status, d_next + 2 * i, Li, l.ctas_per_sm, 0,
-                                    node_elems && l.rows == 1 ? d_node_counts : nullptr);
+        return count_kind(i, Li);
     }));
     KVSMC_CUDA(ctx, scans(L));
     return KVSMC_OK;
+}
+
+cudaError_t StreamBatch::count_kind(size_t i, const kvsmc::Launch& L)
+{
+    const Launch1& l = launches[i];
+    uint32_t* nodes = node_elems && l.rows == 1 ? d_node_counts : nullptr;
+    const kvsmc::PairList* pairs = list_cap && l.listed ? &list : nullptr;
+    if (l.one && !nodes)
+        return kvsmc::launch_count_one(l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts, d_status,
+                                       d_next + 2 * i, L, pairs);
+    return kvsmc::launch_stream(false, l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts, nullptr,
+                                nullptr, d_status, d_next + 2 * i, L, l.ctas_per_sm, 0, nodes, nullptr, pairs);
 }
 
 cudaError_t StreamBatch::scans(const kvsmc::Launch& L)
@@ -398,6 +457,9 @@ kvsmc_status StreamBatch::count_finish()
     const size_t n = isos.size();
     int status;
     std::memcpy(&status, ctx->h_stage, sizeof(int));
+    int over = 0;
+    std::memcpy(&over, static_cast<const char*>(ctx->h_stage) + 8 * sizeof(int), sizeof over);
+    overflowed = over != 0;
     if (status) return fail(ctx, KVSMC_ERR_TIMEOUT, "streaming passes: a shared-memory load did not complete");
     const uint64_t* h = reinterpret_cast<const uint64_t*>(static_cast<const char*>(ctx->h_stage) + 256);
     for (size_t i = 0; i < n; ++i) {
@@ -432,19 +494,33 @@ kvsmc_status StreamBatch::extract()
     if (!st) st = read_enqueue();
     if (st) return st;
     KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return count_finish();
+    if ((st = count_finish())) return st;
+    if (!overflowed || !any) return KVSMC_OK;
+    // the pairs did not fit their list: the listing emit did nothing
+    if ((st = emit_enqueue(d_totals))) return st;
+    return finish();
+}
+
+cudaError_t StreamBatch::emit_kind(size_t i, const kvsmc::Launch& L, const uint64_t* d_fit)
+{
+    const Launch1& l = launches[i];
+    if (list_cap && l.listed && !overflowed)
+        return kvsmc::launch_emit_pairs(l.dtype, d_groups + l.g0, l.ng, l.netasks, d_isos, list, d_unit_offsets,
+                                        d_plane_base, d_status, d_next + 2 * i + 1, L, 0, d_fit);
+    return kvsmc::launch_stream(true, l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts,
+                                d_unit_offsets, d_plane_base, d_status, d_next + 2 * i + 1, L, l.ctas_per_sm, 0, nullptr,
+                                d_fit);
 }
 
 kvsmc_status StreamBatch::emit_enqueue(const uint64_t* d_fit)
 {
     const kvsmc::Launch L = launch_of(ctx);
+    if (overflowed)   // (an emit may have taken the tasks already)
+        KVSMC_CUDA(ctx, cudaMemsetAsync(d_next, 0, launches.size() * 16, ctx->stream));
     KVSMC_CUDA(ctx, fan_out(ctx, ctx->stream, launches.size(), [&](size_t i, cudaStream_t st) {
-        const Launch1& l = launches[i];
         kvsmc::Launch Li = L;
         Li.stream = st;
-        return kvsmc::launch_stream(true, l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts,
-                                    d_unit_offsets, d_plane_base, d_status, d_next + 2 * i + 1, Li, l.ctas_per_sm, 0,
-                                    nullptr, d_fit);
+        return emit_kind(i, Li, d_fit);
     }));
     return KVSMC_OK;
 }
@@ -506,11 +582,16 @@ kvsmc_status StreamBatch::emit_parts(int parts, const std::function<kvsmc_status
     uint64_t c0 = 0;
     for (int p = 0; p < parts; ++p) {
         const uint64_t c1 = zchunks * (uint64_t)(p + 1) / (uint64_t)parts;
-        KVSMC_CUDA(ctx, kvsmc::launch_stream(true, l.dtype, l.rows, d_groups, 1, c1 * per_chunk, d_isos, d_unit_counts,
-                                             d_unit_offsets, d_plane_base, d_status, d_next_parts + p, L,
-                                             l.ctas_per_sm, c0 * per_chunk));
         const uint32_t z0 = (uint32_t)(c0 * g.zchunk);
         const uint32_t z1 = (uint32_t)(c1 * g.zchunk < cz ? c1 * g.zchunk : cz);
+        if (list_cap && l.listed && !overflowed)   // (its blocks are numbered plane-major)
+            KVSMC_CUDA(ctx, kvsmc::launch_emit_pairs(l.dtype, d_groups, 1, (uint64_t)z1 * g.eblocks, d_isos, list,
+                                                     d_unit_offsets, d_plane_base, d_status, d_next_parts + p, L,
+                                                     (uint64_t)z0 * g.eblocks, nullptr));
+        else
+            KVSMC_CUDA(ctx, kvsmc::launch_stream(true, l.dtype, l.rows, d_groups, 1, c1 * per_chunk, d_isos,
+                                                 d_unit_counts, d_unit_offsets, d_plane_base, d_status,
+                                                 d_next_parts + p, L, l.ctas_per_sm, c0 * per_chunk));
         if ((st = after(z0, z1, false))) return st;
         c0 = c1;
     }

@@ -57,6 +57,9 @@ struct StreamBatch {
         int g0, ng;
         uint64_t ntasks;
         int ctas_per_sm;   // 0: as many as fit
+        uint64_t netasks;  // blocks of units of the listing emit
+        bool listed;       // the count lists this kind's pairs
+        bool one;          // every group holds one isolevel
     };
     std::vector<kvsmc::StreamGroup> groups;
     std::vector<kvsmc::StreamIso> isos;
@@ -75,6 +78,16 @@ struct StreamBatch {
     bool one_row = false;
     uint64_t node_elems = 0;
     uint32_t* d_node_counts = nullptr;
+    // the count pass lists the active pairs of the 8/16-bit and float32 groups
+    // for the emit of mc_pairs.cu (set before plan_tables); list_cap: entries
+    // there is room for (0: no list), list_sure: no count can exceed them;
+    // overflowed: the last count did, its emit classifies again
+    bool want_list = false;
+    uint64_t list_cap = 0;
+    bool list_sure = false;
+    bool overflowed = false;
+    uint64_t pair_units = 0;
+    kvsmc::PairList list{};
 
     kvsmc::StreamGroup* d_groups = nullptr;
     kvsmc::StreamIso* d_isos = nullptr;
@@ -118,6 +131,10 @@ struct StreamBatch {
     // complete once the stream reaches that point.
     kvsmc_status emit_parts(int parts, const std::function<kvsmc_status(uint32_t, uint32_t, bool)>& after);
 
+    // One kind's count.
+    cudaError_t count_kind(size_t i, const kvsmc::Launch& L);
+    // One kind's emit: over the listed pairs, or classifying again.
+    cudaError_t emit_kind(size_t i, const kvsmc::Launch& L, const uint64_t* d_fit);
     // The emit launches; d_fit: see launch_stream's d_totals.
     kvsmc_status emit_enqueue(const uint64_t* d_fit);
     // The scans behind a count: unit offsets, plane bases, totals.

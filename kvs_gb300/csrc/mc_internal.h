@@ -114,7 +114,30 @@ struct StreamGroup {
     // node_base + k * node_units + u; node_units == 0: not counted
     uint64_t node_base;
     uint64_t node_units;
+    // the listing emit (mc_pairs.cu): its tasks are blocks of `eblock`
+    // consecutive units of one cell plane, `eblocks` per plane
+    uint64_t etask_begin;    // first block of this group in its launch
+    uint64_t pair_base;      // first of its units' list descriptors
+    uint32_t eblock, eblocks;
+    uint32_t seg_cells;      // cells per unit (256 / rows)
+    uint32_t pad;
 };
+
+// The active (cell, isolevel) pairs found by a count pass: per unit their
+// number and first entry, the entries (cell in the unit's segment | isolevel
+// << 8, in cell order, then isolevel), how many entries there is room for, the
+// next free one, and a word set when the room did not suffice.
+struct PairList {
+    uint16_t* unit_pairs;
+    uint32_t* unit_list;
+    uint16_t* list;
+    uint64_t cap;
+    unsigned long long* cursor;
+    int* overflow;
+};
+// A count's warp takes entries in runs of this many (or one step's, if more).
+constexpr uint32_t kPairRun = 1024;
+constexpr int kPairWarpsPerSm = 24;   // resident warps of the listing emit
 
 // Brick min/max table of a volume: one float2 per (8 cell planes, 2 cell
 // rows, 128 cells) brick, the min and max of its node box ((-inf, +inf) when
@@ -147,12 +170,26 @@ size_t stream_row_elems(int dtype, int rows);
 // launch split by z-chunks).  d_totals (emit): per isolevel record its
 // triangles; a request whose total exceeds its cap_tris writes nothing (null:
 // each request writes up to its cap_tris).  The emit writes nothing when the
-// status word says that the count gave up.
+// status word says that the count gave up.  list (count): also list the pairs.
+// d_only_if (emit): the launch does nothing when this word is zero.
 cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
                           const StreamIso* d_isos, uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
                           const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
                           const Launch& L, int ctas_per_sm = 0, uint64_t task0 = 0,
-                          uint32_t* d_node_counts = nullptr, const uint64_t* d_totals = nullptr);
+                          uint32_t* d_node_counts = nullptr, const uint64_t* d_totals = nullptr,
+                          const PairList* list = nullptr, const int* d_only_if = nullptr);
+// The count of launches whose groups hold one isolevel each, any value type
+// (mc_one.cu); same outputs as launch_stream's.
+cudaError_t launch_count_one(int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
+                             const StreamIso* d_isos, uint16_t* d_unit_counts, int* d_status,
+                             unsigned long long* d_next_task, const Launch& L, const PairList* list);
+// The emit over the pairs that the count listed (launch_stream with `list`):
+// same outputs, same rules for status and totals; does nothing when the list
+// overflowed.  Tasks: the groups' blocks of units.
+cudaError_t launch_emit_pairs(int dtype, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
+                              const StreamIso* d_isos, const PairList& list, const uint32_t* d_unit_offsets,
+                              const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
+                              const Launch& L, uint64_t task0, const uint64_t* d_totals);
 // The same two passes for the 32/64-bit integer and double volumes (one
 // isolevel per group, one row per task); launch_stream calls it for them.
 cudaError_t launch_wide(bool emit, int dtype, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,

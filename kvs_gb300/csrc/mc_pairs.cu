@@ -1,0 +1,337 @@
+// mc_pairs.cu -- the emit pass over listed cells: the count pass has already
+// found every active (cell, isolevel) pair and listed it, so the triangles
+// are written without classifying the volume again.
+//
+// The count writes, per unit (z, y, segment), its pairs in (cell, isolevel)
+// order as 16-bit entries (cell in the segment | isolevel << 8) somewhere in
+// one list, with the unit's first entry and their number.  A warp task here
+// is a block of up to 32 consecutive units of one cell plane: lane u takes
+// unit u's descriptor, a warp scan makes one index space of the block's
+// pairs, and they are taken 32 at a time, one per lane, whatever unit they
+// belong to.  Consecutive units' triangles of one isolevel are consecutive in
+// its output, so an isolevel's position is its first unit's offset plus a
+// running count.  Per round:
+//   * each lane reads its cell's 8 corner values from the volume (L1/L2: a
+//     cell's neighbours share its sectors), forms the corner code by 8
+//     compares and leaves the values in a shared 8 x 32 table;
+//   * lanes of the same isolevel are grouped with __match_any_sync, bit-sliced
+//     ballots give each pair's output position;
+//   * one lane per (pair, used edge) interpolates a vertex (the FP32
+//     certificate of mc_interp.cuh) into a pool, one lane per (pair, triangle)
+//     reads its three and writes the triangle.
+// The rounds are full up to a block's last one (the re-classifying emit took
+// the pairs of one 256-cell segment at a time: 6 of 32 lanes with one
+// isolevel on smooth data), nothing waits for staged planes, and without the
+// ring and the masks 24 warps are resident on an SM instead of 16.
+#include <cuda_runtime.h>
+
+#include "mc_emit.cuh"
+#include "mc_internal.h"
+#include "mc_interp.cuh"
+#include "mc_tables.h"
+#include "tma.cuh"
+
+#ifndef KVSMC_PAIRS_CTAS
+#define KVSMC_PAIRS_CTAS 3
+#endif
+
+namespace kvsmc {
+
+namespace {
+
+constexpr int kPairThreads = 256;
+constexpr int kPairWarps = kPairThreads / 32;
+constexpr int kPairVerts = 192;          // vertex items of one round
+constexpr int kPairTris = 32 * 5;        // triangle items of one round
+constexpr unsigned FULL = 0xffffffffu;
+
+// Case tables indexed by the corner code (bit r: row r's node i above, rows
+// (y, z) (y+1, z) (y, z+1) (y+1, z+1); bit 4 + r: its node i + 1), laid out
+// at compile time and copied into shared memory by one bulk copy per CTA.
+struct alignas(16) PairTables {
+    uint64_t tri_slots[256];   // per triangle corner: its edge's rank among the used edges, 4 bits each
+    uint64_t edge_list[256];   // the used edges in increasing order, 4 bits each
+    uint16_t edge_mask[256];
+    uint8_t ntri[256];
+    uint8_t edge[16];          // corner A | corner B << 3 | axis << 6 (corner: dx + 2 dy + 4 dz)
+};
+static_assert(sizeof(PairTables) % 16 == 0, "copied by a bulk copy");
+
+constexpr uint64_t h_tri[256] = MC_TRI_PACKED_INIT;
+constexpr uint8_t h_ntri[256] = MC_NTRI_INIT;
+constexpr uint16_t h_mask[256] = MC_EDGE_MASK_INIT;
+constexpr uint8_t h_edge[12] = MC_EDGE_PACKED_INIT;
+
+constexpr uint32_t h_case(uint32_t c)
+{
+    return (c & 1u) | (((c >> 4) & 1u) << 1) | (((c >> 5) & 1u) << 2) | (((c >> 1) & 1u) << 3) |
+           (((c >> 2) & 1u) << 4) | (((c >> 6) & 1u) << 5) | (((c >> 7) & 1u) << 6) | (((c >> 3) & 1u) << 7);
+}
+
+constexpr PairTables make_tables()
+{
+    PairTables t{};
+    for (uint32_t code = 0; code < 256; ++code) {
+        const uint32_t cs = h_case(code), em = h_mask[cs];
+        t.ntri[code] = h_ntri[cs];
+        t.edge_mask[code] = (uint16_t)em;
+        int n = 0;
+        for (uint32_t e = 0; e < 12; ++e)
+            if ((em >> e) & 1u) t.edge_list[code] |= (uint64_t)e << (4 * n++);
+        for (int c = 0; c < 3 * (int)h_ntri[cs]; ++c) {
+            const uint32_t e = (uint32_t)(h_tri[cs] >> (4 * c)) & 15u;
+            uint64_t rank = 0;
+            for (uint32_t b = 0; b < e; ++b) rank += (em >> b) & 1u;
+            t.tri_slots[code] |= rank << (4 * c);
+        }
+    }
+    for (int e = 0; e < 12; ++e) {
+        const uint32_t c0 = h_edge[e] & 7u, c1 = h_edge[e] >> 3, d = c0 ^ c1;
+        t.edge[e] = (uint8_t)(c0 | (c1 << 3) | ((d == 1u ? 0u : (d == 2u ? 1u : 2u)) << 6));
+    }
+    return t;
+}
+
+__device__ PairTables d_pair_tables = make_tables();
+
+struct alignas(16) PairWarp {
+    IsoConst ic[kStreamMaxIso];
+    float4 pv[kPairVerts];     // vertex pool: x, y, z, unused (one 16-byte access per vertex)
+    float cv[8][32];           // corner values of the round's cells
+    uint32_t add[32];          // per isolevel: triangles of the round
+    uint8_t item_v[kPairVerts];
+    uint8_t item_t[kPairTris];
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
+    k_emit_pairs(const StreamGroup* __restrict__ groups, int ngroups, uint64_t ntasks,
+                 const StreamIso* __restrict__ isos, PairList pl, const uint32_t* __restrict__ unit_offsets,
+                 const uint64_t* __restrict__ plane_base, int* __restrict__ status,
+                 unsigned long long* __restrict__ next_task, uint32_t wait_polls, uint64_t task0,
+                 const uint64_t* __restrict__ totals)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t bar;
+    PairTables& TB = *reinterpret_cast<PairTables*>(smem_raw);
+    const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    PairWarp& W = reinterpret_cast<PairWarp*>(smem_raw + sizeof(PairTables))[warp];
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        fence_barrier_init();
+        mbar_arrive_expect_tx(&bar, sizeof(PairTables));
+        bulk_copy_g2s(&TB, &d_pair_tables, sizeof(PairTables), &bar);
+    }
+    W.add[lane] = 0;
+    // nothing to write at when the count gave up or its list overflowed (the
+    // caller then runs the re-classifying emit)
+    const bool stop = __syncthreads_or(*status != 0 || *pl.overflow != 0);
+    const bool ok = mbar_wait(&bar, 0, wait_polls);
+    if (!__syncthreads_and(ok) || stop) {
+        if (tid == 0) {
+            if (!stop) atomicExch(status, 1);
+            mbar_wait(&bar, 0, 1u << 16);   // the copy lands before the CTA leaves
+        }
+        return;
+    }
+    const unsigned lt = (1u << lane) - 1u;
+    int gi = 0, gcur = -1;
+    bool live = true;
+    for (;;) {
+        unsigned long long tk = 0;
+        if (lane == 0) tk = atomicAdd(next_task, 1ull);
+        const uint64_t task = task0 + __shfl_sync(FULL, tk, 0);
+        if (task >= ntasks) break;
+        while (gi + 1 < ngroups && task >= groups[gi + 1].etask_begin) ++gi;   // (tasks come in increasing order)
+        const StreamGroup& G = groups[gi];
+        if (G.skip_emit) continue;
+        const int niso = G.niso, iso_begin = G.iso_begin;
+        if (gi != gcur) {
+            __syncwarp();
+            if (lane < (unsigned)niso) fill_iso(W.ic[lane], isos[iso_begin + lane], totals, iso_begin + (int)lane);
+            live = __any_sync(FULL, lane < (unsigned)niso && W.ic[lane & 15u].coords != nullptr);
+            gcur = gi;
+        }
+        if (!live) continue;
+        const uint32_t cy = G.vol.ny - 1, wpr = G.wpr, ub = G.eblock;
+        const uint32_t local = (uint32_t)(task - G.etask_begin);
+        const uint32_t z = local / G.eblocks, u0 = (local - z * G.eblocks) * ub;   // first unit in the plane
+        const uint32_t plane_units = cy * wpr;
+        // lane u: unit u0 + u's pairs and where they are listed
+        uint32_t np = 0, first = 0;
+        const uint32_t un = u0 + lane;
+        if (lane < ub && un < plane_units) {
+            const uint64_t pu = G.pair_base + (uint64_t)z * plane_units + un;
+            np = pl.unit_pairs[pu];
+            if (np) first = pl.unit_list[pu];
+        }
+        uint32_t inc = np;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(FULL, inc, o);
+            if (lane >= (unsigned)o) inc += t;
+        }
+        const uint32_t npairs = __shfl_sync(FULL, inc, 31);
+        if (npairs == 0) continue;
+        first -= inc - np;   // entry of pair p of this unit: list[first + p]
+        const uint32_t uy = un / wpr;
+        const uint32_t ux = (un - uy * wpr) * G.seg_cells;
+        // lane k: the next output triangle of isolevel k
+        uint64_t run = 0;
+        if (lane < (unsigned)niso) {
+            const uint64_t pi = isos[iso_begin + lane].plane_index;
+            run = plane_base[pi + z] - plane_base[pi] +
+                  unit_offsets[G.unit_base + ((uint64_t)z * plane_units + u0) * niso + lane];
+        }
+        const uint64_t pitch = G.vol.pitch, slice = G.vol.slice;
+        const T* vz = static_cast<const T*>(G.vol.data) + (uint64_t)z * slice;
+        const float fz = __uint2float_rn(z);
+        uint32_t taken = 0;
+        for (uint32_t r0 = 0; r0 < npairs; r0 += taken) {
+            // ---- one pair per lane, as many as the vertex pool holds
+            const uint32_t p = r0 + lane;
+            bool has = p < npairs;
+            uint32_t own = 0;   // its unit: the first lane whose inclusive count exceeds p
+#pragma unroll
+            for (int s = 4; s >= 0; --s) {
+                const uint32_t mid = own + (1u << s) - 1u;
+                if (__shfl_sync(FULL, inc, mid) <= p) own = mid + 1;
+            }
+            own &= 31u;   // (lanes past the last pair)
+            const uint32_t at = __shfl_sync(FULL, first, own) + p;
+            const uint32_t y = __shfl_sync(FULL, uy, own);
+            uint32_t x = __shfl_sync(FULL, ux, own);
+            uint32_t k = 0, code = 0;
+            if (has) {
+                const uint32_t e = pl.list[at];
+                x += e & 0xffu;
+                k = e >> 8;
+                const T* c = vz + (uint64_t)y * pitch + x;
+                const float thr = W.ic[k].f.f_thr;
+                const float v0 = (float)__ldg(c), v1 = (float)__ldg(c + 1);
+                const float v2 = (float)__ldg(c + pitch), v3 = (float)__ldg(c + pitch + 1);
+                const float v4 = (float)__ldg(c + slice), v5 = (float)__ldg(c + slice + 1);
+                const float v6 = (float)__ldg(c + slice + pitch), v7 = (float)__ldg(c + slice + pitch + 1);
+                W.cv[0][lane] = v0; W.cv[1][lane] = v1; W.cv[2][lane] = v2; W.cv[3][lane] = v3;
+                W.cv[4][lane] = v4; W.cv[5][lane] = v5; W.cv[6][lane] = v6; W.cv[7][lane] = v7;
+                code = (v0 > thr ? 1u : 0u) | (v2 > thr ? 2u : 0u) | (v4 > thr ? 4u : 0u) | (v6 > thr ? 8u : 0u) |
+                       (v1 > thr ? 16u : 0u) | (v3 > thr ? 32u : 0u) | (v5 > thr ? 64u : 0u) | (v7 > thr ? 128u : 0u);
+            }
+            const uint32_t ne0 = has ? (uint32_t)__popc(TB.edge_mask[code]) : 0u;
+            uint32_t vpre = 0;
+#pragma unroll
+            for (int bit = 0; bit < 4; ++bit)
+                vpre += (uint32_t)__popc(__ballot_sync(FULL, (ne0 >> bit) & 1u) & lt) << bit;
+            has = has && vpre + ne0 <= (uint32_t)kPairVerts;   // a suffix of lanes waits
+            taken = (uint32_t)__popc(__ballot_sync(FULL, has));
+            const uint32_t nv = __shfl_sync(FULL, vpre + ne0, taken - 1);
+            const uint32_t nt = has ? TB.ntri[code] : 0u;
+            const uint32_t ne = has ? ne0 : 0u;
+            const uint32_t pe = x | (k << 12) | (code << 16);   // (x < 4096)
+            // output position of the pair's first triangle: its isolevel's running
+            // count plus the triangles of the earlier lanes of that isolevel
+            const uint32_t grp = niso == 1 ? __ballot_sync(FULL, has) : __match_any_sync(FULL, has ? k : 32u + lane);
+            uint32_t pre = 0, gtot = 0, tpre = 0, ntr = 0;
+#pragma unroll
+            for (int bit = 0; bit < 3; ++bit) {
+                const uint32_t bm = __ballot_sync(FULL, (nt >> bit) & 1u);
+                pre += (uint32_t)__popc(bm & grp & lt) << bit;
+                gtot += (uint32_t)__popc(bm & grp) << bit;
+                tpre += (uint32_t)__popc(bm & lt) << bit;
+                ntr += (uint32_t)__popc(bm) << bit;
+            }
+            const uint64_t obase = __shfl_sync(FULL, run, k) + pre;
+            if (has && (31 - __clz(grp)) == (int)lane) W.add[k] = gtot;
+            for (uint32_t r = 0; r < ne; ++r) W.item_v[vpre + r] = (uint8_t)lane;
+            for (uint32_t t = 0; t < nt; ++t) W.item_t[tpre + t] = (uint8_t)lane;
+            __syncwarp();
+            run += W.add[lane];
+            W.add[lane] = 0;
+            // ---- vertices: one (pair, used edge) per lane
+            for (uint32_t j0 = 0; j0 < nv; j0 += 32) {
+                const uint32_t j = j0 + lane;
+                const bool hv = j < nv;
+                const uint32_t q = hv ? W.item_v[j] : 0u;
+                const uint32_t qe = __shfl_sync(FULL, pe, q);
+                const uint32_t qv = __shfl_sync(FULL, vpre, q);
+                const uint32_t qy = __shfl_sync(FULL, y, q);
+                const uint32_t e = (uint32_t)(TB.edge_list[qe >> 16] >> (4 * ((j - qv) & 15u))) & 15u;
+                const uint32_t ed = TB.edge[e];
+                const uint32_t c0 = ed & 7u, c1 = (ed >> 3) & 7u;
+                const int axis = (int)(ed >> 6);
+                const float va = W.cv[c0][q], vb = W.cv[c1][q];
+                const uint32_t qx = qe & 0xfffu, qk = (qe >> 12) & 15u;
+                // corner coordinates: integers below 2^24, exact as floats
+                const float ax = __uint2float_rn(qx + (c0 & 1u)), ay = __uint2float_rn(qy + ((c0 >> 1) & 1u));
+                const float az = __fadd_rn(fz, (c0 & 4u) ? 1.0f : 0.0f);
+                const float a = axis == 0 ? ax : (axis == 1 ? ay : az);
+                const float b = __fadd_rn(a, c1 > c0 ? 1.0f : -1.0f);
+                const IsoRegs I = load_iso(W.ic[qk]);
+                float3 v;
+                const bool good = edge_vertex_axis_try(I.f, I.mc, I.sc, va, vb, ax, ay, az, axis, b, v);
+                if (hv && !good)   // (about one in 10^5) the exact FP64 sequence
+                    v = edge_vertex_axis(I.f, I.mc, I.sc, isos[iso_begin + qk].ip, va, vb, ax, ay, az, axis, b);
+                if (hv) W.pv[j] = make_float4(v.x, v.y, v.z, 0.0f);
+            }
+            __syncwarp();
+            // ---- triangles: one (pair, triangle) per lane, table order
+            for (uint32_t j0 = 0; j0 < ntr; j0 += 32) {
+                const uint32_t j = j0 + lane;
+                const bool ht = j < ntr;
+                const uint32_t q = ht ? W.item_t[j] : 0u;
+                const uint32_t qe = __shfl_sync(FULL, pe, q);
+                const uint32_t qv = __shfl_sync(FULL, vpre, q);
+                const uint32_t qt = __shfl_sync(FULL, tpre, q);
+                const uint64_t qo = __shfl_sync(FULL, obase, q);
+                if (ht) {
+                    const uint32_t t = j - qt;
+                    const uint32_t sl = (uint32_t)(TB.tri_slots[qe >> 16] >> (12 * t));
+                    const float4 fa = W.pv[qv + (sl & 15u)], fb = W.pv[qv + ((sl >> 4) & 15u)];
+                    const float4 fc = W.pv[qv + ((sl >> 8) & 15u)];
+                    const float3 A = make_float3(fa.x, fa.y, fa.z), B = make_float3(fb.x, fb.y, fb.z);
+                    const float3 C = make_float3(fc.x, fc.y, fc.z);
+                    const IsoConst& IC = W.ic[(qe >> 12) & 15u];
+                    float* const pc = IC.coords;
+                    if (pc && qo + t < IC.cap_tris)
+                        store_triangle(pc + 9 * (qo + t), IC.normals + 3 * (qo + t), A, B, C, tri_normal(A, B, C));
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+}  // namespace
+
+cudaError_t launch_emit_pairs(int dtype, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
+                              const StreamIso* d_isos, const PairList& list, const uint32_t* d_unit_offsets,
+                              const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
+                              const Launch& L, uint64_t task0, const uint64_t* d_totals)
+{
+    if (ntasks <= task0) return cudaSuccess;
+    const size_t smem = sizeof(PairTables) + kPairWarps * sizeof(PairWarp);
+    const uint64_t need = (ntasks - task0 + kPairWarps - 1) / kPairWarps;
+    const void* kern = dtype == 0   ? reinterpret_cast<const void*>(k_emit_pairs<int8_t>)
+                       : dtype == 1 ? reinterpret_cast<const void*>(k_emit_pairs<int16_t>)
+                       : dtype == 4 ? reinterpret_cast<const void*>(k_emit_pairs<uint8_t>)
+                       : dtype == 5 ? reinterpret_cast<const void*>(k_emit_pairs<uint16_t>)
+                       : dtype == 8 ? reinterpret_cast<const void*>(k_emit_pairs<float>)
+                                    : nullptr;
+    if (!kern) return cudaErrorInvalidValue;
+    int per_sm = 0;
+    cudaError_t e = kernel_fit(L, kern, kPairThreads, smem, &per_sm);
+    if (e != cudaSuccess) return e;
+    const uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)L.num_sms;
+    uint32_t polls = L.wait_polls[1];
+    PairList pl = list;
+    void* args[] = {&d_groups, &ngroups, &ntasks, &d_isos, &pl, &d_unit_offsets, &d_plane_base, &d_status,
+                    &d_next_task, &polls, &task0, &d_totals};
+    prof_begin(L, "stream_emit");
+    e = cudaLaunchKernel(kern, dim3((unsigned)(need < resident ? need : resident)), dim3(kPairThreads), args, smem,
+                         L.stream);
+    prof_end(L);
+    *L.counter += 1;
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+}  // namespace kvsmc

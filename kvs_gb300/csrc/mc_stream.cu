@@ -35,6 +35,7 @@
 
 #include <cuda_runtime.h>
 
+#include "mc_emit.cuh"
 #include "mc_internal.h"
 #include "mc_interp.cuh"
 #include "mc_thermo.cuh"
@@ -158,16 +159,6 @@ struct WarpState {
 
 // Per-warp emit buffers: the unit's pairs, and for one round the vertex pool
 // (one entry per (pair, used edge)) and the item -> pair maps.
-// An isolevel's constants as the emit loops read them (copied from the
-// group's StreamIso entries when a warp starts on a group).
-struct __align__(16) IsoConst {
-    FastIso f;
-    float mc[3], sc[3];   // min_coord, scale
-    float* coords;
-    float* normals;
-    uint64_t cap_tris;
-};
-
 struct WarpEmit {
     IsoConst ic[kStreamMaxIso];
     uint32_t pairs_round[32];   // this round's pair entry and vertex base per lane
@@ -187,59 +178,6 @@ __device__ __forceinline__ float3 load_vertex(const WarpEmit* WE, uint32_t j)
 {
     const float4 v = WE->pv[j];
     return make_float3(v.x, v.y, v.z);
-}
-
-// One triangle's 9 coordinates and 3 normal components, as the 8-byte
-// stores the addresses allow: a word whose address is 8-byte aligned pairs
-// with the next one, the odd word out is stored alone (the first word when
-// the array starts off an 8-byte boundary, else the last).  Seven stores
-// instead of twelve; the values are chosen by selects, so lanes with either
-// alignment run the same instructions.
-__device__ __forceinline__ void store_triangle(float* oc, float* on, float3 A, float3 B, float3 C, float3 n)
-{
-    const bool ho = (reinterpret_cast<uintptr_t>(oc) & 4u) != 0;
-    *(ho ? oc : oc + 8) = ho ? A.x : C.z;
-    float2* p2 = reinterpret_cast<float2*>(ho ? oc + 1 : oc);
-    p2[0] = make_float2(ho ? A.y : A.x, ho ? A.z : A.y);
-    p2[1] = make_float2(ho ? B.x : A.z, ho ? B.y : B.x);
-    p2[2] = make_float2(ho ? B.z : B.y, ho ? C.x : B.z);
-    p2[3] = make_float2(ho ? C.y : C.x, ho ? C.z : C.y);
-    const bool hn = (reinterpret_cast<uintptr_t>(on) & 4u) != 0;
-    *(hn ? on : on + 2) = hn ? n.x : n.z;
-    *reinterpret_cast<float2*>(hn ? on + 1 : on) = make_float2(hn ? n.y : n.x, hn ? n.z : n.y);
-}
-
-// An isolevel's interpolation constants in registers, read from its IsoConst
-// with four 16-byte loads.
-struct IsoRegs {
-    FastIso f;
-    float mc[3], sc[3];
-};
-
-static_assert(offsetof(IsoConst, f) == 0 && sizeof(FastIso) == 32 && offsetof(IsoConst, mc) == 32 &&
-                  offsetof(IsoConst, sc) == 44 && sizeof(IsoConst) % 16 == 0,
-              "load_iso reads IsoConst as four float4");
-
-__device__ __forceinline__ IsoRegs load_iso(const IsoConst& c)
-{
-    const float4* p = reinterpret_cast<const float4*>(&c);
-    const float4 a = p[0], b = p[1], m = p[2], n = p[3];
-    IsoRegs r;
-    r.f.ih = a.x;
-    r.f.il = a.y;
-    r.f.iso_err = a.z;
-    r.f.f_thr = a.w;
-    r.f.vmin_f = b.x;
-    r.f.vmax_f = b.y;
-    r.f.fast_ok = __float_as_int(b.z);
-    r.f.pad = 0;
-    r.mc[0] = m.x;
-    r.mc[1] = m.y;
-    r.mc[2] = m.z;
-    r.sc[0] = m.w;
-    r.sc[1] = n.x;
-    r.sc[2] = n.y;
-    return r;
 }
 
 // One vertex item: where its edge's two corner values sit in the warp's ring,
@@ -369,13 +307,16 @@ __device__ __forceinline__ int find_group(const StreamGroup* groups, int ngroups
 // cell row y counts node row y at its planes; on the last cell row also node
 // row y + 1, on the last cell plane also the last node plane.  Groups with
 // node_units == 0 are not counted.
-template <typename T, bool EMIT, int R, bool NODES = false>
+// LIST (count pass): every unit's active pairs are listed for the emit of
+// mc_pairs.cu (a warp scan per step, and one 16-bit entry per pair).
+template <typename T, bool EMIT, int R, bool NODES = false, bool LIST = false>
 __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? KVSMC_EMIT_CTAS : 3)
     k_stream(const StreamGroup* __restrict__ groups, int ngroups, uint64_t ntasks, const StreamIso* __restrict__ isos,
              uint16_t* __restrict__ unit_counts, const uint32_t* __restrict__ unit_offsets,
              const uint64_t* __restrict__ plane_base, int* __restrict__ status,
              unsigned long long* __restrict__ next_task, uint32_t wait_polls, uint64_t task0,
-             uint32_t* __restrict__ node_counts, const uint64_t* __restrict__ totals)
+             uint32_t* __restrict__ node_counts, const uint64_t* __restrict__ totals, PairList pl,
+             const int* __restrict__ only_if)
 {
     static_assert(!NODES || (!EMIT && R == 1), "node counts come from one-row count tasks");
     constexpr int LPR = 32 / R;                 // lanes per cell row
@@ -424,7 +365,7 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
     }
     // the only CTA-wide barrier: tables are read-only from here on (an emit
     // whose count gave up has no offsets to write at)
-    if (__syncthreads_or(EMIT && *status != 0)) return;
+    if (__syncthreads_or(EMIT && (*status != 0 || (only_if && *only_if == 0)))) return;
 
     const size_t wstride = align128(sizeof(WarpState)) + (EMIT ? align128(sizeof(WarpEmit)) : 0) +
                            align128((size_t)3 * plane_elems * sizeof(T));
@@ -443,6 +384,8 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
     uint32_t ph = 0;     // per ring buffer: parity of its next completion
     int gcur = -1;       // group whose tables are in W
     bool live = true;    // emit: some request of the group is written
+    uint64_t lcur = 0, lend = 0;   // this warp's entries of the pair list
+    bool lfull = false;
     for (;;) {
     unsigned long long tk = 0;
     if (lane == 0) tk = atomicAdd(next_task, 1ull);
@@ -484,13 +427,7 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
             W.thr[lane] = t;
             W.thr_bucket[lane] = (int32_t)bucket_index(t, bs, bo);
             if (EMIT) {
-                IsoConst& c = WE->ic[lane];
-                c.f = I.f;
-                for (int a = 0; a < 3; ++a) { c.mc[a] = I.ip.min_coord[a]; c.sc[a] = I.ip.scale[a]; }
-                // a request that does not fit its outputs is not written at all
-                c.coords = totals && totals[iso_begin + lane] > I.cap_tris ? nullptr : I.coords;
-                c.normals = I.normals;
-                c.cap_tris = I.cap_tris;
+                fill_iso(WE->ic[lane], I, totals, iso_begin + (int)lane);
             }
         }
         if (EMIT) live = __any_sync(FULL, lane < (unsigned)niso && WE->ic[lane & 15u].coords != nullptr);
@@ -656,6 +593,34 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
 
         if (!EMIT) {
             // count: one u16 per (unit, isolevel); counters [row][isolevel]
+            uint16_t* entry = nullptr;   // this lane's next list entry
+            if (LIST) {
+                const uint32_t inc = warp_inclusive_scan(m, lane);
+                const uint32_t npairs = __shfl_sync(FULL, inc, 31);
+                if (npairs != 0) {
+                    if (lcur + npairs > lend) {
+                        const uint32_t want = npairs > kPairRun ? npairs : kPairRun;
+                        unsigned long long at = 0;
+                        if (lane == 0) at = atomicAdd(pl.cursor, (unsigned long long)want);
+                        lcur = __shfl_sync(FULL, at, 0);
+                        lend = lcur + want;
+                        if (lend > pl.cap && !lfull) {
+                            lfull = true;
+                            if (lane == 0) atomicExch(pl.overflow, 1);
+                        }
+                    }
+                    entry = lfull ? nullptr : pl.list + lcur + (inc - m);
+                    // each of the step's R units: its pairs, its first entry
+                    const uint32_t before = R == 1 ? 0u : __shfl_sync(FULL, inc, LPR - 1);
+                    if (lane % LPR == 0 && row_ok) {
+                        const uint64_t pu = G.pair_base + ((uint64_t)z * cy + y + half) * wpr + seg;
+                        const uint32_t b = half ? before : 0u;
+                        pl.unit_pairs[pu] = (uint16_t)((R == 1 || half ? npairs : before) - b);
+                        pl.unit_list[pu] = (uint32_t)(lcur + b);
+                    }
+                    lcur += npairs;
+                }
+            }
             if (__any_sync(FULL, m != 0)) {
 #pragma unroll
                 for (int i = 0; i < kLaneCells; ++i) {
@@ -666,6 +631,7 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
                         do {
                             const uint32_t k = __ffs(am) - 1;
                             am &= am - 1;
+                            if (LIST && entry) *entry++ = (uint16_t)((xl + i) | (k << 8));
                             atomicAdd(&W.cnt[half * 16 + k], (uint32_t)TB.ntri[case_code(w0, w1, w2, w3, k)]);
                         } while (am);
                     }
@@ -1127,7 +1093,7 @@ cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_g
                           const StreamIso* d_isos, uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
                           const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
                           const Launch& L, int ctas_per_sm, uint64_t task0, uint32_t* d_node_counts,
-                          const uint64_t* d_totals)
+                          const uint64_t* d_totals, const PairList* list, const int* d_only_if)
 {
     if (ntasks <= task0) return cudaSuccess;
     if (rows != 1 && rows != 2) return cudaErrorInvalidValue;
@@ -1140,8 +1106,10 @@ cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_g
     const uint64_t need = (ntasks - task0 + threads / 32 - 1) / (threads / 32);
     KVSMC_STREAM_SWITCH(dtype, {
         auto kern = emit ? (rows == 1 ? k_stream<T, true, 1> : k_stream<T, true, 2>)
-                         : (rows == 1 ? (d_node_counts ? k_stream<T, false, 1, true> : k_stream<T, false, 1>)
-                                      : k_stream<T, false, 2>);
+                         : (rows == 1 ? (d_node_counts ? k_stream<T, false, 1, true>
+                                         : list        ? k_stream<T, false, 1, false, true>
+                                                       : k_stream<T, false, 1>)
+                                      : (list ? k_stream<T, false, 2, false, true> : k_stream<T, false, 2>));
         int per_sm = 0;
         const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), threads, smem, &per_sm, true);
         if (e != cudaSuccess) return e;
@@ -1153,7 +1121,8 @@ cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_g
         kern<<<(unsigned)nctas, threads, smem, L.stream>>>(d_groups, ngroups, ntasks, d_isos, d_unit_counts,
                                                            d_unit_offsets, d_plane_base, d_status, d_next_task,
                                                            L.wait_polls[emit ? 1 : 0], task0,
-                                                           emit ? nullptr : d_node_counts, emit ? d_totals : nullptr);
+                                                           emit ? nullptr : d_node_counts, emit ? d_totals : nullptr,
+                                                           list ? *list : PairList{}, emit ? d_only_if : nullptr);
         prof_end(L);
     });
     *L.counter += 1;

@@ -55,10 +55,15 @@ cudaError_t record(kvsmc_host::StreamBatch& b, cudaStream_t s, int num_sms, uint
             const auto& l = b.launches[i];
             kvsmc::Launch Li = L;
             Li.stream = st;
-            return kvsmc::launch_stream(emit, l.dtype, l.rows, b.d_groups + l.g0, l.ng, l.ntasks, b.d_isos,
-                                        b.d_unit_counts, emit ? b.d_unit_offsets : nullptr,
-                                        emit ? b.d_plane_base : nullptr, b.d_status, b.d_next + 2 * i + (emit ? 1 : 0),
-                                        Li, l.ctas_per_sm);
+            if (!emit) return b.count_kind(i, Li);
+            const cudaError_t ee = b.emit_kind(i, Li, nullptr);
+            if (ee != cudaSuccess || !b.list_cap || b.list_sure || !l.listed) return ee;
+            // the list may overflow, and a replay has no host between its passes:
+            // the classifying emit stands behind, for that case only
+            return kvsmc::launch_stream(true, l.dtype, l.rows, b.d_groups + l.g0, l.ng, l.ntasks, b.d_isos,
+                                        b.d_unit_counts, b.d_unit_offsets, b.d_plane_base, b.d_status,
+                                        b.d_next + 2 * i + 1, Li, l.ctas_per_sm, 0, nullptr, nullptr, nullptr,
+                                        b.list.overflow);
         });
     };
     cudaError_t e = cudaMemsetAsync(b.d_status, 0, b.zero_bytes, s);
@@ -115,6 +120,7 @@ kvsmc_status kvsmc_plan_create(kvsmc_context* ctx, const kvsmc_request* reqs, in
     StreamBatch b;
     b.ctx = ctx;
     b.items = stream_items;
+    b.want_list = true;
     b.plan_tables();
     for (size_t k = 0; k < b.isos.size(); ++k) {
         Item* it = b.iso_item[k];
@@ -126,6 +132,11 @@ kvsmc_status kvsmc_plan_create(kvsmc_context* ctx, const kvsmc_request* reqs, in
     }
     cudaStream_t cs = nullptr;
     cudaError_t e = kvsmc_host::device_malloc(ctx, &p->d_mem, b.scratch_bytes());
+    if (e == cudaErrorMemoryAllocation && b.list_cap) {   // no room for the pair list: the emit classifies again
+        cudaGetLastError();
+        b.list_cap = 0;
+        e = kvsmc_host::device_malloc(ctx, &p->d_mem, b.scratch_bytes());
+    }
     if (e == cudaSuccess) e = cudaMallocHost(&p->h_out, (b.isos.size() + 1) * sizeof(uint64_t));
     if (e == cudaSuccess) {
         std::memset(p->h_out, 0, (b.isos.size() + 1) * sizeof(uint64_t));

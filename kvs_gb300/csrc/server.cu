@@ -155,6 +155,7 @@ void worker(kvsmc_server* S, int w)
         b.items = live;
         kvsmc_status st = KVSMC_OK;
         if (!live.empty()) {
+            b.want_list = true;
             st = b.plan();
             if (!st) st = b.count();
         }

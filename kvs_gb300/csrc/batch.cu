@@ -47,6 +47,7 @@ kvsmc::FastIso make_fast(double iso, double vmin, double vmax, int dtype)
     f.fast_ok = std::isfinite(iso) && std::fabs(iso) <= lim && std::isfinite(vmin) && std::isfinite(vmax) &&
                 std::fabs(vmin) <= lim && std::fabs(vmax) <= lim && (double)f.vmin_f == vmin &&
                 (double)f.vmax_f == vmax && std::isfinite(f.ih) && std::isfinite(f.il);
+    f.lean_ok = f.fast_ok && f.vmin_f <= f.f_thr && f.f_thr < f.vmax_f;
     return f;
 }
 
@@ -214,7 +215,7 @@ void StreamBatch::plan_tables()
         L.g0 = (int)groups.size();
         L.ntasks = 0;
         L.netasks = 0;
-        L.listed = want_list && stream_dtype(dt);
+        L.listed = want_list;
         L.one = true;
         // one z-chunk for the whole launch: sized by all its warp steps, so a
         // batch of small volumes gets long tasks rather than many short ones

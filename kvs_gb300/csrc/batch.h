@@ -78,8 +78,7 @@ struct StreamBatch {
     bool one_row = false;
     uint64_t node_elems = 0;
     uint32_t* d_node_counts = nullptr;
-    // the count pass lists the active pairs of the 8/16-bit and float32 groups
-    // for the emit of mc_pairs.cu (set before plan_tables); list_cap: entries
+    // the count pass lists the active pairs for the emit of mc_pairs.cu (set before plan_tables); list_cap: entries
     // there is room for (0: no list), list_sure: no count can exceed them;
     // overflowed: the last count did, its emit classifies again
     bool want_list = false;

@@ -42,7 +42,7 @@ __device__ __forceinline__ IsoRegs load_iso(const IsoConst& c)
     r.f.vmin_f = b.x;
     r.f.vmax_f = b.y;
     r.f.fast_ok = __float_as_int(b.z);
-    r.f.pad = 0;
+    r.f.lean_ok = __float_as_int(b.w);
     r.mc[0] = m.x;
     r.mc[1] = m.y;
     r.mc[2] = m.z;

@@ -190,12 +190,12 @@ cudaError_t launch_emit_pairs(int dtype, const StreamGroup* d_groups, int ngroup
                               const StreamIso* d_isos, const PairList& list, const uint32_t* d_unit_offsets,
                               const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
                               const Launch& L, uint64_t task0, const uint64_t* d_totals);
-// The same two passes for the 32/64-bit integer and double volumes (one
-// isolevel per group, one row per task); launch_stream calls it for them.
-cudaError_t launch_wide(bool emit, int dtype, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
-                        const StreamIso* d_isos, uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
+// The emit launch for the 32/64-bit integer and double volumes (one isolevel
+// per group, one row per task); launch_stream calls it for them.
+cudaError_t launch_wide(int dtype, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
+                        const StreamIso* d_isos, const uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
                         const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task, const Launch& L,
-                        uint64_t task0, const uint64_t* d_totals);
+                        uint64_t task0, const uint64_t* d_totals, const int* d_only_if);
 // scan_threads: units per CTA pass (64, 128 or 256; 0 = 256).
 cudaError_t launch_unit_scan(const StreamGroup* d_groups, int ngroups, uint32_t nplanes, const StreamIso* d_isos,
                              const uint16_t* d_unit_counts, uint32_t* d_unit_offsets, uint32_t* d_plane_totals,

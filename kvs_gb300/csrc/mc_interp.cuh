@@ -45,7 +45,7 @@ struct FastIso {
     float f_thr;         // largest float <= iso: v > f_thr <=> double(v) > iso
     float vmin_f, vmax_f;// the clamp range as floats (exact when fast_ok)
     int32_t fast_ok;     // 0: always take the FP64 sequence
-    int32_t pad;
+    int32_t lean_ok;     // fast_ok, and the clamp range spans the threshold (see fast_axis_lean)
 };
 
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e)
@@ -181,6 +181,62 @@ __device__ __forceinline__ bool fast_axis_bf(float v0, float v1, float a, float 
     const bool ok = at_v0 || (den_ok && aq <= 1.5f && (pos_ok || zero_ok));
     out = at_v0 ? a : (zero_ok ? 0.0f : yh);
     return ok;
+}
+
+// fast_axis for an edge that the isolevel crosses (exactly one of va, vb is
+// above f_thr, as of every used edge of a case), in fewer operations: the
+// streaming emit's vertex, 58 instead of 95 instructions.  Same certificate:
+//  * lean_ok: vmin_f <= f_thr < vmax_f, so the clamped values lie on the same
+//    sides as the values themselves (a NaN, which is on neither, is refused),
+//    the ratio is in [0, 1] and |den| <= 2^61; fmin/fmax then clamp as
+//    clampf_ref does, up to the sign of a zero, which no step keeps;
+//  * nh - q1 dh by one FMA: its exact value needs at most 26 bits (q1 is within
+//    4 ulps of nh / dh), so the rounding is below 2^-46 |q|; the bound
+//    1.5 * 2^-43 |R| of q1 + q2 holds with room;
+//  * EXACT_DEN (values that are integers below 2^17): v1 - v0 has no error;
+//  * yh + yl by Fast2Sum, valid for |ya| >= |yb2| (checked: it fails only for
+//    a vertex within a few 2^-24 of coordinate 0);
+//  * the error bound's terms by FMAs, each factor raised by 1.001 against
+//    their roundings, and (a + 2) for max(a, b) + 1;
+//  * instead of the distance to the rounding boundaries: both ends of
+//    [yl - E, yl + E], rounded outwards, added to yh give yh again, so every
+//    real of the interval rounds to yh (rounding is monotone).  At yh = 0 this
+//    never holds, E being positive.
+// A ratio of exactly 0 (iso == v0) gives yh = a like any other.
+template <bool EXACT_DEN>
+__device__ __forceinline__ bool fast_axis_lean(float va, float vb, float a, bool up, const FastIso& f, float& out)
+{
+    const float v0 = fmaxf(fminf(va, f.vmax_f), f.vmin_f), v1 = fmaxf(fminf(vb, f.vmax_f), f.vmin_f);
+    float s, e;
+    two_sum(f.ih, -v0, s, e);
+    const float e2 = __fadd_rn(e, f.il);
+    float nh, nl;
+    two_sum(s, e2, nh, nl);
+    float dh, dl = 0.0f;
+    if (EXACT_DEN) dh = __fsub_rn(v1, v0);
+    else two_sum(v1, -v0, dh, dl);
+    float inv;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(dh));
+    const float q1 = __fmul_rn(nh, inv);
+    const float r1 = __fmaf_rn(-q1, dh, nh);
+    const float rho = __fadd_rn(r1, EXACT_DEN ? nl : __fmaf_rn(-q1, dl, nl));
+    const float q2 = __fmul_rn(rho, inv);
+    const float dq1 = up ? q1 : -q1, dq2 = up ? q2 : -q2;
+    const float ya = __fadd_rn(a, dq1);
+    const float yb = __fsub_rn(dq1, __fsub_rn(ya, a));
+    const float yb2 = __fadd_rn(yb, dq2);
+    const float yh = __fadd_rn(ya, yb2);
+    const float yl = __fsub_rn(yb2, __fsub_rn(yh, ya));
+    const float err_num = __fmaf_rn(fabsf(e2), 1.1932e-07f, f.iso_err);             // 2^-23 |e2| + iso_err
+    float E = __fmaf_rn(a, 8.8907e-16f, 1.77814e-15f);                              // 2^-50 (a + 2)
+    E = __fmaf_rn(__fmul_rn(err_num, 1.0012f), fabsf(inv), E);                      // err(num) / |den|
+    E = __fmaf_rn(fabsf(yb2), 1.1933e-07f, E);                                      // 2^-23 |yb2|
+    E = __fmaf_rn(fabsf(q1), 9.1041e-13f, E);                                       // 2^-40 |q|
+    const float t1 = __fadd_ru(yl, E), t2 = __fadd_rd(yl, -E);
+    out = yh;
+    return __fadd_rn(yh, t1) == yh && __fadd_rn(yh, t2) == yh && fabsf(ya) >= fabsf(yb2) && yh < 1.6e7f &&
+           fabsf(dh) >= 8.67361738e-19f && f.lean_ok != 0 &&
+           (EXACT_DEN || (va == va && vb == vb));
 }
 
 // The fast path of edge_vertex_axis without branches: the vertex, and

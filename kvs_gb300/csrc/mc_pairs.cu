@@ -42,7 +42,6 @@ namespace {
 constexpr int kPairThreads = 256;
 constexpr int kPairWarps = kPairThreads / 32;
 constexpr int kPairVerts = 192;          // vertex items of one round
-constexpr int kPairTris = 32 * 5;        // triangle items of one round
 constexpr unsigned FULL = 0xffffffffu;
 
 // Case tables indexed by the corner code (bit r: row r's node i above, rows
@@ -94,13 +93,22 @@ constexpr PairTables make_tables()
 
 __device__ PairTables d_pair_tables = make_tables();
 
-struct alignas(16) PairWarp {
+// Value types that are floats exactly take the FP32 certificate; the others
+// keep their corner values as doubles and take the FP64 sequence.
+template <typename T> constexpr bool kPairFast = sizeof(T) < 4;
+template <> constexpr bool kPairFast<float> = true;
+template <typename T> struct PairValue { using type = double; };
+template <> struct PairValue<float> { using type = float; };
+template <> struct PairValue<int8_t> { using type = float; };
+template <> struct PairValue<uint8_t> { using type = float; };
+template <> struct PairValue<int16_t> { using type = float; };
+template <> struct PairValue<uint16_t> { using type = float; };
+
+template <typename V> struct alignas(16) PairWarp {
     IsoConst ic[kStreamMaxIso];
     float4 pv[kPairVerts];     // vertex pool: x, y, z, unused (one 16-byte access per vertex)
-    float cv[8][32];           // corner values of the round's cells
+    V cv[8][32];               // corner values of the round's cells
     uint32_t add[32];          // per isolevel: triangles of the round
-    uint8_t item_v[kPairVerts];
-    uint8_t item_t[kPairTris];
 };
 
 template <typename T>
@@ -115,7 +123,8 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
     __shared__ __align__(8) uint64_t bar;
     PairTables& TB = *reinterpret_cast<PairTables*>(smem_raw);
     const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    PairWarp& W = reinterpret_cast<PairWarp*>(smem_raw + sizeof(PairTables))[warp];
+    using V = typename PairValue<T>::type;
+    PairWarp<V>& W = reinterpret_cast<PairWarp<V>*>(smem_raw + sizeof(PairTables))[warp];
     if (tid == 0) {
         mbar_init(&bar, 1);
         fence_barrier_init();
@@ -207,15 +216,21 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
                 x += e & 0xffu;
                 k = e >> 8;
                 const T* c = vz + (uint64_t)y * pitch + x;
-                const float thr = W.ic[k].f.f_thr;
-                const float v0 = (float)__ldg(c), v1 = (float)__ldg(c + 1);
-                const float v2 = (float)__ldg(c + pitch), v3 = (float)__ldg(c + pitch + 1);
-                const float v4 = (float)__ldg(c + slice), v5 = (float)__ldg(c + slice + 1);
-                const float v6 = (float)__ldg(c + slice + pitch), v7 = (float)__ldg(c + slice + pitch + 1);
-                W.cv[0][lane] = v0; W.cv[1][lane] = v1; W.cv[2][lane] = v2; W.cv[3][lane] = v3;
-                W.cv[4][lane] = v4; W.cv[5][lane] = v5; W.cv[6][lane] = v6; W.cv[7][lane] = v7;
-                code = (v0 > thr ? 1u : 0u) | (v2 > thr ? 2u : 0u) | (v4 > thr ? 4u : 0u) | (v6 > thr ? 8u : 0u) |
-                       (v1 > thr ? 16u : 0u) | (v3 > thr ? 32u : 0u) | (v5 > thr ? 64u : 0u) | (v7 > thr ? 128u : 0u);
+                const T v0 = __ldg(c), v1 = __ldg(c + 1), v2 = __ldg(c + pitch), v3 = __ldg(c + pitch + 1);
+                const T v4 = __ldg(c + slice), v5 = __ldg(c + slice + 1);
+                const T v6 = __ldg(c + slice + pitch), v7 = __ldg(c + slice + pitch + 1);
+                auto up = [&](T v) -> bool {
+                    if constexpr (kPairFast<T>) return (float)v > W.ic[k].f.f_thr;
+                    else return above(isos[iso_begin].cls, v);   // (one isolevel per group)
+                };
+                auto val = [&](T v) -> V {
+                    if constexpr (kPairFast<T>) return (float)v;
+                    else return to_double(v);
+                };
+                W.cv[0][lane] = val(v0); W.cv[1][lane] = val(v1); W.cv[2][lane] = val(v2); W.cv[3][lane] = val(v3);
+                W.cv[4][lane] = val(v4); W.cv[5][lane] = val(v5); W.cv[6][lane] = val(v6); W.cv[7][lane] = val(v7);
+                code = (up(v0) ? 1u : 0u) | (up(v2) ? 2u : 0u) | (up(v4) ? 4u : 0u) | (up(v6) ? 8u : 0u) |
+                       (up(v1) ? 16u : 0u) | (up(v3) ? 32u : 0u) | (up(v5) ? 64u : 0u) | (up(v7) ? 128u : 0u);
             }
             const uint32_t ne0 = has ? (uint32_t)__popc(TB.edge_mask[code]) : 0u;
             uint32_t vpre = 0;
@@ -226,7 +241,6 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
             taken = (uint32_t)__popc(__ballot_sync(FULL, has));
             const uint32_t nv = __shfl_sync(FULL, vpre + ne0, taken - 1);
             const uint32_t nt = has ? TB.ntri[code] : 0u;
-            const uint32_t ne = has ? ne0 : 0u;
             const uint32_t pe = x | (k << 12) | (code << 16);   // (x < 4096)
             // output position of the pair's first triangle: its isolevel's running
             // count plus the triangles of the earlier lanes of that isolevel
@@ -241,17 +255,25 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
                 ntr += (uint32_t)__popc(bm) << bit;
             }
             const uint64_t obase = __shfl_sync(FULL, run, k) + pre;
-            if (has && (31 - __clz(grp)) == (int)lane) W.add[k] = gtot;
-            for (uint32_t r = 0; r < ne; ++r) W.item_v[vpre + r] = (uint8_t)lane;
-            for (uint32_t t = 0; t < nt; ++t) W.item_t[tpre + t] = (uint8_t)lane;
-            __syncwarp();
-            run += W.add[lane];
-            W.add[lane] = 0;
-            // ---- vertices: one (pair, used edge) per lane
+            if (niso == 1) {
+                run += ntr;
+            } else {
+                if (has && (31 - __clz(grp)) == (int)lane) W.add[k] = gtot;
+                __syncwarp();
+                run += W.add[lane];
+                W.add[lane] = 0;
+            }
+            __syncwarp();   // the corner values are there
+            // ---- vertices: one (pair, used edge) per lane.  Item j's pair: the
+            // pairs' first items as bits of one word (every pair has items), so
+            // the pair is the number of first items up to j
+            uint32_t seen = 0;
             for (uint32_t j0 = 0; j0 < nv; j0 += 32) {
                 const uint32_t j = j0 + lane;
                 const bool hv = j < nv;
-                const uint32_t q = hv ? W.item_v[j] : 0u;
+                const uint32_t starts = __reduce_or_sync(FULL, has && vpre - j0 < 32u ? 1u << (vpre - j0) : 0u);
+                const uint32_t q = seen + (uint32_t)__popc(starts & (lt | (1u << lane))) - 1u;
+                seen += (uint32_t)__popc(starts);
                 const uint32_t qe = __shfl_sync(FULL, pe, q);
                 const uint32_t qv = __shfl_sync(FULL, vpre, q);
                 const uint32_t qy = __shfl_sync(FULL, y, q);
@@ -259,26 +281,40 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
                 const uint32_t ed = TB.edge[e];
                 const uint32_t c0 = ed & 7u, c1 = (ed >> 3) & 7u;
                 const int axis = (int)(ed >> 6);
-                const float va = W.cv[c0][q], vb = W.cv[c1][q];
+                const V va = W.cv[c0][q], vb = W.cv[c1][q];
                 const uint32_t qx = qe & 0xfffu, qk = (qe >> 12) & 15u;
                 // corner coordinates: integers below 2^24, exact as floats
                 const float ax = __uint2float_rn(qx + (c0 & 1u)), ay = __uint2float_rn(qy + ((c0 >> 1) & 1u));
                 const float az = __fadd_rn(fz, (c0 & 4u) ? 1.0f : 0.0f);
-                const float a = axis == 0 ? ax : (axis == 1 ? ay : az);
-                const float b = __fadd_rn(a, c1 > c0 ? 1.0f : -1.0f);
-                const IsoRegs I = load_iso(W.ic[qk]);
+                const bool up = c1 > c0;
                 float3 v;
-                const bool good = edge_vertex_axis_try(I.f, I.mc, I.sc, va, vb, ax, ay, az, axis, b, v);
-                if (hv && !good)   // (about one in 10^5) the exact FP64 sequence
-                    v = edge_vertex_axis(I.f, I.mc, I.sc, isos[iso_begin + qk].ip, va, vb, ax, ay, az, axis, b);
+                if constexpr (kPairFast<T>) {
+                    const float a = axis == 0 ? ax : (axis == 1 ? ay : az);
+                    const IsoRegs I = load_iso(W.ic[qk]);
+                    float r;
+                    const bool good = fast_axis_lean<(sizeof(T) < 4)>(va, vb, a, up, I.f, r);
+                    v.x = __fmul_rn(__fadd_rn(axis == 0 ? r : ax, I.mc[0]), I.sc[0]);
+                    v.y = __fmul_rn(__fadd_rn(axis == 1 ? r : ay, I.mc[1]), I.sc[1]);
+                    v.z = __fmul_rn(__fadd_rn(axis == 2 ? r : az, I.mc[2]), I.sc[2]);
+                    if (hv && !good)   // (about one in 10^5) the exact FP64 sequence
+                        v = edge_vertex_axis(I.f, I.mc, I.sc, isos[iso_begin + qk].ip, va, vb, ax, ay, az, axis,
+                                             __fadd_rn(a, up ? 1.0f : -1.0f));
+                } else {
+                    const float d = up ? 1.0f : -1.0f;
+                    v = interpolate_exact_axis(isos[iso_begin].ip, va, vb, ax, ay, az, axis == 0 ? __fadd_rn(ax, d) : ax,
+                                               axis == 1 ? __fadd_rn(ay, d) : ay, axis == 2 ? __fadd_rn(az, d) : az, axis);
+                }
                 if (hv) W.pv[j] = make_float4(v.x, v.y, v.z, 0.0f);
             }
             __syncwarp();
             // ---- triangles: one (pair, triangle) per lane, table order
+            seen = 0;
             for (uint32_t j0 = 0; j0 < ntr; j0 += 32) {
                 const uint32_t j = j0 + lane;
                 const bool ht = j < ntr;
-                const uint32_t q = ht ? W.item_t[j] : 0u;
+                const uint32_t starts = __reduce_or_sync(FULL, has && tpre - j0 < 32u ? 1u << (tpre - j0) : 0u);
+                const uint32_t q = seen + (uint32_t)__popc(starts & (lt | (1u << lane))) - 1u;
+                seen += (uint32_t)__popc(starts);
                 const uint32_t qe = __shfl_sync(FULL, pe, q);
                 const uint32_t qv = __shfl_sync(FULL, vpre, q);
                 const uint32_t qt = __shfl_sync(FULL, tpre, q);
@@ -309,14 +345,28 @@ cudaError_t launch_emit_pairs(int dtype, const StreamGroup* d_groups, int ngroup
                               const Launch& L, uint64_t task0, const uint64_t* d_totals)
 {
     if (ntasks <= task0) return cudaSuccess;
-    const size_t smem = sizeof(PairTables) + kPairWarps * sizeof(PairWarp);
     const uint64_t need = (ntasks - task0 + kPairWarps - 1) / kPairWarps;
-    const void* kern = dtype == 0   ? reinterpret_cast<const void*>(k_emit_pairs<int8_t>)
-                       : dtype == 1 ? reinterpret_cast<const void*>(k_emit_pairs<int16_t>)
-                       : dtype == 4 ? reinterpret_cast<const void*>(k_emit_pairs<uint8_t>)
-                       : dtype == 5 ? reinterpret_cast<const void*>(k_emit_pairs<uint16_t>)
-                       : dtype == 8 ? reinterpret_cast<const void*>(k_emit_pairs<float>)
-                                    : nullptr;
+    const void* kern = nullptr;
+    size_t smem = sizeof(PairTables);
+#define KVSMC_PAIR_CASE(CODE, T)                                                     \
+    case CODE:                                                                       \
+        kern = reinterpret_cast<const void*>(k_emit_pairs<T>);                       \
+        smem += kPairWarps * sizeof(PairWarp<typename PairValue<T>::type>);          \
+        break;
+    switch (dtype) {
+        KVSMC_PAIR_CASE(0, int8_t)
+        KVSMC_PAIR_CASE(1, int16_t)
+        KVSMC_PAIR_CASE(2, int32_t)
+        KVSMC_PAIR_CASE(3, long long)
+        KVSMC_PAIR_CASE(4, uint8_t)
+        KVSMC_PAIR_CASE(5, uint16_t)
+        KVSMC_PAIR_CASE(6, uint32_t)
+        KVSMC_PAIR_CASE(7, unsigned long long)
+        KVSMC_PAIR_CASE(8, float)
+        KVSMC_PAIR_CASE(9, double)
+    default: break;
+    }
+#undef KVSMC_PAIR_CASE
     if (!kern) return cudaErrorInvalidValue;
     int per_sm = 0;
     cudaError_t e = kernel_fit(L, kern, kPairThreads, smem, &per_sm);

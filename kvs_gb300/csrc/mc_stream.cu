@@ -1098,9 +1098,9 @@ cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_g
     if (ntasks <= task0) return cudaSuccess;
     if (rows != 1 && rows != 2) return cudaErrorInvalidValue;
     if (dtype == 2 || dtype == 3 || dtype == 6 || dtype == 7 || dtype == 9)
-        return rows == 1 ? launch_wide(emit, dtype, d_groups, ngroups, ntasks, d_isos, d_unit_counts, d_unit_offsets,
-                                       d_plane_base, d_status, d_next_task, L, task0, d_totals)
-                         : cudaErrorInvalidValue;
+        return emit && rows == 1 ? launch_wide(dtype, d_groups, ngroups, ntasks, d_isos, d_unit_counts, d_unit_offsets,
+                                               d_plane_base, d_status, d_next_task, L, task0, d_totals, d_only_if)
+                                 : cudaErrorInvalidValue;
     const size_t smem = stream_shared_bytes(dtype, emit, rows);
     const int threads = emit ? kEmitThreads : kStreamThreads;
     const uint64_t need = (ntasks - task0 + threads / 32 - 1) / (threads / 32);

@@ -1,21 +1,16 @@
-// mc_wide.cu -- duplicated-vertex extraction of 32/64-bit integer and double
-// volumes on the streaming layout (count and emit; the unit scan and the
-// shared-vertex passes are the narrow types').
+// mc_wide.cu -- the classifying emit of 32/64-bit integer and double volumes
+// (duplicated mode): for counts whose pair list overflowed or had no room.
+// (The count is mc_one.cu's, the emit over listed pairs mc_pairs.cu's.)
 //
 // A warp task is a streaming cell task with one row per task: a chunk of cell
 // planes, one cell row, a 256-cell segment, the two node rows of each node
 // plane arriving in the warp's three-buffer ring through bulk copies.  Lane l
 // owns cells 8 l .. 8 l + 7.  One isolevel per group: each node is classified
-// by one integer compare (Classifier: 64-bit values and doubles through
-// order-preserving keys, so the FP64 units are not asked), the 8 cells' cases
-// come out of four 9-bit row masks by an 8 x 8 bit transpose, and the upper
-// plane's masks are the next step's lower ones.  The emit spreads a step's
-// triangles over the lanes, one lane a triangle, its vertices by the FP64
-// sequence (the values are no floats, so the FP32 certificate does not apply).
-//
-// It replaces one thread per cell with 8 scattered loads and a serial walk of
-// its triangles: 201 x 173 x 187 doubles, 488 k triangles, count 132 us and
-// emit 1628 us there.
+// by one integer compare (Classifier), the 8 cells' cases come out of four
+// 9-bit row masks by an 8 x 8 bit transpose, and the upper plane's masks are
+// the next step's lower ones.  A step's triangles are spread over the lanes,
+// one lane a triangle, its vertices by the FP64 sequence (201 x 173 x 187
+// doubles, 488 k triangles: 175 us; over listed pairs 81 us).
 #include <cuda_runtime.h>
 
 #include "mc_internal.h"
@@ -35,13 +30,13 @@ __constant__ uint8_t c_w_edge[12] = MC_EDGE_PACKED_INIT;
 
 __host__ __device__ __forceinline__ size_t w_align(size_t v) { return (v + 127) / 128 * 128; }
 
-template <typename T, bool EMIT>
+template <typename T>
 __global__ void __launch_bounds__(kWideThreads)
     k_wide(const StreamGroup* __restrict__ groups, int ngroups, uint64_t ntasks, const StreamIso* __restrict__ isos,
-           uint16_t* __restrict__ unit_counts, const uint32_t* __restrict__ unit_offsets,
+           const uint16_t* __restrict__ unit_counts, const uint32_t* __restrict__ unit_offsets,
            const uint64_t* __restrict__ plane_base, int* __restrict__ status,
            unsigned long long* __restrict__ next_task, uint32_t wait_polls, uint64_t task0,
-           const uint64_t* __restrict__ totals)
+           const uint64_t* __restrict__ totals, const int* __restrict__ only_if)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ uint64_t s_tri[256];
@@ -54,7 +49,7 @@ __global__ void __launch_bounds__(kWideThreads)
         if (c < 12) s_edge[c] = c_w_edge[c];
     }
     // the only CTA-wide barrier (an emit whose count gave up writes nothing)
-    if (__syncthreads_or(EMIT && *status != 0)) return;
+    if (__syncthreads_or(*status != 0 || (only_if && *only_if == 0))) return;
     const uint32_t row_elems = groups[0].seg_elems;
     const size_t plane_elems = 2 * (size_t)row_elems;
     unsigned char* wbase = smem_raw + (size_t)warp * (128 + w_align(3 * plane_elems * sizeof(T)));
@@ -74,12 +69,12 @@ __global__ void __launch_bounds__(kWideThreads)
         if (task >= ntasks) break;
         while (gi + 1 < ngroups && task >= groups[gi + 1].task_begin) ++gi;   // (tasks come in increasing order)
         const StreamGroup& G = groups[gi];
-        if (EMIT && G.skip_emit) continue;
+        if (G.skip_emit) continue;
         const StreamIso& I = isos[G.iso_begin];
-        float* const out_c = EMIT ? I.coords : nullptr;
-        float* const out_n = EMIT ? I.normals : nullptr;
-        const uint64_t cap = EMIT ? I.cap_tris : 0;
-        if (EMIT && (!out_c || (totals && totals[G.iso_begin] > cap))) continue;   // not written at all
+        float* const out_c = I.coords;
+        float* const out_n = I.normals;
+        const uint64_t cap = I.cap_tris;
+        if (!out_c || (totals && totals[G.iso_begin] > cap)) continue;   // not written at all
         const Classifier cls = I.cls;
         const uint64_t local = task - G.task_begin;
         const uint32_t cx = G.vol.nx - 1, cy = G.vol.ny - 1, cz = G.vol.nz - 1, wpr = G.wpr;
@@ -116,13 +111,13 @@ __global__ void __launch_bounds__(kWideThreads)
         bool dead = false;
         const int lim = (int)cx - (int)((uint32_t)xoff + 8 * lane);   // this lane's cells inside the row (if < 8)
         auto unit_of = [&](uint32_t zz) -> uint64_t { return G.unit_base + ((uint64_t)zz * cy + y) * wpr + seg; };
-        const uint64_t first_plane = EMIT ? plane_base[I.plane_index] : 0;
+        const uint64_t first_plane = plane_base[I.plane_index];
         auto unit_first = [&](uint32_t zz) -> uint64_t {
             return plane_base[I.plane_index + zz] - first_plane + unit_offsets[unit_of(zz)];
         };
         // the unit's triangles and first triangle, loaded one step ahead
-        uint32_t next_count = EMIT ? unit_counts[unit_of(z0)] : 0;
-        uint64_t next_first = EMIT ? unit_first(z0) : 0;
+        uint32_t next_count = unit_counts[unit_of(z0)];
+        uint64_t next_first = unit_first(z0);
         uint32_t ma = 0;        // rows y, y + 1 of plane z: this lane's 9 nodes above (bits 0-8, 16-24)
         bool have_a = false;
         auto row_mask = [&](const T* p) -> uint32_t {
@@ -138,7 +133,7 @@ __global__ void __launch_bounds__(kWideThreads)
             const uint32_t st = z - z0;
             const uint32_t count_now = next_count;
             const uint64_t tbase = next_first;
-            if (EMIT && z + 1 < z1) {
+            if (z + 1 < z1) {
                 next_count = unit_counts[unit_of(z + 1)];
                 next_first = unit_first(z + 1);
             }
@@ -153,7 +148,7 @@ __global__ void __launch_bounds__(kWideThreads)
                 issued = st + 3 < nplanes ? st + 3 : nplanes;
                 break;
             }
-            if (EMIT && count_now == 0) {
+            if (count_now == 0) {
                 have_a = false;
             } else {
                 const T* a = ring + (size_t)(st % 3u) * plane_elems + 8 * lane;
@@ -181,10 +176,7 @@ __global__ void __launch_bounds__(kWideThreads)
 #pragma unroll
                     for (int i = 0; i < 8; ++i) n += s_ntri[(uint32_t)(cw >> (8 * i)) & 0xffu];
                 }
-                if (!EMIT) {
-                    const uint32_t t = __reduce_add_sync(FULL, n);
-                    if (lane == 0) unit_counts[unit_of(z)] = (uint16_t)t;
-                } else {
+                {
                     uint32_t inc = n;
 #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) {
@@ -269,24 +261,24 @@ __global__ void __launch_bounds__(kWideThreads)
     default: return cudaErrorInvalidValue;                           \
     }
 
-cudaError_t launch_wide(bool emit, int dtype, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
-                        const StreamIso* d_isos, uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
+cudaError_t launch_wide(int dtype, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
+                        const StreamIso* d_isos, const uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
                         const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task, const Launch& L,
-                        uint64_t task0, const uint64_t* d_totals)
+                        uint64_t task0, const uint64_t* d_totals, const int* d_only_if)
 {
     const size_t smem =
         (size_t)kWideWarps * (128 + w_align(3 * 2 * stream_row_elems(dtype, 1) * dtype_size(dtype)));
     const uint64_t need = (ntasks - task0 + kWideWarps - 1) / kWideWarps;
     KVSMC_WIDE_SWITCH(dtype, {
-        auto kern = emit ? k_wide<T, true> : k_wide<T, false>;
+        auto kern = k_wide<T>;
         int per_sm = 0;
         const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), kWideThreads, smem, &per_sm, true);
         if (e != cudaSuccess) return e;
         const uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)L.num_sms;
-        prof_begin(L, emit ? "wide_emit" : "wide_count");
+        prof_begin(L, "wide_emit");
         kern<<<(unsigned)(need < resident ? need : resident), kWideThreads, smem, L.stream>>>(
             d_groups, ngroups, ntasks, d_isos, d_unit_counts, d_unit_offsets, d_plane_base, d_status, d_next_task,
-            L.wait_polls[emit ? 1 : 0], task0, emit ? d_totals : nullptr);
+            L.wait_polls[1], task0, d_totals, d_only_if);
         prof_end(L);
     });
     *L.counter += 1;

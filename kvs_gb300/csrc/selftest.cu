@@ -68,7 +68,7 @@ __global__ void k_selftest(uint64_t n, uint64_t seed, unsigned long long* counte
         f.iso_err = (float)fabs(rep) * 1.0001f;
         f.f_thr = thr;
         f.vmin_f = -3.0e38f; f.vmax_f = 3.0e38f;
-        f.fast_ok = 1; f.pad = 0;
+        f.fast_ok = 1; f.lean_ok = 1;
         Interp j;
         j.iso = iso;
         j.vmin = -3.0e38; j.vmax = 3.0e38;
@@ -94,9 +94,15 @@ __global__ void k_selftest(uint64_t n, uint64_t seed, unsigned long long* counte
         const bool ok = fast_axis(v0, v1, *pa, *pb, f, r);
         const bool okb = fast_axis_bf(v0, v1, *pa, *pb, f, rb);
         const float3 fv = edge_vertex_fast(j, f, va, vb, ax, ay, az, bx, by, bz, axis);
+        // the streaming emit's form, and its variant for small integers
+        float rl, ri = want;
+        const bool okl = fast_axis_lean<false>(v0, v1, *pa, *pb > *pa, f, rl);
+        const bool oki = (kind == 2 || kind == 3 || kind == 7) && fast_axis_lean<true>(v0, v1, *pa, *pb > *pa, f, ri);
         ++tested;
-        if (!okb) ++fall;
-        if (__float_as_int(ex.x) != __float_as_int(fv.x) || __float_as_int(ex.y) != __float_as_int(fv.y) ||
+        if (!okb || !okl) ++fall;
+        if ((okl && __float_as_int(rl) != __float_as_int(want)) || (oki && __float_as_int(ri) != __float_as_int(want)))
+            ++mism;
+        else if (__float_as_int(ex.x) != __float_as_int(fv.x) || __float_as_int(ex.y) != __float_as_int(fv.y) ||
             __float_as_int(ex.z) != __float_as_int(fv.z) ||
             (ok && __float_as_int(r) != __float_as_int(want)) || (okb && __float_as_int(rb) != __float_as_int(want)))
             ++mism;
@@ -164,7 +170,7 @@ __global__ void k_selftest_cells(uint64_t n, uint64_t seed, unsigned long long* 
         f.iso_err = (float)fabs(rep) * 1.0001f;
         f.f_thr = thr;
         f.vmin_f = -3.0e38f; f.vmax_f = 3.0e38f;
-        f.fast_ok = 1; f.pad = 0;
+        f.fast_ok = 1; f.lean_ok = 1;
         const double q = __ddiv_rn(__dsub_rn(iso, (double)va), __dsub_rn((double)vb, (double)va));
         const double r = q < 0.0 ? -q : q;
         const float want = __double2float_rn(__dadd_rn((double)c0, __dmul_rn(r, (double)__fsub_rn(c1, c0))));

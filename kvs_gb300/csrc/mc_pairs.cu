@@ -13,7 +13,8 @@
 // running count.  Per round:
 //   * each lane reads its cell's 8 corner values from the volume (L1/L2: a
 //     cell's neighbours share its sectors), forms the corner code by 8
-//     compares and leaves the values in a shared 8 x 32 table;
+//     compares and leaves the values in a shared table, 9 words a cell, so that
+//     the lanes of one cell reading its corners meet in different banks;
 //   * lanes of the same isolevel are grouped with __match_any_sync, bit-sliced
 //     ballots give each pair's output position;
 //   * one lane per (pair, used edge) interpolates a vertex (the FP32
@@ -22,7 +23,16 @@
 // The rounds are full up to a block's last one (the re-classifying emit took
 // the pairs of one 256-cell segment at a time: 6 of 32 lanes with one
 // isolevel on smooth data), nothing waits for staged planes, and without the
-// ring and the masks 24 warps are resident on an SM instead of 16.
+// ring and the masks 32 warps are resident on an SM instead of 16.  What
+// bounds it is the issue of about 1200 instructions a round and the latency of
+// shuffles and shared memory between them (24 warps kept the issue slots 66%
+// busy; DRAM writes are a third of its time).  So a pair's cell, code, isolevel
+// and vertex base are one word, its output place and first triangle another (a
+// task writes less than 2^16 triangles, so places are counted from the task's
+// start and the isolevels' 64-bit addresses are formed once per task), and an
+// edge's corners and axis are one byte of one table.  640x704x600 f32, 16
+// isolevels: 3810 -> 3635 us (40% of the 9 GB it writes at the copy rate);
+// 768x768x640 u16, 4 isolevels: 2519 -> 2296 us.
 #include <cuda_runtime.h>
 
 #include "mc_emit.cuh"
@@ -32,7 +42,7 @@
 #include "tma.cuh"
 
 #ifndef KVSMC_PAIRS_CTAS
-#define KVSMC_PAIRS_CTAS 3
+#define KVSMC_PAIRS_CTAS 4
 #endif
 
 namespace kvsmc {
@@ -49,10 +59,9 @@ constexpr unsigned FULL = 0xffffffffu;
 // at compile time and copied into shared memory by one bulk copy per CTA.
 struct alignas(16) PairTables {
     uint64_t tri_slots[256];   // per triangle corner: its edge's rank among the used edges, 4 bits each
-    uint64_t edge_list[256];   // the used edges in increasing order, 4 bits each
-    uint16_t edge_mask[256];
-    uint8_t ntri[256];
-    uint8_t edge[16];          // corner A | corner B << 3 | axis << 6 (corner: dx + 2 dy + 4 dz)
+    uint8_t edges[256][12];    // the used edges in increasing order: corner A | corner B << 3 | axis << 6
+                               // (corner: dx + 2 dy + 4 dz)
+    uint8_t counts[256];       // triangles | used edges << 3
 };
 static_assert(sizeof(PairTables) % 16 == 0, "copied by a bulk copy");
 
@@ -72,21 +81,19 @@ constexpr PairTables make_tables()
     PairTables t{};
     for (uint32_t code = 0; code < 256; ++code) {
         const uint32_t cs = h_case(code), em = h_mask[cs];
-        t.ntri[code] = h_ntri[cs];
-        t.edge_mask[code] = (uint16_t)em;
         int n = 0;
         for (uint32_t e = 0; e < 12; ++e)
-            if ((em >> e) & 1u) t.edge_list[code] |= (uint64_t)e << (4 * n++);
+            if ((em >> e) & 1u) {
+                const uint32_t c0 = h_edge[e] & 7u, c1 = h_edge[e] >> 3, d = c0 ^ c1;
+                t.edges[code][n++] = (uint8_t)(c0 | (c1 << 3) | ((d == 1u ? 0u : (d == 2u ? 1u : 2u)) << 6));
+            }
+        t.counts[code] = (uint8_t)(h_ntri[cs] | (n << 3));
         for (int c = 0; c < 3 * (int)h_ntri[cs]; ++c) {
             const uint32_t e = (uint32_t)(h_tri[cs] >> (4 * c)) & 15u;
             uint64_t rank = 0;
             for (uint32_t b = 0; b < e; ++b) rank += (em >> b) & 1u;
             t.tri_slots[code] |= rank << (4 * c);
         }
-    }
-    for (int e = 0; e < 12; ++e) {
-        const uint32_t c0 = h_edge[e] & 7u, c1 = h_edge[e] >> 3, d = c0 ^ c1;
-        t.edge[e] = (uint8_t)(c0 | (c1 << 3) | ((d == 1u ? 0u : (d == 2u ? 1u : 2u)) << 6));
     }
     return t;
 }
@@ -104,10 +111,17 @@ template <> struct PairValue<uint8_t> { using type = float; };
 template <> struct PairValue<int16_t> { using type = float; };
 template <> struct PairValue<uint16_t> { using type = float; };
 
+struct alignas(16) PairOut {
+    float* coords;
+    float* normals;
+};
+
 template <typename V> struct alignas(16) PairWarp {
     IsoConst ic[kStreamMaxIso];
     float4 pv[kPairVerts];     // vertex pool: x, y, z, unused (one 16-byte access per vertex)
-    V cv[8][32];               // corner values of the round's cells
+    PairOut out[kStreamMaxIso];   // per isolevel: where the task's triangles go
+    uint32_t room[kStreamMaxIso]; // and how many of them may be written
+    V cv[32][9];               // corner values of the round's cells (9: a cell's corners in different banks)
     uint32_t add[32];          // per isolevel: triangles of the round
 };
 
@@ -185,13 +199,19 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
         first -= inc - np;   // entry of pair p of this unit: list[first + p]
         const uint32_t uy = un / wpr;
         const uint32_t ux = (un - uy * wpr) * G.seg_cells;
-        // lane k: the next output triangle of isolevel k
-        uint64_t run = 0;
+        // per isolevel: where the task's first triangle goes and how many fit
+        __syncwarp();
         if (lane < (unsigned)niso) {
             const uint64_t pi = isos[iso_begin + lane].plane_index;
-            run = plane_base[pi + z] - plane_base[pi] +
-                  unit_offsets[G.unit_base + ((uint64_t)z * plane_units + u0) * niso + lane];
+            const uint64_t at = plane_base[pi + z] - plane_base[pi] +
+                                unit_offsets[G.unit_base + ((uint64_t)z * plane_units + u0) * niso + lane];
+            const IsoConst& c = W.ic[lane];
+            W.out[lane] = PairOut{c.coords + 9 * at, c.normals + 3 * at};
+            W.room[lane] = !c.coords || c.cap_tris <= at ? 0u
+                           : c.cap_tris - at < 0xffffu ? (uint32_t)(c.cap_tris - at) : 0xffffu;
         }
+        __syncwarp();
+        uint32_t run = 0;   // lane k: the task's triangles of isolevel k so far (at most 32 * 256 * 5)
         const uint64_t pitch = G.vol.pitch, slice = G.vol.slice;
         const T* vz = static_cast<const T*>(G.vol.data) + (uint64_t)z * slice;
         const float fz = __uint2float_rn(z);
@@ -227,12 +247,14 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
                     if constexpr (kPairFast<T>) return (float)v;
                     else return to_double(v);
                 };
-                W.cv[0][lane] = val(v0); W.cv[1][lane] = val(v1); W.cv[2][lane] = val(v2); W.cv[3][lane] = val(v3);
-                W.cv[4][lane] = val(v4); W.cv[5][lane] = val(v5); W.cv[6][lane] = val(v6); W.cv[7][lane] = val(v7);
+                V* cv = W.cv[lane];
+                cv[0] = val(v0); cv[1] = val(v1); cv[2] = val(v2); cv[3] = val(v3);
+                cv[4] = val(v4); cv[5] = val(v5); cv[6] = val(v6); cv[7] = val(v7);
                 code = (up(v0) ? 1u : 0u) | (up(v2) ? 2u : 0u) | (up(v4) ? 4u : 0u) | (up(v6) ? 8u : 0u) |
                        (up(v1) ? 16u : 0u) | (up(v3) ? 32u : 0u) | (up(v5) ? 64u : 0u) | (up(v7) ? 128u : 0u);
             }
-            const uint32_t ne0 = has ? (uint32_t)__popc(TB.edge_mask[code]) : 0u;
+            const uint32_t cnt = has ? TB.counts[code] : 0u;
+            const uint32_t ne0 = cnt >> 3;
             uint32_t vpre = 0;
 #pragma unroll
             for (int bit = 0; bit < 4; ++bit)
@@ -240,8 +262,8 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
             has = has && vpre + ne0 <= (uint32_t)kPairVerts;   // a suffix of lanes waits
             taken = (uint32_t)__popc(__ballot_sync(FULL, has));
             const uint32_t nv = __shfl_sync(FULL, vpre + ne0, taken - 1);
-            const uint32_t nt = has ? TB.ntri[code] : 0u;
-            const uint32_t pe = x | (k << 12) | (code << 16);   // (x < 4096)
+            const uint32_t nt = has ? cnt & 7u : 0u;
+            const uint32_t pe = x | (k << 12) | (code << 16) | (vpre << 24);   // (x < 4096; vpre < kPairVerts)
             // output position of the pair's first triangle: its isolevel's running
             // count plus the triangles of the earlier lanes of that isolevel
             const uint32_t grp = niso == 1 ? __ballot_sync(FULL, has) : __match_any_sync(FULL, has ? k : 32u + lane);
@@ -254,7 +276,7 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
                 tpre += (uint32_t)__popc(bm & lt) << bit;
                 ntr += (uint32_t)__popc(bm) << bit;
             }
-            const uint64_t obase = __shfl_sync(FULL, run, k) + pre;
+            const uint32_t ot = __shfl_sync(FULL, run, k) + pre + (tpre << 16);   // (both below 2^16)
             if (niso == 1) {
                 run += ntr;
             } else {
@@ -275,13 +297,11 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
                 const uint32_t q = seen + (uint32_t)__popc(starts & (lt | (1u << lane))) - 1u;
                 seen += (uint32_t)__popc(starts);
                 const uint32_t qe = __shfl_sync(FULL, pe, q);
-                const uint32_t qv = __shfl_sync(FULL, vpre, q);
                 const uint32_t qy = __shfl_sync(FULL, y, q);
-                const uint32_t e = (uint32_t)(TB.edge_list[qe >> 16] >> (4 * ((j - qv) & 15u))) & 15u;
-                const uint32_t ed = TB.edge[e];
+                const uint32_t ed = TB.edges[(qe >> 16) & 255u][hv ? j - (qe >> 24) : 0u];
                 const uint32_t c0 = ed & 7u, c1 = (ed >> 3) & 7u;
                 const int axis = (int)(ed >> 6);
-                const V va = W.cv[c0][q], vb = W.cv[c1][q];
+                const V va = W.cv[q][c0], vb = W.cv[q][c1];
                 const uint32_t qx = qe & 0xfffu, qk = (qe >> 12) & 15u;
                 // corner coordinates: integers below 2^24, exact as floats
                 const float ax = __uint2float_rn(qx + (c0 & 1u)), ay = __uint2float_rn(qy + ((c0 >> 1) & 1u));
@@ -316,20 +336,18 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
                 const uint32_t q = seen + (uint32_t)__popc(starts & (lt | (1u << lane))) - 1u;
                 seen += (uint32_t)__popc(starts);
                 const uint32_t qe = __shfl_sync(FULL, pe, q);
-                const uint32_t qv = __shfl_sync(FULL, vpre, q);
-                const uint32_t qt = __shfl_sync(FULL, tpre, q);
-                const uint64_t qo = __shfl_sync(FULL, obase, q);
+                const uint32_t qo = __shfl_sync(FULL, ot, q);
                 if (ht) {
-                    const uint32_t t = j - qt;
-                    const uint32_t sl = (uint32_t)(TB.tri_slots[qe >> 16] >> (12 * t));
-                    const float4 fa = W.pv[qv + (sl & 15u)], fb = W.pv[qv + ((sl >> 4) & 15u)];
-                    const float4 fc = W.pv[qv + ((sl >> 8) & 15u)];
+                    const uint32_t t = j - (qo >> 16), o = (qo & 0xffffu) + t, qk = (qe >> 12) & 15u;
+                    const uint32_t sl = (uint32_t)(TB.tri_slots[(qe >> 16) & 255u] >> (12 * t));
+                    const float4* pv = W.pv + (qe >> 24);
+                    const float4 fa = pv[sl & 15u], fb = pv[(sl >> 4) & 15u], fc = pv[(sl >> 8) & 15u];
                     const float3 A = make_float3(fa.x, fa.y, fa.z), B = make_float3(fb.x, fb.y, fb.z);
                     const float3 C = make_float3(fc.x, fc.y, fc.z);
-                    const IsoConst& IC = W.ic[(qe >> 12) & 15u];
-                    float* const pc = IC.coords;
-                    if (pc && qo + t < IC.cap_tris)
-                        store_triangle(pc + 9 * (qo + t), IC.normals + 3 * (qo + t), A, B, C, tri_normal(A, B, C));
+                    if (o < W.room[qk]) {
+                        const PairOut to = W.out[qk];
+                        store_triangle(to.coords + 9 * o, to.normals + 3 * o, A, B, C, tri_normal(A, B, C));
+                    }
                 }
             }
             __syncwarp();

@@ -426,8 +426,11 @@ cudaError_t StreamBatch::count_kind(size_t i, const kvsmc::Launch& L)
     if (l.one && !nodes)
         return kvsmc::launch_count_one(l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts, d_status,
                                        d_next + 2 * i, L, pairs);
+    if (!nodes)
+        return kvsmc::launch_count_many(l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts,
+                                        d_status, d_next + 2 * i, L, l.ctas_per_sm, pairs);
     return kvsmc::launch_stream(false, l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts, nullptr,
-                                nullptr, d_status, d_next + 2 * i, L, l.ctas_per_sm, 0, nodes, nullptr, pairs);
+                                nullptr, d_status, d_next + 2 * i, L, l.ctas_per_sm, 0, nodes);
 }
 
 cudaError_t StreamBatch::scans(const kvsmc::Launch& L)

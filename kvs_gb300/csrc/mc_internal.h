@@ -170,21 +170,25 @@ size_t stream_row_elems(int dtype, int rows);
 // launch split by z-chunks).  d_totals (emit): per isolevel record its
 // triangles; a request whose total exceeds its cap_tris writes nothing (null:
 // each request writes up to its cap_tris).  The emit writes nothing when the
-// status word says that the count gave up.  list (count): also list the pairs.
+// status word says that the count gave up.
 // d_only_if (emit): the launch does nothing when this word is zero.
 cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
                           const StreamIso* d_isos, uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
                           const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
                           const Launch& L, int ctas_per_sm = 0, uint64_t task0 = 0,
                           uint32_t* d_node_counts = nullptr, const uint64_t* d_totals = nullptr,
-                          const PairList* list = nullptr, const int* d_only_if = nullptr);
+                          const int* d_only_if = nullptr);
 // The count of launches whose groups hold one isolevel each, any value type
 // (mc_one.cu); same outputs as launch_stream's.
 cudaError_t launch_count_one(int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
                              const StreamIso* d_isos, uint16_t* d_unit_counts, int* d_status,
                              unsigned long long* d_next_task, const Launch& L, const PairList* list);
-// The emit over the pairs that the count listed (launch_stream with `list`):
-// same outputs, same rules for status and totals; does nothing when the list
+// The count of launches with several isolevels a volume, the narrow types
+// (mc_many.cu); same outputs.
+cudaError_t launch_count_many(int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
+                              const StreamIso* d_isos, uint16_t* d_unit_counts, int* d_status,
+                              unsigned long long* d_next_task, const Launch& L, int ctas_per_sm, const PairList* list);
+// The emit over the pairs that the count listed: same outputs, same rules for status and totals; does nothing when the list
 // overflowed.  Tasks: the groups' blocks of units.
 cudaError_t launch_emit_pairs(int dtype, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
                               const StreamIso* d_isos, const PairList& list, const uint32_t* d_unit_offsets,

@@ -115,12 +115,12 @@ __global__ void __launch_bounds__(kOneThreads)
         const uint32_t z1 = z0 + G.zchunk < cz ? z0 + G.zchunk : cz;   // cell planes [z0, z1)
         // empty space: a brick whose node range lies on one side of the threshold
         const float2* bricks = G.bricks;
-        const uint32_t nby = (cy + 1) / 2;
+        const uint32_t nby = (cy + 1) / 2, brick_wpr = G.brick_wpr;
+        const float thr = isos[G.iso_begin].f.f_thr;
         auto brick_empty = [&](uint32_t z) -> bool {
-            const float thr = isos[G.iso_begin].f.f_thr;
-            const float2* row = bricks + ((uint64_t)(z / kBrickPlanes) * nby + (y >> 1)) * G.brick_wpr;
+            const float2* row = bricks + ((uint64_t)(z / kBrickPlanes) * nby + (y >> 1)) * brick_wpr;
             float2 mm = row[R == 2 ? seg : 2 * seg];
-            if (R == 1 && 2 * seg + 1 < G.brick_wpr) {   // a 256-cell segment spans two bricks
+            if (R == 1 && 2 * seg + 1 < brick_wpr) {   // a 256-cell segment spans two bricks
                 const float2 m1 = row[2 * seg + 1];
                 mm.x = fminf(mm.x, m1.x);
                 mm.y = fmaxf(mm.y, m1.y);
@@ -158,6 +158,13 @@ __global__ void __launch_bounds__(kOneThreads)
             for (uint32_t i = 0; i < nplanes && i < 3; ++i) issue(i);
         }
         const bool row_ok = y + half < cy;
+        // the lane's unit and (isolevel, unit) counter at plane z0 (the group's
+        // fields are read once per task: the stores below could alias them)
+        const uint32_t plane_units = cy * wpr;
+        const uint64_t unit0 = ((uint64_t)z0 * cy + y + half) * wpr + seg;
+        uint16_t* const ucount = unit_counts + G.unit_base + unit0;
+        uint16_t* upairs = LIST ? pl.unit_pairs + G.pair_base + unit0 : nullptr;
+        uint32_t* ulist = LIST ? pl.unit_list + G.pair_base + unit0 : nullptr;
         // this lane's cells inside the volume, as a mask
         const int lim = row_ok ? (int)cx - (int)((uint32_t)xoff + xl) : 0;
         const uint32_t inside = lim >= 8 ? 0xffu : (lim <= 0 ? 0u : (1u << lim) - 1u);
@@ -216,10 +223,9 @@ __global__ void __launch_bounds__(kOneThreads)
                         entry = lfull ? nullptr : pl.list + lcur + (inc - m);
                         const uint32_t before = R == 1 ? 0u : __shfl_sync(FULL, inc, LPR - 1);
                         if (lane % LPR == 0 && row_ok) {
-                            const uint64_t pu = G.pair_base + ((uint64_t)z * cy + y + half) * wpr + seg;
                             const uint32_t b = half ? before : 0u;
-                            pl.unit_pairs[pu] = (uint16_t)((R == 1 || half ? npairs : before) - b);
-                            pl.unit_list[pu] = (uint32_t)(lcur + b);
+                            upairs[(uint64_t)s * plane_units] = (uint16_t)((R == 1 || half ? npairs : before) - b);
+                            ulist[(uint64_t)s * plane_units] = (uint32_t)lcur + b;
                         }
                         lcur += npairs;
                     }
@@ -251,7 +257,7 @@ __global__ void __launch_bounds__(kOneThreads)
                         for (int d = LPR / 2; d > 0; d >>= 1) sum += __shfl_xor_sync(FULL, sum, d);
                     }
                     if (lane % LPR == 0 && row_ok && sum)
-                        unit_counts[G.unit_base + ((uint64_t)z * cy + y + half) * wpr + seg] = (uint16_t)sum;
+                        ucount[(uint64_t)s * plane_units] = (uint16_t)sum;
                 }
                 a0 = b0;
                 a1 = b1;

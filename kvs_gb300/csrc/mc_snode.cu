@@ -328,10 +328,7 @@ __global__ void __launch_bounds__(kSnThreads, KVSMC_SNODE_MULTI_CTAS)
     if (warp == 0) {
         float t = 0.0f;
         if (lane < (unsigned)niso) t = isos[lane].f.f_thr;
-        __shared__ float s_thr[kStreamMaxIso];
-        if (lane < (unsigned)niso) s_thr[lane] = t;
-        __syncwarp();
-        thermo_build(C.th, s_thr, niso, bs, bo, lane);
+        thermo_build(C.th, t, niso, bs, bo, lane);
     }
     for (unsigned i = threadIdx.x; i < (unsigned)niso; i += blockDim.x) C.iso[i] = isos[i];
     __syncthreads();   // the only CTA-wide barrier: the tables are read-only from here on
@@ -425,10 +422,10 @@ __global__ void __launch_bounds__(kSnThreads, KVSMC_SNODE_MULTI_CTAS)
                     const uint64_t x = xoff + xl;
                     uint32_t cx = 0, cy = 0, cz = 0;
                     if (x < nx) {
-                        const uint32_t a = thermo_mask(C.th, niso, bs, bo, (float)ra[xl]);
-                        if (x + 1 < nx) cx = a ^ thermo_mask(C.th, niso, bs, bo, (float)ra[xl + 1]);
-                        if (has_y) cy = a ^ thermo_mask(C.th, niso, bs, bo, (float)rb[xl]);
-                        if (has_z) cz = a ^ thermo_mask(C.th, niso, bs, bo, (float)rz[xl]);
+                        const uint32_t a = thermo_mask(C.th, bs, bo, (float)ra[xl]);
+                        if (x + 1 < nx) cx = a ^ thermo_mask(C.th, bs, bo, (float)ra[xl + 1]);
+                        if (has_y) cy = a ^ thermo_mask(C.th, bs, bo, (float)rb[xl]);
+                        if (has_z) cz = a ^ thermo_mask(C.th, bs, bo, (float)rz[xl]);
                     }
                     CX[i >> 1] |= cx << (16 * (i & 1));
                     CY[i >> 1] |= cy << (16 * (i & 1));
@@ -866,10 +863,9 @@ __global__ void __launch_bounds__(kSnThreads, 3)
         if (c < (unsigned)niso) C.iso[c] = conn[c];
     }
     if (warp == 0) {
-        __shared__ float s_thr[kStreamMaxIso];
-        if (lane < (unsigned)niso) s_thr[lane] = isos[G.iso_begin + lane].f.f_thr;
-        __syncwarp();
-        thermo_build(C.th, s_thr, niso, bs, bo, lane);
+        float t = 0.0f;
+        if (lane < (unsigned)niso) t = isos[G.iso_begin + lane].f.f_thr;
+        thermo_build(C.th, t, niso, bs, bo, lane);
     }
     __syncthreads();   // the only CTA-wide barrier: the tables are read-only from here on
     if (lane == 0) {
@@ -965,7 +961,7 @@ __global__ void __launch_bounds__(kSnThreads, 3)
                     const T* row = (r < 2 ? pa : pb) + (r & 1) * row_elems + xl;
                     uint32_t e[9];
 #pragma unroll
-                    for (int i = 0; i < 9; ++i) e[i] = thermo_mask(C.th, niso, bs, bo, (float)row[i]);
+                    for (int i = 0; i < 9; ++i) e[i] = thermo_mask(C.th, bs, bo, (float)row[i]);
                     P[r][0] = e[0] | (e[1] << 16);
                     P[r][1] = e[2] | (e[3] << 16);
                     P[r][2] = e[4] | (e[5] << 16);

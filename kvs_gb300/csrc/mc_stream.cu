@@ -1,5 +1,9 @@
-// mc_stream.cu -- the streaming kernels: duplicated-vertex extraction of many
-// (volume, isolevel) requests in fused launches (count, unit scan, emit).
+// mc_stream.cu -- the streaming layout's kernels that classify the volume
+// themselves: the shared-vertex modes' count (triangles and vertices in one
+// pass), the duplicated mode's emit for requests whose crossed cells could not
+// all be listed and for extractions without a list, and the unit scan.  The
+// duplicated mode counts in mc_one.cu and mc_many.cu and emits in mc_pairs.cu
+// on the same tasks and units.
 //
 // Work decomposition: every warp is an independent worker.
 //   * A warp task = (volume, z-chunk, cell row y, 256-cell x-segment).  The
@@ -9,13 +13,11 @@
 //     a per-buffer mbarrier), so a plane is read from HBM once per pass and
 //     the next one is in flight while the warp works.  No CTA-wide barrier:
 //     warps never wait for each other.
-//   * Classification works on each node's isolevel index q = #{thresholds < v}
-//     (isolevels sorted by threshold; a monotone bucket table plus exact
-//     compares in the rare shared bucket).  Since v > t_k exactly when q > k,
-//     a cell is active for isolevel k exactly when min(q) <= k < max(q) over
-//     its 8 corners, and its case bits are (q_c > k).  Each lane owns 8
-//     consecutive cells; q of the new plane's nodes is computed once per
-//     step and carried (packed bytes) to the next step.
+//   * Classification works on each node's isolevel mask (bit k set when the
+//     value is above isolevel k; mc_thermo.cuh): a cell is active for isolevel
+//     k exactly when bit k differs among its 8 corners, and its case bits are
+//     theirs.  Each lane owns 8 consecutive cells; the masks of the new plane's
+//     nodes are computed once per step and carried to the next step.
 //   * A "unit" = (z, y, segment): a contiguous piece of the reference's linear
 //     cell order.  The count kernel writes one u16 triangle count per (unit,
 //     isolevel); the unit-scan kernel turns them into u32 offsets inside each
@@ -73,49 +75,6 @@ __constant__ uint8_t c_ntri[256] = MC_NTRI_INIT;
 __constant__ uint16_t c_edge_mask[256] = MC_EDGE_MASK_INIT;
 __constant__ uint8_t c_edge_packed[12] = MC_EDGE_PACKED_INIT;
 
-// ------------------------------------------------------------ value access
-
-// 8 consecutive values of a shared-memory row as floats (x0 multiple of 8).
-template <typename T> __device__ __forceinline__ void load8(const T* row, uint32_t x0, float* o);
-template <> __device__ __forceinline__ void load8<float>(const float* row, uint32_t x0, float* o)
-{
-    const float4 a = *reinterpret_cast<const float4*>(row + x0);
-    const float4 b = *reinterpret_cast<const float4*>(row + x0 + 4);
-    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
-}
-template <> __device__ __forceinline__ void load8<uint16_t>(const uint16_t* row, uint32_t x0, float* o)
-{
-    const uint4 a = *reinterpret_cast<const uint4*>(row + x0);
-    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { o[2 * i] = (float)(w[i] & 0xffffu); o[2 * i + 1] = (float)(w[i] >> 16); }
-}
-template <> __device__ __forceinline__ void load8<int16_t>(const int16_t* row, uint32_t x0, float* o)
-{
-    const uint4 a = *reinterpret_cast<const uint4*>(row + x0);
-    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        o[2 * i] = (float)(int16_t)(w[i] & 0xffffu);
-        o[2 * i + 1] = (float)(int16_t)(w[i] >> 16);
-    }
-}
-template <> __device__ __forceinline__ void load8<uint8_t>(const uint8_t* row, uint32_t x0, float* o)
-{
-    const uint2 a = *reinterpret_cast<const uint2*>(row + x0);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { o[i] = (float)((a.x >> (8 * i)) & 255u); o[4 + i] = (float)((a.y >> (8 * i)) & 255u); }
-}
-template <> __device__ __forceinline__ void load8<int8_t>(const int8_t* row, uint32_t x0, float* o)
-{
-    const uint2 a = *reinterpret_cast<const uint2*>(row + x0);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        o[i] = (float)(int8_t)((a.x >> (8 * i)) & 255u);
-        o[4 + i] = (float)(int8_t)((a.y >> (8 * i)) & 255u);
-    }
-}
-
 // ------------------------------------------------------------ shared layout
 
 constexpr int kMaxVerts = KVSMC_EMIT_MAX_VERTS;   // vertex items of one round (rounds end before it is exceeded)
@@ -148,13 +107,9 @@ static_assert(3 * 3 * (kSegCells + 16) < (1 << 14), "edge_off packs ring offsets
 // Per-warp state.
 struct WarpState {
     uint64_t bar[3];
-    float thr[kStreamMaxIso];
-    int32_t thr_bucket[kStreamMaxIso];
+    ThermoTables th;
     uint32_t cnt[32];                        // count: triangles of the current units, [row][isolevel]
     uint32_t add[32];                        // emit: per-(row, isolevel) advance of the current round
-    // bucket -> (thermometer mask of the thresholds in lower buckets | kMultiThr,
-    //            bits of the bucket's first threshold, +inf when it has none)
-    uint2 lut[kLut];
 };
 
 // Per-warp emit buffers: the unit's pairs, and for one round the vertex pool
@@ -215,60 +170,6 @@ __device__ __forceinline__ EdgeItem edge_item(const Tables& TB, uint32_t qe, uin
 
 __host__ __device__ __forceinline__ size_t align128(size_t v) { return (v + 127) / 128 * 128; }
 
-// Thermometer masks of the 9 nodes x0 .. x0+8 of a staged row: bit k set when
-// the value is above isolevel k's threshold (v > t_k; thresholds sorted, so
-// the set bits are 0 .. q-1), packed two nodes per word (node 2m in the low
-// half of word m, node 2m+1 in the high half; word 4 holds node 8).  A bucket
-// holding one threshold needs one compare (branch-free); only a bucket holding
-// several takes the exact loop.
-template <typename T>
-__device__ __forceinline__ void row_masks(const T* row, uint32_t x0, const WarpState& W, int niso, float bs, float bo,
-                                          uint32_t* P)
-{
-    float v[9];
-    load8<T>(row, x0, v);
-    v[8] = (float)row[x0 + 8];
-    uint32_t e[9];
-    uint32_t any = 0;
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-        const uint2 l = W.lut[bucket_index(v[i], bs, bo)];
-        e[i] = (v[i] > __int_as_float((int)l.y)) ? 2u * l.x + 1u : l.x;
-        any |= l.x;
-    }
-    if (any & kMultiThr) {
-#pragma unroll
-        for (int i = 0; i < 9; ++i) {
-            const uint32_t b = bucket_index(v[i], bs, bo);
-            const uint32_t lx = W.lut[b].x;
-            if (lx & kMultiThr) {
-                int k = __popc(lx & 0xffffu);
-                while (k < niso && (uint32_t)W.thr_bucket[k] == b && W.thr[k] < v[i]) ++k;
-                e[i] = (1u << k) - 1u;
-            }
-        }
-    }
-    P[0] = __byte_perm(e[0], e[1], 0x5410);
-    P[1] = __byte_perm(e[2], e[3], 0x5410);
-    P[2] = __byte_perm(e[4], e[5], 0x5410);
-    P[3] = __byte_perm(e[6], e[7], 0x5410);
-    P[4] = e[8];
-}
-
-// Thermometer mask of one value (the per-node rule of row_masks).
-__device__ __forceinline__ uint32_t value_mask(const WarpState& W, int niso, float bs, float bo, float v)
-{
-    const uint32_t b = bucket_index(v, bs, bo);
-    const uint2 l = W.lut[b];
-    uint32_t e = (v > __int_as_float((int)l.y)) ? 2u * l.x + 1u : l.x;
-    if (l.x & kMultiThr) {
-        int k = __popc(l.x & 0xffffu);
-        while (k < niso && (uint32_t)W.thr_bucket[k] == b && W.thr[k] < v) ++k;
-        e = (1u << k) - 1u;
-    }
-    return e & 0xffffu;
-}
-
 __device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v, unsigned lane)
 {
 #pragma unroll
@@ -300,25 +201,23 @@ __device__ __forceinline__ int find_group(const StreamGroup* groups, int ngroups
 // whose other warps still run.  Tasks come out in increasing order; the
 // group's isolevel tables are rebuilt when a warp crosses a group boundary.
 //
-// NODES (count pass, one row per task): the pass also counts, per isolevel,
-// the vertices of the shared-vertex modes' node units (plane, node row,
+// The count (one row per task) is the shared-vertex modes': it also counts, per
+// isolevel, the vertices of their node units (plane, node row,
 // 256-node segment): the cut x, y and z edges from each node to its upper
 // neighbours, the edges whose two ends' threshold masks differ.  A task of
 // cell row y counts node row y at its planes; on the last cell row also node
 // row y + 1, on the last cell plane also the last node plane.  Groups with
 // node_units == 0 are not counted.
-// LIST (count pass): every unit's active pairs are listed for the emit of
-// mc_pairs.cu (a warp scan per step, and one 16-bit entry per pair).
-template <typename T, bool EMIT, int R, bool NODES = false, bool LIST = false>
+template <typename T, bool EMIT, int R>
 __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? KVSMC_EMIT_CTAS : 3)
     k_stream(const StreamGroup* __restrict__ groups, int ngroups, uint64_t ntasks, const StreamIso* __restrict__ isos,
              uint16_t* __restrict__ unit_counts, const uint32_t* __restrict__ unit_offsets,
              const uint64_t* __restrict__ plane_base, int* __restrict__ status,
              unsigned long long* __restrict__ next_task, uint32_t wait_polls, uint64_t task0,
-             uint32_t* __restrict__ node_counts, const uint64_t* __restrict__ totals, PairList pl,
+             uint32_t* __restrict__ node_counts, const uint64_t* __restrict__ totals,
              const int* __restrict__ only_if)
 {
-    static_assert(!NODES || (!EMIT && R == 1), "node counts come from one-row count tasks");
+    static_assert(EMIT || R == 1, "node counts come from one-row count tasks");
     constexpr int LPR = 32 / R;                 // lanes per cell row
     constexpr int SEG = kSegCells / R;          // cells per row segment
     constexpr int SEG_SHIFT = R == 1 ? 8 : 7;   // log2(SEG)
@@ -384,8 +283,6 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
     uint32_t ph = 0;     // per ring buffer: parity of its next completion
     int gcur = -1;       // group whose tables are in W
     bool live = true;    // emit: some request of the group is written
-    uint64_t lcur = 0, lend = 0;   // this warp's entries of the pair list
-    bool lfull = false;
     for (;;) {
     unsigned long long tk = 0;
     if (lane == 0) tk = atomicAdd(next_task, 1ull);
@@ -421,27 +318,17 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
     if (EMIT && G.skip_emit) continue;   // nothing of this group is written in this launch
     if (gi != gcur) {
         // the group's thresholds and bucket table
+        float t = 0.0f;
         if (lane < (unsigned)niso) {
             const StreamIso& I = isos[iso_begin + lane];
-            const float t = I.f.f_thr;
-            W.thr[lane] = t;
-            W.thr_bucket[lane] = (int32_t)bucket_index(t, bs, bo);
+            t = I.f.f_thr;
             if (EMIT) {
                 fill_iso(WE->ic[lane], I, totals, iso_begin + (int)lane);
             }
         }
         if (EMIT) live = __any_sync(FULL, lane < (unsigned)niso && WE->ic[lane & 15u].coords != nullptr);
         __syncwarp();
-        for (unsigned b = lane; b < (unsigned)kLut; b += 32) {
-            uint32_t below = 0, in = 0;
-            for (int k = 0; k < niso; ++k) {
-                below += (uint32_t)W.thr_bucket[k] < b ? 1u : 0u;
-                in += (uint32_t)W.thr_bucket[k] == b ? 1u : 0u;
-            }
-            const float first = in ? W.thr[below] : __int_as_float(0x7f800000);
-            W.lut[b] = make_uint2(((1u << below) - 1u) | (in > 1 ? kMultiThr : 0u), (uint32_t)__float_as_int(first));
-        }
-        __syncwarp();
+        thermo_build(W.th, t, niso, bs, bo, lane);
         gcur = gi;
     }
     if (EMIT && !live) continue;
@@ -464,7 +351,7 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
                 mm.y = fmaxf(mm.y, m1.y);
             }
         }
-        return value_mask(W, niso, bs, bo, mm.x) == value_mask(W, niso, bs, bo, mm.y);
+        return thermo_rank(W.th, bs, bo, mm.x) == thermo_rank(W.th, bs, bo, mm.y);
     };
     if (bricks) {
         bool all_empty = true;
@@ -557,12 +444,12 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
 
         // ---------------- phase 1: node masks, per-cell active isolevels
         if (!pa_valid) {
-            row_masks<T>(ra0, xl, W, niso, bs, bo, PA0);
-            row_masks<T>(ra1, xl, W, niso, bs, bo, PA1);
+            row_masks<T>(ra0, xl, W.th, bs, bo, PA0);
+            row_masks<T>(ra1, xl, W.th, bs, bo, PA1);
         }
         uint32_t PB0[5], PB1[5];
-        row_masks<T>(rb0, xl, W, niso, bs, bo, PB0);
-        row_masks<T>(rb1, xl, W, niso, bs, bo, PB1);
+        row_masks<T>(rb0, xl, W.th, bs, bo, PB0);
+        row_masks<T>(rb1, xl, W.th, bs, bo, PB1);
         // per node column: OR / AND of the 4 corners' masks (thermometer codes:
         // OR = the highest, AND = the lowest); per cell: the isolevels whose
         // threshold lies between its lowest and highest corner
@@ -593,34 +480,6 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
 
         if (!EMIT) {
             // count: one u16 per (unit, isolevel); counters [row][isolevel]
-            uint16_t* entry = nullptr;   // this lane's next list entry
-            if (LIST) {
-                const uint32_t inc = warp_inclusive_scan(m, lane);
-                const uint32_t npairs = __shfl_sync(FULL, inc, 31);
-                if (npairs != 0) {
-                    if (lcur + npairs > lend) {
-                        const uint32_t want = npairs > kPairRun ? npairs : kPairRun;
-                        unsigned long long at = 0;
-                        if (lane == 0) at = atomicAdd(pl.cursor, (unsigned long long)want);
-                        lcur = __shfl_sync(FULL, at, 0);
-                        lend = lcur + want;
-                        if (lend > pl.cap && !lfull) {
-                            lfull = true;
-                            if (lane == 0) atomicExch(pl.overflow, 1);
-                        }
-                    }
-                    entry = lfull ? nullptr : pl.list + lcur + (inc - m);
-                    // each of the step's R units: its pairs, its first entry
-                    const uint32_t before = R == 1 ? 0u : __shfl_sync(FULL, inc, LPR - 1);
-                    if (lane % LPR == 0 && row_ok) {
-                        const uint64_t pu = G.pair_base + ((uint64_t)z * cy + y + half) * wpr + seg;
-                        const uint32_t b = half ? before : 0u;
-                        pl.unit_pairs[pu] = (uint16_t)((R == 1 || half ? npairs : before) - b);
-                        pl.unit_list[pu] = (uint32_t)(lcur + b);
-                    }
-                    lcur += npairs;
-                }
-            }
             if (__any_sync(FULL, m != 0)) {
 #pragma unroll
                 for (int i = 0; i < kLaneCells; ++i) {
@@ -631,13 +490,12 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
                         do {
                             const uint32_t k = __ffs(am) - 1;
                             am &= am - 1;
-                            if (LIST && entry) *entry++ = (uint16_t)((xl + i) | (k << 8));
                             atomicAdd(&W.cnt[half * 16 + k], (uint32_t)TB.ntri[case_code(w0, w1, w2, w3, k)]);
                         } while (am);
                     }
                 }
                 __syncwarp();
-                if (NODES && G.node_units) {
+                if (G.node_units) {
                     // (a node edge that is cut for isolevel k belongs to a cell active
                     // for k, so a step without active cells has no vertices either)
                     const int nlim = (int)G.vol.nx - (int)((uint32_t)xoff + xl);   // this lane's nodes in the row
@@ -1093,7 +951,7 @@ cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_g
                           const StreamIso* d_isos, uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
                           const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
                           const Launch& L, int ctas_per_sm, uint64_t task0, uint32_t* d_node_counts,
-                          const uint64_t* d_totals, const PairList* list, const int* d_only_if)
+                          const uint64_t* d_totals, const int* d_only_if)
 {
     if (ntasks <= task0) return cudaSuccess;
     if (rows != 1 && rows != 2) return cudaErrorInvalidValue;
@@ -1101,15 +959,12 @@ cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_g
         return emit && rows == 1 ? launch_wide(dtype, d_groups, ngroups, ntasks, d_isos, d_unit_counts, d_unit_offsets,
                                                d_plane_base, d_status, d_next_task, L, task0, d_totals, d_only_if)
                                  : cudaErrorInvalidValue;
+    if (!emit && (rows != 1 || !d_node_counts)) return cudaErrorInvalidValue;   // (the other counts: mc_one.cu, mc_many.cu)
     const size_t smem = stream_shared_bytes(dtype, emit, rows);
     const int threads = emit ? kEmitThreads : kStreamThreads;
     const uint64_t need = (ntasks - task0 + threads / 32 - 1) / (threads / 32);
     KVSMC_STREAM_SWITCH(dtype, {
-        auto kern = emit ? (rows == 1 ? k_stream<T, true, 1> : k_stream<T, true, 2>)
-                         : (rows == 1 ? (d_node_counts ? k_stream<T, false, 1, true>
-                                         : list        ? k_stream<T, false, 1, false, true>
-                                                       : k_stream<T, false, 1>)
-                                      : (list ? k_stream<T, false, 2, false, true> : k_stream<T, false, 2>));
+        auto kern = emit ? (rows == 1 ? k_stream<T, true, 1> : k_stream<T, true, 2>) : k_stream<T, false, 1>;
         int per_sm = 0;
         const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), threads, smem, &per_sm, true);
         if (e != cudaSuccess) return e;
@@ -1122,7 +977,7 @@ cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_g
                                                            d_unit_offsets, d_plane_base, d_status, d_next_task,
                                                            L.wait_polls[emit ? 1 : 0], task0,
                                                            emit ? nullptr : d_node_counts, emit ? d_totals : nullptr,
-                                                           list ? *list : PairList{}, emit ? d_only_if : nullptr);
+                                                           emit ? d_only_if : nullptr);
         prof_end(L);
     });
     *L.counter += 1;

@@ -4,11 +4,15 @@
 //
 // With the isolevels' thresholds sorted (t_0 <= t_1 <= ...), a value's mask
 // has bit k set when v > t_k, so its set bits are 0 .. q-1.  A bucket index
-// floor(kStreamBuckets * sat(v * bs + bo)) is monotone in v; a lookup table
-// per bucket holds the mask of the thresholds in lower buckets and the
-// bucket's first threshold, so one float compare finishes the mask; only a
-// bucket holding two or more thresholds runs an exact loop.  NaN saturates to
-// bucket 0 and is above no threshold, as in the reference's double compare.
+// floor(kStreamBuckets * sat(v * bs + bo)) is monotone in v; a table of bytes
+// holds the number of thresholds in lower buckets, and one compare with the
+// next threshold finishes q: when that threshold lies in a higher bucket the
+// compare is false by itself.  Only when some bucket holds two or more
+// thresholds does a loop go on comparing.  NaN saturates to bucket 0 and is
+// above no threshold, as in the reference's double compare.
+// Byte and threshold lookups spread over few words (33 and 17), so 32 lanes'
+// random ones meet in no more than two rows of a shared-memory bank; one table
+// of 8-byte (mask, threshold) entries cost 4 to 5 wavefronts a lookup.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -18,8 +22,6 @@
 namespace kvsmc {
 
 constexpr int kLut = kStreamBuckets + 1;   // bucket indices 0 .. kStreamBuckets
-constexpr uint32_t kMultiThr = 1u << 31;   // LUT flag: two or more thresholds lie in this bucket
-
 // Monotone (non-decreasing) bucket of a value in [0, kStreamBuckets]:
 // floor(kStreamBuckets * sat(v * bs + bo)).  Thresholds and node values go
 // through exactly this function, so a threshold in a lower bucket than v is
@@ -36,46 +38,114 @@ __device__ __forceinline__ uint32_t bucket_index(float v, float bs, float bo)
 
 // A group's threshold tables (shared memory).
 struct ThermoTables {
-    float thr[kStreamMaxIso];
-    int32_t thr_bucket[kStreamMaxIso];
-    // bucket -> (thermometer mask of the thresholds in lower buckets | kMultiThr,
-    //            bits of the bucket's first threshold, +inf when it has none)
-    uint2 lut[kLut];
+    float thr[kStreamMaxIso + 1];   // sorted; +inf after the last one (no value is above it)
+    uint32_t several;               // some bucket holds two or more thresholds
+    uint8_t lut[(kLut + 3) / 4 * 4];   // bucket -> number of thresholds in lower buckets
 };
 
-// Fill W from the sorted thresholds t[0 .. niso): called by all 32 lanes of
-// one warp (the caller synchronizes before W is read by others).
-__device__ __forceinline__ void thermo_build(ThermoTables& W, const float* t, int niso, float bs, float bo,
-                                             unsigned lane)
+// Fill W from the sorted thresholds, lane k holding t_k for k < niso: called by
+// all 32 lanes of one warp (the caller synchronizes before W is read by others).
+__device__ __forceinline__ void thermo_build(ThermoTables& W, float t, int niso, float bs, float bo, unsigned lane)
 {
-    if (lane < (unsigned)niso) {
-        W.thr[lane] = t[lane];
-        W.thr_bucket[lane] = (int32_t)bucket_index(t[lane], bs, bo);
+    const uint32_t bucket = bucket_index(t, bs, bo);
+    if (lane <= (unsigned)niso) W.thr[lane] = lane < (unsigned)niso ? t : __int_as_float(0x7f800000);
+    const uint32_t before = __shfl_up_sync(0xffffffffu, bucket, 1);
+    const bool several = __any_sync(0xffffffffu, lane > 0 && lane < (unsigned)niso && before == bucket);
+    if (lane == 0) W.several = several ? 1u : 0u;
+    for (unsigned b0 = 0; b0 < (unsigned)kLut; b0 += 32) {
+        uint32_t below = 0;
+        for (int k = 0; k < niso; ++k) below += __shfl_sync(0xffffffffu, bucket, k) < b0 + lane ? 1u : 0u;
+        if (b0 + lane < (unsigned)kLut) W.lut[b0 + lane] = (uint8_t)below;
     }
     __syncwarp();
-    for (unsigned b = lane; b < (unsigned)kLut; b += 32) {
-        uint32_t below = 0, in = 0;
-        for (int k = 0; k < niso; ++k) {
-            below += (uint32_t)W.thr_bucket[k] < b ? 1u : 0u;
-            in += (uint32_t)W.thr_bucket[k] == b ? 1u : 0u;
-        }
-        const float first = in ? W.thr[below] : __int_as_float(0x7f800000);
-        W.lut[b] = make_uint2(((1u << below) - 1u) | (in > 1 ? kMultiThr : 0u), (uint32_t)__float_as_int(first));
+}
+
+// The number of thresholds below v.
+__device__ __forceinline__ uint32_t thermo_rank(const ThermoTables& W, float bs, float bo, float v)
+{
+    uint32_t q = W.lut[bucket_index(v, bs, bo)];
+    if (W.several) {
+        while (v > W.thr[q]) ++q;   // (ends at the +inf after the last one)
+    } else {
+        q += v > W.thr[q] ? 1u : 0u;
     }
+    return q;
 }
 
 // The mask of one value: bit k set when v > t_k.
-__device__ __forceinline__ uint32_t thermo_mask(const ThermoTables& W, int niso, float bs, float bo, float v)
+__device__ __forceinline__ uint32_t thermo_mask(const ThermoTables& W, float bs, float bo, float v)
 {
-    const uint32_t b = bucket_index(v, bs, bo);
-    const uint2 l = W.lut[b];
-    uint32_t e = (v > __int_as_float((int)l.y)) ? 2u * l.x + 1u : l.x;
-    if (l.x & kMultiThr) {
-        int k = __popc(l.x & 0xffffu);
-        while (k < niso && (uint32_t)W.thr_bucket[k] == b && W.thr[k] < v) ++k;
-        e = (1u << k) - 1u;
+    return (1u << thermo_rank(W, bs, bo, v)) - 1u;
+}
+
+// 8 consecutive values of a shared-memory row as floats (x0 multiple of 8).
+template <typename T> __device__ __forceinline__ void load8(const T* row, uint32_t x0, float* o);
+template <> __device__ __forceinline__ void load8<float>(const float* row, uint32_t x0, float* o)
+{
+    const float4 a = *reinterpret_cast<const float4*>(row + x0);
+    const float4 b = *reinterpret_cast<const float4*>(row + x0 + 4);
+    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+}
+template <> __device__ __forceinline__ void load8<uint16_t>(const uint16_t* row, uint32_t x0, float* o)
+{
+    const uint4 a = *reinterpret_cast<const uint4*>(row + x0);
+    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { o[2 * i] = (float)(w[i] & 0xffffu); o[2 * i + 1] = (float)(w[i] >> 16); }
+}
+template <> __device__ __forceinline__ void load8<int16_t>(const int16_t* row, uint32_t x0, float* o)
+{
+    const uint4 a = *reinterpret_cast<const uint4*>(row + x0);
+    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        o[2 * i] = (float)(int16_t)(w[i] & 0xffffu);
+        o[2 * i + 1] = (float)(int16_t)(w[i] >> 16);
     }
-    return e & 0xffffu;
+}
+template <> __device__ __forceinline__ void load8<uint8_t>(const uint8_t* row, uint32_t x0, float* o)
+{
+    const uint2 a = *reinterpret_cast<const uint2*>(row + x0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { o[i] = (float)((a.x >> (8 * i)) & 255u); o[4 + i] = (float)((a.y >> (8 * i)) & 255u); }
+}
+template <> __device__ __forceinline__ void load8<int8_t>(const int8_t* row, uint32_t x0, float* o)
+{
+    const uint2 a = *reinterpret_cast<const uint2*>(row + x0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        o[i] = (float)(int8_t)((a.x >> (8 * i)) & 255u);
+        o[4 + i] = (float)(int8_t)((a.y >> (8 * i)) & 255u);
+    }
+}
+
+// Thermometer masks of the 9 nodes x0 .. x0+8 of a staged row: bit k set when
+// the value is above isolevel k's threshold (v > t_k; thresholds sorted, so
+// the set bits are 0 .. q-1), packed two nodes per word (node 2m in the low
+// half of word m, node 2m+1 in the high half; word 4 holds node 8).
+template <typename T>
+__device__ __forceinline__ void row_masks(const T* row, uint32_t x0, const ThermoTables& W, float bs, float bo,
+                                          uint32_t* P)
+{
+    float v[9];
+    load8<T>(row, x0, v);
+    v[8] = (float)row[x0 + 8];
+    uint32_t q[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) q[i] = W.lut[bucket_index(v[i], bs, bo)];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) q[i] += v[i] > W.thr[q[i]] ? 1u : 0u;
+    if (W.several) {
+#pragma unroll
+        for (int i = 0; i < 9; ++i)
+            while (v[i] > W.thr[q[i]]) ++q[i];   // (ends at the +inf after the last one)
+    }
+    // (1 << a) - 1 in the low and (1 << b) - 1 in the high half (a, b <= 16: the
+    // sum is right modulo 2^32)
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+        P[m] = (1u << q[2 * m]) + ((1u << q[2 * m + 1]) << 16) - 0x10001u;
+    P[4] = (1u << q[8]) - 1u;
 }
 
 // The row word of cell i (0..7): node i in the low half, node i+1 in the high half.

@@ -186,7 +186,7 @@ extern "C" kvsmc_status kvsmc_extract_noalloc(const void* d_values, kvsmc_dtype 
         cudaMemcpyAsync(d_status, &zero, sizeof zero, cudaMemcpyHostToDevice, s) != cudaSuccess ||
         cudaMemsetAsync(d_unit_counts, 0, units * sizeof(uint16_t), s) != cudaSuccess ||
         cudaMemsetAsync(d_next, 0, 2 * sizeof(unsigned long long), s) != cudaSuccess ||
-        launch_stream(false, dtype, rows, d_group, 1, ntasks, d_iso, d_unit_counts, nullptr, nullptr, d_status, d_next, L) !=
+        launch_count_one(dtype, rows, d_group, 1, ntasks, d_iso, d_unit_counts, d_status, d_next, L, nullptr) !=
             cudaSuccess ||
         launch_unit_scan(d_group, 1, cz, d_iso, d_unit_counts, d_unit_offsets, d_plane_totals, L) != cudaSuccess ||
         launch_scan(d_plane_totals, d_plane_base, cz, d_scan, d_total, L) != cudaSuccess ||

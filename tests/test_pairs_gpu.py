@@ -53,6 +53,29 @@ def test_single_isolevel_on_and_between_integer_values(kvsmc_ctx, oracle_lib):
         vol.free()
 
 
+@pytest.mark.parametrize("mode", [0, 2])
+def test_crowded_isolevels_and_extreme_values(kvsmc_ctx, mode):
+    """Equal isolevels and several in one bucket of the threshold table beside
+    far ones, values at both ends of the float range, infinities and NaN:
+    together and alone (one isolevel's plain compares)."""
+    rng = np.random.default_rng(7 + mode)
+    v = rng.random((7, 9, 300)).astype(np.float32)
+    flat = v.reshape(-1)
+    for i, x in enumerate((3.4e38, -3.4e38, np.inf, -np.inf, np.nan, -0.0, 1e-45)):
+        flat[rng.integers(0, flat.size, 40)] = np.float32(x)
+    vol = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+    for isos in ([0.5] * 9 + [0.5 + 1e-9, 0.5 + 6e-8, 0.50001, 0.7, 0.7, -1e30, 1e30],
+                 [np.nextafter(np.float32(0.25), np.float32(1)), 0.25, 0.25, 1.0]):
+        params = [_abi.make_params(float(x), mode) for x in isos]
+        together = extract_batch(kvsmc_ctx, [vol] * len(isos), params, _abi.PATH_AUTO)
+        for x, p, o in zip(isos, params, together):
+            alone = extract_batch(kvsmc_ctx, [vol], [p], _abi.PATH_AUTO)[0]
+            assert o["status"] == alone["status"] == _abi.OK
+            assert all(same_bits(o[k], alone[k]) for k in ("coords", "normals")), (mode, x)
+            assert np.array_equal(o["connections"], alone["connections"]), (mode, x)
+    vol.free()
+
+
 def test_a_list_that_overflows(kvsmc_ctx):
     """16 isolevels of noise cross nearly every cell: 6e8 pairs, more than the
     list holds, so the triangles come from the classifying emit, in a batch and

@@ -19,11 +19,12 @@
 // normal per triangle (v1 - v0) x (v2 - v0).  Duplicated vertices only (the
 // reference's shared-vertex branch is not built, :164-206).
 //
-// Two passes over groups of 32 cells, a warp per group: count, an exclusive
-// scan of the group counts, emit (a warp scan of each cell's triangle
-// count); the emit pass skips the groups that counted no triangle without
-// reading their cells.  A
-// connection index outside the nodes sets a flag and reads node 0 instead.
+// Two passes, a warp per block of up to 32 groups of 32 cells: count (per group
+// a word of which cells have triangles, per block their number), an exclusive
+// scan over the blocks, emit.  An emitting warp takes the block's cut cells by
+// the words' bits, 32 at a time whatever groups they are in, so its lanes stay
+// busy where a surface passes a few cells of each group.  A connection index
+// outside the nodes sets a flag and reads node 0 instead.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -34,6 +35,7 @@
 #include "context.h"
 #include "batch.h"
 #include "mc_device.cuh"
+#include "mc_emit.cuh"
 #include "mc_interp.cuh"
 #include "slice_common.cuh"
 
@@ -41,66 +43,112 @@ namespace kvsmc {
 
 namespace {
 
-__constant__ uint8_t c_tet_ntri[CELL_TETRA_CASES] = CELL_TETRA_NTRI_INIT;
-__constant__ uint64_t c_tet_tri[CELL_TETRA_CASES] = CELL_TETRA_TRI_INIT;
-__constant__ uint8_t c_tet_edge[CELL_TETRA_EDGES] = CELL_TETRA_EDGE_INIT;
-__constant__ uint8_t c_hex_ntri[CELL_HEXA_CASES] = CELL_HEXA_NTRI_INIT;
-__constant__ uint64_t c_hex_tri[CELL_HEXA_CASES] = CELL_HEXA_TRI_INIT;
-__constant__ uint8_t c_hex_edge[CELL_HEXA_EDGES] = CELL_HEXA_EDGE_INIT;
-__constant__ uint8_t c_pyr_ntri[CELL_PYRAMID_CASES] = CELL_PYRAMID_NTRI_INIT;
-__constant__ uint64_t c_pyr_tri[CELL_PYRAMID_CASES] = CELL_PYRAMID_TRI_INIT;
-__constant__ uint8_t c_pyr_edge[CELL_PYRAMID_EDGES] = CELL_PYRAMID_EDGE_INIT;
-__constant__ uint8_t c_pri_ntri[CELL_PRISM_CASES] = CELL_PRISM_NTRI_INIT;
-__constant__ uint64_t c_pri_tri[CELL_PRISM_CASES] = CELL_PRISM_TRI_INIT;
-__constant__ uint8_t c_pri_edge[CELL_PRISM_EDGES] = CELL_PRISM_EDGE_INIT;
+// A cell type's case tables, laid out at compile time: per case the triangle
+// corners as ranks among the case's edges (4 bits each, table order), the edges
+// (local nodes, 4 bits each) and triangles | edges << 4.
+template <int CASES> struct alignas(16) CellTables {
+    static constexpr int kCases = CASES;
+    uint64_t slots[CASES];
+    uint8_t edges[CASES][12];
+    uint8_t counts[CASES];
+};
+
+template <int CASES>
+constexpr CellTables<CASES> make_cell_tables(const uint8_t* ntri, const uint64_t* tri, const uint8_t* edge)
+{
+    CellTables<CASES> t{};
+    for (int c = 0; c < CASES; ++c) {
+        int n = 0;
+        uint64_t of[12] = {};
+        for (int k = 0; k < 3 * (int)ntri[c]; ++k) {
+            const uint64_t e = (tri[c] >> (4 * k)) & 15u;
+            int r = 0;
+            while (r < n && of[r] != e) ++r;
+            if (r == n) {
+                of[n] = e;
+                t.edges[c][n++] = edge[e];
+            }
+            t.slots[c] |= (uint64_t)r << (4 * k);
+        }
+        t.counts[c] = (uint8_t)(ntri[c] | (n << 4));
+    }
+    return t;
+}
+
+constexpr uint8_t h_tet_ntri[CELL_TETRA_CASES] = CELL_TETRA_NTRI_INIT;
+constexpr uint64_t h_tet_tri[CELL_TETRA_CASES] = CELL_TETRA_TRI_INIT;
+constexpr uint8_t h_tet_edge[CELL_TETRA_EDGES] = CELL_TETRA_EDGE_INIT;
+constexpr uint8_t h_hex_ntri[CELL_HEXA_CASES] = CELL_HEXA_NTRI_INIT;
+constexpr uint64_t h_hex_tri[CELL_HEXA_CASES] = CELL_HEXA_TRI_INIT;
+constexpr uint8_t h_hex_edge[CELL_HEXA_EDGES] = CELL_HEXA_EDGE_INIT;
+constexpr uint8_t h_pyr_ntri[CELL_PYRAMID_CASES] = CELL_PYRAMID_NTRI_INIT;
+constexpr uint64_t h_pyr_tri[CELL_PYRAMID_CASES] = CELL_PYRAMID_TRI_INIT;
+constexpr uint8_t h_pyr_edge[CELL_PYRAMID_EDGES] = CELL_PYRAMID_EDGE_INIT;
+constexpr uint8_t h_pri_ntri[CELL_PRISM_CASES] = CELL_PRISM_NTRI_INIT;
+constexpr uint64_t h_pri_tri[CELL_PRISM_CASES] = CELL_PRISM_TRI_INIT;
+constexpr uint8_t h_pri_edge[CELL_PRISM_EDGES] = CELL_PRISM_EDGE_INIT;
+
+__device__ const CellTables<CELL_TETRA_CASES> d_tet_tables =
+    make_cell_tables<CELL_TETRA_CASES>(h_tet_ntri, h_tet_tri, h_tet_edge);
+__device__ const CellTables<CELL_HEXA_CASES> d_hex_tables =
+    make_cell_tables<CELL_HEXA_CASES>(h_hex_ntri, h_hex_tri, h_hex_edge);
+__device__ const CellTables<CELL_PYRAMID_CASES> d_pyr_tables =
+    make_cell_tables<CELL_PYRAMID_CASES>(h_pyr_ntri, h_pyr_tri, h_pyr_edge);
+__device__ const CellTables<CELL_PRISM_CASES> d_pri_tables =
+    make_cell_tables<CELL_PRISM_CASES>(h_pri_ntri, h_pri_tri, h_pri_edge);
 
 constexpr int kCellThreads = 256;
-constexpr int kCountGroups = 4;    // 32-cell groups per warp step of the count pass
+// 32-cell groups per warp step of the count pass
+template <int CT> constexpr int kCountGroups = CT == KVSMC_TETRAHEDRA ? 4 : 2;
+constexpr unsigned FULL = 0xffffffffu;
 
 template <int CT> struct CellTraits;
 template <> struct CellTraits<KVSMC_TETRAHEDRA> {
     static constexpr int kNodes = 4;
+    using Tables = CellTables<CELL_TETRA_CASES>;
     __device__ static int node(int k) { return k; }
-    __device__ static uint32_t ntri(unsigned c) { return c_tet_ntri[c]; }
-    __device__ static uint64_t tri(unsigned c) { return c_tet_tri[c]; }
-    __device__ static unsigned edge(int e) { return c_tet_edge[e]; }
+    __device__ static const Tables& tables() { return d_tet_tables; }
 };
 template <> struct CellTraits<KVSMC_HEXAHEDRA> {
     static constexpr int kNodes = 8;
+    using Tables = CellTables<CELL_HEXA_CASES>;
     __device__ static int node(int k) { return k < 4 ? k + 4 : k - 4; }   // MarchingHexahedra.cpp:105-112
-    __device__ static uint32_t ntri(unsigned c) { return c_hex_ntri[c]; }
-    __device__ static uint64_t tri(unsigned c) { return c_hex_tri[c]; }
-    __device__ static unsigned edge(int e) { return c_hex_edge[e]; }
+    __device__ static const Tables& tables() { return d_hex_tables; }
 };
 template <> struct CellTraits<KVSMC_PYRAMID> {
     static constexpr int kNodes = 5;
+    using Tables = CellTables<CELL_PYRAMID_CASES>;
     __device__ static int node(int k) { return k; }
-    __device__ static uint32_t ntri(unsigned c) { return c < CELL_PYRAMID_CASES ? c_pyr_ntri[c] : 0u; }
-    __device__ static uint64_t tri(unsigned c) { return c < CELL_PYRAMID_CASES ? c_pyr_tri[c] : 0ull; }
-    __device__ static unsigned edge(int e) { return c_pyr_edge[e]; }
+    __device__ static const Tables& tables() { return d_pyr_tables; }
 };
 template <> struct CellTraits<KVSMC_PRISM> {
     static constexpr int kNodes = 6;
+    using Tables = CellTables<CELL_PRISM_CASES>;
     __device__ static int node(int k) { return k; }
-    __device__ static uint32_t ntri(unsigned c) { return c_pri_ntri[c]; }
-    __device__ static uint64_t tri(unsigned c) { return c_pri_tri[c]; }
-    __device__ static unsigned edge(int e) { return c_pri_edge[e]; }
+    __device__ static const Tables& tables() { return d_pri_tables; }
 };
+
+// Copy the cell type's tables into shared memory (whole CTA; the caller
+// synchronizes).
+template <typename TB> __device__ __forceinline__ void load_tables(TB& dst, const TB& src)
+{
+    static_assert(sizeof(TB) % 16 == 0, "copied as 16-byte words");
+    for (unsigned i = threadIdx.x; i < sizeof(TB) / 16; i += kCellThreads)
+        reinterpret_cast<uint4*>(&dst)[i] = reinterpret_cast<const uint4*>(&src)[i];
+}
 
 template <typename T> __device__ __forceinline__ double dval(const void* v, uint64_t i)
 {
     return to_double(static_cast<const T*>(v)[i]);
 }
 
-// The cell's local node indices (checked against the node count): one or two
-// 16-byte loads per cell when the connections allow it (tetrahedra,
-// hexahedra on a 16-byte aligned array), else 32-bit loads.
+// The cell's connections: one or two 16-byte loads when they allow it
+// (tetrahedra, hexahedra on a 16-byte aligned array), else 32-bit loads.
 template <int CT>
-__device__ __forceinline__ void cell_nodes(const CellJob& j, uint64_t cell, uint32_t* nodes)
+__device__ __forceinline__ void cell_conn(const CellJob& j, uint64_t cell, uint32_t* raw)
 {
     using Tr = CellTraits<CT>;
     const uint32_t* conn = j.conn + (uint64_t)Tr::kNodes * cell;
-    uint32_t raw[Tr::kNodes];
     if ((CT == KVSMC_TETRAHEDRA || CT == KVSMC_HEXAHEDRA) && j.conn_vec16) {
 #pragma unroll
         for (int q = 0; q < Tr::kNodes / 4; ++q) {
@@ -111,6 +159,13 @@ __device__ __forceinline__ void cell_nodes(const CellJob& j, uint64_t cell, uint
 #pragma unroll
         for (int k = 0; k < Tr::kNodes; ++k) raw[k] = __ldg(conn + k);
     }
+}
+
+// The local node indices of a cell's connections, checked against the node count.
+template <int CT>
+__device__ __forceinline__ void cell_nodes_of(const CellJob& j, const uint32_t* raw, uint32_t* nodes)
+{
+    using Tr = CellTraits<CT>;
 #pragma unroll
     for (int k = 0; k < Tr::kNodes; ++k) {
         uint32_t n = raw[Tr::node(k)];
@@ -120,6 +175,14 @@ __device__ __forceinline__ void cell_nodes(const CellJob& j, uint64_t cell, uint
         }
         nodes[k] = n;
     }
+}
+
+template <int CT>
+__device__ __forceinline__ void cell_nodes(const CellJob& j, uint64_t cell, uint32_t* nodes)
+{
+    uint32_t raw[CellTraits<CT>::kNodes];
+    cell_conn<CT>(j, cell, raw);
+    cell_nodes_of<CT>(j, raw, nodes);
 }
 
 // The case: bit k iff double(value of local node k) > isolevel, decided
@@ -148,23 +211,13 @@ __device__ __forceinline__ unsigned case_of(const Classifier& cls, double iso, c
     return c;
 }
 
-// The cell's nodes and their values.
+// The nodes' values.
 template <int CT, typename T>
-__device__ __forceinline__ void cell_load(const CellJob& j, uint64_t cell, uint32_t* nodes, T* v)
+__device__ __forceinline__ void cell_values(const CellJob& j, const uint32_t* nodes, T* v)
 {
-    using Tr = CellTraits<CT>;
-    cell_nodes<CT>(j, cell, nodes);
     const T* vals = static_cast<const T*>(j.values);
 #pragma unroll
-    for (int k = 0; k < Tr::kNodes; ++k) v[k] = __ldg(vals + nodes[k]);
-}
-
-template <int CT, typename T>
-__device__ __forceinline__ unsigned cell_case(const CellJob& j, uint64_t cell, uint32_t* nodes)
-{
-    T v[CellTraits<CT>::kNodes];
-    cell_load<CT, T>(j, cell, nodes, v);
-    return case_of<CT, T>(j.cls, j.iso, v);
+    for (int k = 0; k < CellTraits<CT>::kNodes; ++k) v[k] = __ldg(vals + nodes[k]);
 }
 
 // The reference's FP64 sequence, out of line (it runs for the vertices the
@@ -215,110 +268,6 @@ __device__ __forceinline__ float3 cell_vertex(const CellJob& j, const FastIso& f
     return cell_vertex_exact<T>(j, iso, n0, n1);
 }
 
-// Both passes work on groups of 32 consecutive cells, one warp per group
-// (grid-stride over groups): the count pass writes each group's triangle
-// count, the emit pass skips the groups that counted none without reading
-// their cells and places the others' triangles by a warp scan.
-template <int CT, typename T>
-__global__ void __launch_bounds__(kCellThreads) k_cells_count(CellJob j)
-{
-    using Tr = CellTraits<CT>;
-    const unsigned lane = threadIdx.x & 31u;
-    const uint64_t warps = (uint64_t)gridDim.x * (kCellThreads / 32);
-    const uint64_t groups = (j.ncells + 31) / 32;
-    // kCountGroups groups per step (their loads in flight together)
-    constexpr int G = kCountGroups;
-    for (uint64_t g = ((uint64_t)blockIdx.x * (kCellThreads / 32) + (threadIdx.x >> 5)) * G; g < groups;
-         g += warps * G) {
-        uint32_t n[G];
-#pragma unroll
-        for (int q = 0; q < G; ++q) {
-            const uint64_t c = (g + q) * 32 + lane;
-            uint32_t nodes[Tr::kNodes];
-            n[q] = c < j.ncells ? Tr::ntri(cell_case<CT, T>(j, c, nodes)) : 0u;
-        }
-#pragma unroll
-        for (int q = 0; q < G; ++q) {
-            const uint32_t t = __reduce_add_sync(0xffffffffu, n[q]);
-            if (lane == 0 && g + q < groups) j.tile_counts[g + q] = t;
-        }
-    }
-}
-
-template <int CT, typename T>
-__global__ void __launch_bounds__(kCellThreads) k_cells_emit(CellJob j)
-{
-    using Tr = CellTraits<CT>;
-    // launched before the host knows the total: nothing is written unless all fits
-    if (j.d_total && *j.d_total > j.cap_tris) return;
-    const unsigned lane = threadIdx.x & 31u;
-    const uint64_t warps = (uint64_t)gridDim.x * (kCellThreads / 32);
-    const uint64_t groups = (j.ncells + 31) / 32;
-    // a warp takes 32 groups at a time: one coalesced read of their counts,
-    // then only the groups with triangles (ballot)
-    for (uint64_t g0 = ((uint64_t)blockIdx.x * (kCellThreads / 32) + (threadIdx.x >> 5)) * 32; g0 < groups;
-         g0 += warps * 32) {
-        const uint64_t mine = g0 + lane;
-        unsigned todo = __ballot_sync(0xffffffffu, mine < groups && j.tile_counts[mine] != 0);
-        while (todo) {
-        const uint64_t g = g0 + (unsigned)(__ffs(todo) - 1);
-        todo &= todo - 1;
-        const uint64_t cell = g * 32 + lane;
-        uint32_t nodes[Tr::kNodes] = {};
-        unsigned c = 0;
-        uint32_t n = 0;
-        if (cell < j.ncells) {
-            c = cell_case<CT, T>(j, cell, nodes);
-            n = Tr::ntri(c);
-        }
-        uint32_t inc = n;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= (unsigned)o) inc += y;
-        }
-        // the group's triangles spread over the lanes: lane l builds triangles
-        // l, l + 32, ... of the group; its cell is the first lane whose
-        // inclusive count exceeds the index (a 5-step search over shuffles)
-        const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
-        const uint64_t base = j.tile_offsets[g];
-        for (uint32_t first = 0; first < total; first += 32) {   // warp-uniform: every lane shuffles
-            const uint32_t tri = first + lane;
-            unsigned lo = 0;
-#pragma unroll
-            for (unsigned step = 16; step > 0; step >>= 1) {
-                const uint32_t probe = __shfl_sync(0xffffffffu, inc, lo + step - 1);
-                if (probe <= tri) lo += step;
-            }
-            // lo: the owning lane (inc[lo] > tri, inc[lo - 1] <= tri)
-            const uint32_t own_inc = __shfl_sync(0xffffffffu, inc, lo);
-            const uint32_t own_n = __shfl_sync(0xffffffffu, n, lo);
-            const unsigned own_c = __shfl_sync(0xffffffffu, c, lo);
-            uint32_t own_nodes[Tr::kNodes];
-#pragma unroll
-            for (int k = 0; k < Tr::kNodes; ++k) own_nodes[k] = __shfl_sync(0xffffffffu, nodes[k], lo);
-            const uint64_t t = base + tri;
-            if (tri >= total || t >= j.cap_tris) continue;   // never past the group or the outputs
-            const uint32_t k = tri - (own_inc - own_n);
-            const uint64_t pk = Tr::tri(own_c) >> (12 * k);
-            float3 v[3];
-#pragma unroll
-            for (int s = 0; s < 3; ++s) {
-                const unsigned ed = Tr::edge((int)((pk >> (4 * s)) & 15u));
-                v[s] = cell_vertex<T>(j, j.f, j.iso, own_nodes[ed & 15u], own_nodes[ed >> 4]);
-            }
-            float* o = j.out_coords + 9 * t;
-            o[0] = v[0].x; o[1] = v[0].y; o[2] = v[0].z;
-            o[3] = v[1].x; o[4] = v[1].y; o[5] = v[1].z;
-            o[6] = v[2].x; o[7] = v[2].y; o[8] = v[2].z;
-            const float3 nn = tri_normal(v[0], v[1], v[2]);
-            float* q = j.out_normals + 3 * t;
-            q[0] = nn.x; q[1] = nn.y; q[2] = nn.z;
-        }
-        }
-    }
-}
-
 // ---- kvs::SlicePlane on unstructured volumes (SlicePlane.cpp:291-800):
 // per cell type, a case from the plane's sign at the cell's node coordinates
 // (calculate_*_table_index, :828-942; no pyramid re-mapping), the cell type's
@@ -337,40 +286,33 @@ __device__ __forceinline__ float3 node_xyz(const CellJob& j, uint32_t n)
 }
 
 template <int CT>
-__device__ __forceinline__ unsigned slice_cell_case(const CellJob& j, uint64_t cell, uint32_t* nodes)
+__device__ __forceinline__ unsigned slice_cell_case(const CellJob& j, const uint32_t* nodes)
 {
-    using Tr = CellTraits<CT>;
-    cell_nodes<CT>(j, cell, nodes);
     unsigned c = 0;
 #pragma unroll
-    for (int k = 0; k < Tr::kNodes; ++k) {
+    for (int k = 0; k < CellTraits<CT>::kNodes; ++k) {
         const float3 p = node_xyz<CT>(j, nodes[k]);
         c |= plane_at(j, p.x, p.y, p.z) > 0.0f ? (1u << k) : 0u;
     }
     return c;
 }
 
-template <int CT, typename T>
-__global__ void __launch_bounds__(kCellThreads) k_cells_slice_count(CellJob j)
+// A cell's case: of an isolevel, or of the plane.
+template <int CT, typename T, bool SLICE>
+__device__ __forceinline__ unsigned cell_case(const CellJob& j, const Classifier& cls, double iso, const uint32_t* nodes)
 {
-    using Tr = CellTraits<CT>;
-    const unsigned lane = threadIdx.x & 31u;
-    const uint64_t warps = (uint64_t)gridDim.x * (kCellThreads / 32);
-    const uint64_t groups = (j.ncells + 31) / 32;
-    for (uint64_t g = (uint64_t)blockIdx.x * (kCellThreads / 32) + (threadIdx.x >> 5); g < groups; g += warps) {
-        const uint64_t cell = g * 32 + lane;
-        uint32_t n = 0;
-        if (cell < j.ncells) {
-            uint32_t nodes[Tr::kNodes];
-            n = Tr::ntri(slice_cell_case<CT>(j, cell, nodes));
-        }
-        const uint32_t t = __reduce_add_sync(0xffffffffu, n);
-        if (lane == 0) j.tile_counts[g] = t;
+    if constexpr (SLICE) {
+        return slice_cell_case<CT>(j, nodes);
+    } else {
+        T v[CellTraits<CT>::kNodes];
+        cell_values<CT, T>(j, nodes, v);
+        return case_of<CT, T>(cls, iso, v);
     }
 }
 
 template <typename T>
-__device__ __forceinline__ void slice_cell_vertex(const CellJob& j, uint32_t n0, uint32_t n1, float3& v, uchar3& rgb)
+__device__ __forceinline__ void slice_cell_vertex(const CellJob& j, const float* unit, uint32_t n0, uint32_t n1,
+                                                  float3& v, uchar3& rgb)
 {
     const float3 a = node_xyz<0>(j, n0), b = node_xyz<0>(j, n1);
     const float p0 = plane_at(j, a.x, a.y, a.z), p1 = plane_at(j, b.x, b.y, b.z);
@@ -380,83 +322,227 @@ __device__ __forceinline__ void slice_cell_vertex(const CellJob& j, uint32_t n0,
     v.y = __fadd_rn(__fmul_rn(s, a.y), __fmul_rn(r, b.y));
     v.z = __fadd_rn(__fmul_rn(s, a.z), __fmul_rn(r, b.z));
     const T* vals = static_cast<const T*>(j.values);
-    rgb = color_at(j, slice_value(vals[n0], vals[n1], r));
+    rgb = color_at(j, unit, slice_value(vals[n0], vals[n1], r));
 }
 
-template <int CT, typename T>
-__global__ void __launch_bounds__(kCellThreads) k_cells_slice_emit(CellJob j)
+// ---- the two passes.  A warp's work is a block of 2^block_shift consecutive
+// groups of 32 cells (at most 32 groups; fewer on small meshes, so that every
+// warp the GPU holds gets one, see cells_block_shift).
+//
+// Count: per group the word of its cells with triangles, per block the number
+// of its triangles; kCountGroups groups' loads are in flight together.
+// Bound by the latency of two dependent reads (connections, then values): 9.1e6
+// tetrahedra (146 MB of connections) take 40 us, 57% of the copy rate; more
+// groups in flight (8), or reading the next step's connections ahead (60 us:
+// twice the registers), do not help.
+template <int CT, typename T, bool SLICE>
+__global__ void __launch_bounds__(kCellThreads) k_cells_count(CellJob j)
+{
+    using Tr = CellTraits<CT>;
+    __shared__ typename Tr::Tables TB;
+    load_tables(TB, Tr::tables());
+    __syncthreads();
+    const unsigned lane = threadIdx.x & 31u;
+    const uint64_t groups = (j.ncells + 31) / 32;
+    const uint64_t blk = (uint64_t)blockIdx.x * (kCellThreads / 32) + (threadIdx.x >> 5);
+    const uint64_t g0 = blk << j.block_shift;
+    if (g0 >= groups) return;
+    const uint32_t ng = (uint32_t)(groups - g0 < (1ull << j.block_shift) ? groups - g0 : 1ull << j.block_shift);
+    constexpr int G = kCountGroups<CT>;
+    uint32_t sum = 0, mine = 0;   // this lane's triangles; the word of group g0 + lane
+    for (uint32_t g = 0; g < ng; g += G) {
+        uint32_t n[G];
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            const uint64_t c = (g0 + g + q) * 32 + lane;
+            n[q] = 0;
+            if (g + q < ng && c < j.ncells) {
+                uint32_t nodes[Tr::kNodes];
+                cell_nodes<CT>(j, c, nodes);
+                n[q] = TB.counts[cell_case<CT, T, SLICE>(j, j.cls, j.iso, nodes)] & 15u;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            const uint32_t word = __ballot_sync(FULL, n[q] != 0);
+            if (lane == g + q) mine = word;
+            sum += n[q];
+        }
+    }
+    sum = __reduce_add_sync(FULL, sum);
+    if (lane < ng) j.cut_words[g0 + lane] = mine;
+    if (lane == 0) j.block_counts[blk] = sum;
+}
+
+// A warp's shared memory in the emit pass: the nodes of a round's cells (an
+// odd stride: a column meets 32 banks) and the round's vertices.
+template <int CT> struct alignas(16) CellWarp {
+    static constexpr uint32_t kVerts = CT == KVSMC_TETRAHEDRA ? 128 : 192;
+    float4 pv[kVerts];   // x, y, z, colour (slices)
+    uint32_t nodes[32][CellTraits<CT>::kNodes | 1];
+};
+
+__device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t n)
+{
+    uint32_t pos = 0;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+        const uint32_t c = (uint32_t)__popc(m & ((1u << s) - 1u));
+        if (n >= c) {
+            n -= c;
+            m >>= s;
+            pos += s;
+        }
+    }
+    return pos;
+}
+
+// Emit one block: lane u holds the cut cells' word of group u; their bits are
+// one index space, taken 32 cells at a time, one per lane.  A round's vertices
+// are then computed one per lane (each edge a cell uses once, whatever number
+// of its triangles share it), and its triangles written one per lane, in cell
+// and table order from `run` on.
+template <int CT, typename T, bool SLICE>
+__device__ __forceinline__ void emit_block(const CellJob& j, const Classifier& cls, double iso, const FastIso& f,
+                                           float* out_coords, float* out_normals, uint64_t cap,
+                                           const typename CellTraits<CT>::Tables& TB, CellWarp<CT>& W,
+                                           const float* unit, uint32_t word, uint64_t g0, uint64_t run, unsigned lane)
 {
     using Tr = CellTraits<CT>;
     // hexahedra and pyramids are packed in the mappers' [i], [i+2], [i+1]
     // order; the slicer takes [i], [i+1], [i+2]
-    constexpr bool kSwapped = CT == KVSMC_HEXAHEDRA || CT == KVSMC_PYRAMID;
-    if (j.d_total && *j.d_total > j.cap_tris) return;
-    const unsigned lane = threadIdx.x & 31u;
-    const uint64_t warps = (uint64_t)gridDim.x * (kCellThreads / 32);
-    const uint64_t groups = (j.ncells + 31) / 32;
-    for (uint64_t g0 = ((uint64_t)blockIdx.x * (kCellThreads / 32) + (threadIdx.x >> 5)) * 32; g0 < groups;
-         g0 += warps * 32) {
-        const uint64_t mine = g0 + lane;
-        unsigned todo = __ballot_sync(0xffffffffu, mine < groups && j.tile_counts[mine] != 0);
-        while (todo) {
-            const uint64_t g = g0 + (unsigned)(__ffs(todo) - 1);
-            todo &= todo - 1;
-            const uint64_t cell = g * 32 + lane;
-            uint32_t nodes[Tr::kNodes] = {};
-            unsigned c = 0;
-            uint32_t n = 0;
-            if (cell < j.ncells) {
-                c = slice_cell_case<CT>(j, cell, nodes);
-                n = Tr::ntri(c);
-            }
-            uint32_t inc = n;
+    constexpr bool kSwapped = SLICE && (CT == KVSMC_HEXAHEDRA || CT == KVSMC_PYRAMID);
+    const unsigned lt = (1u << lane) - 1u;
+    const uint32_t cut = (uint32_t)__popc(word);
+    uint32_t inc = cut;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= (unsigned)o) inc += y;
-            }
-            const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
-            const uint64_t base = j.tile_offsets[g];
-            for (uint32_t first = 0; first < total; first += 32) {   // warp-uniform: every lane shuffles
-                const uint32_t tri = first + lane;
-                unsigned lo = 0;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(FULL, inc, o);
+        if (lane >= (unsigned)o) inc += t;
+    }
+    const uint32_t ncut = __shfl_sync(FULL, inc, 31);
+    uint32_t taken = 0;
+    for (uint32_t r0 = 0; r0 < ncut; r0 += taken) {
+        const uint32_t p = r0 + lane;
+        bool has = p < ncut;
+        uint32_t own = 0;   // its group: the first lane whose inclusive count exceeds p
 #pragma unroll
-                for (unsigned step = 16; step > 0; step >>= 1) {
-                    const uint32_t probe = __shfl_sync(0xffffffffu, inc, lo + step - 1);
-                    if (probe <= tri) lo += step;
+        for (int s = 4; s >= 0; --s) {
+            const uint32_t mid = own + (1u << s) - 1u;
+            if (__shfl_sync(FULL, inc, mid) <= p) own = mid + 1;
+        }
+        own &= 31u;   // (lanes past the last cell)
+        const uint32_t first = __shfl_sync(FULL, inc - cut, own), bits = __shfl_sync(FULL, word, own);
+        unsigned code = 0;
+        if (has) {
+            const uint64_t cell = (g0 + own) * 32 + nth_set_bit(bits, p - first);
+            uint32_t nodes[Tr::kNodes];
+            cell_nodes<CT>(j, cell, nodes);
+            code = cell_case<CT, T, SLICE>(j, cls, iso, nodes);
+#pragma unroll
+            for (int k = 0; k < Tr::kNodes; ++k) W.nodes[lane][k] = nodes[k];
+        }
+        const uint32_t cnt = has ? TB.counts[code] : 0u, ne = cnt >> 4;
+        uint32_t vpre = 0;
+#pragma unroll
+        for (int bit = 0; bit < 4; ++bit) vpre += (uint32_t)__popc(__ballot_sync(FULL, (ne >> bit) & 1u) & lt) << bit;
+        has = has && vpre + ne <= CellWarp<CT>::kVerts;   // a suffix of lanes waits
+        taken = (uint32_t)__popc(__ballot_sync(FULL, has));
+        const uint32_t nv = __shfl_sync(FULL, vpre + ne, taken - 1);
+        const uint32_t nt = has ? cnt & 15u : 0u;
+        uint32_t tpre = 0, ntr = 0;
+#pragma unroll
+        for (int bit = 0; bit < 3; ++bit) {
+            const uint32_t bm = __ballot_sync(FULL, (nt >> bit) & 1u);
+            tpre += (uint32_t)__popc(bm & lt) << bit;
+            ntr += (uint32_t)__popc(bm) << bit;
+        }
+        const uint32_t pe = code | (vpre << 8) | (tpre << 20);
+        __syncwarp();   // the nodes are there
+        uint32_t seen = 0;
+        for (uint32_t j0 = 0; j0 < nv; j0 += 32) {
+            const uint32_t i = j0 + lane;
+            // the cells' first items as bits: an item's cell is the number of first items up to it
+            const uint32_t starts = __reduce_or_sync(FULL, has && vpre - j0 < 32u ? 1u << (vpre - j0) : 0u);
+            const uint32_t q = seen + (uint32_t)__popc(starts & (lt | (1u << lane))) - 1u;
+            seen += (uint32_t)__popc(starts);
+            const uint32_t qe = __shfl_sync(FULL, pe, q);
+            if (i < nv) {
+                const uint32_t r = i - ((qe >> 8) & 0xfffu);
+                const uint32_t ed = TB.edges[qe & 255u][r < 11u ? r : 11u];
+                const uint32_t n0 = W.nodes[q][ed & 15u], n1 = W.nodes[q][ed >> 4];
+                if constexpr (SLICE) {
+                    float3 v;
+                    uchar3 rgb;
+                    slice_cell_vertex<T>(j, unit, n0, n1, v, rgb);
+                    W.pv[i] = make_float4(v.x, v.y, v.z, __uint_as_float((uint32_t)rgb.x | ((uint32_t)rgb.y << 8) |
+                                                                         ((uint32_t)rgb.z << 16)));
+                } else {
+                    const float3 v = cell_vertex<T>(j, f, iso, n0, n1);
+                    W.pv[i] = make_float4(v.x, v.y, v.z, 0.0f);
                 }
-                const uint32_t own_inc = __shfl_sync(0xffffffffu, inc, lo);
-                const uint32_t own_n = __shfl_sync(0xffffffffu, n, lo);
-                const unsigned own_c = __shfl_sync(0xffffffffu, c, lo);
-                uint32_t own_nodes[Tr::kNodes];
-#pragma unroll
-                for (int k = 0; k < Tr::kNodes; ++k) own_nodes[k] = __shfl_sync(0xffffffffu, nodes[k], lo);
-                const uint64_t t = base + tri;
-                if (tri >= total || t >= j.cap_tris) continue;
-                const uint32_t k = tri - (own_inc - own_n);
-                const uint64_t pk = Tr::tri(own_c) >> (12 * k);
-                float3 v[3];
-                uchar3 rgb[3];
-#pragma unroll
-                for (int sl = 0; sl < 3; ++sl) {
-                    const int src = kSwapped ? (sl == 0 ? 0 : 3 - sl) : sl;
-                    const unsigned ed = Tr::edge((int)((pk >> (4 * src)) & 15u));
-                    slice_cell_vertex<T>(j, own_nodes[ed & 15u], own_nodes[ed >> 4], v[sl], rgb[sl]);
-                }
-                float* o = j.out_coords + 9 * t;
-                o[0] = v[0].x; o[1] = v[0].y; o[2] = v[0].z;
-                o[3] = v[1].x; o[4] = v[1].y; o[5] = v[1].z;
-                o[6] = v[2].x; o[7] = v[2].y; o[8] = v[2].z;
-                uint8_t* q = j.out_colors + 9 * t;
-                q[0] = rgb[0].x; q[1] = rgb[0].y; q[2] = rgb[0].z;
-                q[3] = rgb[1].x; q[4] = rgb[1].y; q[5] = rgb[1].z;
-                q[6] = rgb[2].x; q[7] = rgb[2].y; q[8] = rgb[2].z;
-                const float3 nn = slice_normal(v[0], v[1], v[2]);
-                float* w = j.out_normals + 3 * t;
-                w[0] = nn.x; w[1] = nn.y; w[2] = nn.z;
             }
         }
+        __syncwarp();
+        seen = 0;
+        for (uint32_t j0 = 0; j0 < ntr; j0 += 32) {
+            const uint32_t i = j0 + lane;
+            const uint32_t starts = __reduce_or_sync(FULL, has && tpre - j0 < 32u ? 1u << (tpre - j0) : 0u);
+            const uint32_t q = seen + (uint32_t)__popc(starts & (lt | (1u << lane))) - 1u;
+            seen += (uint32_t)__popc(starts);
+            const uint32_t qe = __shfl_sync(FULL, pe, q);
+            const uint64_t t = run + i;
+            if (i < ntr && t < cap) {   // never past the outputs
+                const uint32_t sl = (uint32_t)(TB.slots[qe & 255u] >> (12 * (i - (qe >> 20))));
+                const float4* pv = W.pv + ((qe >> 8) & 0xfffu);
+                const float4 fa = pv[sl & 15u], fb = pv[(sl >> (kSwapped ? 8 : 4)) & 15u];
+                const float4 fc = pv[(sl >> (kSwapped ? 4 : 8)) & 15u];
+                const float3 A = make_float3(fa.x, fa.y, fa.z), B = make_float3(fb.x, fb.y, fb.z);
+                const float3 C = make_float3(fc.x, fc.y, fc.z);
+                store_triangle(out_coords + 9 * t, out_normals + 3 * t, A, B, C,
+                               SLICE ? slice_normal(A, B, C) : tri_normal(A, B, C));
+                if constexpr (SLICE) {
+                    uint8_t* o = j.out_colors + 9 * t;
+                    const float4 corner[3] = {fa, fb, fc};
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        const uint32_t w = __float_as_uint(corner[k].w);
+                        o[3 * k] = (uint8_t)w;
+                        o[3 * k + 1] = (uint8_t)(w >> 8);
+                        o[3 * k + 2] = (uint8_t)(w >> 16);
+                    }
+                }
+            }
+        }
+        run += ntr;
+        __syncwarp();
     }
+}
+
+// Emit, one isolevel or a slice: a warp per block.  9.1e6 tetrahedra, 6% of
+// them cut: 88 us with a warp to each group of 32 cells and three vertices a
+// triangle, 47 us.  Bound by latency: two or three rounds a warp, each a chain
+// of dependent reads (connections, values, coordinates).
+template <int CT, typename T, bool SLICE>
+__global__ void __launch_bounds__(kCellThreads) k_cells_emit(CellJob j)
+{
+    using Tr = CellTraits<CT>;
+    __shared__ typename Tr::Tables TB;
+    __shared__ CellWarp<CT> sw[kCellThreads / 32];
+    __shared__ float s_unit[SLICE ? 256 : 1];
+    // launched before the host knows the total: nothing is written unless all fits
+    if (j.d_total && *j.d_total > j.cap_tris) return;
+    load_tables(TB, Tr::tables());
+    if (SLICE) fill_unit(s_unit);
+    __syncthreads();
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint64_t groups = (j.ncells + 31) / 32;
+    const uint64_t blk = (uint64_t)blockIdx.x * (kCellThreads / 32) + warp;
+    const uint64_t g0 = blk << j.block_shift;
+    if (g0 >= groups) return;
+    const uint32_t ng = (uint32_t)(groups - g0 < (1ull << j.block_shift) ? groups - g0 : 1ull << j.block_shift);
+    emit_block<CT, T, SLICE>(j, j.cls, j.iso, j.f, j.out_coords, j.out_normals, j.cap_tris, TB, sw[warp], s_unit,
+                             lane < ng ? j.cut_words[g0 + lane] : 0u, g0, j.block_offsets[blk], lane);
 }
 
 // ---- min/max over the cells' nodes (GetMinMaxValues with connections,
@@ -667,119 +753,74 @@ template <int CT, typename T>
 __global__ void __launch_bounds__(kCellThreads) k_cells_sweep_count(CellJob j)
 {
     using Tr = CellTraits<CT>;
+    __shared__ typename Tr::Tables TB;
     __shared__ CellIso s_iso[kCellSweepMax];
+    load_tables(TB, Tr::tables());
     for (int i = threadIdx.x; i < j.niso; i += blockDim.x) s_iso[i] = j.isos[i];
     __syncthreads();
     const unsigned lane = threadIdx.x & 31u;
-    const uint64_t warps = (uint64_t)gridDim.x * (kCellThreads / 32);
-    const uint64_t groups = (j.ncells + 31) / 32;
-    for (uint64_t g = (uint64_t)blockIdx.x * (kCellThreads / 32) + (threadIdx.x >> 5); g < groups; g += warps) {
-        const uint64_t cell = g * 32 + lane;
+    const uint64_t groups = (j.ncells + 31) / 32, blocks = (groups + (1ull << j.block_shift) - 1) >> j.block_shift;
+    const uint64_t blk = (uint64_t)blockIdx.x * (kCellThreads / 32) + (threadIdx.x >> 5);
+    const uint64_t g0 = blk << j.block_shift;
+    if (g0 >= groups) return;
+    const uint32_t ng = (uint32_t)(groups - g0 < (1ull << j.block_shift) ? groups - g0 : 1ull << j.block_shift);
+    uint32_t sum[2] = {0, 0};   // lane l: the block's triangles of isolevels l and l + 32
+    for (uint32_t g = 0; g < ng; ++g) {
+        const uint64_t cell = (g0 + g) * 32 + lane;
         const bool ok = cell < j.ncells;
         uint32_t nodes[Tr::kNodes];
         T v[Tr::kNodes];
-        if (ok) cell_load<CT, T>(j, cell, nodes, v);
-        for (int k = 0; k < j.niso; ++k) {
-            const uint32_t n = ok ? Tr::ntri(case_of<CT, T>(s_iso[k].cls, s_iso[k].iso, v)) : 0u;
-            const uint32_t t = __reduce_add_sync(0xffffffffu, n);
-            if (lane == 0) j.tile_counts[(uint64_t)k * groups + g] = t;
+        if (ok) {
+            cell_nodes<CT>(j, cell, nodes);
+            cell_values<CT, T>(j, nodes, v);
         }
+        uint32_t words[2] = {0, 0};
+        for (int k = 0; k < j.niso; ++k) {
+            const uint32_t n = ok ? TB.counts[case_of<CT, T>(s_iso[k].cls, s_iso[k].iso, v)] & 15u : 0u;
+            const uint32_t w = __ballot_sync(FULL, n != 0), t = __reduce_add_sync(FULL, n);
+            if (lane == (unsigned)(k & 31)) {
+                if (k < 32) { words[0] = w; sum[0] += t; }
+                else { words[1] = w; sum[1] += t; }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if ((int)lane + 32 * h < j.niso) j.cut_words[(lane + 32 * h) * groups + g0 + g] = words[h];
     }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        if ((int)lane + 32 * h < j.niso) j.block_counts[(lane + 32 * h) * blocks + blk] = sum[h];
 }
 
 template <int CT, typename T>
 __global__ void __launch_bounds__(kCellThreads) k_cells_sweep_emit(CellJob j)
 {
     using Tr = CellTraits<CT>;
-    __shared__ CellIso s_iso[kCellSweepMax];
-    for (int i = threadIdx.x; i < j.niso; i += blockDim.x) s_iso[i] = j.isos[i];
+    __shared__ typename Tr::Tables TB;
+    __shared__ CellWarp<CT> sw[kCellThreads / 32];
+    load_tables(TB, Tr::tables());
     __syncthreads();
-    const unsigned lane = threadIdx.x & 31u;
-    const uint64_t warps = (uint64_t)gridDim.x * (kCellThreads / 32);
-    const uint64_t groups = (j.ncells + 31) / 32;
-    const uint64_t nchunks = (groups + 31) / 32;
-    const uint64_t items = nchunks * (uint64_t)j.niso;
-    for (uint64_t it = (uint64_t)blockIdx.x * (kCellThreads / 32) + (threadIdx.x >> 5); it < items; it += warps) {
-        const int k = (int)(it / nchunks);
-        const uint64_t g0 = (it - (uint64_t)k * nchunks) * 32;
-        const CellIso& I = s_iso[k];
-        const uint32_t* counts = j.tile_counts + (uint64_t)k * groups;
-        const uint64_t* offsets = j.tile_offsets + (uint64_t)k * groups;
-        const uint64_t mine = g0 + lane;
-        unsigned todo = __ballot_sync(0xffffffffu, mine < groups && counts[mine] != 0);
-        while (todo) {
-            const uint64_t g = g0 + (unsigned)(__ffs(todo) - 1);
-            todo &= todo - 1;
-            const uint64_t cell = g * 32 + lane;
-            uint32_t nodes[Tr::kNodes] = {};
-            unsigned c = 0;
-            uint32_t n = 0;
-            if (cell < j.ncells) {
-                T v[Tr::kNodes];
-                cell_load<CT, T>(j, cell, nodes, v);
-                c = case_of<CT, T>(I.cls, I.iso, v);
-                n = Tr::ntri(c);
-            }
-            uint32_t inc = n;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= (unsigned)o) inc += y;
-            }
-            const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
-            const uint64_t base = offsets[g] - I.base;
-            for (uint32_t first = 0; first < total; first += 32) {   // warp-uniform: every lane shuffles
-                const uint32_t tri = first + lane;
-                unsigned lo = 0;
-#pragma unroll
-                for (unsigned step = 16; step > 0; step >>= 1) {
-                    const uint32_t probe = __shfl_sync(0xffffffffu, inc, lo + step - 1);
-                    if (probe <= tri) lo += step;
-                }
-                const uint32_t own_inc = __shfl_sync(0xffffffffu, inc, lo);
-                const uint32_t own_n = __shfl_sync(0xffffffffu, n, lo);
-                const unsigned own_c = __shfl_sync(0xffffffffu, c, lo);
-                uint32_t own_nodes[Tr::kNodes];
-#pragma unroll
-                for (int q = 0; q < Tr::kNodes; ++q) own_nodes[q] = __shfl_sync(0xffffffffu, nodes[q], lo);
-                const uint64_t t = base + tri;
-                if (tri >= total || t >= I.cap_tris) continue;
-                const uint32_t kk = tri - (own_inc - own_n);
-                const uint64_t pk = Tr::tri(own_c) >> (12 * kk);
-                float3 vx[3];
-#pragma unroll
-                for (int sl = 0; sl < 3; ++sl) {
-                    const unsigned ed = Tr::edge((int)((pk >> (4 * sl)) & 15u));
-                    vx[sl] = cell_vertex<T>(j, I.f, I.iso, own_nodes[ed & 15u], own_nodes[ed >> 4]);
-                }
-                float* o = I.out_coords + 9 * t;
-                o[0] = vx[0].x; o[1] = vx[0].y; o[2] = vx[0].z;
-                o[3] = vx[1].x; o[4] = vx[1].y; o[5] = vx[1].z;
-                o[6] = vx[2].x; o[7] = vx[2].y; o[8] = vx[2].z;
-                const float3 nn = tri_normal(vx[0], vx[1], vx[2]);
-                float* q = I.out_normals + 3 * t;
-                q[0] = nn.x; q[1] = nn.y; q[2] = nn.z;
-            }
-        }
-    }
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint64_t groups = (j.ncells + 31) / 32, blocks = (groups + (1ull << j.block_shift) - 1) >> j.block_shift;
+    const uint64_t it = (uint64_t)blockIdx.x * (kCellThreads / 32) + warp;   // (isolevel, block)
+    const uint64_t k = it / blocks, blk = it - k * blocks;
+    if (k >= (uint64_t)j.niso) return;
+    const uint64_t g0 = blk << j.block_shift;
+    const uint32_t ng = (uint32_t)(groups - g0 < (1ull << j.block_shift) ? groups - g0 : 1ull << j.block_shift);
+    const CellIso& I = j.isos[k];
+    emit_block<CT, T, false>(j, I.cls, I.iso, I.f, I.out_coords, I.out_normals, I.cap_tris, TB, sw[warp], nullptr,
+                             lane < ng ? j.cut_words[k * groups + g0 + lane] : 0u, g0,
+                             j.block_offsets[k * blocks + blk] - I.base, lane);
 }
 
 // base[k] = the first scanned offset of isolevel k, base[niso] = the total.
-__global__ void k_sweep_bases(const uint64_t* offsets, uint64_t groups, int niso, const uint64_t* total, uint64_t* out)
+__global__ void k_sweep_bases(const uint64_t* offsets, uint64_t blocks, int niso, const uint64_t* total, uint64_t* out)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        for (int k = 0; k < niso; ++k) out[k] = groups ? offsets[(uint64_t)k * groups] : 0;
-        out[niso] = *total;
-    }
+    for (int k = threadIdx.x; k <= niso; k += blockDim.x) out[k] = k < niso ? offsets[(uint64_t)k * blocks] : *total;
 }
 
-// Blocks of 8 warps, one warp per 32-cell group, at most 8 blocks per SM.
-unsigned cell_grid(uint64_t groups, const Launch& L)
-{
-    const uint64_t blocks = (groups + kCellThreads / 32 - 1) / (kCellThreads / 32);
-    const uint64_t cap = (uint64_t)L.num_sms * 8;
-    return (unsigned)(blocks < cap ? (blocks ? blocks : 1) : cap);
-}
+// CTAs for `items` warps (at most (2^32 / 32 groups) x 64 isolevels: 2^30).
+unsigned cell_grid(uint64_t items) { return (unsigned)((items + kCellThreads / 32 - 1) / (kCellThreads / 32)); }
 
 #define KVSMC_CELL_SWITCH(CTV, DT, ...)                                                     \
     switch (CTV) {                                                                          \
@@ -810,10 +851,10 @@ unsigned cell_grid(uint64_t groups, const Launch& L)
 cudaError_t launch_cells_count(const CellJob& j, const Launch& L)
 {
     if (j.ncells == 0) return cudaSuccess;
-    const uint64_t tiles = cells_tiles(j.ncells);
     prof_begin(L, "cells_count");
-    KVSMC_CELL_SWITCH(j.cell_type, j.dtype,
-                      { k_cells_count<CT, T><<<cell_grid(tiles, L), kCellThreads, 0, L.stream>>>(j); });
+    KVSMC_CELL_SWITCH(j.cell_type, j.dtype, {
+        k_cells_count<CT, T, false><<<cell_grid(cells_blocks(j.ncells, j.block_shift)), kCellThreads, 0, L.stream>>>(j);
+    });
     prof_end(L);
     *L.counter += 1;
     return cudaGetLastError();
@@ -822,23 +863,22 @@ cudaError_t launch_cells_count(const CellJob& j, const Launch& L)
 cudaError_t launch_cells_emit(const CellJob& j, const Launch& L)
 {
     if (j.ncells == 0) return cudaSuccess;
-    const uint64_t tiles = cells_tiles(j.ncells);
     prof_begin(L, "cells_emit");
-    KVSMC_CELL_SWITCH(j.cell_type, j.dtype,
-                      { k_cells_emit<CT, T><<<cell_grid(tiles, L), kCellThreads, 0, L.stream>>>(j); });
+    KVSMC_CELL_SWITCH(j.cell_type, j.dtype, {
+        k_cells_emit<CT, T, false><<<cell_grid(cells_blocks(j.ncells, j.block_shift)), kCellThreads, 0, L.stream>>>(j);
+    });
     prof_end(L);
     *L.counter += 1;
     return cudaGetLastError();
 }
 
-
 cudaError_t launch_cells_slice_count(const CellJob& j, const Launch& L)
 {
     if (j.ncells == 0) return cudaSuccess;
-    const uint64_t tiles = cells_tiles(j.ncells);
     prof_begin(L, "cells_slice_count");
-    KVSMC_CELL_SWITCH(j.cell_type, j.dtype,
-                      { k_cells_slice_count<CT, T><<<cell_grid(tiles, L), kCellThreads, 0, L.stream>>>(j); });
+    KVSMC_CELL_SWITCH(j.cell_type, j.dtype, {
+        k_cells_count<CT, T, true><<<cell_grid(cells_blocks(j.ncells, j.block_shift)), kCellThreads, 0, L.stream>>>(j);
+    });
     prof_end(L);
     *L.counter += 1;
     return cudaGetLastError();
@@ -847,10 +887,10 @@ cudaError_t launch_cells_slice_count(const CellJob& j, const Launch& L)
 cudaError_t launch_cells_slice_emit(const CellJob& j, const Launch& L)
 {
     if (j.ncells == 0) return cudaSuccess;
-    const uint64_t tiles = cells_tiles(j.ncells);
     prof_begin(L, "cells_slice_emit");
-    KVSMC_CELL_SWITCH(j.cell_type, j.dtype,
-                      { k_cells_slice_emit<CT, T><<<cell_grid(tiles, L), kCellThreads, 0, L.stream>>>(j); });
+    KVSMC_CELL_SWITCH(j.cell_type, j.dtype, {
+        k_cells_emit<CT, T, true><<<cell_grid(cells_blocks(j.ncells, j.block_shift)), kCellThreads, 0, L.stream>>>(j);
+    });
     prof_end(L);
     *L.counter += 1;
     return cudaGetLastError();
@@ -859,10 +899,10 @@ cudaError_t launch_cells_slice_emit(const CellJob& j, const Launch& L)
 cudaError_t launch_cells_sweep_count(const CellJob& j, const Launch& L)
 {
     if (j.ncells == 0 || j.niso <= 0) return cudaSuccess;
-    const uint64_t tiles = cells_tiles(j.ncells);
     prof_begin(L, "cells_sweep_count");
-    KVSMC_CELL_SWITCH(j.cell_type, j.dtype,
-                      { k_cells_sweep_count<CT, T><<<cell_grid(tiles, L), kCellThreads, 0, L.stream>>>(j); });
+    KVSMC_CELL_SWITCH(j.cell_type, j.dtype, {
+        k_cells_sweep_count<CT, T><<<cell_grid(cells_blocks(j.ncells, j.block_shift)), kCellThreads, 0, L.stream>>>(j);
+    });
     prof_end(L);
     *L.counter += 1;
     return cudaGetLastError();
@@ -871,19 +911,19 @@ cudaError_t launch_cells_sweep_count(const CellJob& j, const Launch& L)
 cudaError_t launch_cells_sweep_emit(const CellJob& j, const Launch& L)
 {
     if (j.ncells == 0 || j.niso <= 0) return cudaSuccess;
-    const uint64_t items = (cells_tiles(j.ncells) + 31) / 32 * (uint64_t)j.niso;
     prof_begin(L, "cells_sweep_emit");
-    KVSMC_CELL_SWITCH(j.cell_type, j.dtype,
-                      { k_cells_sweep_emit<CT, T><<<cell_grid(items * 32, L), kCellThreads, 0, L.stream>>>(j); });
+    KVSMC_CELL_SWITCH(j.cell_type, j.dtype, {
+        k_cells_sweep_emit<CT, T><<<cell_grid(cells_blocks(j.ncells, j.block_shift) * (uint64_t)j.niso), kCellThreads, 0, L.stream>>>(j);
+    });
     prof_end(L);
     *L.counter += 1;
     return cudaGetLastError();
 }
 
-cudaError_t launch_sweep_bases(const uint64_t* offsets, uint64_t groups, int niso, const uint64_t* total,
+cudaError_t launch_sweep_bases(const uint64_t* offsets, uint64_t blocks, int niso, const uint64_t* total,
                                uint64_t* out, const Launch& L)
 {
-    k_sweep_bases<<<1, 32, 0, L.stream>>>(offsets, groups, niso, total, out);
+    k_sweep_bases<<<1, 96, 0, L.stream>>>(offsets, blocks, niso, total, out);
     *L.counter += 1;
     return cudaGetLastError();
 }
@@ -929,7 +969,24 @@ cudaError_t launch_cells_minmax(const CellJob& j, void* scratch, double* d_out, 
     return cudaGetLastError();
 }
 
-uint64_t cells_tiles(uint64_t ncells) { return (ncells + 31) / 32; }
+uint64_t cells_groups(uint64_t ncells) { return (ncells + 31) / 32; }
+
+uint64_t cells_blocks(uint64_t ncells, int block_shift)
+{
+    return (cells_groups(ncells) + (1ull << block_shift) - 1) >> block_shift;
+}
+
+// Groups per block (a power of two, at most 32, a lane each): as many as leave
+// every SM 64 blocks, a block or two for each warp that an SM holds.  Larger
+// blocks fill the emit's rounds and shorten the scan; fewer of them would leave
+// warps idle: a mesh of 1e4 cells in blocks of one group takes 37 us a call,
+// where one warp to 32 groups in turn took 90.
+int cells_block_shift(uint64_t ncells, int num_sms)
+{
+    int s = 0;
+    while (s < 5 && (cells_groups(ncells) >> (s + 1)) >= (uint64_t)num_sms * 64) ++s;
+    return s;
+}
 
 }  // namespace kvsmc
 
@@ -964,13 +1021,13 @@ kvsmc_status check_args(kvsmc_context* ctx, int cell_type, int dtype, uint64_t n
     return KVSMC_OK;
 }
 
-// The count pass's scratch (group counts, offsets, scan scratch, a tail for
+// The count pass's scratch (group words, block counts, offsets, scan scratch, a tail for
 // the total or the min/max) in the context's arena, and the bad-index flag.
 struct CellsScratch {
     void* d_scan;
     uint64_t* d_tail;
-    uint64_t tiles;      // 32-cell groups
-    uint64_t nscan;      // scanned entries: groups x isolevels
+    uint64_t blocks;     // of one isolevel
+    uint64_t nscan;      // scanned entries: blocks x isolevels
     void* d_extra;       // sweep: isolevel records (kCellSweepMax) and bases (kCellSweepMax + 1)
 };
 
@@ -980,18 +1037,22 @@ kvsmc_status cells_prepare(kvsmc_context* ctx, kvsmc::CellJob& j, CellsScratch* 
     if (!ctx->d_flag) KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->d_flag, sizeof(int)));
     j.bad_index = ctx->d_flag;
     KVSMC_CUDA(ctx, cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream));
-    sc->tiles = kvsmc::cells_tiles(j.ncells);
-    sc->nscan = sc->tiles * (uint64_t)niso;
-    const size_t bc = align_up(sc->nscan * 4, 256), bo = align_up(sc->nscan * 8, 256),
+    j.block_shift = kvsmc::cells_block_shift(j.ncells, ctx->num_sms);
+    sc->blocks = kvsmc::cells_blocks(j.ncells, j.block_shift);
+    sc->nscan = sc->blocks * (uint64_t)niso;
+    const size_t bw = align_up(kvsmc::cells_groups(j.ncells) * (uint64_t)niso * 4, 256),
+                 bc = align_up(sc->nscan * 4, 256), bo = align_up(sc->nscan * 8, 256),
                  bs = align_up(std::max(std::max(kvsmc::scan_scratch_bytes(sc->nscan),
                                                  kvsmc::cells_minmax_scratch_bytes(ctx->num_sms)),
                                         kvsmc::minmax_scratch_bytes(ctx->num_sms)), 256),
                  be = align_up(kvsmc::kCellSweepMax * sizeof(kvsmc::CellIso) + (kvsmc::kCellSweepMax + 1) * 8, 256);
-    kvsmc_status st = ensure_scratch(ctx, bc + bo + bs + 256 + be);
+    kvsmc_status st = ensure_scratch(ctx, bw + bc + bo + bs + 256 + be);
     if (st) return st;
     char* base = static_cast<char*>(ctx->scratch);
-    j.tile_counts = reinterpret_cast<uint32_t*>(base);
-    j.tile_offsets = reinterpret_cast<uint64_t*>(base + bc);
+    j.cut_words = reinterpret_cast<uint32_t*>(base);
+    base += bw;
+    j.block_counts = reinterpret_cast<uint32_t*>(base);
+    j.block_offsets = reinterpret_cast<uint64_t*>(base + bc);
     sc->d_scan = base + bc + bo;
     sc->d_tail = reinterpret_cast<uint64_t*>(base + bc + bo + bs);
     sc->d_extra = base + bc + bo + bs + 256;
@@ -1058,7 +1119,7 @@ kvsmc_status cells_passes(kvsmc_context* ctx, kvsmc::CellJob& j, const CellsScra
     using namespace kvsmc_host;
     const kvsmc::Launch L = launch_of(ctx);
     KVSMC_CUDA(ctx, kvsmc::launch_cells_count(j, L));
-    KVSMC_CUDA(ctx, kvsmc::launch_scan(j.tile_counts, j.tile_offsets, sc.nscan, sc.d_scan, sc.d_tail, L));
+    KVSMC_CUDA(ctx, kvsmc::launch_scan(j.block_counts, j.block_offsets, sc.nscan, sc.d_scan, sc.d_tail, L));
     if (emit) {
         j.d_total = sc.d_tail;
         KVSMC_CUDA(ctx, kvsmc::launch_cells_emit(j, L));
@@ -1237,7 +1298,7 @@ kvsmc_status kvsmc_slice_cells_host(kvsmc_context* ctx, kvsmc_cell_type cell_typ
     if ((st = cells_prepare(ctx, j, &sc))) return done(st);
     const kvsmc::Launch L = launch_of(ctx);
     e = kvsmc::launch_cells_slice_count(j, L);
-    if (e == cudaSuccess) e = kvsmc::launch_scan(j.tile_counts, j.tile_offsets, sc.nscan, sc.d_scan, sc.d_tail, L);
+    if (e == cudaSuccess) e = kvsmc::launch_scan(j.block_counts, j.block_offsets, sc.nscan, sc.d_scan, sc.d_tail, L);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_small, sc.d_tail, sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_small + 2, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -1368,8 +1429,8 @@ kvsmc_status kvsmc_marching_cells_sweep_device(kvsmc_context* ctx, kvsmc_cell_ty
     KVSMC_CUDA(ctx, cudaMemcpyAsync(d_isos, isos.data(), sizeof(kvsmc::CellIso) * niso, cudaMemcpyHostToDevice,
                                     ctx->stream));
     KVSMC_CUDA(ctx, kvsmc::launch_cells_sweep_count(j, L));
-    KVSMC_CUDA(ctx, kvsmc::launch_scan(j.tile_counts, j.tile_offsets, sc.nscan, sc.d_scan, sc.d_tail, L));
-    KVSMC_CUDA(ctx, kvsmc::launch_sweep_bases(j.tile_offsets, sc.tiles, niso, sc.d_tail, d_bases, L));
+    KVSMC_CUDA(ctx, kvsmc::launch_scan(j.block_counts, j.block_offsets, sc.nscan, sc.d_scan, sc.d_tail, L));
+    KVSMC_CUDA(ctx, kvsmc::launch_sweep_bases(j.block_offsets, sc.blocks, niso, sc.d_tail, d_bases, L));
     std::vector<uint64_t> bases((size_t)niso + 1);
     int bad = 0;
     KVSMC_CUDA(ctx, cudaMemcpyAsync(bases.data(), d_bases, 8 * ((size_t)niso + 1), cudaMemcpyDeviceToHost, ctx->stream));

@@ -570,6 +570,81 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const uint32_t* coun
     }
 }
 
+// The whole scan in one CTA, for counts that one CTA reads and writes in less
+// time than three launches take to run one after the other: a warp takes one
+// contiguous range, 128 counts (a 16-byte vector a lane) at a time, all its
+// loads in flight at once, so n <= kScanOneMax (7.5e3 counts: 8 us against 16;
+// 1.8e4: 12 against 16)
+constexpr int kScanOneVecs = 8;
+constexpr uint64_t kScanOneMax = (uint64_t)(kScanThreads / 32) * 128 * kScanOneVecs;
+
+__global__ void __launch_bounds__(kScanThreads) k_scan_one(const uint32_t* counts, uint32_t n, uint32_t vecs,
+                                                          uint64_t* offsets, uint64_t* d_total)
+{
+    __shared__ uint64_t ws[33];
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t base = warp * 128 * vecs + 4 * lane;   // vecs * 128 counts a warp
+    uint4 v[kScanOneVecs];
+#pragma unroll
+    for (int k = 0; k < kScanOneVecs; ++k) {
+        const uint32_t i = base + 128 * k;
+        v[k] = make_uint4(0, 0, 0, 0);
+        if (k < (int)vecs && i < n) {
+            if (i + 4 <= n) {
+                v[k] = *reinterpret_cast<const uint4*>(counts + i);
+            } else {
+                v[k].x = counts[i];
+                if (i + 1 < n) v[k].y = counts[i + 1];
+                if (i + 2 < n) v[k].z = counts[i + 2];
+            }
+        }
+    }
+    uint64_t run = 0;   // the warp's counts so far
+    uint64_t e[kScanOneVecs];
+#pragma unroll
+    for (int k = 0; k < kScanOneVecs; ++k) {
+        if (k >= (int)vecs) break;
+        const uint64_t s = (uint64_t)v[k].x + v[k].y + v[k].z + v[k].w;
+        uint64_t inc = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= (unsigned)o) inc += t;
+        }
+        e[k] = run + inc - s;
+        run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) ws[warp] = run;
+    __syncthreads();
+    if (warp == 0) {
+        const uint64_t w = ws[lane];
+        uint64_t inc = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= (unsigned)o) inc += t;
+        }
+        ws[lane] = inc - w;
+        if (lane == 31) *d_total = inc;
+    }
+    __syncthreads();
+    const uint64_t before = ws[warp];
+#pragma unroll
+    for (int k = 0; k < kScanOneVecs; ++k) {
+        const uint32_t i = base + 128 * k;
+        if (k >= (int)vecs || i >= n) break;
+        const uint64_t a = before + e[k], b = a + v[k].x, c = b + v[k].y, d = c + v[k].z;
+        if (i + 4 <= n) {
+            *reinterpret_cast<ulonglong2*>(offsets + i) = make_ulonglong2(a, b);
+            *reinterpret_cast<ulonglong2*>(offsets + i + 2) = make_ulonglong2(c, d);
+        } else {
+            offsets[i] = a;
+            if (i + 1 < n) offsets[i + 1] = b;
+            if (i + 2 < n) offsets[i + 2] = c;
+        }
+    }
+}
+
 }  // namespace
 
 // ------------------------------------------------------------ host side
@@ -634,6 +709,13 @@ cudaError_t launch_scan(const uint32_t* counts, uint64_t* offsets, uint64_t n, v
     if (nb == 0) nb = 1;
     uint64_t* bs = static_cast<uint64_t*>(scratch);
     prof_begin(L, "scan");
+    if (n <= kScanOneMax && ((reinterpret_cast<uintptr_t>(counts) | reinterpret_cast<uintptr_t>(offsets)) & 15u) == 0) {
+        const uint32_t per = (kScanThreads / 32) * 128;
+        k_scan_one<<<1, kScanThreads, 0, L.stream>>>(counts, (uint32_t)n, (uint32_t)(n + per - 1) / per, offsets, d_total);
+        prof_end(L);
+        *L.counter += 1;
+        return cudaGetLastError();
+    }
     k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, L.stream>>>(counts, n, bs);
     k_scan_top<<<1, kScanThreads, 0, L.stream>>>(bs, nb, d_total);
     k_scan_down<<<(unsigned)nb, kScanThreads, 0, L.stream>>>(counts, n, bs, offsets);

@@ -288,8 +288,10 @@ struct SliceJob {
     int32_t tf_res;
     const uint8_t* table;     // device colour table, tf_res x RGB
     uint64_t nrows;           // (ny - 1) (nz - 1)
-    uint32_t* row_counts;     // count pass: triangles per row
-    uint64_t* row_offsets;    // emit pass: exclusive scan of row_counts
+    int32_t group_shift;      // 2^group_shift consecutive rows per group
+    uint32_t* group_counts;   // count pass: triangles per group
+    uint64_t* group_offsets;  // their exclusive scan
+    uint64_t* d_total;        // and their sum
     float* coords;            // 9 T
     uint8_t* colors;          // 9 T (RGB per vertex)
     float* normals;           // 3 T
@@ -308,7 +310,7 @@ struct CellIso {
     float* out_coords;        // 9 T
     float* out_normals;       // 3 T
     uint64_t cap_tris;
-    uint64_t base;            // sweep: its first slot in the scanned group offsets
+    uint64_t base;            // sweep: its first slot in the scanned block offsets
 };
 constexpr int kCellSweepMax = 64;   // isolevels of one sweep
 struct CellJob {
@@ -323,8 +325,10 @@ struct CellJob {
     Classifier cls;           // exact thresholds of the isolevel (no FP64 for float / 32-bit values)
     FastIso f;                // constants of the FP32 vertex certificate (emit pass)
     int32_t conn_vec16;       // connections 16-byte aligned: vector loads for tetrahedra / hexahedra
-    uint32_t* tile_counts;    // per 32-cell group
-    uint64_t* tile_offsets;
+    int32_t block_shift;      // 2^block_shift 32-cell groups per block
+    uint32_t* cut_words;      // per group: which of its cells have triangles
+    uint32_t* block_counts;   // per block: its triangles
+    uint64_t* block_offsets;  // and their exclusive scan
     float* out_coords;        // 9 T
     float* out_normals;       // 3 T
     uint64_t cap_tris;
@@ -336,17 +340,19 @@ struct CellJob {
     int32_t tf_res;
     const uint8_t* table;     // device colour table, tf_res x RGB
     uint8_t* out_colors;      // 9 T (RGB per vertex)
-    // isolevel sweep: niso records in device memory, group counts / offsets
-    // of isolevel k at [k * groups, (k + 1) * groups)
+    // isolevel sweep: niso records in device memory; isolevel k's group words
+    // at k * groups, its block counts and offsets at k * blocks
     const CellIso* isos;
     int32_t niso;
 };
 cudaError_t launch_cells_count(const CellJob& j, const Launch& L);
 cudaError_t launch_cells_emit(const CellJob& j, const Launch& L);
-uint64_t cells_tiles(uint64_t ncells);
+uint64_t cells_groups(uint64_t ncells);
+uint64_t cells_blocks(uint64_t ncells, int block_shift);
+int cells_block_shift(uint64_t ncells, int num_sms);
 cudaError_t launch_cells_sweep_count(const CellJob& j, const Launch& L);
 cudaError_t launch_cells_sweep_emit(const CellJob& j, const Launch& L);
-cudaError_t launch_sweep_bases(const uint64_t* offsets, uint64_t groups, int niso, const uint64_t* total,
+cudaError_t launch_sweep_bases(const uint64_t* offsets, uint64_t blocks, int niso, const uint64_t* total,
                                uint64_t* out, const Launch& L);
 cudaError_t launch_cells_slice_count(const CellJob& j, const Launch& L);
 cudaError_t launch_cells_slice_emit(const CellJob& j, const Launch& L);

@@ -10,16 +10,18 @@
 // triangle's normal is (n0 + n1 + n2) / 3 in float, in that order
 // (PolygonExporter.cpp:133-152, kvs::Vector3 operator+ and operator/).
 //
-// Duplicated meshes with 16-byte aligned arrays: a persistent CTA walks tiles
-// of 256 triangles through a two-stage pipeline of bulk asynchronous copies
-// (TMA): the next tile's 9,216 coordinate and 3,072 normal bytes load into
-// shared memory (mbarrier completion) while the current tile's 12,800 record
-// bytes are composed there and leave by one bulk shared-to-global copy.  The
-// last partial tile, shared-vertex meshes (gathers through the connections)
-// and unaligned arrays take the plain kernel: coalesced loads, the records
-// composed in shared memory, 16-byte stores (a tile's records start at a
-// multiple of 12,800 bytes, so every store is aligned).  HBM-bound: 48 bytes
-// read and 50 written per triangle for a duplicated mesh.
+// A warp's work is a tile of 64 consecutive triangles, two per lane: their
+// records are 100 bytes, 25 whole words, so they are composed from registers
+// with 25 word stores at an odd stride, free of bank conflicts, and a tile's
+// 3,200 bytes leave by one bulk shared-to-global copy.  Duplicated meshes with
+// 16-byte aligned arrays arrive through a ring of two tiles a warp (TMA bulk
+// copies, mbarrier completion): 16 warps an SM keep 98 KB in flight and none
+// waits for another.  Shared-vertex meshes (gathers through the connections),
+// unaligned arrays and the last partial tile load straight into registers.
+// Bound by HBM: 48 bytes read and 50 written per triangle of a duplicated
+// mesh.  4,000,037 triangles: 75.6 us with CTA-wide tiles of
+// 256 and half-word stores, 68.6 us, 86% of the copy rate (three or four tiles
+// a ring: 68.6 to 69.6); 661 triangles, in one launch: 30 -> 18 us a call.
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -31,204 +33,248 @@ namespace kvsmc {
 
 namespace {
 
-constexpr int kStlTile = 256;
-constexpr int kStlRecord = 50;
+constexpr uint32_t kStlTile = 64;   // triangles
+constexpr uint32_t kStlRecord = 50;
+constexpr uint32_t kStlPollLimit = 1u << 22;
+constexpr unsigned FULL = 0xffffffffu;
 
-__device__ __forceinline__ void put_float(uint16_t* r, int slot, float f)
-{
-    const uint32_t b = __float_as_uint(f);
-    r[2 * slot] = (uint16_t)(b & 0xffffu);
-    r[2 * slot + 1] = (uint16_t)(b >> 16);
-}
+constexpr int kStlStages = 2;
+constexpr int kStlThreads = 256;
 
-// mode: KVSMC_DUP_POLYGON_NORMAL / KVSMC_SHARED_POLYGON_NORMAL / KVSMC_SHARED_VERTEX_NORMAL.
-__global__ void __launch_bounds__(kStlTile)
-    k_stl_records(const float* __restrict__ coords, const float* __restrict__ normals,
-                  const uint32_t* __restrict__ conn, uint64_t nverts, uint64_t ntri, int mode,
-                  uint8_t* __restrict__ out, int* __restrict__ bad_index)
-{
-    __shared__ float sc[kStlTile * 9];
-    __shared__ float sn[kStlTile * 3];
-    __shared__ __align__(16) uint16_t rec[kStlTile * kStlRecord / 2];
-    const unsigned tid = threadIdx.x;
-    for (uint64_t tile = blockIdx.x; tile * kStlTile < ntri; tile += gridDim.x) {
-        const uint64_t t0 = tile * kStlTile;
-        const uint32_t n = (uint32_t)(ntri - t0 < (uint64_t)kStlTile ? ntri - t0 : (uint64_t)kStlTile);
-        if (mode == KVSMC_DUP_POLYGON_NORMAL) {
-            const float* cs = coords + 9 * t0;
-            for (uint32_t i = tid; i < 9 * n; i += kStlTile) sc[i] = cs[i];
-            const float* ns = normals + 3 * t0;
-            for (uint32_t i = tid; i < 3 * n; i += kStlTile) sn[i] = ns[i];
-        } else {
-            // one (triangle, corner) per thread pass: its vertex through the connections
-            const uint32_t* cn = conn + 3 * t0;
-            for (uint32_t i = tid; i < 3 * n; i += kStlTile) {
-                uint64_t v = cn[i];
-                if (v >= nverts) {
-                    atomicExch(bad_index, 1);
-                    v = 0;
-                }
-                sc[3 * i + 0] = coords[3 * v + 0];
-                sc[3 * i + 1] = coords[3 * v + 1];
-                sc[3 * i + 2] = coords[3 * v + 2];
-            }
-            if (mode == KVSMC_SHARED_POLYGON_NORMAL) {
-                const float* ns = normals + 3 * t0;
-                for (uint32_t i = tid; i < 3 * n; i += kStlTile) sn[i] = ns[i];
-            } else if (tid < n) {
-                // ( normal0 + normal1 + normal2 ) / 3.0f, component by component
-                uint64_t v0 = cn[3 * tid], v1 = cn[3 * tid + 1], v2 = cn[3 * tid + 2];
-                v0 = v0 < nverts ? v0 : 0;
-                v1 = v1 < nverts ? v1 : 0;
-                v2 = v2 < nverts ? v2 : 0;
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const float s = __fadd_rn(__fadd_rn(normals[3 * v0 + k], normals[3 * v1 + k]), normals[3 * v2 + k]);
-                    sn[3 * tid + k] = __fdiv_rn(s, 3.0f);
-                }
-            }
-        }
-        __syncthreads();
-        if (tid < n) {
-            uint16_t* r = rec + tid * (kStlRecord / 2);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) put_float(r, k, sn[3 * tid + k]);
-#pragma unroll
-            for (int k = 0; k < 9; ++k) put_float(r, 3 + k, sc[9 * tid + k]);
-            r[24] = 0;   // the unused 2-byte attribute
-        }
-        __syncthreads();
-        const uint32_t bytes = (uint32_t)kStlRecord * n;
-        uint8_t* dst = out + (uint64_t)kStlRecord * t0;
-        const uint4* src4 = reinterpret_cast<const uint4*>(rec);
-        uint4* dst4 = reinterpret_cast<uint4*>(dst);
-        for (uint32_t i = tid; i < bytes / 16; i += kStlTile) dst4[i] = src4[i];
-        const uint8_t* src1 = reinterpret_cast<const uint8_t*>(rec);
-        for (uint32_t i = bytes / 16 * 16 + tid; i < bytes; i += kStlTile) dst[i] = src1[i];
-        __syncthreads();
-    }
-}
-
-// Shared memory of the pipelined kernel: two stages of tile inputs and of
-// composed records, and one mbarrier per input stage.
-struct StlPipe {
-    float c[2][kStlTile * 9];
-    float n[2][kStlTile * 3];
-    uint16_t rec[2][kStlTile * kStlRecord / 2];
-    uint64_t bar[2];
+// Warp shared memory: composed records of two tiles and, for bulk loads, the
+// ring of input tiles.
+struct alignas(16) StlOut {
+    uint32_t rec[2][kStlTile * kStlRecord / 4];
+};
+struct alignas(16) StlIn {
+    float c[kStlStages][kStlTile * 9];
+    float n[kStlStages][kStlTile * 3];
+    uint64_t bar[kStlStages];
 };
 
-constexpr uint32_t kStlPollLimit = 1u << 22;
-
-// Full tiles [0, ntiles) of a duplicated mesh; coords, normals, out 16-byte
-// aligned.  status: set to 2 when a load did not complete within the poll
-// limit (the CTA then drains its own copies and stops).
-__global__ void __launch_bounds__(kStlTile)
-    k_stl_records_tma(const float* __restrict__ coords, const float* __restrict__ normals, uint64_t ntiles,
-                      uint8_t* __restrict__ out, int* __restrict__ status)
+// Two triangles' 24 floats (each 3 of the normal, 9 of the corners) as 25
+// record words: the first record's 48 bytes and two zero bytes, the second's
+// shifted by half a word.
+__device__ __forceinline__ void stl_compose(uint32_t* r, const float* f)
 {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    StlPipe& P = *reinterpret_cast<StlPipe*>(smem_raw);
-    const unsigned tid = threadIdx.x;
-    constexpr uint32_t kInBytes = kStlTile * 12 * sizeof(float);
-    auto issue = [&](uint64_t tile, int b) {
-        mbar_arrive_expect_tx(&P.bar[b], kInBytes);
-        bulk_copy_g2s(P.c[b], coords + (uint64_t)kStlTile * 9 * tile, kStlTile * 9 * sizeof(float), &P.bar[b]);
-        bulk_copy_g2s(P.n[b], normals + (uint64_t)kStlTile * 3 * tile, kStlTile * 3 * sizeof(float), &P.bar[b]);
-    };
-    if (tid == 0) {
-        mbar_init(&P.bar[0], 1);
-        mbar_init(&P.bar[1], 1);
-        fence_barrier_init();
+    uint32_t before = 0;
+#pragma unroll
+    for (int i = 0; i < 12; ++i) r[i] = __float_as_uint(f[i]);
+#pragma unroll
+    for (int i = 0; i < 12; ++i) {
+        const uint32_t w = __float_as_uint(f[12 + i]);
+        r[12 + i] = __funnelshift_l(before, w, 16);
+        before = w;
     }
-    __syncthreads();
-    uint64_t tile = blockIdx.x;
-    if (tid == 0 && tile < ntiles) issue(tile, 0);
-    uint32_t ph = 0;            // per input stage: parity of its next completion
-    uint32_t pending = 0;       // per input stage: a load was issued and not yet waited for
-    if (tile < ntiles) pending = 1u;
-    for (uint32_t k = 0; tile < ntiles; tile += gridDim.x, ++k) {
-        const int b = (int)(k & 1u);
-        const uint64_t next = tile + gridDim.x;
-        if (tid == 0 && next < ntiles) {
-            fence_proxy_async();   // the stage was read by every thread in the previous step
-            issue(next, b ^ 1);
-        }
-        if (next < ntiles) pending |= 1u << (b ^ 1);
-        const bool ok = mbar_wait(&P.bar[b], (ph >> b) & 1u, kStlPollLimit);
-        if (!__syncthreads_and(ok)) {
-            if (tid == 0) atomicExch(status, 2);
-            break;
-        }
-        ph ^= 1u << b;
-        pending &= ~(1u << b);
-        // this stage's records were handed to a bulk store two steps ago
-        if (tid == 0) bulk_wait_read<1>();
-        __syncthreads();
-        uint16_t* r = P.rec[b] + tid * (kStlRecord / 2);
+    r[24] = before >> 16;
+}
+
+// The lane's two triangles (t, t + 1; those below ntri) straight from memory.
+template <int MODE>
+__device__ __forceinline__ void stl_load(const float* __restrict__ coords, const float* __restrict__ normals,
+                                         const uint32_t* __restrict__ conn, uint64_t nverts, uint64_t t, uint64_t ntri,
+                                         int* bad_index, float* f)
+{
 #pragma unroll
-        for (int j = 0; j < 3; ++j) put_float(r, j, P.n[b][3 * tid + j]);
+    for (int h = 0; h < 2; ++h) {
+        float* g = f + 12 * h;
+        const uint64_t tri = t + h;
+        if (tri >= ntri) {
 #pragma unroll
-        for (int j = 0; j < 9; ++j) put_float(r, 3 + j, P.c[b][9 * tid + j]);
-        r[24] = 0;
+            for (int k = 0; k < 12; ++k) g[k] = 0.0f;
+            continue;
+        }
+        if (MODE != KVSMC_SHARED_VERTEX_NORMAL) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) g[k] = __ldg(normals + 3 * tri + k);
+        }
+        if (MODE == KVSMC_DUP_POLYGON_NORMAL) {
+#pragma unroll
+            for (int k = 0; k < 9; ++k) g[3 + k] = __ldg(coords + 9 * tri + k);
+            continue;
+        }
+        uint64_t v[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            v[k] = __ldg(conn + 3 * tri + k);
+            if (v[k] >= nverts) {
+                atomicExch(bad_index, 1);
+                v[k] = 0;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 9; ++k) g[3 + k] = __ldg(coords + 3 * v[k / 3] + k % 3);
+        if (MODE == KVSMC_SHARED_VERTEX_NORMAL) {
+            // ( normal0 + normal1 + normal2 ) / 3.0f, component by component
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                g[k] = __fdiv_rn(__fadd_rn(__fadd_rn(__ldg(normals + 3 * v[0] + k), __ldg(normals + 3 * v[1] + k)),
+                                           __ldg(normals + 3 * v[2] + k)), 3.0f);
+        }
+    }
+}
+
+// Compose a tile's records in `rec` (no bulk store reads it any more) and
+// send them: a whole tile by one bulk store of lane 0, a partial one by the
+// lanes.  dst is 16-byte aligned.
+__device__ __forceinline__ void stl_send(uint32_t* rec, const float* f, uint8_t* dst, uint32_t ntris, unsigned lane)
+{
+    stl_compose(rec + 25 * lane, f);
+    if (ntris == kStlTile) {
         fence_proxy_async();   // the records, written by this thread, are read by the async proxy
-        __syncthreads();
-        if (tid == 0) {
-            bulk_copy_s2g(out + (uint64_t)kStlTile * kStlRecord * tile, P.rec[b], kStlTile * kStlRecord);
+        __syncwarp();
+        if (lane == 0) {
+            bulk_copy_s2g(dst, rec, kStlTile * kStlRecord);
             bulk_commit();
         }
+        return;
     }
-    if (tid == 0) {
-        // after a timeout: the loads still in flight land (bounded) before the CTA exits
-        for (int b = 0; b < 2; ++b)
-            if ((pending >> b) & 1u) mbar_wait(&P.bar[b], (ph >> b) & 1u, kStlPollLimit);
+    __syncwarp();
+    const uint32_t bytes = kStlRecord * ntris;
+    for (uint32_t i = lane; i < bytes / 16; i += 32)
+        reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(rec)[i];
+    for (uint32_t i = bytes / 16 * 8 + lane; i < bytes / 2; i += 32)
+        reinterpret_cast<uint16_t*>(dst)[i] = reinterpret_cast<const uint16_t*>(rec)[i];
+    __syncwarp();
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kStlThreads)
+    k_stl_direct(const float* __restrict__ coords, const float* __restrict__ normals,
+                 const uint32_t* __restrict__ conn, uint64_t nverts, uint64_t ntri, uint8_t* __restrict__ out,
+                 int* __restrict__ bad_index)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    StlOut& O = reinterpret_cast<StlOut*>(smem_raw)[warp];
+    const uint64_t tiles = (ntri + kStlTile - 1) / kStlTile, warps = (uint64_t)gridDim.x * (kStlThreads / 32);
+    uint32_t b = 0;
+    for (uint64_t tile = (uint64_t)blockIdx.x * (kStlThreads / 32) + warp; tile < tiles; tile += warps, b ^= 1u) {
+        const uint64_t t0 = tile * kStlTile;
+        float f[24];
+        stl_load<MODE>(coords, normals, conn, nverts, t0 + 2 * lane, ntri, bad_index, f);
+        if (lane == 0) bulk_wait_read<1>();   // rec[b] was sent two tiles ago
+        __syncwarp();
+        stl_send(O.rec[b], f, out + kStlRecord * t0, (uint32_t)(ntri - t0 < kStlTile ? ntri - t0 : kStlTile), lane);
+    }
+    if (lane == 0) bulk_wait<0>();
+}
+
+// A duplicated mesh; coords, normals, out 16-byte aligned.  status: set to 2
+// when a load did not complete within the poll limit (the warp then drains its
+// own copies and stops).
+__global__ void __launch_bounds__(kStlThreads)
+    k_stl_ring(const float* __restrict__ coords, const float* __restrict__ normals, uint64_t ntri,
+               uint8_t* __restrict__ out, int* __restrict__ status)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    constexpr int kWarps = kStlThreads / 32;
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    StlIn& I = reinterpret_cast<StlIn*>(smem_raw)[warp];
+    StlOut& O = reinterpret_cast<StlOut*>(smem_raw + kWarps * sizeof(StlIn))[warp];
+    const uint64_t full = ntri / kStlTile, warps = (uint64_t)gridDim.x * kWarps;
+    const uint64_t first = (uint64_t)blockIdx.x * kWarps + warp;
+    auto issue = [&](uint64_t tile, int s) {
+        mbar_arrive_expect_tx(&I.bar[s], kStlTile * 12 * sizeof(float));
+        bulk_copy_g2s(I.c[s], coords + kStlTile * 9 * tile, kStlTile * 9 * sizeof(float), &I.bar[s]);
+        bulk_copy_g2s(I.n[s], normals + kStlTile * 3 * tile, kStlTile * 3 * sizeof(float), &I.bar[s]);
+    };
+    if (lane == 0) {
+        for (int s = 0; s < kStlStages; ++s) mbar_init(&I.bar[s], 1);
+        fence_barrier_init();
+        for (int s = 0; s < kStlStages; ++s)
+            if (first + s * warps < full) issue(first + s * warps, s);
+    }
+    __syncwarp();
+    uint32_t ph = 0, pending = 0;   // per stage: parity of its next completion; a load is in flight
+    for (int s = 0; s < kStlStages; ++s)
+        if (first + s * warps < full) pending |= 1u << s;
+    int s = 0;
+    uint32_t b = 0;
+    for (uint64_t tile = first; tile < full; tile += warps) {
+        const bool ok = mbar_wait(&I.bar[s], (ph >> s) & 1u, kStlPollLimit);
+        if (!__all_sync(FULL, ok)) {
+            if (lane == 0) atomicExch(status, 2);
+            break;
+        }
+        ph ^= 1u << s;
+        pending &= ~(1u << s);
+        float f[24];
+        const float2* c2 = reinterpret_cast<const float2*>(I.c[s] + 18 * lane);
+        const float2* n2 = reinterpret_cast<const float2*>(I.n[s] + 6 * lane);
+        float c[18], n[6];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) { c[2 * k] = c2[k].x; c[2 * k + 1] = c2[k].y; }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { n[2 * k] = n2[k].x; n[2 * k + 1] = n2[k].y; }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) f[12 * h + k] = n[3 * h + k];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) f[12 * h + 3 + k] = c[9 * h + k];
+        }
+        __syncwarp();   // the stage is read
+        const uint64_t next = tile + kStlStages * warps;
+        if (next < full) {
+            if (lane == 0) {
+                fence_proxy_async();
+                issue(next, s);
+            }
+            pending |= 1u << s;
+        }
+        if (lane == 0) bulk_wait_read<1>();   // rec[b] was sent two tiles ago
+        __syncwarp();
+        stl_send(O.rec[b], f, out + kStlTile * kStlRecord * tile, kStlTile, lane);
+        b ^= 1u;
+        s = s + 1 < kStlStages ? s + 1 : 0;
+    }
+    if (full * kStlTile < ntri && full % warps == first) {   // the last partial tile
+        float f[24];
+        stl_load<KVSMC_DUP_POLYGON_NORMAL>(coords, normals, nullptr, 0, full * kStlTile + 2 * lane, ntri, status, f);
+        if (lane == 0) bulk_wait_read<0>();
+        __syncwarp();
+        stl_send(O.rec[0], f, out + kStlTile * kStlRecord * full, (uint32_t)(ntri - full * kStlTile), lane);
+    }
+    if (lane == 0) {
+        // after a timeout: the loads still in flight land (bounded) before the warp leaves
+        for (int q = 0; q < kStlStages; ++q)
+            if ((pending >> q) & 1u) mbar_wait(&I.bar[q], (ph >> q) & 1u, kStlPollLimit);
         bulk_wait<0>();
     }
 }
 
 }  // namespace
 
+// out is 16-byte aligned.
 cudaError_t launch_stl_records(const float* coords, const float* normals, const uint32_t* conn, uint64_t nverts,
                                uint64_t ntri, int mode, uint8_t* out, int* bad_index, const Launch& L)
 {
     if (ntri == 0) return cudaSuccess;
+    if (reinterpret_cast<uintptr_t>(out) & 15u) return cudaErrorInvalidValue;
+    const bool ring = mode == KVSMC_DUP_POLYGON_NORMAL &&
+                      ((reinterpret_cast<uintptr_t>(coords) | reinterpret_cast<uintptr_t>(normals)) & 15u) == 0;
+    const void* kern = ring ? reinterpret_cast<const void*>(k_stl_ring)
+                     : mode == KVSMC_DUP_POLYGON_NORMAL
+                         ? reinterpret_cast<const void*>(k_stl_direct<KVSMC_DUP_POLYGON_NORMAL>)
+                     : mode == KVSMC_SHARED_POLYGON_NORMAL
+                         ? reinterpret_cast<const void*>(k_stl_direct<KVSMC_SHARED_POLYGON_NORMAL>)
+                         : reinterpret_cast<const void*>(k_stl_direct<KVSMC_SHARED_VERTEX_NORMAL>);
+    constexpr int warps = kStlThreads / 32;
+    const size_t smem = warps * (sizeof(StlOut) + (ring ? sizeof(StlIn) : 0));
+    int per_sm = 0;
+    cudaError_t e = kernel_fit(L, kern, kStlThreads, smem, &per_sm, true);
+    if (e != cudaSuccess) return e;
+    const uint64_t tiles = (ntri + kStlTile - 1) / kStlTile, need = (tiles + warps - 1) / warps;
+    const uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)L.num_sms;
+    void* direct[] = {&coords, &normals, &conn, &nverts, &ntri, &out, &bad_index};
+    void* tma[] = {&coords, &normals, &ntri, &out, &bad_index};
     prof_begin(L, "stl_records");
-    uint64_t done = 0;
-    cudaError_t e = cudaSuccess;
-    const bool aligned = ((reinterpret_cast<uintptr_t>(coords) | reinterpret_cast<uintptr_t>(normals) |
-                           reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
-    if (mode == KVSMC_DUP_POLYGON_NORMAL && aligned && ntri >= (uint64_t)kStlTile) {
-        const uint64_t full = ntri / kStlTile;
-        const int smem = (int)sizeof(StlPipe);
-        e = cudaFuncSetAttribute(k_stl_records_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        int per_sm = 0;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stl_records_tma, kStlTile, smem);
-        if (e == cudaSuccess) {
-            const uint64_t cap = (uint64_t)(per_sm > 0 ? per_sm : 1) * L.num_sms;
-            k_stl_records_tma<<<(unsigned)(full < cap ? full : cap), kStlTile, smem, L.stream>>>(coords, normals, full,
-                                                                                              out, bad_index);
-            e = cudaGetLastError();
-            *L.counter += 1;
-        }
-        done = full * kStlTile;
-    }
-    if (e == cudaSuccess && done < ntri) {
-        const uint64_t rest = ntri - done;
-        const uint64_t tiles = (rest + kStlTile - 1) / kStlTile;
-        // resident CTAs: 25 KB of shared memory and 256 threads each, a few per SM
-        const uint64_t cap = (uint64_t)L.num_sms * 8;
-        const unsigned grid = (unsigned)(tiles < cap ? tiles : cap);
-        const bool dup = mode == KVSMC_DUP_POLYGON_NORMAL;
-        k_stl_records<<<grid, kStlTile, 0, L.stream>>>(dup ? coords + 9 * done : coords,
-                                                       (mode == KVSMC_SHARED_VERTEX_NORMAL) ? normals
-                                                                                            : normals + 3 * done,
-                                                       dup ? conn : conn + 3 * done, nverts, rest, mode,
-                                                       out + kStlRecord * done, bad_index);
-        e = cudaGetLastError();
-        *L.counter += 1;
-    }
+    e = cudaLaunchKernel(kern, dim3((unsigned)(need < resident ? need : resident)), dim3(kStlThreads),
+                         ring ? tma : direct, smem, L.stream);
     prof_end(L);
-    return e;
+    *L.counter += 1;
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace kvsmc
@@ -266,9 +312,10 @@ kvsmc_status kvsmc_stl_records(kvsmc_context* ctx, int32_t mode, const float* d_
     KVSMC_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(int), ctx->stream));
     KVSMC_CUDA(ctx, kvsmc::launch_stl_records(d_coords, d_normals, d_connections, nvertices, ntriangles, mode,
                                               static_cast<uint8_t*>(d_out), bad, kvsmc_host::launch_of(ctx)));
-    int h_bad = 0;
-    KVSMC_CUDA(ctx, cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    KVSMC_CUDA(ctx, cudaMemcpyAsync(ctx->h_small, bad, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    int h_bad = 0;
+    std::memcpy(&h_bad, ctx->h_small, sizeof(int));
     if (h_bad == 2) return fail(ctx, KVSMC_ERR_TIMEOUT, "stl: a shared-memory load did not complete");
     if (h_bad) return fail(ctx, KVSMC_ERR_INVALID_ARGUMENT, "stl: a connection index is >= nvertices");
     return KVSMC_OK;

@@ -1,5 +1,5 @@
-"""Unstructured cells and structured slices, at the edges of their warps'
-blocks of cells and groups of rows, against the oracles."""
+"""Unstructured cells, structured slices and STL records, at the edges of their
+warps' blocks of cells, groups of rows and tiles, against the oracles."""
 import numpy as np
 import pytest
 
@@ -7,6 +7,7 @@ from kvs_gb300 import _abi
 from kvs_gb300.marching_cubes import StructuredVolumeObject, TransferFunction
 from kvs_gb300.slice_plane import SlicePlane
 from oracle import cells as ocells
+from oracle import export as oexport
 from oracle import slice as oslice
 
 from . import cell_meshes as cm
@@ -55,3 +56,24 @@ def test_slice_planes(kvsmc_ctx, shape):
         assert same_bits(s.coords(), c), (coef, first_diff(s.coords(), c))
         assert np.array_equal(s.colors(), rgb), coef
         assert same_bits(s.normals(), n), coef
+
+
+@pytest.mark.parametrize("ntri", [1, 2, 63, 64, 65, 128, 5000, 700003])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_stl_records_in_tiles(kvsmc_ctx, ntri, shift):
+    """Partial and whole tiles, two and more a warp, from arrays on and off a
+    16-byte boundary; nothing is written past the last record."""
+    rng = np.random.default_rng(ntri)
+    coords = rng.standard_normal(9 * ntri).astype(np.float32)
+    normals = rng.standard_normal(3 * ntri).astype(np.float32)
+    want = oexport.stl_binary(coords, normals, np.zeros(0, np.uint32), oexport.POLYGON_NORMAL)[84:]
+    c = torch.zeros(9 * ntri + 4, device="cuda")
+    n = torch.zeros(3 * ntri + 4, device="cuda")
+    c[shift:shift + 9 * ntri] = torch.from_numpy(coords).cuda()
+    n[shift:shift + 3 * ntri] = torch.from_numpy(normals).cuda()
+    out = torch.full((50 * ntri + 64,), 7, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_stl_records(kvsmc_ctx.handle, _abi.MODE_DUP_POLYGON_NORMAL, c[shift:].data_ptr(),
+                                                    n[shift:].data_ptr(), None, 3 * ntri, ntri, out.data_ptr()), "records")
+    got = out.cpu().numpy()
+    assert got[:50 * ntri].tobytes() == want and (got[50 * ntri:] == 7).all()

@@ -168,6 +168,7 @@ extern "C" kvsmc_status kvsmc_extract_noalloc(const void* d_values, kvsmc_dtype 
     StreamIso iso;
     std::memset(&iso, 0, sizeof iso);
     iso.f = kvsmc_host::make_fast(p->isolevel, vmin, vmax, dtype);
+    iso.cls = kvsmc_host::make_classifier(p->isolevel);   // (the count reads it)
     iso.ip.iso = p->isolevel;
     iso.ip.vmin = vmin;
     iso.ip.vmax = vmax;

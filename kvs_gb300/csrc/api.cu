@@ -206,6 +206,12 @@ struct Plan {
     // normals are (VertexNormal), kept until its vertex normals
     bool conn_done = false;
     float* tri_normals = nullptr;
+    // its count lists the pairs for the connection pass (set by the caller
+    // before gather_count, for a request that will be emitted)
+    bool want_list = false;
+    // the connections go over listed pairs; where its vertex normals' slots are
+    bool pairs() const { return sconn && sb && sb->list_cap && !sb->overflowed; }
+    kvsmc::VertexSlots vs{};
 };
 
 uint32_t rows_for(uint32_t width, uint32_t limit)
@@ -270,6 +276,7 @@ void gather_setup(kvsmc_context* ctx, Plan& pl)
             pl.batch->items = {pl.item};
             pl.batch->want_nodes = true;
             pl.batch->one_row = true;
+            pl.batch->want_list = pl.want_list;
             pl.batch->plan_tables();
             pl.sconn = true;
             j.cell_tiles = 0;
@@ -362,12 +369,19 @@ kvsmc_status gather_count_at(kvsmc_context* ctx, Plan& pl, char* base)
 }
 
 // Count pass of one gather request in the context's scratch arena.
-kvsmc_status gather_count(kvsmc_context* ctx, Plan& pl)
+kvsmc_status gather_count(kvsmc_context* ctx, Plan& pl, bool emit)
 {
+    pl.want_list = emit;
     gather_setup(ctx, pl);
-    const size_t need =
-        gather_own_bytes(pl) + (pl.sconn && pl.batch ? align_up(pl.batch->scratch_bytes(), 256) : 0);
-    kvsmc_status st = ensure_scratch(ctx, need);
+    auto need = [&] {
+        return gather_own_bytes(pl) + (pl.sconn && pl.batch ? align_up(pl.batch->scratch_bytes(), 256) : 0);
+    };
+    kvsmc_status st = ensure_scratch(ctx, need());
+    if (st == KVSMC_ERR_OUT_OF_MEMORY && pl.batch && pl.batch->list_cap) {   // no room for the list: classify again
+        cudaGetLastError();
+        pl.batch->list_cap = 0;
+        st = ensure_scratch(ctx, need());
+    }
     if (st) return st;
     return gather_count_at(ctx, pl, static_cast<char*>(ctx->scratch));
 }
@@ -393,6 +407,25 @@ void gather_sizes(const Plan& pl, const Item& it, kvsmc_sizes* s)
     }
 }
 
+// The request's record for the connection pass.
+kvsmc::ConnIso conn_iso(const Plan& pl, float* coords, uint32_t* conn, float* normals)
+{
+    const bool vertex = pl.job.mode == KVSMC_SHARED_VERTEX_NORMAL;
+    kvsmc::ConnIso c{};
+    c.rank = pl.job.rank;
+    c.coords = coords;
+    c.connections = conn;
+    c.tri_out = vertex ? pl.tri_normals : normals;
+    c.nvert = pl.nvert;
+    c.ntri = pl.ntri;
+    c.enabled = 1;
+    if (vertex && pl.pairs()) {
+        c.tri4 = pl.vs.tri4;
+        c.slots = pl.vs.slots;
+    }
+    return c;
+}
+
 kvsmc_status gather_emit(kvsmc_context* ctx, Plan& pl, float* coords, float* normals, uint32_t* conn)
 {
     Job& j = pl.job;
@@ -411,7 +444,8 @@ kvsmc_status gather_emit(kvsmc_context* ctx, Plan& pl, float* coords, float* nor
         if (pl.ntri > 0xffffffffull)
             return fail(ctx, KVSMC_ERR_TOO_LARGE, "%llu triangles exceed 32-bit triangle ids of the vertex normals",
                         (unsigned long long)pl.ntri);
-        const size_t need = kvsmc::vertex_normals_scratch_bytes(pl.ntri, pl.nvert);
+        const size_t need = pl.pairs() ? (pl.conn_done ? 0 : kvsmc::vertex_slots_bytes(pl.ntri, pl.nvert))
+                                       : kvsmc::vertex_normals_scratch_bytes(pl.ntri, pl.nvert);
         if (need > ctx->arena2_bytes) {
             KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             if (ctx->arena2) cudaFree(ctx->arena2);
@@ -421,8 +455,13 @@ kvsmc_status gather_emit(kvsmc_context* ctx, Plan& pl, float* coords, float* nor
             KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->arena2, want));
             ctx->arena2_bytes = want;
         }
-        kvsmc::vertex_normals_carve(j, pl.ntri, pl.nvert, ctx->arena2);
-        if (pl.conn_done) j.tri_normals = pl.tri_normals;   // written by the connection pass already
+        if (!pl.pairs()) {
+            kvsmc::vertex_normals_carve(j, pl.ntri, pl.nvert, ctx->arena2);
+            if (pl.conn_done) j.tri_normals = pl.tri_normals;   // written by the connection pass already
+        } else if (!pl.conn_done) {
+            pl.vs = kvsmc::vertex_slots_carve(pl.ntri, pl.nvert, ctx->arena2);
+            j.slots = pl.vs.slots;
+        }
     } else {
         j.tri_normals = nullptr;
     }
@@ -442,6 +481,14 @@ kvsmc_status gather_emit(kvsmc_context* ctx, Plan& pl, float* coords, float* nor
     }
     if (pl.conn_done) {
         // written already
+    } else if (pl.ntri && pl.pairs()) {
+        const StreamBatch& b = *pl.sb;
+        const kvsmc::StreamGroup& G = b.groups[pl.sb_group];
+        kvsmc::ConnTable t{};
+        t.iso[pl.sb_iso] = conn_iso(pl, coords, conn, normals);
+        KVSMC_CUDA(ctx, kvsmc::launch_connect_pairs(b.d_groups + pl.sb_group, b.d_isos, t, j.vol.dtype, j.words_per_row,
+                                                    b.list, b.d_unit_offsets, b.d_plane_base,
+                                                    (uint64_t)(G.vol.nz - 1) * G.eblocks, pl.d_status, pl.d_next + 2, L));
     } else if (pl.ntri && pl.sconn) {
         StreamBatch& b = *pl.sb;
         KVSMC_CUDA(ctx, kvsmc::launch_sconnect(j, b.d_groups + pl.sb_group, b.d_isos, b.d_unit_counts,
@@ -450,7 +497,9 @@ kvsmc_status gather_emit(kvsmc_context* ctx, Plan& pl, float* coords, float* nor
     } else if (pl.ntri) {
         KVSMC_CUDA(ctx, launch_connect(j, L));
     }
-    if (vertex_normals) {
+    if (vertex_normals && pl.pairs()) {
+        KVSMC_CUDA(ctx, kvsmc::launch_vertex_slots(pl.vs, pl.ntri, pl.nvert, normals, L));
+    } else if (vertex_normals) {
         KVSMC_CUDA(ctx, launch_vertex_normals(j, pl.ntri, pl.nvert, L));
     } else if (pl.nvert && j.mode == KVSMC_SHARED_VERTEX_NORMAL) {
         // vertices without any triangle (a volume one node thick): zero normals
@@ -504,7 +553,7 @@ struct SharedCount {
     }
 };
 
-kvsmc_status shared_count(kvsmc_context* ctx, const std::vector<Item*>& items, SharedCount& sc)
+kvsmc_status shared_count(kvsmc_context* ctx, const std::vector<Item*>& items, SharedCount& sc, bool emit)
 {
     for (Item* it : items) {
         const int m = it->params.mode, dt = it->vol->view.dtype;
@@ -523,15 +572,23 @@ kvsmc_status shared_count(kvsmc_context* ctx, const std::vector<Item*>& items, S
     b.items = sc.cand;
     b.want_nodes = true;
     b.one_row = true;
+    b.want_list = emit;
     b.plan_tables();
-    const size_t need = b.scratch_bytes();
+    size_t need = b.scratch_bytes();
     if (need > ctx->arena3_bytes) {
         KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         if (ctx->arena3) cudaFree(ctx->arena3);
         ctx->arena3 = nullptr;
         ctx->arena3_bytes = 0;
-        const size_t want = align_up(need, 1 << 20);
-        if (kvsmc_host::device_malloc(ctx, &ctx->arena3, want) != cudaSuccess) {
+        size_t want = align_up(need, 1 << 20);
+        cudaError_t e = kvsmc_host::device_malloc(ctx, &ctx->arena3, want);
+        if (e != cudaSuccess && b.list_cap) {   // no room for the list: the connection pass classifies again
+            cudaGetLastError();
+            b.list_cap = 0;
+            want = align_up(need = b.scratch_bytes(), 1 << 20);
+            e = kvsmc_host::device_malloc(ctx, &ctx->arena3, want);
+        }
+        if (e != cudaSuccess) {
             // no room for the shared count: each request counts on its own
             cudaGetLastError();
             ctx->arena3 = nullptr;
@@ -672,9 +729,12 @@ kvsmc_status grouped_shared(kvsmc_context* ctx, const SharedCount& sc, std::vect
     // the VertexNormal requests' per-triangle normals, written by the
     // connection pass, summed by their vertex normals afterwards
     size_t tn_total = 0;
+    auto tn_bytes = [&](const Plan& pl) -> size_t {
+        return pl.pairs() ? kvsmc::vertex_slots_bytes(pl.ntri, pl.nvert) : align_up(12 * pl.ntri, 256);
+    };
     for (size_t i = 0; i < items.size(); ++i)
         if (!items[i]->status && items[i]->emit && plans[i].job.mode == KVSMC_SHARED_VERTEX_NORMAL)
-            tn_total += align_up(12 * plans[i].ntri, 256);
+            tn_total += tn_bytes(plans[i]);
     if (tn_total > ctx->arena5_bytes) {
         KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         if (ctx->arena5) cudaFree(ctx->arena5);
@@ -692,8 +752,12 @@ kvsmc_status grouped_shared(kvsmc_context* ctx, const SharedCount& sc, std::vect
         size_t o = 0;
         for (size_t i = 0; i < items.size(); ++i)
             if (!items[i]->status && items[i]->emit && plans[i].job.mode == KVSMC_SHARED_VERTEX_NORMAL) {
-                plans[i].tri_normals = reinterpret_cast<float*>(static_cast<char*>(ctx->arena5) + o);
-                o += align_up(12 * plans[i].ntri, 256);
+                char* at = static_cast<char*>(ctx->arena5) + o;
+                if (!plans[i].pairs()) plans[i].tri_normals = reinterpret_cast<float*>(at);
+                // (more triangles than 32-bit ids: no slots, refused by gather_emit)
+                else if (plans[i].ntri <= 0xffffffffull)
+                    plans[i].vs = kvsmc::vertex_slots_carve(plans[i].ntri, plans[i].nvert, at);
+                o += tn_bytes(plans[i]);
             }
     }
     // one node emit and one connection pass per group: its requests in
@@ -743,6 +807,7 @@ kvsmc_status grouped_shared(kvsmc_context* ctx, const SharedCount& sc, std::vect
             h[k].rank = pl.job.rank;
             h[k].offsets = pl.job.vtile_offsets;
             h[k].counts = pl.sb_nodes;
+            h[k].slots = pl.vs.slots;
         }
         const Plan& p0 = *gp[0];
         int* d_status = reinterpret_cast<int*>(d_status_all + 64 * g);
@@ -769,16 +834,17 @@ kvsmc_status grouped_shared(kvsmc_context* ctx, const SharedCount& sc, std::vect
             if (f == plan_of.end()) continue;
             const Plan& pl = *f->second;
             if (std::find(gp.begin(), gp.end(), f->second) == gp.end() || !pl.ntri) continue;
-            hc[k].rank = pl.job.rank;
-            hc[k].coords = it->d_coords;
-            hc[k].connections = it->d_conn;
-            hc[k].tri_out = pl.job.mode == KVSMC_SHARED_VERTEX_NORMAL ? pl.tri_normals : it->d_normals;
-            hc[k].nvert = pl.nvert;
-            hc[k].ntri = pl.ntri;
-            hc[k].enabled = 1;
+            hc[k] = conn_iso(pl, it->d_coords, it->d_conn, it->d_normals);
             tasks = pl.sb_tasks;
         }
-        if (!st && tasks) {
+        if (!st && tasks && p0.pairs()) {
+            kvsmc::ConnTable t{};
+            std::copy(hc, hc + G.niso, t.iso);
+            KVSMC_CUDA(ctx, kvsmc::launch_connect_pairs(b.d_groups + g, b.d_isos, t, p0.job.vol.dtype,
+                                                        p0.job.words_per_row, b.list, b.d_unit_offsets, b.d_plane_base,
+                                                        (uint64_t)(G.vol.nz - 1) * G.eblocks, d_status, d_next + 1, L));
+            if (ready && !(st = read_status())) st = group_status(g);
+        } else if (!st && tasks) {
             KVSMC_CUDA(ctx, cudaMemcpyAsync(d_conn, hc, (size_t)G.niso * sizeof(kvsmc::ConnIso),
                                             cudaMemcpyHostToDevice, ctx->stream));
             KVSMC_CUDA(ctx, kvsmc::launch_sconnect_multi(b.d_groups + g, b.d_isos, d_conn, p0.job.vol.dtype,
@@ -860,7 +926,7 @@ kvsmc_status run_items(kvsmc_context* ctx, std::vector<Item*>& items, bool emit)
         }
     }
     SharedCount sc;
-    if (kvsmc_status st = shared_count(ctx, gather_items, sc)) {
+    if (kvsmc_status st = shared_count(ctx, gather_items, sc, emit)) {
         for (Item* it : sc.cand) it->status = st;
         if (!first) first = st;
     }
@@ -892,7 +958,7 @@ kvsmc_status run_items(kvsmc_context* ctx, std::vector<Item*>& items, bool emit)
         Plan pl;
         gather_plan(*it, pl);
         sc.attach(it, pl);
-        kvsmc_status st = gather_count(ctx, pl);
+        kvsmc_status st = gather_count(ctx, pl, emit);
         if (!st) {
             gather_sizes(pl, *it, &it->sizes);
             if (emit) {
@@ -1193,7 +1259,7 @@ kvsmc_status kvsmc_marching_cubes_host(kvsmc_context* ctx, const void* host, kvs
         written = it.sizes.ntriangles <= cap;
     } else {
         gather_plan(it, pl);
-        if ((st = gather_count(ctx, pl))) return st;
+        if ((st = gather_count(ctx, pl, true))) return st;
         gather_sizes(pl, it, &it.sizes);
     }
     *sizes = it.sizes;
@@ -1407,7 +1473,7 @@ kvsmc_status kvsmc_extract_batch_host(kvsmc_context* ctx, const void* host, kvsm
         }
     }
     SharedCount sc;
-    if ((st = shared_count(ctx, g_items, sc))) {
+    if ((st = shared_count(ctx, g_items, sc, true))) {
         for (Item* it : sc.cand) it->status = st;
         if (!first) first = st;
     }
@@ -1472,7 +1538,7 @@ kvsmc_status kvsmc_extract_batch_host(kvsmc_context* ctx, const void* host, kvsm
         Plan pl;
         gather_plan(*it, pl);
         sc.attach(it, pl);
-        st = gather_count(ctx, pl);
+        st = gather_count(ctx, pl, true);
         if (!st) {
             gather_sizes(pl, *it, &it->sizes);
             std::vector<Item*> one{it};

@@ -140,8 +140,8 @@ bool stream_volume_eligible(const kvsmc_context* ctx, const Item& it)
     if ((double)(v.nx - 1) * (double)(v.ny - 1) * 5.0 >= 4294967295.0) return false;
     const double iso = it.params.isolevel;
     if (!std::isfinite(iso) || std::fabs(iso) > 1.0e30) return false;
-    return kvsmc::stream_shared_bytes(v.dtype, true, 1) <= (size_t)227 * 1024 &&
-           kvsmc::stream_shared_bytes(v.dtype, true, 2) <= (size_t)227 * 1024;
+    return kvsmc::stream_shared_bytes(v.dtype, 1) <= (size_t)227 * 1024 &&
+           kvsmc::stream_shared_bytes(v.dtype, 2) <= (size_t)227 * 1024;
 }
 
 void StreamBatch::plan_tables()
@@ -252,7 +252,7 @@ void StreamBatch::plan_tables()
             L.ntasks += stream_tasks(v, rows, g.wpr, g.zchunk);
             g.seg_elems = (uint32_t)kvsmc::stream_row_elems(dt, rows);
             g.seg_copy_bytes = g.seg_elems * (uint32_t)kvsmc::dtype_size(dt);
-            g.warp_smem_bytes = (uint32_t)kvsmc::stream_warp_smem_bytes(dt, true, rows);
+            g.warp_smem_bytes = (uint32_t)kvsmc::stream_warp_smem_bytes(dt, rows);
             g.warp_smem_offset = (uint32_t)kvsmc::stream_warp_smem_offset();
             // isolevels sorted by threshold
             std::vector<std::pair<float, Item*>> sorted;
@@ -426,11 +426,8 @@ cudaError_t StreamBatch::count_kind(size_t i, const kvsmc::Launch& L)
     if (l.one && !nodes)
         return kvsmc::launch_count_one(l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts, d_status,
                                        d_next + 2 * i, L, pairs);
-    if (!nodes)
-        return kvsmc::launch_count_many(l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts,
-                                        d_status, d_next + 2 * i, L, l.ctas_per_sm, pairs);
-    return kvsmc::launch_stream(false, l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts, nullptr,
-                                nullptr, d_status, d_next + 2 * i, L, l.ctas_per_sm, 0, nodes);
+    return kvsmc::launch_count_many(l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts, d_status,
+                                    d_next + 2 * i, L, l.ctas_per_sm, pairs, nodes);
 }
 
 cudaError_t StreamBatch::scans(const kvsmc::Launch& L)
@@ -511,9 +508,9 @@ cudaError_t StreamBatch::emit_kind(size_t i, const kvsmc::Launch& L, const uint6
     if (list_cap && l.listed && !overflowed)
         return kvsmc::launch_emit_pairs(l.dtype, d_groups + l.g0, l.ng, l.netasks, d_isos, list, d_unit_offsets,
                                         d_plane_base, d_status, d_next + 2 * i + 1, L, 0, d_fit);
-    return kvsmc::launch_stream(true, l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts,
-                                d_unit_offsets, d_plane_base, d_status, d_next + 2 * i + 1, L, l.ctas_per_sm, 0, nullptr,
-                                d_fit);
+    return kvsmc::launch_stream_emit(l.dtype, l.rows, d_groups + l.g0, l.ng, l.ntasks, d_isos, d_unit_counts,
+                                      d_unit_offsets, d_plane_base, d_status, d_next + 2 * i + 1, L, l.ctas_per_sm, 0,
+                                      d_fit);
 }
 
 kvsmc_status StreamBatch::emit_enqueue(const uint64_t* d_fit)
@@ -593,9 +590,9 @@ kvsmc_status StreamBatch::emit_parts(int parts, const std::function<kvsmc_status
                                                      d_unit_offsets, d_plane_base, d_status, d_next_parts + p, L,
                                                      (uint64_t)z0 * g.eblocks, nullptr));
         else
-            KVSMC_CUDA(ctx, kvsmc::launch_stream(true, l.dtype, l.rows, d_groups, 1, c1 * per_chunk, d_isos,
-                                                 d_unit_counts, d_unit_offsets, d_plane_base, d_status,
-                                                 d_next_parts + p, L, l.ctas_per_sm, c0 * per_chunk));
+            KVSMC_CUDA(ctx, kvsmc::launch_stream_emit(l.dtype, l.rows, d_groups, 1, c1 * per_chunk, d_isos,
+                                                      d_unit_counts, d_unit_offsets, d_plane_base, d_status,
+                                                      d_next_parts + p, L, l.ctas_per_sm, c0 * per_chunk));
         if ((st = after(z0, z1, false))) return st;
         c0 = c1;
     }

@@ -134,7 +134,7 @@ struct StreamBatch {
     cudaError_t count_kind(size_t i, const kvsmc::Launch& L);
     // One kind's emit: over the listed pairs, or classifying again.
     cudaError_t emit_kind(size_t i, const kvsmc::Launch& L, const uint64_t* d_fit);
-    // The emit launches; d_fit: see launch_stream's d_totals.
+    // The emit launches; d_fit: see launch_stream_emit's d_totals.
     kvsmc_status emit_enqueue(const uint64_t* d_fit);
     // The scans behind a count: unit offsets, plane bases, totals.
     cudaError_t scans(const kvsmc::Launch& L);

@@ -87,6 +87,7 @@ struct Job {
     float* tri_normals;
     uint32_t* vcount;         // triangles per vertex
     uint32_t* vlist;          // their ids, slot-major (slot s of vertex v at s * nvert + v)
+    uint2* slots;             // over listed pairs instead: the vertices' slots (node emit zeroes the faces')
 };
 
 // ------------------------------------------------------------------- values

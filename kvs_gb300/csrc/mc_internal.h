@@ -158,36 +158,37 @@ struct IngestOut {
 // src: the values, dense, copied into v's layout (null: they are in place).
 cudaError_t launch_ingest(const VolumeView& v, const void* src, float2* bricks, IngestOut* d_out, const Launch& L);
 
-size_t stream_shared_bytes(int dtype, bool emit, int rows);
-size_t stream_warp_smem_bytes(int dtype, bool emit, int rows);
+size_t stream_shared_bytes(int dtype, int rows);
+size_t stream_warp_smem_bytes(int dtype, int rows);
 size_t stream_warp_smem_offset();
 size_t stream_row_elems(int dtype, int rows);
+// The emit that classifies the volume again.
 // d_next_task: a zeroed u64 per launch (the persistent warps' task counter).
-// d_unit_counts: written by the count launch; read by the emit launch to skip
-// steps without triangles.  ctas_per_sm: resident CTAs per SM of the
-// persistent grid (0: as many as fit; never more than fit).  The launch runs
-// the warp tasks [task0, ntasks) of its groups (task0 > 0: a later part of a
-// launch split by z-chunks).  d_totals (emit): per isolevel record its
-// triangles; a request whose total exceeds its cap_tris writes nothing (null:
-// each request writes up to its cap_tris).  The emit writes nothing when the
-// status word says that the count gave up.
-// d_only_if (emit): the launch does nothing when this word is zero.
-cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
-                          const StreamIso* d_isos, uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
-                          const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
-                          const Launch& L, int ctas_per_sm = 0, uint64_t task0 = 0,
-                          uint32_t* d_node_counts = nullptr, const uint64_t* d_totals = nullptr,
-                          const int* d_only_if = nullptr);
+// d_unit_counts: the count's, read to skip steps without triangles.
+// ctas_per_sm: resident CTAs per SM of the persistent grid (0: as many as fit;
+// never more than fit).  The launch runs the warp tasks [task0, ntasks) of its
+// groups (task0 > 0: a later part of a launch split by z-chunks).  d_totals:
+// per isolevel record its triangles; a request whose total exceeds its
+// cap_tris writes nothing (null: each request writes up to its cap_tris).
+// Nothing is written when the status word says that the count gave up, or when
+// the word at d_only_if is zero.
+cudaError_t launch_stream_emit(int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
+                               const StreamIso* d_isos, const uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
+                               const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
+                               const Launch& L, int ctas_per_sm = 0, uint64_t task0 = 0,
+                               const uint64_t* d_totals = nullptr, const int* d_only_if = nullptr);
 // The count of launches whose groups hold one isolevel each, any value type
-// (mc_one.cu); same outputs as launch_stream's.
+// (mc_one.cu): triangles per (unit, isolevel), and with a list the pairs.
 cudaError_t launch_count_one(int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
                              const StreamIso* d_isos, uint16_t* d_unit_counts, int* d_status,
                              unsigned long long* d_next_task, const Launch& L, const PairList* list);
 // The count of launches with several isolevels a volume, the narrow types
-// (mc_many.cu); same outputs.
+// (mc_many.cu); same outputs, and the vertices of the groups' node units when
+// d_node_counts is given (one row per task).
 cudaError_t launch_count_many(int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
                               const StreamIso* d_isos, uint16_t* d_unit_counts, int* d_status,
-                              unsigned long long* d_next_task, const Launch& L, int ctas_per_sm, const PairList* list);
+                              unsigned long long* d_next_task, const Launch& L, int ctas_per_sm, const PairList* list,
+                              uint32_t* d_node_counts);
 // The emit over the pairs that the count listed: same outputs, same rules for status and totals; does nothing when the list
 // overflowed.  Tasks: the groups' blocks of units.
 cudaError_t launch_emit_pairs(int dtype, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
@@ -195,7 +196,7 @@ cudaError_t launch_emit_pairs(int dtype, const StreamGroup* d_groups, int ngroup
                               const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
                               const Launch& L, uint64_t task0, const uint64_t* d_totals);
 // The emit launch for the 32/64-bit integer and double volumes (one isolevel
-// per group, one row per task); launch_stream calls it for them.
+// per group, one row per task); launch_stream_emit calls it for them.
 cudaError_t launch_wide(int dtype, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
                         const StreamIso* d_isos, const uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
                         const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task, const Launch& L,
@@ -237,6 +238,7 @@ struct NodeIso {
     uint4* rank;                // its rank words (nz * ny * words_per_row)
     const uint64_t* offsets;    // per node unit: its first vertex id + offsets[0]
     const uint32_t* counts;     // per node unit: its vertices
+    uint2* slots;               // vertex normals over listed pairs: its vertices' slots (null: none)
 };
 size_t snode_multi_shared_bytes(int dtype);
 
@@ -244,13 +246,38 @@ size_t snode_multi_shared_bytes(int dtype);
 // streaming count group, in its isolevel order).
 struct ConnIso {
     const uint4* rank;       // its rank words
-    const float* coords;     // its vertices
+    float* coords;           // its vertices
     uint32_t* connections;   // its triangles' vertex ids
     float* tri_out;          // polygon normals, or the per-triangle normals its vertex normals sum
     uint64_t nvert, ntri;
     uint32_t enabled;        // 0: nothing of it is written
     uint32_t pad;
+    // over listed pairs, vertex normals instead of tri_out: per triangle its
+    // normal, per vertex the triangles of its four cells (see VertexSlots)
+    float4* tri4;
+    uint2* slots;
 };
+struct ConnTable {
+    ConnIso iso[kStreamMaxIso];
+};
+// connect_isopoints over the pairs that streaming count group d_group listed
+// (mc_connect.cu), for its enabled requests; ntasks: the group's blocks of
+// units.  Same outputs and rules as launch_sconnect_multi.
+cudaError_t launch_connect_pairs(const StreamGroup* d_group, const StreamIso* d_isos, const ConnTable& conn, int dtype,
+                                 uint32_t words_per_row, const PairList& list, const uint32_t* unit_offsets,
+                                 const uint64_t* plane_base, uint64_t ntasks, int* status,
+                                 unsigned long long* next_task, const Launch& L);
+// The vertex normals from what it left: a vertex on an edge has four slots,
+// one for each cell around the edge in z, y, x order (zero where there is no
+// cell: the node emit writes those of the volume's faces), of the cell's first
+// triangle and, as bits, which of its triangles use the edge.
+struct VertexSlots {
+    float4* tri4;
+    uint2* slots;
+};
+size_t vertex_slots_bytes(uint64_t ntri, uint64_t nvert);
+VertexSlots vertex_slots_carve(uint64_t ntri, uint64_t nvert, void* scratch);
+cudaError_t launch_vertex_slots(const VertexSlots& v, uint64_t ntri, uint64_t nvert, float* normals, const Launch& L);
 size_t sconnect_multi_shared_bytes(int dtype);
 // The connection pass of every enabled request of streaming count group
 // d_group (one-row tasks) at once: the group's tasks, its counters and scans.

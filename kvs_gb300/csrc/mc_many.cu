@@ -1,6 +1,6 @@
 // mc_many.cu -- the count pass for several isolevels of a volume at once
 // (8/16-bit and float32 values): triangles per (unit, isolevel) and, with a
-// list, the active (cell, isolevel) pairs for the emit of mc_pairs.cu.
+// list, the active (cell, isolevel) pairs for mc_pairs.cu and mc_connect.cu.
 //
 // Tasks, units and threshold masks are the streaming kernels' (mc_stream.cu,
 // mc_thermo.cuh): a warp walks a chunk of cell planes of R cell rows, lane l on
@@ -22,6 +22,12 @@
 // an SM (64 registers, 56 KB) instead of three: 1% and 3%.  640x704x600 f32, 16
 // isolevels: 1532 us with the lanes' loops, 1500 us; 1024x768x640 u16, 4
 // isolevels: 2735 -> 2312 us.
+//
+// NODES: the shared-vertex modes' vertices per node unit too (plane, node row,
+// 256-node segment; those whose node segments are their cell segments).  A
+// node's cut edges are its cell's lower ones, so a pair adds them to its key
+// beside its triangles; the last cell of a row, the last row and the last plane
+// add the nodes behind them.
 #include <cuda_runtime.h>
 
 #include "mc_internal.h"
@@ -48,23 +54,29 @@ template <int R> constexpr uint32_t kMaskRow = 256 / R + 8;
 template <int R> struct alignas(16) ManyWarp {
     uint16_t mask[2][R + 1][kMaskRow<R>];   // node masks of the lower and the upper plane (plane & 1)
     uint16_t buf[kManyBuf];                 // cell in the warp (8 bits) | isolevel << 8
-    uint32_t cnt[32];                       // triangles of the current units, [row][isolevel]
+    // [row][isolevel]: triangles | vertices << 16 of the current units; with
+    // vertices (R = 1) 16 + k: those of the node units past the last cell row,
+    // past the last cell plane and past both, 10 bits each
+    uint32_t cnt[32];
     uint64_t bar[2];
     ThermoTables th;
 };
 
-template <typename T, int R, bool LIST>
+template <typename T, int R, bool LIST, bool NODES>
 __global__ void __launch_bounds__(kManyThreads, 4)
     k_count_many(const StreamGroup* __restrict__ groups, int ngroups, uint64_t ntasks,
                  const StreamIso* __restrict__ isos, uint16_t* __restrict__ unit_counts, int* __restrict__ status,
-                 unsigned long long* __restrict__ next_task, uint32_t wait_polls, PairList pl)
+                 unsigned long long* __restrict__ next_task, uint32_t wait_polls, PairList pl,
+                 uint32_t* __restrict__ node_counts)
 {
+    static_assert(!NODES || R == 1, "node units are one row");
     constexpr int LPR = 32 / R;                     // lanes per cell row
     constexpr uint32_t SEG = kStreamSegCells / R;   // cells per row segment
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ uint8_t s_ntri[256];   // by corner code
+    __shared__ uint8_t s_tab[256];   // by corner code: triangles | the lower node's cut edges << 3
     const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    s_ntri[tid] = d_many_ntri[code_to_case(tid)];
+    s_tab[tid] = (uint8_t)(d_many_ntri[code_to_case(tid)] |
+                           ((((tid ^ (tid >> 4)) & 1u) + ((tid ^ (tid >> 1)) & 1u) + ((tid ^ (tid >> 2)) & 1u)) << 3));
     __syncthreads();   // the only CTA-wide barrier
     const uint32_t row_elems = groups[0].seg_elems;
     const uint32_t plane_elems = (R + 1) * row_elems;
@@ -163,6 +175,12 @@ __global__ void __launch_bounds__(kManyThreads, 4)
             unit_counts + G.unit_base + (((uint64_t)z0 * cy + y + ch) * wpr + seg) * (uint32_t)niso + ck;
         uint16_t* upairs = LIST ? pl.unit_pairs + G.pair_base + unit0 : nullptr;
         uint32_t* ulist = LIST ? pl.unit_list + G.pair_base + unit0 : nullptr;
+        // with vertices: lane k's counter of isolevel k's node unit at plane z0
+        const bool last_row = y + 1 == cy;
+        const uint64_t plane_nodes = (uint64_t)G.vol.ny * wpr;
+        uint32_t* const ncount = NODES && G.node_units ? node_counts + G.node_base + lane * G.node_units +
+                                                             ((uint64_t)z0 * G.vol.ny + y) * wpr + seg
+                                                       : nullptr;
         const int lim = row_ok ? (int)cx - (int)((uint32_t)xoff + xl) : 0;   // this lane's cells inside the volume (if < 8)
         // masks of this lane's nodes in rows half and half + 1 of plane i, in
         // registers and in the plane's mask rows
@@ -296,19 +314,48 @@ __global__ void __launch_bounds__(kManyThreads, 4)
                     a += kMaskRow<R>;
                     b += kMaskRow<R>;
                     const uint32_t w1 = a[0] | ((uint32_t)a[1] << 16), w3 = b[0] | ((uint32_t)b[1] << 16);
-                    const uint32_t nt = has ? s_ntri[case_code(w0, w1, w2, w3, k)] : 0u;
+                    const uint32_t code = case_code(w0, w1, w2, w3, k);
+                    const uint32_t tab = has ? s_tab[code] : 0u, nt = tab & 7u;
                     const uint32_t key = R == 1 ? k : h * 16 + k;
                     const uint32_t grp = __match_any_sync(FULL, has ? key : 32u + lane);
                     uint32_t sum = 0;
 #pragma unroll
                     for (int bit = 0; bit < 3; ++bit)
                         sum += (uint32_t)__popc(__ballot_sync(FULL, (nt >> bit) & 1u) & grp) << bit;
+                    if (NODES) {
+                        // the cut edges of the cell's lower node, and in the row's last cell
+                        // of the node behind it
+                        uint32_t nv = tab >> 3;
+                        const bool last = has && xoff + x == cx - 1;
+                        if (last) nv += (((code >> 4) ^ (code >> 5)) & 1u) + (((code >> 4) ^ (code >> 6)) & 1u);
+#pragma unroll
+                        for (int bit = 0; bit < 3; ++bit)
+                            sum += (uint32_t)__popc(__ballot_sync(FULL, (nv >> bit) & 1u) & grp) << (16 + bit);
+                        if (has && (last_row || z + 1 == cz)) {
+                            auto cut = [&](int i, int j) -> uint32_t { return ((code >> i) ^ (code >> j)) & 1u; };
+                            uint32_t v = 0;
+                            if (last_row) v += cut(1, 5) + cut(1, 3) + (last ? cut(5, 7) : 0u);
+                            if (z + 1 == cz) v += (cut(2, 6) + cut(2, 3) + (last ? cut(6, 7) : 0u)) << 10;
+                            if (last_row && z + 1 == cz) v += cut(3, 7) << 20;
+                            if (v) atomicAdd(&W.cnt[16 + k], v);
+                        }
+                    }
                     if (has && (grp & lt) == 0) W.cnt[key] += sum;   // one lane per distinct key
                     __syncwarp();
                 }
             }
             lcur += npairs;
-            if (my_count) ucount[(uint64_t)s * plane_units * (uint32_t)niso] = (uint16_t)W.cnt[lane];
+            if (my_count) {
+                ucount[(uint64_t)s * plane_units * (uint32_t)niso] = (uint16_t)W.cnt[lane];
+                if (NODES && ncount) {
+                    ncount[s * plane_nodes] = W.cnt[lane] >> 16;
+                    const uint32_t v = W.cnt[16 + lane];
+                    if (last_row) ncount[s * plane_nodes + wpr] = v & 0x3ffu;
+                    if (z + 1 == cz) ncount[(s + 1) * plane_nodes] = (v >> 10) & 0x3ffu;
+                    if (last_row && z + 1 == cz) ncount[(s + 1) * plane_nodes + wpr] = v >> 20;
+                }
+            }
+            __syncwarp();
             W.cnt[lane] = 0;
             __syncwarp();
         }
@@ -335,17 +382,19 @@ __global__ void __launch_bounds__(kManyThreads, 4)
 
 cudaError_t launch_count_many(int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
                               const StreamIso* d_isos, uint16_t* d_unit_counts, int* d_status,
-                              unsigned long long* d_next_task, const Launch& L, int ctas_per_sm, const PairList* list)
+                              unsigned long long* d_next_task, const Launch& L, int ctas_per_sm, const PairList* list,
+                              uint32_t* d_node_counts)
 {
     if (ntasks == 0) return cudaSuccess;
-    if (rows != 1 && rows != 2) return cudaErrorInvalidValue;
+    if (rows != 1 && (rows != 2 || d_node_counts)) return cudaErrorInvalidValue;
     const size_t warp = many_align(rows == 1 ? sizeof(ManyWarp<1>) : sizeof(ManyWarp<2>)) +
                         many_align(2 * (size_t)(rows + 1) * stream_row_elems(dtype, rows) * dtype_size(dtype));
     const size_t smem = kManyWarps * warp;
     const uint64_t need = (ntasks + kManyWarps - 1) / kManyWarps;
     KVSMC_MANY_SWITCH(dtype, {
-        auto kern = rows == 1 ? (list ? k_count_many<T, 1, true> : k_count_many<T, 1, false>)
-                              : (list ? k_count_many<T, 2, true> : k_count_many<T, 2, false>);
+        auto kern = d_node_counts ? (list ? k_count_many<T, 1, true, true> : k_count_many<T, 1, false, true>)
+                    : rows == 1   ? (list ? k_count_many<T, 1, true, false> : k_count_many<T, 1, false, false>)
+                                  : (list ? k_count_many<T, 2, true, false> : k_count_many<T, 2, false, false>);
         int per_sm = 0;
         const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), kManyThreads, smem, &per_sm, true);
         if (e != cudaSuccess) return e;
@@ -354,7 +403,7 @@ cudaError_t launch_count_many(int dtype, int rows, const StreamGroup* d_groups, 
         prof_begin(L, "count_many");
         kern<<<(unsigned)(need < resident ? need : resident), kManyThreads, smem, L.stream>>>(
             d_groups, ngroups, ntasks, d_isos, d_unit_counts, d_status, d_next_task, L.wait_polls[0],
-            list ? *list : PairList{});
+            list ? *list : PairList{}, d_node_counts);
         prof_end(L);
     });
     *L.counter += 1;

@@ -38,7 +38,7 @@
 #include "mc_emit.cuh"
 #include "mc_internal.h"
 #include "mc_interp.cuh"
-#include "mc_tables.h"
+#include "mc_pairs.cuh"
 #include "tma.cuh"
 
 #ifndef KVSMC_PAIRS_CTAS
@@ -49,67 +49,7 @@ namespace kvsmc {
 
 namespace {
 
-constexpr int kPairThreads = 256;
-constexpr int kPairWarps = kPairThreads / 32;
-constexpr int kPairVerts = 192;          // vertex items of one round
-constexpr unsigned FULL = 0xffffffffu;
-
-// Case tables indexed by the corner code (bit r: row r's node i above, rows
-// (y, z) (y+1, z) (y, z+1) (y+1, z+1); bit 4 + r: its node i + 1), laid out
-// at compile time and copied into shared memory by one bulk copy per CTA.
-struct alignas(16) PairTables {
-    uint64_t tri_slots[256];   // per triangle corner: its edge's rank among the used edges, 4 bits each
-    uint8_t edges[256][12];    // the used edges in increasing order: corner A | corner B << 3 | axis << 6
-                               // (corner: dx + 2 dy + 4 dz)
-    uint8_t counts[256];       // triangles | used edges << 3
-};
-static_assert(sizeof(PairTables) % 16 == 0, "copied by a bulk copy");
-
-constexpr uint64_t h_tri[256] = MC_TRI_PACKED_INIT;
-constexpr uint8_t h_ntri[256] = MC_NTRI_INIT;
-constexpr uint16_t h_mask[256] = MC_EDGE_MASK_INIT;
-constexpr uint8_t h_edge[12] = MC_EDGE_PACKED_INIT;
-
-constexpr uint32_t h_case(uint32_t c)
-{
-    return (c & 1u) | (((c >> 4) & 1u) << 1) | (((c >> 5) & 1u) << 2) | (((c >> 1) & 1u) << 3) |
-           (((c >> 2) & 1u) << 4) | (((c >> 6) & 1u) << 5) | (((c >> 7) & 1u) << 6) | (((c >> 3) & 1u) << 7);
-}
-
-constexpr PairTables make_tables()
-{
-    PairTables t{};
-    for (uint32_t code = 0; code < 256; ++code) {
-        const uint32_t cs = h_case(code), em = h_mask[cs];
-        int n = 0;
-        for (uint32_t e = 0; e < 12; ++e)
-            if ((em >> e) & 1u) {
-                const uint32_t c0 = h_edge[e] & 7u, c1 = h_edge[e] >> 3, d = c0 ^ c1;
-                t.edges[code][n++] = (uint8_t)(c0 | (c1 << 3) | ((d == 1u ? 0u : (d == 2u ? 1u : 2u)) << 6));
-            }
-        t.counts[code] = (uint8_t)(h_ntri[cs] | (n << 3));
-        for (int c = 0; c < 3 * (int)h_ntri[cs]; ++c) {
-            const uint32_t e = (uint32_t)(h_tri[cs] >> (4 * c)) & 15u;
-            uint64_t rank = 0;
-            for (uint32_t b = 0; b < e; ++b) rank += (em >> b) & 1u;
-            t.tri_slots[code] |= rank << (4 * c);
-        }
-    }
-    return t;
-}
-
-__device__ PairTables d_pair_tables = make_tables();
-
-// Value types that are floats exactly take the FP32 certificate; the others
-// keep their corner values as doubles and take the FP64 sequence.
-template <typename T> constexpr bool kPairFast = sizeof(T) < 4;
-template <> constexpr bool kPairFast<float> = true;
-template <typename T> struct PairValue { using type = double; };
-template <> struct PairValue<float> { using type = float; };
-template <> struct PairValue<int8_t> { using type = float; };
-template <> struct PairValue<uint8_t> { using type = float; };
-template <> struct PairValue<int16_t> { using type = float; };
-template <> struct PairValue<uint16_t> { using type = float; };
+__device__ PairTables d_pair_tables = make_pair_tables();
 
 struct alignas(16) PairOut {
     float* coords;
@@ -176,35 +116,15 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
             gcur = gi;
         }
         if (!live) continue;
-        const uint32_t cy = G.vol.ny - 1, wpr = G.wpr, ub = G.eblock;
-        const uint32_t local = (uint32_t)(task - G.etask_begin);
-        const uint32_t z = local / G.eblocks, u0 = (local - z * G.eblocks) * ub;   // first unit in the plane
-        const uint32_t plane_units = cy * wpr;
-        // lane u: unit u0 + u's pairs and where they are listed
-        uint32_t np = 0, first = 0;
-        const uint32_t un = u0 + lane;
-        if (lane < ub && un < plane_units) {
-            const uint64_t pu = G.pair_base + (uint64_t)z * plane_units + un;
-            np = pl.unit_pairs[pu];
-            if (np) first = pl.unit_list[pu];
-        }
-        uint32_t inc = np;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(FULL, inc, o);
-            if (lane >= (unsigned)o) inc += t;
-        }
-        const uint32_t npairs = __shfl_sync(FULL, inc, 31);
-        if (npairs == 0) continue;
-        first -= inc - np;   // entry of pair p of this unit: list[first + p]
-        const uint32_t uy = un / wpr;
-        const uint32_t ux = (un - uy * wpr) * G.seg_cells;
+        const PairBlock B = pair_block(G, pl, (uint32_t)(task - G.etask_begin), lane);
+        if (B.npairs == 0) continue;
+        const uint32_t z = B.z;
         // per isolevel: where the task's first triangle goes and how many fit
         __syncwarp();
         if (lane < (unsigned)niso) {
             const uint64_t pi = isos[iso_begin + lane].plane_index;
             const uint64_t at = plane_base[pi + z] - plane_base[pi] +
-                                unit_offsets[G.unit_base + ((uint64_t)z * plane_units + u0) * niso + lane];
+                                unit_offsets[G.unit_base + ((uint64_t)z * ((G.vol.ny - 1) * G.wpr) + B.u0) * niso + lane];
             const IsoConst& c = W.ic[lane];
             W.out[lane] = PairOut{c.coords + 9 * at, c.normals + 3 * at};
             W.room[lane] = !c.coords || c.cap_tris <= at ? 0u
@@ -216,42 +136,20 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
         const T* vz = static_cast<const T*>(G.vol.data) + (uint64_t)z * slice;
         const float fz = __uint2float_rn(z);
         uint32_t taken = 0;
-        for (uint32_t r0 = 0; r0 < npairs; r0 += taken) {
+        for (uint32_t r0 = 0; r0 < B.npairs; r0 += taken) {
             // ---- one pair per lane, as many as the vertex pool holds
-            const uint32_t p = r0 + lane;
-            bool has = p < npairs;
-            uint32_t own = 0;   // its unit: the first lane whose inclusive count exceeds p
-#pragma unroll
-            for (int s = 4; s >= 0; --s) {
-                const uint32_t mid = own + (1u << s) - 1u;
-                if (__shfl_sync(FULL, inc, mid) <= p) own = mid + 1;
-            }
-            own &= 31u;   // (lanes past the last pair)
-            const uint32_t at = __shfl_sync(FULL, first, own) + p;
-            const uint32_t y = __shfl_sync(FULL, uy, own);
-            uint32_t x = __shfl_sync(FULL, ux, own);
+            bool has = r0 + lane < B.npairs;
+            uint32_t x, y;
+            const uint32_t at = pair_entry(B, r0 + lane, x, y);
             uint32_t k = 0, code = 0;
             if (has) {
                 const uint32_t e = pl.list[at];
                 x += e & 0xffu;
                 k = e >> 8;
-                const T* c = vz + (uint64_t)y * pitch + x;
-                const T v0 = __ldg(c), v1 = __ldg(c + 1), v2 = __ldg(c + pitch), v3 = __ldg(c + pitch + 1);
-                const T v4 = __ldg(c + slice), v5 = __ldg(c + slice + 1);
-                const T v6 = __ldg(c + slice + pitch), v7 = __ldg(c + slice + pitch + 1);
-                auto up = [&](T v) -> bool {
+                code = pair_corners<T, V>(vz + (uint64_t)y * pitch + x, pitch, slice, W.cv[lane], [&](T v) -> bool {
                     if constexpr (kPairFast<T>) return (float)v > W.ic[k].f.f_thr;
                     else return above(isos[iso_begin].cls, v);   // (one isolevel per group)
-                };
-                auto val = [&](T v) -> V {
-                    if constexpr (kPairFast<T>) return (float)v;
-                    else return to_double(v);
-                };
-                V* cv = W.cv[lane];
-                cv[0] = val(v0); cv[1] = val(v1); cv[2] = val(v2); cv[3] = val(v3);
-                cv[4] = val(v4); cv[5] = val(v5); cv[6] = val(v6); cv[7] = val(v7);
-                code = (up(v0) ? 1u : 0u) | (up(v2) ? 2u : 0u) | (up(v4) ? 4u : 0u) | (up(v6) ? 8u : 0u) |
-                       (up(v1) ? 16u : 0u) | (up(v3) ? 32u : 0u) | (up(v5) ? 64u : 0u) | (up(v7) ? 128u : 0u);
+                });
             }
             const uint32_t cnt = has ? TB.counts[code] : 0u;
             const uint32_t ne0 = cnt >> 3;

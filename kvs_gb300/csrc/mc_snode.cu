@@ -63,6 +63,17 @@ constexpr unsigned FULL = 0xffffffffu;
 
 __host__ __device__ __forceinline__ size_t sn_align(size_t v) { return (v + 127) / 128 * 128; }
 
+// A vertex of a node on the volume's faces may lack cells around its edge: its
+// slots start from zero (the connection pass writes the ones there are).
+__device__ __forceinline__ void clear_face_slots(uint2* slots, uint64_t id, uint32_t x, uint32_t y, uint32_t z,
+                                                 uint32_t nx, uint32_t ny, uint32_t nz)
+{
+    if (x != 0 && y != 0 && z != 0 && x + 1 != nx && y + 1 != ny && z + 1 != nz) return;
+    uint4* s = reinterpret_cast<uint4*>(slots + 4 * id);
+    s[0] = make_uint4(0, 0, 0, 0);
+    s[1] = make_uint4(0, 0, 0, 0);
+}
+
 template <typename T, bool EMIT>
 __global__ void __launch_bounds__(kSnThreads, EMIT ? KVSMC_SNODE_EMIT_CTAS : 1)
     k_snode(Job j, FastIso f, uint32_t wprn, uint32_t zchunk, uint64_t ntasks, uint32_t row_elems,
@@ -253,6 +264,7 @@ __global__ void __launch_bounds__(kSnThreads, EMIT ? KVSMC_SNODE_EMIT_CTAS : 1)
                                                    axis);
                     float* o = j.coords + 3 * (base + q);
                     o[0] = p.x; o[1] = p.y; o[2] = p.z;
+                    if (j.slots) clear_face_slots(j.slots, base + q, (uint32_t)xoff + xl, y, z, nx, ny, nz);
                 }
             }
             // plane z is consumed: refill its buffer with plane z + 3
@@ -519,6 +531,7 @@ __global__ void __launch_bounds__(kSnThreads, KVSMC_SNODE_MULTI_CTAS)
                     const float3 p = edge_vertex_fast(I.ip, I.f, v0, v1, ax, fyf, fzf, bxf, byf, bzf, axis);
                     float* o = I.coords + 3 * (M.base[m] + r0q);
                     o[0] = p.x; o[1] = p.y; o[2] = p.z;
+                    if (I.slots) clear_face_slots(I.slots, M.base[m] + r0q, (uint32_t)xoff + xl, y, z, nx, ny, nz);
                 }
             }
             // plane z is consumed: refill its buffer with plane z + 3

@@ -1,9 +1,8 @@
-// mc_stream.cu -- the streaming layout's kernels that classify the volume
-// themselves: the shared-vertex modes' count (triangles and vertices in one
-// pass), the duplicated mode's emit for requests whose crossed cells could not
-// all be listed and for extractions without a list, and the unit scan.  The
-// duplicated mode counts in mc_one.cu and mc_many.cu and emits in mc_pairs.cu
-// on the same tasks and units.
+// mc_stream.cu -- the streaming layout's emit that classifies the volume itself
+// (for requests whose crossed cells could not all be listed, and for
+// extractions without a list) and the unit scan.  The counts are in mc_one.cu
+// and mc_many.cu, the emit over listed pairs in mc_pairs.cu, on the same tasks
+// and units.
 //
 // Work decomposition: every warp is an independent worker.
 //   * A warp task = (volume, z-chunk, cell row y, 256-cell x-segment).  The
@@ -62,7 +61,6 @@ namespace kvsmc {
 
 namespace {
 
-constexpr int kWarps = kStreamThreads / 32;
 constexpr int kEmitThreads = 32 * KVSMC_EMIT_WARPS;
 constexpr int kEmitWarps = KVSMC_EMIT_WARPS;
 constexpr int kLaneCells = 8;
@@ -108,7 +106,6 @@ static_assert(3 * 3 * (kSegCells + 16) < (1 << 14), "edge_off packs ring offsets
 struct WarpState {
     uint64_t bar[3];
     ThermoTables th;
-    uint32_t cnt[32];                        // count: triangles of the current units, [row][isolevel]
     uint32_t add[32];                        // emit: per-(row, isolevel) advance of the current round
 };
 
@@ -200,24 +197,14 @@ __device__ __forceinline__ int find_group(const StreamGroup* groups, int ngroups
 // so warps that skip empty tasks go on at once instead of idling in a CTA
 // whose other warps still run.  Tasks come out in increasing order; the
 // group's isolevel tables are rebuilt when a warp crosses a group boundary.
-//
-// The count (one row per task) is the shared-vertex modes': it also counts, per
-// isolevel, the vertices of their node units (plane, node row,
-// 256-node segment): the cut x, y and z edges from each node to its upper
-// neighbours, the edges whose two ends' threshold masks differ.  A task of
-// cell row y counts node row y at its planes; on the last cell row also node
-// row y + 1, on the last cell plane also the last node plane.  Groups with
-// node_units == 0 are not counted.
-template <typename T, bool EMIT, int R>
-__global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? KVSMC_EMIT_CTAS : 3)
+template <typename T, int R>
+__global__ void __launch_bounds__(kEmitThreads, KVSMC_EMIT_CTAS)
     k_stream(const StreamGroup* __restrict__ groups, int ngroups, uint64_t ntasks, const StreamIso* __restrict__ isos,
-             uint16_t* __restrict__ unit_counts, const uint32_t* __restrict__ unit_offsets,
+             const uint16_t* __restrict__ unit_counts, const uint32_t* __restrict__ unit_offsets,
              const uint64_t* __restrict__ plane_base, int* __restrict__ status,
              unsigned long long* __restrict__ next_task, uint32_t wait_polls, uint64_t task0,
-             uint32_t* __restrict__ node_counts, const uint64_t* __restrict__ totals,
-             const int* __restrict__ only_if)
+             const uint64_t* __restrict__ totals, const int* __restrict__ only_if)
 {
-    static_assert(EMIT || R == 1, "node counts come from one-row count tasks");
     constexpr int LPR = 32 / R;                 // lanes per cell row
     constexpr int SEG = kSegCells / R;          // cells per row segment
     constexpr int SEG_SHIFT = R == 1 ? 8 : 7;   // log2(SEG)
@@ -234,21 +221,19 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
         TB.ntri[code] = c_ntri[cs];
         const uint32_t em = c_edge_mask[cs];
         TB.edge_mask[code] = (uint16_t)em;
-        if (EMIT) {
-            uint64_t list = 0;
-            int n = 0;
-            for (int e = 0; e < 12; ++e)
-                if ((em >> e) & 1u) list |= (uint64_t)e << (4 * n++);
-            TB.edge_list[code] = list;
-            const uint64_t tp = c_tri_packed[cs];
-            uint64_t slots = 0;
-            for (int c = 0; c < 3 * (int)c_ntri[cs]; ++c) {
-                const uint32_t e = (uint32_t)(tp >> (4 * c)) & 15u;
-                slots |= (uint64_t)__popc(em & ((1u << e) - 1u)) << (4 * c);
-            }
-            TB.tri_slots[code] = slots;
+        uint64_t list = 0;
+        int n = 0;
+        for (int e = 0; e < 12; ++e)
+            if ((em >> e) & 1u) list |= (uint64_t)e << (4 * n++);
+        TB.edge_list[code] = list;
+        const uint64_t tp = c_tri_packed[cs];
+        uint64_t slots = 0;
+        for (int c = 0; c < 3 * (int)c_ntri[cs]; ++c) {
+            const uint32_t e = (uint32_t)(tp >> (4 * c)) & 15u;
+            slots |= (uint64_t)__popc(em & ((1u << e) - 1u)) << (4 * c);
         }
-        if (EMIT && code < 36) {
+        TB.tri_slots[code] = slots;
+        if (code < 36) {
             const uint32_t e = code % 12u, ph = code / 12u;
             const uint32_t ep = c_edge_packed[e], c0 = ep & 7u, c1 = ep >> 3, d = c0 ^ c1;
             const uint32_t axis = d == 1u ? 0u : (d == 2u ? 1u : 2u);
@@ -264,19 +249,18 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
     }
     // the only CTA-wide barrier: tables are read-only from here on (an emit
     // whose count gave up has no offsets to write at)
-    if (__syncthreads_or(EMIT && (*status != 0 || (only_if && *only_if == 0)))) return;
+    if (__syncthreads_or(*status != 0 || (only_if && *only_if == 0))) return;
 
-    const size_t wstride = align128(sizeof(WarpState)) + (EMIT ? align128(sizeof(WarpEmit)) : 0) +
+    const size_t wstride = align128(sizeof(WarpState)) + align128(sizeof(WarpEmit)) +
                            align128((size_t)3 * plane_elems * sizeof(T));
     unsigned char* wbase = smem_raw + align128(sizeof(Tables)) + (size_t)warp * wstride;
     WarpState& W = *reinterpret_cast<WarpState*>(wbase);
     WarpEmit* WE = reinterpret_cast<WarpEmit*>(wbase + align128(sizeof(WarpState)));
-    T* ring = reinterpret_cast<T*>(wbase + align128(sizeof(WarpState)) + (EMIT ? align128(sizeof(WarpEmit)) : 0));
+    T* ring = reinterpret_cast<T*>(wbase + align128(sizeof(WarpState)) + align128(sizeof(WarpEmit)));
     if (lane == 0) {
         for (int b = 0; b < 3; ++b) mbar_init(&W.bar[b], 1);
         fence_barrier_init();
     }
-    W.cnt[lane] = 0;
     W.add[lane] = 0;
     __syncwarp();
 
@@ -315,23 +299,21 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
     const uint32_t row_bytes = (uint32_t)(avail < G.seg_copy_bytes ? avail : G.seg_copy_bytes);
     const T* vol = static_cast<const T*>(G.vol.data);
 
-    if (EMIT && G.skip_emit) continue;   // nothing of this group is written in this launch
+    if (G.skip_emit) continue;   // nothing of this group is written in this launch
     if (gi != gcur) {
         // the group's thresholds and bucket table
         float t = 0.0f;
         if (lane < (unsigned)niso) {
             const StreamIso& I = isos[iso_begin + lane];
             t = I.f.f_thr;
-            if (EMIT) {
-                fill_iso(WE->ic[lane], I, totals, iso_begin + (int)lane);
-            }
+            fill_iso(WE->ic[lane], I, totals, iso_begin + (int)lane);
         }
-        if (EMIT) live = __any_sync(FULL, lane < (unsigned)niso && WE->ic[lane & 15u].coords != nullptr);
+        live = __any_sync(FULL, lane < (unsigned)niso && WE->ic[lane & 15u].coords != nullptr);
         __syncwarp();
         thermo_build(W.th, t, niso, bs, bo, lane);
         gcur = gi;
     }
-    if (EMIT && !live) continue;
+    if (!live) continue;
 
     // empty space: a brick whose node min and max have the same mask (no
     // threshold between them) holds no active cell for any isolevel
@@ -356,7 +338,7 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
     if (bricks) {
         bool all_empty = true;
         for (uint32_t z = z0; z < z1 && all_empty; z = (z / kBrickPlanes + 1) * kBrickPlanes) all_empty = brick_empty(z);
-        if (all_empty) continue;   // nothing to count or emit (counts are zeroed before the count pass)
+        if (all_empty) continue;   // nothing to emit
     }
 
     // plane i of this task goes to ring buffer i % 3
@@ -396,11 +378,11 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
     // emit: whether this lane's (row, isolevel) unit of step z has triangles,
     // loaded one step ahead so the load's latency hides behind a step's work
     const uint32_t uh = lane >> 4, uk = lane & 15u;
-    const bool u_lane = EMIT && uh < (uint32_t)R && uk < (uint32_t)niso && y + uh < cy;
+    const bool u_lane = uh < (uint32_t)R && uk < (uint32_t)niso && y + uh < cy;
     auto unit_nonzero = [&](uint32_t zz) -> bool {
         return u_lane && unit_counts[unit_base + (((uint64_t)zz * cy + y + uh) * wpr + seg) * niso + uk] != 0;
     };
-    bool next_any = EMIT ? unit_nonzero(z0) : false;
+    bool next_any = unit_nonzero(z0);
 
     for (uint32_t z = z0; z < z1; ++z) {
         const uint32_t s = z - z0;
@@ -426,12 +408,10 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
         const float fz = __uint2float_rn(z);
         if (bricks && (s == 0 || z % kBrickPlanes == 0)) brick_skip = brick_empty(z);
         bool skip = brick_skip;
-        if (EMIT) {
-            // the count pass found no triangle in this step's units: nothing to emit
-            const bool any = next_any;
-            next_any = z + 1 < z1 ? unit_nonzero(z + 1) : false;
-            if (!skip) skip = !__any_sync(FULL, any);
-        }
+        // the count pass found no triangle in this step's units: nothing to emit
+        const bool any = next_any;
+        next_any = z + 1 < z1 ? unit_nonzero(z + 1) : false;
+        if (!skip) skip = !__any_sync(FULL, any);
         if (skip) {
             pa_valid = false;
             __syncwarp();
@@ -478,76 +458,7 @@ __global__ void __launch_bounds__(EMIT ? kEmitThreads : kStreamThreads, EMIT ? K
 #pragma unroll
         for (int w = 0; w < 4; ++w) m += __popc(act[w]);
 
-        if (!EMIT) {
-            // count: one u16 per (unit, isolevel); counters [row][isolevel]
-            if (__any_sync(FULL, m != 0)) {
-#pragma unroll
-                for (int i = 0; i < kLaneCells; ++i) {
-                    uint32_t am = (act[i >> 1] >> (16 * (i & 1))) & 0xffffu;
-                    if (am) {
-                        const uint32_t w0 = cell_word(PA0, i), w1 = cell_word(PA1, i);
-                        const uint32_t w2 = cell_word(PB0, i), w3 = cell_word(PB1, i);
-                        do {
-                            const uint32_t k = __ffs(am) - 1;
-                            am &= am - 1;
-                            atomicAdd(&W.cnt[half * 16 + k], (uint32_t)TB.ntri[case_code(w0, w1, w2, w3, k)]);
-                        } while (am);
-                    }
-                }
-                __syncwarp();
-                if (G.node_units) {
-                    // (a node edge that is cut for isolevel k belongs to a cell active
-                    // for k, so a step without active cells has no vertices either)
-                    const int nlim = (int)G.vol.nx - (int)((uint32_t)xoff + xl);   // this lane's nodes in the row
-                    // vertices of node row (plane zn, row yn): masks Pn, and the rows
-                    // across its y edges (Py) and z edges (Pz) when it has them
-                    auto node_unit = [&](const uint32_t* Pn, const uint32_t* Py, const uint32_t* Pz, bool has_y,
-                                         bool has_z, uint32_t zn, uint32_t yn) {
-                        uint32_t X[4], Y[4], Z[4], U = 0;
-#pragma unroll
-                        for (int w = 0; w < 4; ++w) {
-                            // halves: nodes 2w (low) and 2w + 1 (high)
-                            const uint32_t vn = (2 * w < nlim ? 0xffffu : 0u) | (2 * w + 1 < nlim ? 0xffff0000u : 0u);
-                            const uint32_t vx =
-                                (2 * w + 1 < nlim ? 0xffffu : 0u) | (2 * w + 2 < nlim ? 0xffff0000u : 0u);
-                            X[w] = (Pn[w] ^ __funnelshift_r(Pn[w], Pn[w + 1], 16)) & vx;
-                            Y[w] = has_y ? (Pn[w] ^ Py[w]) & vn : 0u;
-                            Z[w] = has_z ? (Pn[w] ^ Pz[w]) & vn : 0u;
-                            U |= X[w] | Y[w] | Z[w];
-                        }
-                        uint32_t am = (U | (U >> 16)) & 0xffffu;
-                        if (!__any_sync(FULL, am != 0)) return;
-                        while (am) {
-                            const uint32_t k = __ffs(am) - 1;
-                            am &= am - 1;
-                            const uint32_t mk = 0x10001u << k;
-                            uint32_t c = 0;
-#pragma unroll
-                            for (int w = 0; w < 4; ++w) c += __popc(X[w] & mk) + __popc(Y[w] & mk) + __popc(Z[w] & mk);
-                            atomicAdd(&W.add[k], c);
-                        }
-                        __syncwarp();
-                        if (lane < (unsigned)niso) {
-                            const uint64_t un = ((uint64_t)zn * G.vol.ny + yn) * wpr + seg;
-                            node_counts[G.node_base + (uint64_t)lane * G.node_units + un] = W.add[lane];
-                            W.add[lane] = 0;
-                        }
-                        __syncwarp();
-                    };
-                    const bool last_row = y + 1 == cy, last_plane = z + 1 == cz;
-                    node_unit(PA0, PA1, PB0, true, true, z, y);
-                    if (last_row) node_unit(PA1, PA1, PB1, false, true, z, y + 1);
-                    if (last_plane) node_unit(PB0, PB1, PB0, true, false, z + 1, y);
-                    if (last_row && last_plane) node_unit(PB1, PB1, PB1, false, false, z + 1, y + 1);
-                }
-            }
-            const uint32_t h = lane >> 4, k = lane & 15u;
-            if (h < (uint32_t)R && k < (uint32_t)niso && y + h < cy) {
-                const uint64_t unit = ((uint64_t)z * cy + y + h) * wpr + seg;
-                unit_counts[unit_base + unit * niso + k] = (uint16_t)W.cnt[lane];
-                W.cnt[lane] = 0;
-            }
-        } else {
+        {
             // ---------------- phase 2: pairs, positions, vertices, triangles
             const uint32_t inc = warp_inclusive_scan(m, lane);
             const uint32_t npairs = __shfl_sync(FULL, inc, 31);
@@ -916,17 +827,17 @@ size_t stream_row_elems(int dtype, int rows)
     return ((((size_t)kSegCells / rows + 1) * es + 15) / 16) * 16 / es;
 }
 
-size_t stream_warp_smem_bytes(int dtype, bool emit, int rows)
+size_t stream_warp_smem_bytes(int dtype, int rows)
 {
     const size_t plane = (size_t)(rows + 1) * stream_row_elems(dtype, rows) * dtype_size(dtype);
-    return align128(sizeof(WarpState)) + (emit ? align128(sizeof(WarpEmit)) : 0) + align128(3 * plane);
+    return align128(sizeof(WarpState)) + align128(sizeof(WarpEmit)) + align128(3 * plane);
 }
 
 size_t stream_warp_smem_offset() { return align128(sizeof(Tables)); }
 
-size_t stream_shared_bytes(int dtype, bool emit, int rows)
+size_t stream_shared_bytes(int dtype, int rows)
 {
-    return stream_warp_smem_offset() + (size_t)(emit ? kEmitWarps : kWarps) * stream_warp_smem_bytes(dtype, emit, rows);
+    return stream_warp_smem_offset() + (size_t)kEmitWarps * stream_warp_smem_bytes(dtype, rows);
 }
 
 uint64_t brick_count(const VolumeView& v)
@@ -947,37 +858,33 @@ uint64_t brick_count(const VolumeView& v)
     default: return cudaErrorInvalidValue;              \
     }
 
-cudaError_t launch_stream(bool emit, int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
-                          const StreamIso* d_isos, uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
-                          const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
-                          const Launch& L, int ctas_per_sm, uint64_t task0, uint32_t* d_node_counts,
-                          const uint64_t* d_totals, const int* d_only_if)
+cudaError_t launch_stream_emit(int dtype, int rows, const StreamGroup* d_groups, int ngroups, uint64_t ntasks,
+                               const StreamIso* d_isos, const uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
+                               const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task,
+                               const Launch& L, int ctas_per_sm, uint64_t task0, const uint64_t* d_totals,
+                               const int* d_only_if)
 {
     if (ntasks <= task0) return cudaSuccess;
     if (rows != 1 && rows != 2) return cudaErrorInvalidValue;
     if (dtype == 2 || dtype == 3 || dtype == 6 || dtype == 7 || dtype == 9)
-        return emit && rows == 1 ? launch_wide(dtype, d_groups, ngroups, ntasks, d_isos, d_unit_counts, d_unit_offsets,
-                                               d_plane_base, d_status, d_next_task, L, task0, d_totals, d_only_if)
-                                 : cudaErrorInvalidValue;
-    if (!emit && (rows != 1 || !d_node_counts)) return cudaErrorInvalidValue;   // (the other counts: mc_one.cu, mc_many.cu)
-    const size_t smem = stream_shared_bytes(dtype, emit, rows);
-    const int threads = emit ? kEmitThreads : kStreamThreads;
-    const uint64_t need = (ntasks - task0 + threads / 32 - 1) / (threads / 32);
+        return rows == 1 ? launch_wide(dtype, d_groups, ngroups, ntasks, d_isos, d_unit_counts, d_unit_offsets,
+                                       d_plane_base, d_status, d_next_task, L, task0, d_totals, d_only_if)
+                         : cudaErrorInvalidValue;
+    const size_t smem = stream_shared_bytes(dtype, rows);
+    const uint64_t need = (ntasks - task0 + kEmitWarps - 1) / kEmitWarps;
     KVSMC_STREAM_SWITCH(dtype, {
-        auto kern = emit ? (rows == 1 ? k_stream<T, true, 1> : k_stream<T, true, 2>) : k_stream<T, false, 1>;
+        auto kern = rows == 1 ? k_stream<T, 1> : k_stream<T, 2>;
         int per_sm = 0;
-        const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), threads, smem, &per_sm, true);
+        const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), kEmitThreads, smem, &per_sm, true);
         if (e != cudaSuccess) return e;
         if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
         // persistent: as many CTAs as are resident at once (never more than the tasks need)
         const uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)L.num_sms;
         const uint64_t nctas = need < resident ? need : resident;
-        prof_begin(L, emit ? "stream_emit" : "stream_count");
-        kern<<<(unsigned)nctas, threads, smem, L.stream>>>(d_groups, ngroups, ntasks, d_isos, d_unit_counts,
-                                                           d_unit_offsets, d_plane_base, d_status, d_next_task,
-                                                           L.wait_polls[emit ? 1 : 0], task0,
-                                                           emit ? nullptr : d_node_counts, emit ? d_totals : nullptr,
-                                                           emit ? d_only_if : nullptr);
+        prof_begin(L, "stream_emit");
+        kern<<<(unsigned)nctas, kEmitThreads, smem, L.stream>>>(d_groups, ngroups, ntasks, d_isos, d_unit_counts,
+                                                                d_unit_offsets, d_plane_base, d_status, d_next_task,
+                                                                L.wait_polls[1], task0, d_totals, d_only_if);
         prof_end(L);
     });
     *L.counter += 1;

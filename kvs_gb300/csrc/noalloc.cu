@@ -115,7 +115,7 @@ extern "C" kvsmc_status kvsmc_extract_noalloc(const void* d_values, kvsmc_dtype 
     const int rows = kvsmc_host::stream_rows(nx - 1);
     g.rows = (uint32_t)rows;
     g.wpr = kvsmc_host::segments_per_row(v, rows);
-    if (stream_shared_bytes(dtype, true, rows) > (size_t)227 * 1024 ||
+    if (stream_shared_bytes(dtype, rows) > (size_t)227 * 1024 ||
         (double)(nx - 1) * (double)(ny - 1) * 5.0 >= 4294967295.0)
         return KVSMC_ERR_TOO_LARGE;
     const uint32_t cy = ny - 1, cz = nz - 1;
@@ -128,7 +128,7 @@ extern "C" kvsmc_status kvsmc_extract_noalloc(const void* d_values, kvsmc_dtype 
     g.plane_begin = 0;
     g.seg_elems = (uint32_t)stream_row_elems(dtype, rows);
     g.seg_copy_bytes = g.seg_elems * (uint32_t)es;
-    g.warp_smem_bytes = (uint32_t)stream_warp_smem_bytes(dtype, true, rows);
+    g.warp_smem_bytes = (uint32_t)stream_warp_smem_bytes(dtype, rows);
     g.warp_smem_offset = (uint32_t)stream_warp_smem_offset();
 
     // carve the static array
@@ -210,7 +210,7 @@ extern "C" kvsmc_status kvsmc_extract_noalloc(const void* d_values, kvsmc_dtype 
     iso.normals = d_normals;
     iso.cap_tris = total;
     if (cudaMemcpyAsync(d_iso, &iso, sizeof iso, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-        launch_stream(true, dtype, rows, d_group, 1, ntasks, d_iso, d_unit_counts, d_unit_offsets, d_plane_base, d_status, d_next + 1, L) !=
+        launch_stream_emit(dtype, rows, d_group, 1, ntasks, d_iso, d_unit_counts, d_unit_offsets, d_plane_base, d_status, d_next + 1, L) !=
             cudaSuccess ||
         cudaMemcpyAsync(&status, d_status, sizeof status, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)

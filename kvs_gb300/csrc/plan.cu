@@ -60,10 +60,9 @@ cudaError_t record(kvsmc_host::StreamBatch& b, cudaStream_t s, int num_sms, uint
             if (ee != cudaSuccess || !b.list_cap || b.list_sure || !l.listed) return ee;
             // the list may overflow, and a replay has no host between its passes:
             // the classifying emit stands behind, for that case only
-            return kvsmc::launch_stream(true, l.dtype, l.rows, b.d_groups + l.g0, l.ng, l.ntasks, b.d_isos,
-                                        b.d_unit_counts, b.d_unit_offsets, b.d_plane_base, b.d_status,
-                                        b.d_next + 2 * i + 1, Li, l.ctas_per_sm, 0, nullptr, nullptr,
-                                        b.list.overflow);
+            return kvsmc::launch_stream_emit(l.dtype, l.rows, b.d_groups + l.g0, l.ng, l.ntasks, b.d_isos,
+                                              b.d_unit_counts, b.d_unit_offsets, b.d_plane_base, b.d_status,
+                                              b.d_next + 2 * i + 1, Li, l.ctas_per_sm, 0, nullptr, b.list.overflow);
         });
     };
     cudaError_t e = cudaMemsetAsync(b.d_status, 0, b.zero_bytes, s);

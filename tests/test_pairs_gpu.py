@@ -121,3 +121,68 @@ def test_a_list_that_overflows(kvsmc_ctx):
         assert all(torch.equal(a, b) for a, b in zip(got[i], want[i])), i
     plan.close()
     vol.free()
+
+
+def test_a_list_that_overflows_in_the_shared_modes(kvsmc_ctx):
+    """The same noise with shared vertices: together the pairs overflow their
+    list (the connections classify again, the vertex normals sort), alone they
+    do not (connections over pairs, normals by cell).  Only two requests have
+    outputs."""
+    n = 341
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    v = torch.randint(0, 256, (n, n, n), generator=gen, device="cuda", dtype=torch.uint8)
+    torch.cuda.synchronize()
+    vol = _abi.DeviceVolume.from_device(kvsmc_ctx, v.data_ptr(), np.uint8, (n, n, n))
+    params = [_abi.make_params(110.5 + 2.0 * k, 1 if k == 3 else 2) for k in range(16)]
+
+    def outputs(s):
+        t = (torch.zeros(s.ncoords, device="cuda"), torch.zeros(s.nnormals, device="cuda"),
+             torch.zeros(s.nconnections, dtype=torch.int32, device="cuda"))
+        torch.cuda.synchronize()
+        return t
+
+    want = {}
+    for i in (3, 12):
+        o = _abi.Sizes()
+        kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_count(kvsmc_ctx.handle, vol.handle, params[i], o), "count")
+        c, m, k = outputs(o)
+        kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_extract_device(kvsmc_ctx.handle, vol.handle, params[i], c.data_ptr(), o.ncoords,
+                                                           m.data_ptr(), o.nnormals, k.data_ptr(), o.nconnections, o),
+                        "extract")
+        want[i] = (c, m, k, o)
+    reqs = (_abi.Request * 16)()
+    got = {i: outputs(want[i][3]) for i in want}
+    for i in range(16):
+        reqs[i].volume, reqs[i].params = vol.handle, params[i]
+        if i in got:
+            c, m, k = got[i]
+            reqs[i].d_coords, reqs[i].coords_capacity = c.data_ptr(), c.numel()
+            reqs[i].d_normals, reqs[i].normals_capacity = m.data_ptr(), m.numel()
+            reqs[i].d_connections, reqs[i].connections_capacity = k.data_ptr(), k.numel()
+    assert kvsmc_ctx.lib.kvsmc_extract_batch(kvsmc_ctx.handle, reqs, 16) == _abi.ERR_CAPACITY
+    for i in want:
+        assert reqs[i].status == _abi.OK
+        assert all(torch.equal(a, b) for a, b in zip(got[i], want[i])), i
+    vol.free()
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.int16, np.float32, np.float64])
+@pytest.mark.parametrize("shape", [(2, 2, 2), (2, 3, 33), (3, 2, 257), (5, 4, 256), (4, 34, 70), (40, 3, 9)])
+def test_shared_modes_over_listed_pairs(kvsmc_ctx, oracle_lib, dtype, shape):
+    """Volumes that are mostly faces (vertices that lack cells around their
+    edge, node rows and planes past the last cells), every cell crossed: one
+    request, three and sixteen in a batch."""
+    rng = np.random.default_rng(sum(shape))
+    v = rng.random(shape).astype(dtype) if np.dtype(dtype).kind == "f" else rng.integers(0, 100, shape).astype(dtype)
+    lo, hi = float(v.min()), float(v.max())
+    vol = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+    for n in (1, 3, 16):
+        isos = [lo + (hi - lo) * (k + 0.37) / n for k in range(n)]
+        modes = [1 + (k & 1) if n > 1 else 2 for k in range(n)]
+        out = extract_batch(kvsmc_ctx, [vol] * n, [_abi.make_params(x, m) for x, m in zip(isos, modes)], _abi.PATH_AUTO)
+        for x, m, o in zip(isos, modes, out):
+            ref = oracle_lib.extract(v, x, m, lo, hi)
+            assert same_bits(o["coords"], ref["coords"]), (shape, n, x, first_diff(o["coords"], ref["coords"]))
+            assert same_bits(o["normals"], ref["normals"]), (shape, n, x, m)
+            assert np.array_equal(o["connections"], ref["connections"].view(np.uint32)), (shape, n, x)
+    vol.free()

@@ -407,6 +407,9 @@ void gather_sizes(const Plan& pl, const Item& it, kvsmc_sizes* s)
     }
 }
 
+// Tasks of a group's node emit over listed pairs.
+uint64_t nodes_tasks(const kvsmc::StreamGroup& G) { return (uint64_t)G.vol.nz * (G.eblocks + 1); }
+
 // The request's record for the connection pass.
 kvsmc::ConnIso conn_iso(const Plan& pl, float* coords, uint32_t* conn, float* normals)
 {
@@ -472,6 +475,13 @@ kvsmc_status gather_emit(kvsmc_context* ctx, Plan& pl, float* coords, float* nor
     const bool own_passes = pl.snode && !pl.nodes_done && pl.nvert;
     if (pl.nodes_done) {
         // written already
+    } else if (pl.nvert && pl.snode && pl.pairs() && pl.sb_nodes) {
+        const StreamBatch& b = *pl.sb;
+        kvsmc::NodeTable t{};
+        t.iso[pl.sb_iso] = kvsmc::NodeOut{coords, j.rank, j.vtile_offsets, j.slots};
+        KVSMC_CUDA(ctx, kvsmc::launch_nodes_pairs(b.d_groups + pl.sb_group, b.d_isos, t, j.vol.dtype, j.words_per_row,
+                                                  b.list, nodes_tasks(b.groups[pl.sb_group]), pl.d_status,
+                                                  pl.d_next + 1, L));
     } else if (pl.nvert && pl.snode) {
         uint32_t* counts = const_cast<uint32_t*>(pl.sb_nodes ? pl.sb_nodes : j.vtile_counts);
         KVSMC_CUDA(ctx, kvsmc::launch_snode(true, j, pl.f, pl.wprn, pl.zchunk, pl.ntasks, counts, j.vtile_offsets,
@@ -812,10 +822,18 @@ kvsmc_status grouped_shared(kvsmc_context* ctx, const SharedCount& sc, std::vect
         const Plan& p0 = *gp[0];
         int* d_status = reinterpret_cast<int*>(d_status_all + 64 * g);
         unsigned long long* d_next = reinterpret_cast<unsigned long long*>(d_status_all + 64 * g + 16);
-        KVSMC_CUDA(ctx, cudaMemcpyAsync(d_node, h, gp.size() * sizeof(kvsmc::NodeIso), cudaMemcpyHostToDevice,
-                                        ctx->stream));
-        KVSMC_CUDA(ctx, kvsmc::launch_snode_multi(p0.job.vol, d_node, (int)gp.size(), G.bs, G.bo, p0.wprn, p0.zchunk,
-                                                  p0.ntasks, p0.job.words_per_row, d_status, d_next, L));
+        if (p0.pairs()) {
+            kvsmc::NodeTable t{};
+            for (const Plan* pl : gp)
+                t.iso[pl->sb_iso] = kvsmc::NodeOut{pl->item->d_coords, pl->job.rank, pl->job.vtile_offsets, pl->vs.slots};
+            KVSMC_CUDA(ctx, kvsmc::launch_nodes_pairs(b.d_groups + g, b.d_isos, t, p0.job.vol.dtype,
+                                                      p0.job.words_per_row, b.list, nodes_tasks(G), d_status, d_next, L));
+        } else {
+            KVSMC_CUDA(ctx, cudaMemcpyAsync(d_node, h, gp.size() * sizeof(kvsmc::NodeIso), cudaMemcpyHostToDevice,
+                                            ctx->stream));
+            KVSMC_CUDA(ctx, kvsmc::launch_snode_multi(p0.job.vol, d_node, (int)gp.size(), G.bs, G.bo, p0.wprn, p0.zchunk,
+                                                      p0.ntasks, p0.job.words_per_row, d_status, d_next, L));
+        }
         kvsmc_status st = KVSMC_OK;
         if (ready) {   // the vertices leave while the connections are written
             if (!(st = read_status())) st = group_status(g);

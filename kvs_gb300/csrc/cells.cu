@@ -37,6 +37,7 @@
 #include "mc_device.cuh"
 #include "mc_emit.cuh"
 #include "mc_interp.cuh"
+#include "mc_slots.cuh"
 #include "slice_common.cuh"
 
 namespace kvsmc {
@@ -381,21 +382,6 @@ template <int CT> struct alignas(16) CellWarp {
     float4 pv[kVerts];   // x, y, z, colour (slices)
     uint32_t nodes[32][CellTraits<CT>::kNodes | 1];
 };
-
-__device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t n)
-{
-    uint32_t pos = 0;
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-        const uint32_t c = (uint32_t)__popc(m & ((1u << s) - 1u));
-        if (n >= c) {
-            n -= c;
-            m >>= s;
-            pos += s;
-        }
-    }
-    return pos;
-}
 
 // Emit one block: lane u holds the cut cells' word of group u; their bits are
 // one index space, taken 32 cells at a time, one per lane.  A round's vertices

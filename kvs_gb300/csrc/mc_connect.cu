@@ -1,9 +1,8 @@
-// mc_connect.cu -- connect_isopoints (MarchingCubes.cpp:456-521) and the vertex
-// normals (:569-605) of the shared-vertex modes over listed pairs: the count
-// pass has listed the crossed cells, the node emit has written vertices and
-// rank words (mc_snode.cu).
+// mc_connect.cu -- the shared-vertex modes over listed pairs: calculate_isopoints
+// (MarchingCubes.cpp:366-446), connect_isopoints (:456-521) and the vertex
+// normals (:569-605) from the crossed cells that the count pass listed.
 //
-// Tasks, blocks and rounds are mc_pairs.cu's.  A round's vertex items (one per
+// Tasks, blocks and rounds are mc_pairs.cu's.  In the connection pass a round's vertex items (one per
 // (pair, used edge), 4 to 5 a pair) each read the rank word of the edge's lower
 // node, which gives the vertex id, and have the vertex itself by interpolating
 // it again from the corner values at hand (the same certified bits; a read of
@@ -31,6 +30,7 @@
 #include "mc_internal.h"
 #include "mc_interp.cuh"
 #include "mc_pairs.cuh"
+#include "mc_slots.cuh"
 #include "tma.cuh"
 
 namespace kvsmc {
@@ -142,14 +142,14 @@ __global__ void __launch_bounds__(kPairThreads, 3)
         if (lane == 0) tk = atomicAdd(next_task, 1ull);
         const uint64_t task = __shfl_sync(FULL, tk, 0);
         if (task >= ntasks) break;
-        const PairBlock B = pair_block(G, pl, (uint32_t)task, lane);
+        const uint32_t z = (uint32_t)task / G.eblocks, u0 = ((uint32_t)task - z * G.eblocks) * G.eblock;
+        const PairBlock B = pair_block(G, pl, z, u0, G.eblock, lane);
         if (B.npairs == 0) continue;
-        const uint32_t z = B.z;
         __syncwarp();
         if (lane < niso) {
             const uint64_t pi = isos[iso_begin + lane].plane_index;
             W.first[lane] = plane_base[pi + z] - plane_base[pi] +
-                            unit_offsets[G.unit_base + ((uint64_t)z * ((ny - 1) * G.wpr) + B.u0) * niso + lane];
+                            unit_offsets[G.unit_base + ((uint64_t)z * ((ny - 1) * G.wpr) + u0) * niso + lane];
         }
         __syncwarp();
         uint32_t run = 0;   // lane k: the task's triangles of isolevel k so far (at most 32 * 256 * 5)
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kPairThreads, 3)
                 const uint32_t starts = __reduce_or_sync(FULL, item && vpre - j0 < 32u ? 1u << (vpre - j0) : 0u);
                 uint32_t q = seen + (uint32_t)__popc(starts & (lt | (1u << lane))) - 1u;
                 seen += (uint32_t)__popc(starts);
-                if (gaps) q = __fns(items, 0, (int)q + 1);
+                if (gaps) q = nth_set_bit(items, q) & 31u;
                 const uint32_t qe = __shfl_sync(FULL, pe, q);
                 const uint32_t qy = __shfl_sync(FULL, y, q);
                 const uint32_t qo = __shfl_sync(FULL, ot, q);
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kPairThreads, 3)
                 const uint32_t starts = __reduce_or_sync(FULL, item && tpre - j0 < 32u ? 1u << (tpre - j0) : 0u);
                 uint32_t q = seen + (uint32_t)__popc(starts & (lt | (1u << lane))) - 1u;
                 seen += (uint32_t)__popc(starts);
-                if (gaps) q = __fns(items, 0, (int)q + 1);
+                if (gaps) q = nth_set_bit(items, q) & 31u;
                 const uint32_t qe = __shfl_sync(FULL, pe, q);
                 const uint32_t qo = __shfl_sync(FULL, ot, q);
                 if (j < ntr) {
@@ -297,6 +297,232 @@ __global__ void __launch_bounds__(kPairThreads, 3)
                 }
             }
             __syncwarp();
+        }
+    }
+}
+
+// calculate_isopoints (MarchingCubes.cpp:366-446) over listed pairs: the
+// vertices and rank words that mc_snode.cu's kernels write, from the cells that
+// the count found.  A node's cut edges make its cell (the one it is the lower
+// corner of) a listed pair; the nodes behind the last cell of a row belong to
+// that cell's item list, those of the last row and plane to tasks of their own,
+// which walk the last cell row's or plane's pairs for the nodes at their far
+// side.  So a task's pairs are its vertices in id order, and a round numbers
+// them as the emit numbers triangles.  A round's pairs of one (unit, isolevel,
+// 32-node word) collect the word's flags in shared memory; the first of them
+// stores the word, with its own first vertex as the word's; a word that goes on
+// in the next round gets the rest by atomics.
+// 385x320x352 f32, 8 isolevels: 711 us classifying every node again, 302 us.
+struct __align__(16) NodeConst {
+    FastIso f;
+    float mc[3], sc[3];
+    float* coords;
+    uint4* rank;
+    uint2* slots;
+    const uint64_t* offsets;
+    uint64_t pad[3];
+};
+static_assert(sizeof(NodeConst) == 112, "bank stride");
+
+template <typename V> struct alignas(16) NodeWarp {
+    V cv[32][9];                    // corner values of the round's cells
+    uint64_t first[kStreamMaxIso];  // per isolevel: the task's first vertex
+    uint32_t add[kStreamMaxIso];    // per isolevel: vertices of the round,
+    uint32_t last[kStreamMaxIso];   // and the word of its last pair so far
+    uint32_t flags[32][3];          // per leading lane: the word's x, y, z flags
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kPairThreads, 4)
+    k_nodes_pairs(const StreamGroup* __restrict__ groups, const StreamIso* __restrict__ isos,
+                  const __grid_constant__ NodeTable nodes, PairList pl, uint64_t ntasks, uint32_t words_per_row,
+                  int* __restrict__ status, unsigned long long* __restrict__ next_task)
+{
+    using V = typename PairValue<T>::type;
+    __shared__ NodeConst s_iso[kStreamMaxIso];
+    __shared__ NodeWarp<V> sw[kPairWarps];
+    const unsigned tid = threadIdx.x, lane = tid & 31u;
+    NodeWarp<V>& W = sw[tid >> 5];
+    const StreamGroup& G = groups[0];
+    const uint32_t niso = (uint32_t)G.niso;
+    const int iso_begin = G.iso_begin;
+    if (tid < niso) {
+        const StreamIso& I = isos[iso_begin + tid];
+        const NodeOut& o = nodes.iso[tid];
+        NodeConst& k = s_iso[tid];
+        k.f = I.f;
+        for (int a = 0; a < 3; ++a) { k.mc[a] = I.ip.min_coord[a]; k.sc[a] = I.ip.scale[a]; }
+        k.coords = o.coords;
+        k.rank = o.rank;
+        k.slots = o.slots;
+        k.offsets = o.offsets;
+    }
+    if (__syncthreads_or(*status != 0 || *pl.overflow != 0)) return;   // the list is not complete
+    const unsigned lt = (1u << lane) - 1u;
+    const uint32_t nx = G.vol.nx, ny = G.vol.ny, nz = G.vol.nz, wpr = G.wpr;
+    const uint64_t pitch = G.vol.pitch, slice = G.vol.slice;
+    for (;;) {
+        unsigned long long tk = 0;
+        if (lane == 0) tk = atomicAdd(next_task, 1ull);
+        const uint64_t task = __shfl_sync(FULL, tk, 0);
+        if (task >= ntasks) break;
+        // (node plane, block of units); the last block of a plane is the nodes
+        // behind the last cell row, the last plane those behind the last cell plane
+        const uint32_t per = G.eblocks + 1;
+        const uint32_t zn = (uint32_t)task / per, e = (uint32_t)task - zn * per;
+        const bool far_y = e == G.eblocks, far_z = zn == nz - 1;
+        const uint32_t z = far_z ? zn - 1 : zn;   // cell plane
+        const uint32_t u0 = far_y ? (ny - 2) * wpr : e * G.eblock;
+        const PairBlock B = pair_block(G, pl, z, u0, far_y ? wpr : G.eblock, lane);
+        if (B.npairs == 0) continue;
+        const uint32_t row = (far_y ? 1u : 0u) | (far_z ? 2u : 0u);   // the node's row among the cell's four
+        __syncwarp();
+        if (lane < niso) {
+            const uint64_t* off = s_iso[lane].offsets;
+            W.first[lane] = s_iso[lane].coords ? off[((uint64_t)zn * ny + (u0 / wpr + (far_y ? 1u : 0u))) * wpr + u0 % wpr] - off[0] : 0;
+            W.last[lane] = 0xffffffffu;
+            W.add[lane] = 0;
+        }
+        __syncwarp();
+        uint32_t run = 0;   // lane k: the task's vertices of isolevel k so far
+        const T* vz = static_cast<const T*>(G.vol.data) + (uint64_t)z * slice;
+        const float fz = __uint2float_rn(zn);
+        for (uint32_t r0 = 0; r0 < B.npairs; r0 += 32) {
+            // ---- one pair per lane
+            bool has = r0 + lane < B.npairs;
+            uint32_t x, y;
+            const uint32_t at = pair_entry(B, r0 + lane, x, y);
+            uint32_t k = 0, cut = 0;
+            if (has) {
+                const uint32_t ent = pl.list[at];
+                x += ent & 0xffu;
+                k = ent >> 8;
+                const uint32_t code = pair_corners<T, V>(vz + (uint64_t)y * pitch + x, pitch, slice, W.cv[lane],
+                                                         [&](T v) -> bool {
+                    if constexpr (kPairFast<T>) return (float)v > s_iso[k].f.f_thr;
+                    else return above(isos[iso_begin].cls, v);   // (one isolevel per group)
+                });
+                has = s_iso[k].coords != nullptr;
+                // the node's cut edges (code bit r: row r at x, 4 + r: at x + 1)
+                const uint32_t n = code >> row, f = code >> (4 + row);
+                cut = (n ^ f) & 1u;
+                if (!far_y) cut |= ((n ^ (n >> 1)) & 1u) << 1;
+                if (!far_z) cut |= ((n ^ (n >> 2)) & 1u) << 2;
+                if (x + 2 == nx) {   // and those of the row's last node
+                    if (!far_y) cut |= ((f ^ (f >> 1)) & 1u) << 3;
+                    if (!far_z) cut |= ((f ^ (f >> 2)) & 1u) << 4;
+                }
+                if (!has) cut = 0;
+            }
+            y += far_y ? 1u : 0u;   // the node's
+            const uint32_t nv0 = (uint32_t)__popc(cut);
+            const uint32_t kgrp = niso == 1 ? __ballot_sync(FULL, has) : __match_any_sync(FULL, has ? k : 32u + lane);
+            uint32_t pre = 0, gtot = 0, vpre = 0, nv = 0;
+#pragma unroll
+            for (int bit = 0; bit < 3; ++bit) {
+                const uint32_t bm = __ballot_sync(FULL, (nv0 >> bit) & 1u);
+                pre += (uint32_t)__popc(bm & kgrp & lt) << bit;
+                gtot += (uint32_t)__popc(bm & kgrp) << bit;
+                vpre += (uint32_t)__popc(bm & lt) << bit;
+                nv += (uint32_t)__popc(bm) << bit;
+            }
+            const uint32_t start = __shfl_sync(FULL, run, k) + pre;   // the pair's first vertex, from the task's
+            // ---- rank words
+            const uint32_t word = y * words_per_row + (x >> 5);   // (in the node plane)
+            const uint32_t wgrp = __match_any_sync(FULL, has ? word : 0xffffffffu - lane) & kgrp;
+            const int leader = __ffs(wgrp) - 1;
+            W.flags[lane][0] = 0;
+            W.flags[lane][1] = 0;
+            W.flags[lane][2] = 0;
+            __syncwarp();
+            const bool split = (x & 31u) == 31u;   // the row's last node opens a word of its own
+            if (has) {
+                const uint32_t bit = 1u << (x & 31u);
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+                    if ((cut >> a) & 1u) atomicOr(&W.flags[leader][a], bit);
+                if ((cut >> 3) && !split) {
+                    if (cut & 8u) atomicOr(&W.flags[leader][1], bit << 1);
+                    if (cut & 16u) atomicOr(&W.flags[leader][2], bit << 1);
+                }
+            }
+            __syncwarp();
+            if (has && (int)lane == leader) {
+                const NodeConst& I = s_iso[k];
+                uint4* R = I.rank + (uint64_t)zn * ny * words_per_row + word;
+                const uint32_t fx = W.flags[lane][0], fy = W.flags[lane][1], fz3 = W.flags[lane][2];
+                if (W.last[k] != word) {
+                    *R = make_uint4(fx, fy, fz3, (uint32_t)(W.first[k] + start));
+                } else {   // begun in the round before
+                    if (fx) atomicOr(&R->x, fx);
+                    if (fy) atomicOr(&R->y, fy);
+                    if (fz3) atomicOr(&R->z, fz3);
+                }
+            }
+            if ((cut >> 3) && split)
+                s_iso[k].rank[(uint64_t)zn * ny * words_per_row + word + 1] =
+                    make_uint4(0, (cut >> 3) & 1u, cut >> 4, (uint32_t)(W.first[k] + start) + (uint32_t)__popc(cut & 7u));
+            __syncwarp();   // the words before are read
+            if (has && (31 - __clz(kgrp)) == (int)lane) {
+                W.add[k] = gtot;
+                W.last[k] = word;
+            }
+            __syncwarp();
+            if (lane < kStreamMaxIso) {
+                run += W.add[lane];
+                W.add[lane] = 0;
+            }
+            __syncwarp();
+            // ---- vertices: one per lane, from the corner values
+            const uint32_t pe = x | (k << 12) | (cut << 16) | (vpre << 21);   // (x < 4096; vpre <= 160)
+            const uint32_t items = __ballot_sync(FULL, nv0 != 0);
+            uint32_t seen = 0;
+            for (uint32_t j0 = 0; j0 < nv; j0 += 32) {
+                const uint32_t j = j0 + lane;
+                const uint32_t starts = __reduce_or_sync(FULL, nv0 && vpre - j0 < 32u ? 1u << (vpre - j0) : 0u);
+                const uint32_t nth = seen + (uint32_t)__popc(starts & (lt | (1u << lane)));   // 1 ..
+                seen += (uint32_t)__popc(starts);
+                const uint32_t q = nth_set_bit(items, nth - 1u) & 31u;
+                const uint32_t qe = __shfl_sync(FULL, pe, q), qy = __shfl_sync(FULL, y, q);
+                const uint32_t qs = __shfl_sync(FULL, start, q);
+                if (j < nv) {
+                    const uint32_t r = j - (qe >> 21), qk = (qe >> 12) & 15u;
+                    uint32_t m = (qe >> 16) & 31u;
+#pragma unroll
+                    for (uint32_t i = 0; i < 4; ++i)
+                        if (i < r) m &= m - 1u;
+                    const uint32_t ed = (uint32_t)__ffs(m) - 1u;          // 0 .. 2 the node's, 3, 4 the last node's y and z
+                    const uint32_t far_x = ed >= 3u ? 1u : 0u, axis = ed - 2u * far_x;
+                    const uint32_t c0 = far_x | ((row & 1u) << 1) | ((row & 2u) << 1);
+                    const V va = W.cv[q][c0], vb = W.cv[q][c0 | (1u << axis)];
+                    const uint32_t lx = (qe & 0xfffu) + far_x;
+                    const float ax = __uint2float_rn(lx), ay = __uint2float_rn(qy);
+                    const NodeConst& I = s_iso[qk];
+                    float3 v;
+                    bool good = false;
+                    if constexpr (kPairFast<T>) {
+                        const float a = axis == 0 ? ax : (axis == 1 ? ay : fz);
+                        float w;
+                        good = fast_axis_lean<(sizeof(T) < 4)>(va, vb, a, true, I.f, w);
+                        v.x = __fmul_rn(__fadd_rn(axis == 0 ? w : ax, I.mc[0]), I.sc[0]);
+                        v.y = __fmul_rn(__fadd_rn(axis == 1 ? w : ay, I.mc[1]), I.sc[1]);
+                        v.z = __fmul_rn(__fadd_rn(axis == 2 ? w : fz, I.mc[2]), I.sc[2]);
+                    }
+                    if (!good) {   // the exact FP64 sequence
+                        const float bx = axis == 0 ? __fadd_rn(ax, 1.0f) : ax, by = axis == 1 ? __fadd_rn(ay, 1.0f) : ay;
+                        const float bz = axis == 2 ? __fadd_rn(fz, 1.0f) : fz;
+                        if constexpr (kPairFast<T>)
+                            v = edge_vertex_fast(isos[iso_begin + qk].ip, I.f, va, vb, ax, ay, fz, bx, by, bz, (int)axis);
+                        else
+                            v = interpolate_exact_axis(isos[iso_begin].ip, va, vb, ax, ay, fz, bx, by, bz, (int)axis);
+                    }
+                    const uint64_t id = W.first[qk] + qs + r;
+                    float* o = I.coords + 3 * id;
+                    o[0] = v.x; o[1] = v.y; o[2] = v.z;
+                    if (I.slots) clear_face_slots(I.slots, id, lx, qy, zn, nx, ny, nz);
+                }
+            }
+            __syncwarp();   // the corner values and first vertices are read
         }
     }
 }
@@ -392,6 +618,33 @@ cudaError_t launch_connect_pairs(const StreamGroup* d_group, const StreamIso* d_
     prof_begin(L, "connect_pairs");
     e = cudaLaunchKernel(kern, dim3((unsigned)(need < resident ? need : resident)), dim3(kPairThreads), args, smem,
                          L.stream);
+    prof_end(L);
+    *L.counter += 1;
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+cudaError_t launch_nodes_pairs(const StreamGroup* d_group, const StreamIso* d_isos, const NodeTable& nodes, int dtype,
+                               uint32_t words_per_row, const PairList& list, uint64_t ntasks, int* status,
+                               unsigned long long* next_task, const Launch& L)
+{
+    if (ntasks == 0) return cudaSuccess;
+    const void* kern = dtype == 0   ? reinterpret_cast<const void*>(k_nodes_pairs<int8_t>)
+                       : dtype == 1 ? reinterpret_cast<const void*>(k_nodes_pairs<int16_t>)
+                       : dtype == 4 ? reinterpret_cast<const void*>(k_nodes_pairs<uint8_t>)
+                       : dtype == 5 ? reinterpret_cast<const void*>(k_nodes_pairs<uint16_t>)
+                       : dtype == 8 ? reinterpret_cast<const void*>(k_nodes_pairs<float>)
+                                    : nullptr;   // (the wide types' node units are not counted with their pairs)
+    if (!kern) return cudaErrorInvalidValue;
+    int per_sm = 0;
+    cudaError_t e = kernel_fit(L, kern, kPairThreads, 0, &per_sm);
+    if (e != cudaSuccess) return e;
+    const uint64_t need = (ntasks + kPairWarps - 1) / kPairWarps;
+    const uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)L.num_sms;
+    PairList pl = list;
+    NodeTable table = nodes;
+    void* args[] = {&d_group, &d_isos, &table, &pl, &ntasks, &words_per_row, &status, &next_task};
+    prof_begin(L, "nodes_pairs");
+    e = cudaLaunchKernel(kern, dim3((unsigned)(need < resident ? need : resident)), dim3(kPairThreads), args, 0, L.stream);
     prof_end(L);
     *L.counter += 1;
     return e != cudaSuccess ? e : cudaGetLastError();

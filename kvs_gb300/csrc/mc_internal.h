@@ -260,6 +260,24 @@ struct ConnIso {
 struct ConnTable {
     ConnIso iso[kStreamMaxIso];
 };
+// One request of the node emit over listed pairs: coords null when nothing of
+// it is written; offsets, slots as in NodeIso.
+struct NodeOut {
+    float* coords;
+    uint4* rank;
+    const uint64_t* offsets;
+    uint2* slots;
+};
+struct NodeTable {
+    NodeOut iso[kStreamMaxIso];
+};
+// calculate_isopoints over the pairs that streaming count group d_group listed
+// (8/16-bit and float32, a group with node_units); ntasks: (nz node planes) x
+// (the group's blocks of units per plane + 1).  Same outputs as
+// launch_snode_multi.
+cudaError_t launch_nodes_pairs(const StreamGroup* d_group, const StreamIso* d_isos, const NodeTable& nodes, int dtype,
+                               uint32_t words_per_row, const PairList& list, uint64_t ntasks, int* status,
+                               unsigned long long* next_task, const Launch& L);
 // connect_isopoints over the pairs that streaming count group d_group listed
 // (mc_connect.cu), for its enabled requests; ntasks: the group's blocks of
 // units.  Same outputs and rules as launch_sconnect_multi.

@@ -116,15 +116,16 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
             gcur = gi;
         }
         if (!live) continue;
-        const PairBlock B = pair_block(G, pl, (uint32_t)(task - G.etask_begin), lane);
+        const uint32_t local = (uint32_t)(task - G.etask_begin);
+        const uint32_t z = local / G.eblocks, u0 = (local - z * G.eblocks) * G.eblock;   // first unit in the plane
+        const PairBlock B = pair_block(G, pl, z, u0, G.eblock, lane);
         if (B.npairs == 0) continue;
-        const uint32_t z = B.z;
         // per isolevel: where the task's first triangle goes and how many fit
         __syncwarp();
         if (lane < (unsigned)niso) {
             const uint64_t pi = isos[iso_begin + lane].plane_index;
             const uint64_t at = plane_base[pi + z] - plane_base[pi] +
-                                unit_offsets[G.unit_base + ((uint64_t)z * ((G.vol.ny - 1) * G.wpr) + B.u0) * niso + lane];
+                                unit_offsets[G.unit_base + ((uint64_t)z * ((G.vol.ny - 1) * G.wpr) + u0) * niso + lane];
             const IsoConst& c = W.ic[lane];
             W.out[lane] = PairOut{c.coords + 9 * at, c.normals + 3 * at};
             W.room[lane] = !c.coords || c.cap_tris <= at ? 0u

@@ -79,23 +79,22 @@ template <> struct PairValue<uint16_t> { using type = float; };
 // A task's pairs as one index space: lane u holds unit u's (a warp scan of
 // their numbers), and its row and first cell.
 struct PairBlock {
-    uint32_t z, u0;       // cell plane, first unit in it
     uint32_t inc, first;  // pairs up to and with this lane's unit; entry of pair p of it: list[first + p]
     uint32_t npairs;
     uint32_t uy, ux;
 };
 
-__device__ __forceinline__ PairBlock pair_block(const StreamGroup& G, const PairList& pl, uint32_t local, unsigned lane)
+// Units u0 .. u0 + units - 1 (at most 32; those there are) of cell plane z.
+__device__ __forceinline__ PairBlock pair_block(const StreamGroup& G, const PairList& pl, uint32_t z, uint32_t u0,
+                                                uint32_t units, unsigned lane)
 {
     PairBlock b;
-    const uint32_t cy = G.vol.ny - 1, wpr = G.wpr, plane_units = cy * wpr;
-    b.z = local / G.eblocks;
-    b.u0 = (local - b.z * G.eblocks) * G.eblock;
+    const uint32_t wpr = G.wpr, plane_units = (G.vol.ny - 1) * wpr;
     uint32_t np = 0;
     b.first = 0;
-    const uint32_t un = b.u0 + lane;
-    if (lane < G.eblock && un < plane_units) {
-        const uint64_t pu = G.pair_base + (uint64_t)b.z * plane_units + un;
+    const uint32_t un = u0 + lane;
+    if (lane < units && un < plane_units) {
+        const uint64_t pu = G.pair_base + (uint64_t)z * plane_units + un;
         np = pl.unit_pairs[pu];
         if (np) b.first = pl.unit_list[pu];
     }

@@ -1,4 +1,8 @@
-// mc_snode.cu -- the shared-vertex modes' node passes as streaming kernels.
+// mc_snode.cu -- the shared-vertex modes' node and connection passes as
+// streaming kernels that classify the volume themselves: for requests whose
+// pairs are not listed (a list that overflowed or had no room), and the node
+// passes of the wide types and of rows whose last node opens a segment.  The
+// passes over listed pairs are in mc_connect.cu.
 //
 // calculate_isopoints (MarchingCubes.cpp:366-446) visits every node in z, y, x
 // order and gives each of its x-, y- and z-edges (inside the grid) that the
@@ -19,6 +23,7 @@
 
 #include "mc_internal.h"
 #include "mc_interp.cuh"
+#include "mc_slots.cuh"
 #include "mc_thermo.cuh"
 #include "tma.cuh"
 
@@ -62,17 +67,6 @@ constexpr unsigned FULL = 0xffffffffu;
 #endif
 
 __host__ __device__ __forceinline__ size_t sn_align(size_t v) { return (v + 127) / 128 * 128; }
-
-// A vertex of a node on the volume's faces may lack cells around its edge: its
-// slots start from zero (the connection pass writes the ones there are).
-__device__ __forceinline__ void clear_face_slots(uint2* slots, uint64_t id, uint32_t x, uint32_t y, uint32_t z,
-                                                 uint32_t nx, uint32_t ny, uint32_t nz)
-{
-    if (x != 0 && y != 0 && z != 0 && x + 1 != nx && y + 1 != ny && z + 1 != nz) return;
-    uint4* s = reinterpret_cast<uint4*>(slots + 4 * id);
-    s[0] = make_uint4(0, 0, 0, 0);
-    s[1] = make_uint4(0, 0, 0, 0);
-}
 
 template <typename T, bool EMIT>
 __global__ void __launch_bounds__(kSnThreads, EMIT ? KVSMC_SNODE_EMIT_CTAS : 1)

@@ -101,11 +101,11 @@ kvsmc_tune_choice stream_shape(const kvsmc_context* ctx, const kvsmc::VolumeView
     return c;
 }
 
-uint32_t stream_zchunk(uint64_t warp_steps, int num_sms, int tasks_per_sm)
+uint32_t stream_zchunk(uint64_t warp_steps, int num_sms, int tasks_per_sm, uint32_t least)
 {
     const uint64_t want_tasks = (uint64_t)num_sms * (uint64_t)(tasks_per_sm > 0 ? tasks_per_sm : kDefaultTasksPerSm);
     uint64_t zc = (warp_steps + want_tasks - 1) / want_tasks;
-    if (zc < 4) zc = 4;
+    if (zc < least) zc = least;
     if (zc > 64) zc = 64;
     return (uint32_t)zc;
 }
@@ -230,7 +230,13 @@ void StreamBatch::plan_tables()
         }
         const kvsmc_tune_choice& bs_shape = shape[big];
         L.ctas_per_sm = bs_shape.ctas_per_sm;
-        const uint32_t zchunk = stream_zchunk(steps, ctx->num_sms, bs_shape.tasks_per_sm);
+        // a small launch's time is one task's: a step over several isolevels or
+        // with vertices is three times a plain one's (99x130x83 u16, shared
+        // vertices: 32 us with tasks of four planes, 25.6 of two), while a plain
+        // one gains nothing from a third plane read for every two
+        bool plain = !want_nodes;
+        for (auto& l : lists) plain = plain && (kind_of(l) != kd || l.size() == 1);
+        const uint32_t zchunk = stream_zchunk(steps, ctx->num_sms, bs_shape.tasks_per_sm, plain ? 4 : 2);
         // units per block of the listing emit: enough blocks for every resident
         // warp to take two, at most a warp's lanes, at least two
         const uint32_t eblock = (uint32_t)std::min<uint64_t>(

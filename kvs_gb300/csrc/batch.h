@@ -16,7 +16,7 @@ void bucket_params(float t0, float t1, float& bs, float& bo);
 // steps in all: about tasks_per_sm tasks per SM (the built-in rule: 96),
 // 4 to 64 planes per task (the one-plane halo a task re-reads stays small).
 constexpr int kDefaultTasksPerSm = 96;
-uint32_t stream_zchunk(uint64_t warp_steps, int num_sms, int tasks_per_sm = kDefaultTasksPerSm);
+uint32_t stream_zchunk(uint64_t warp_steps, int num_sms, int tasks_per_sm = kDefaultTasksPerSm, uint32_t least = 4);
 
 // Cell rows per warp task for rows of cx cells: 2 (128-cell segments) when
 // that idles fewer lanes than 256-cell segments, else 1.

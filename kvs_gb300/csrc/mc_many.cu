@@ -51,7 +51,7 @@ __host__ __device__ __forceinline__ size_t many_align(size_t v) { return (v + 12
 // Mask rows: SEG + 1 nodes and padding to 16 bytes.
 template <int R> constexpr uint32_t kMaskRow = 256 / R + 8;
 
-template <int R> struct alignas(16) ManyWarp {
+template <typename T, int R> struct alignas(16) ManyWarp {
     uint16_t mask[2][R + 1][kMaskRow<R>];   // node masks of the lower and the upper plane (plane & 1)
     uint16_t buf[kManyBuf];                 // cell in the warp (8 bits) | isolevel << 8
     // [row][isolevel]: triangles | vertices << 16 of the current units; with
@@ -59,7 +59,7 @@ template <int R> struct alignas(16) ManyWarp {
     // past the last cell plane and past both, 10 bits each
     uint32_t cnt[32];
     uint64_t bar[2];
-    ThermoTables th;
+    ThermoTables<T> th;
 };
 
 template <typename T, int R, bool LIST, bool NODES>
@@ -80,9 +80,9 @@ __global__ void __launch_bounds__(kManyThreads, 4)
     __syncthreads();   // the only CTA-wide barrier
     const uint32_t row_elems = groups[0].seg_elems;
     const uint32_t plane_elems = (R + 1) * row_elems;
-    const size_t wstride = many_align(sizeof(ManyWarp<R>)) + many_align((size_t)2 * plane_elems * sizeof(T));
-    ManyWarp<R>& W = *reinterpret_cast<ManyWarp<R>*>(smem_raw + (size_t)warp * wstride);
-    T* ring = reinterpret_cast<T*>(smem_raw + (size_t)warp * wstride + many_align(sizeof(ManyWarp<R>)));
+    const size_t wstride = many_align(sizeof(ManyWarp<T, R>)) + many_align((size_t)2 * plane_elems * sizeof(T));
+    ManyWarp<T, R>& W = *reinterpret_cast<ManyWarp<T, R>*>(smem_raw + (size_t)warp * wstride);
+    T* ring = reinterpret_cast<T*>(smem_raw + (size_t)warp * wstride + many_align(sizeof(ManyWarp<T, R>)));
     if (lane == 0) {
         mbar_init(&W.bar[0], 1);
         mbar_init(&W.bar[1], 1);
@@ -387,11 +387,10 @@ cudaError_t launch_count_many(int dtype, int rows, const StreamGroup* d_groups, 
 {
     if (ntasks == 0) return cudaSuccess;
     if (rows != 1 && (rows != 2 || d_node_counts)) return cudaErrorInvalidValue;
-    const size_t warp = many_align(rows == 1 ? sizeof(ManyWarp<1>) : sizeof(ManyWarp<2>)) +
-                        many_align(2 * (size_t)(rows + 1) * stream_row_elems(dtype, rows) * dtype_size(dtype));
-    const size_t smem = kManyWarps * warp;
     const uint64_t need = (ntasks + kManyWarps - 1) / kManyWarps;
     KVSMC_MANY_SWITCH(dtype, {
+        const size_t smem = kManyWarps * (many_align(rows == 1 ? sizeof(ManyWarp<T, 1>) : sizeof(ManyWarp<T, 2>)) +
+                                          many_align(2 * (size_t)(rows + 1) * stream_row_elems(dtype, rows) * sizeof(T)));
         auto kern = d_node_counts ? (list ? k_count_many<T, 1, true, true> : k_count_many<T, 1, false, true>)
                     : rows == 1   ? (list ? k_count_many<T, 1, true, false> : k_count_many<T, 1, false, false>)
                                   : (list ? k_count_many<T, 2, true, false> : k_count_many<T, 2, false, false>);

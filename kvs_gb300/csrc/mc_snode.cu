@@ -305,7 +305,7 @@ struct SnMulti {
 
 // Per-CTA tables: the thresholds' bucket map and the requests' constants.
 struct SnMultiCta {
-    ThermoTables th;
+    ThermoTables<float> th;   // (values as floats)
     NodeIso iso[kStreamMaxIso];
 };
 
@@ -813,7 +813,7 @@ __global__ void __launch_bounds__(kSnThreads)
 constexpr int kScPairCap = 128;   // listed (cell, request) pairs per warp at a time
 
 struct ScMultiCta {
-    ThermoTables th;
+    ThermoTables<float> th;   // (values as floats)
     ConnIso iso[kStreamMaxIso];
     uint64_t tri[256];   // per reference case: edges per triangle, 4 bits each
     uint8_t ntri[256];

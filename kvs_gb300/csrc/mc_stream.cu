@@ -103,9 +103,9 @@ struct Tables {
 static_assert(3 * 3 * (kSegCells + 16) < (1 << 14), "edge_off packs ring offsets into 14 bits");
 
 // Per-warp state.
-struct WarpState {
+template <typename T> struct WarpState {
     uint64_t bar[3];
-    ThermoTables th;
+    ThermoTables<T> th;
     uint32_t add[32];                        // emit: per-(row, isolevel) advance of the current round
 };
 
@@ -251,12 +251,12 @@ __global__ void __launch_bounds__(kEmitThreads, KVSMC_EMIT_CTAS)
     // whose count gave up has no offsets to write at)
     if (__syncthreads_or(*status != 0 || (only_if && *only_if == 0))) return;
 
-    const size_t wstride = align128(sizeof(WarpState)) + align128(sizeof(WarpEmit)) +
+    const size_t wstride = align128(sizeof(WarpState<T>)) + align128(sizeof(WarpEmit)) +
                            align128((size_t)3 * plane_elems * sizeof(T));
     unsigned char* wbase = smem_raw + align128(sizeof(Tables)) + (size_t)warp * wstride;
-    WarpState& W = *reinterpret_cast<WarpState*>(wbase);
-    WarpEmit* WE = reinterpret_cast<WarpEmit*>(wbase + align128(sizeof(WarpState)));
-    T* ring = reinterpret_cast<T*>(wbase + align128(sizeof(WarpState)) + align128(sizeof(WarpEmit)));
+    WarpState<T>& W = *reinterpret_cast<WarpState<T>*>(wbase);
+    WarpEmit* WE = reinterpret_cast<WarpEmit*>(wbase + align128(sizeof(WarpState<T>)));
+    T* ring = reinterpret_cast<T*>(wbase + align128(sizeof(WarpState<T>)) + align128(sizeof(WarpEmit)));
     if (lane == 0) {
         for (int b = 0; b < 3; ++b) mbar_init(&W.bar[b], 1);
         fence_barrier_init();
@@ -830,7 +830,8 @@ size_t stream_row_elems(int dtype, int rows)
 size_t stream_warp_smem_bytes(int dtype, int rows)
 {
     const size_t plane = (size_t)(rows + 1) * stream_row_elems(dtype, rows) * dtype_size(dtype);
-    return align128(sizeof(WarpState)) + align128(sizeof(WarpEmit)) + align128(3 * plane);
+    const size_t state = dtype_size(dtype) == 1 ? sizeof(WarpState<uint8_t>) : sizeof(WarpState<float>);
+    return align128(state) + align128(sizeof(WarpEmit)) + align128(3 * plane);
 }
 
 size_t stream_warp_smem_offset() { return align128(sizeof(Tables)); }

@@ -53,6 +53,22 @@ def test_single_isolevel_on_and_between_integer_values(kvsmc_ctx, oracle_lib):
         vol.free()
 
 
+def test_several_isolevels_on_and_past_integer_values(kvsmc_ctx, oracle_lib):
+    rng = np.random.default_rng(9)
+    for dtype in (np.int8, np.uint8, np.int16, np.uint16):
+        i = np.iinfo(dtype)
+        v = rng.integers(i.min, i.max, (5, 6, 140), endpoint=True).astype(dtype)
+        v[0, 0, :4] = (i.min, i.max, 0, 1)
+        vol = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+        isos = [-1e30, i.min - 1.0, i.min, i.min + 0.5, -1.0, -0.0, 0.5, 1.0, 2.999999, 3.0, i.max - 0.5, float(i.max),
+                i.max + 1.0, 1e30]
+        out = extract_batch(kvsmc_ctx, [vol] * len(isos), [_abi.make_params(x, 0) for x in isos], _abi.PATH_AUTO)
+        for x, o in zip(isos, out):
+            ref = oracle_lib.extract(v, x, 0, float(i.min), float(i.max))
+            assert same_bits(o["coords"], ref["coords"]) and same_bits(o["normals"], ref["normals"]), (dtype, x)
+        vol.free()
+
+
 @pytest.mark.parametrize("mode", [0, 2])
 def test_crowded_isolevels_and_extreme_values(kvsmc_ctx, mode):
     """Equal isolevels and several in one bucket of the threshold table beside

@@ -18,10 +18,12 @@
 //   * a staged plane's values are not needed once its masks are formed, so two
 //     buffers a warp suffice, and the next copies start before the pairs are
 //     worked on.
-// Bound by instruction issue (70% busy) and shared-memory latency.  Four CTAs
-// an SM (64 registers, 56 KB) instead of three: 1% and 3%.  640x704x600 f32, 16
-// isolevels: 1532 us with the lanes' loops, 1500 us; 1024x768x640 u16, 4
-// isolevels: 2735 -> 2312 us.
+// Bound by instruction issue (70% busy) and shared-memory latency, and above all
+// it must not spill: 32 warps an SM at 64 registers took 1500 and 2312 us below,
+// 24 at 80 take 1220 and 1884, with the lower plane's masks read back from
+// shared memory and the task's addresses kept there.  640x704x600 f32, 16
+// isolevels: 1532 us with the lanes' loops, 1220 us; 1024x768x640 u16, 4
+// isolevels: 2735 -> 1884 us.
 //
 // NODES: the shared-vertex modes' vertices per node unit too (plane, node row,
 // 256-node segment; those whose node segments are their cell segments).  A
@@ -59,11 +61,15 @@ template <typename T, int R> struct alignas(16) ManyWarp {
     // past the last cell plane and past both, 10 bits each
     uint32_t cnt[32];
     uint64_t bar[2];
+    uint16_t* counts;                       // the task's counters, pair numbers, list entries and node counters
+    uint16_t* pairs;
+    uint32_t* list;
+    uint32_t* nodes;
     ThermoTables<T> th;
 };
 
 template <typename T, int R, bool LIST, bool NODES>
-__global__ void __launch_bounds__(kManyThreads, 4)
+__global__ void __launch_bounds__(kManyThreads, 3)
     k_count_many(const StreamGroup* __restrict__ groups, int ngroups, uint64_t ntasks,
                  const StreamIso* __restrict__ isos, uint16_t* __restrict__ unit_counts, int* __restrict__ status,
                  unsigned long long* __restrict__ next_task, uint32_t wait_polls, PairList pl,
@@ -92,7 +98,7 @@ __global__ void __launch_bounds__(kManyThreads, 4)
     __syncwarp();
     const uint32_t half = lane / LPR, xl = (lane % LPR) * 8;   // this lane's row of the task and first cell
     const unsigned lt = (1u << lane) - 1u;
-    uint64_t lcur = 0, lend = 0;   // this warp's entries of the pair list
+    uint32_t lcur = 0, lend = 0;   // this warp's entries of the pair list (less than 2^31 while it is not full)
     bool lfull = false;
     uint32_t ph = 0;   // per ring buffer: parity of its next completion
     int gi = 0, gcur = -1;
@@ -164,42 +170,40 @@ __global__ void __launch_bounds__(kManyThreads, 4)
             for (uint32_t i = 0; i < issued; ++i) issue(i);
         }
         const bool row_ok = y + half < cy;
-        // the lane's unit and (isolevel, unit) counter at plane z0 (the group's
-        // fields are read once per task: the stores below could alias them)
+        // where the task's counters at plane z0 and row y lie (in shared memory: the
+        // loop below has no registers to spare)
         const uint32_t plane_units = cy * wpr;
-        const uint64_t unit0 = ((uint64_t)z0 * cy + y + half) * wpr + seg;
+        if (lane == 0) {
+            const uint64_t unit0 = ((uint64_t)z0 * cy + y) * wpr + seg;
+            W.counts = unit_counts + G.unit_base + unit0 * (uint32_t)niso;
+            if (LIST) {
+                W.pairs = pl.unit_pairs + G.pair_base + unit0;
+                W.list = pl.unit_list + G.pair_base + unit0;
+            }
+            if (NODES)
+                W.nodes = G.node_units ? node_counts + G.node_base + ((uint64_t)z0 * G.vol.ny + y) * wpr + seg : nullptr;
+        }
         // lane 16 h + k: the counter of isolevel k in row y + h
         const uint32_t ch = lane >> 4, ck = lane & 15u;
         const bool my_count = ch < (uint32_t)R && ck < (uint32_t)niso && y + ch < cy;
-        uint16_t* const ucount =
-            unit_counts + G.unit_base + (((uint64_t)z0 * cy + y + ch) * wpr + seg) * (uint32_t)niso + ck;
-        uint16_t* upairs = LIST ? pl.unit_pairs + G.pair_base + unit0 : nullptr;
-        uint32_t* ulist = LIST ? pl.unit_list + G.pair_base + unit0 : nullptr;
-        // with vertices: lane k's counter of isolevel k's node unit at plane z0
         const bool last_row = y + 1 == cy;
-        const uint64_t plane_nodes = (uint64_t)G.vol.ny * wpr;
-        uint32_t* const ncount = NODES && G.node_units ? node_counts + G.node_base + lane * G.node_units +
-                                                             ((uint64_t)z0 * G.vol.ny + y) * wpr + seg
-                                                       : nullptr;
         const int lim = row_ok ? (int)cx - (int)((uint32_t)xoff + xl) : 0;   // this lane's cells inside the volume (if < 8)
-        // masks of this lane's nodes in rows half and half + 1 of plane i, in
-        // registers and in the plane's mask rows
+        // masks of plane i's nodes into its mask rows: each lane's 8 in rows half
+        // and half + 1 (left in P0, P1 too), a lane per row for the node behind the
+        // last cell
         auto plane_masks = [&](uint32_t i, uint32_t* P0, uint32_t* P1) {
-            const T* p = ring + (i & 1u) * plane_elems + half * row_elems;
-            row_masks<T>(p, xl, W.th, bs, bo, P0);
-            row_masks<T>(p + row_elems, xl, W.th, bs, bo, P1);
-            uint16_t* m = W.mask[i & 1u][half];
-            *reinterpret_cast<uint4*>(m + xl) = make_uint4(P0[0], P0[1], P0[2], P0[3]);
-            if (xl + 8 == SEG) m[SEG] = (uint16_t)P0[4];
-            if (half == R - 1) {
-                m += kMaskRow<R>;
-                *reinterpret_cast<uint4*>(m + xl) = make_uint4(P1[0], P1[1], P1[2], P1[3]);
-                if (xl + 8 == SEG) m[SEG] = (uint16_t)P1[4];
-            }
+            const T* p = ring + (i & 1u) * plane_elems;
+            uint16_t* m = W.mask[i & 1u][0];
+            row_masks<T, 8>(p + half * row_elems, xl, W.th, bs, bo, P0);
+            *reinterpret_cast<uint4*>(m + half * kMaskRow<R> + xl) = make_uint4(P0[0], P0[1], P0[2], P0[3]);
+            row_masks<T, 8>(p + (half + 1) * row_elems, xl, W.th, bs, bo, P1);
+            if (half == R - 1)
+                *reinterpret_cast<uint4*>(m + R * kMaskRow<R> + xl) = make_uint4(P1[0], P1[1], P1[2], P1[3]);
+            if (lane <= (unsigned)R)
+                m[lane * kMaskRow<R> + SEG] = (uint16_t)thermo_mask(W.th, bs, bo, (float)p[lane * row_elems + SEG]);
         };
         bool dead = false, pa_valid = false, brick_skip = false;
         uint32_t acq = 0;
-        uint32_t PA0[5], PA1[5];   // masks of plane z, this lane's rows (carried from the previous step)
         for (uint32_t z = z0; z < z1; ++z) {
             const uint32_t s = z - z0;
             bool ok = true;
@@ -213,9 +217,9 @@ __global__ void __launch_bounds__(kManyThreads, 4)
                 break;
             }
             if (bricks && (s == 0 || z % kBrickPlanes == 0)) brick_skip = brick_empty(z);
-            uint32_t PB0[5], PB1[5];
+            uint32_t PB0[4], PB1[4];
             if (!brick_skip) {
-                if (!pa_valid) plane_masks(s, PA0, PA1);
+                if (!pa_valid) plane_masks(s, PB0, PB1);
                 plane_masks(s + 1, PB0, PB1);
             }
             // plane z's values are consumed, and plane z + 1's once their masks are
@@ -238,12 +242,17 @@ __global__ void __launch_bounds__(kManyThreads, 4)
             // highest corner (thermometer codes: OR = the highest, AND = the lowest)
             uint32_t act[4], m = 0;
             {
-                uint32_t co[5], ca[5];
-#pragma unroll
-                for (int w = 0; w < 5; ++w) {
-                    co[w] = PA0[w] | PA1[w] | PB0[w] | PB1[w];
-                    ca[w] = PA0[w] & PA1[w] & PB0[w] & PB1[w];
-                }
+                // (plane z's masks come back from shared memory: carried in registers
+                // they made the compiler spill)
+                const uint16_t* ma = W.mask[s & 1u][half] + xl;
+                const uint16_t* mb = W.mask[(s + 1) & 1u][half] + xl;
+                const uint4 A0 = *reinterpret_cast<const uint4*>(ma);
+                const uint4 A1 = *reinterpret_cast<const uint4*>(ma + kMaskRow<R>);
+                const uint32_t a0 = ma[8], a1 = ma[kMaskRow<R> + 8], b0 = mb[8], b1 = mb[kMaskRow<R> + 8];
+                const uint32_t co[5] = {A0.x | A1.x | PB0[0] | PB1[0], A0.y | A1.y | PB0[1] | PB1[1],
+                                        A0.z | A1.z | PB0[2] | PB1[2], A0.w | A1.w | PB0[3] | PB1[3], a0 | a1 | b0 | b1};
+                const uint32_t ca[5] = {A0.x & A1.x & PB0[0] & PB1[0], A0.y & A1.y & PB0[1] & PB1[1],
+                                        A0.z & A1.z & PB0[2] & PB1[2], A0.w & A1.w & PB0[3] & PB1[3], a0 & a1 & b0 & b1};
 #pragma unroll
                 for (int w = 0; w < 4; ++w) {
                     const uint32_t o = co[w] | __funnelshift_r(co[w], co[w + 1], 16);
@@ -253,8 +262,6 @@ __global__ void __launch_bounds__(kManyThreads, 4)
                     m += __popc(act[w]);
                 }
             }
-#pragma unroll
-            for (int w = 0; w < 5; ++w) { PA0[w] = PB0[w]; PA1[w] = PB1[w]; }
             pa_valid = true;
             uint32_t inc = m;
 #pragma unroll
@@ -269,9 +276,10 @@ __global__ void __launch_bounds__(kManyThreads, 4)
                     const uint32_t want = npairs > kPairRun ? npairs : kPairRun;
                     unsigned long long at = 0;
                     if (lane == 0) at = atomicAdd(pl.cursor, (unsigned long long)want);
-                    lcur = __shfl_sync(FULL, at, 0);
+                    at = __shfl_sync(FULL, at, 0);
+                    lcur = (uint32_t)at;
                     lend = lcur + want;
-                    if (lend > pl.cap && !lfull) {
+                    if (at + want > pl.cap && !lfull) {
                         lfull = true;
                         if (lane == 0) atomicExch(pl.overflow, 1);
                     }
@@ -280,8 +288,9 @@ __global__ void __launch_bounds__(kManyThreads, 4)
                 const uint32_t before = R == 1 ? 0u : __shfl_sync(FULL, inc, LPR - 1);
                 if (lane % LPR == 0 && row_ok) {
                     const uint32_t b = half ? before : 0u;
-                    upairs[(uint64_t)s * plane_units] = (uint16_t)((R == 1 || half ? npairs : before) - b);
-                    ulist[(uint64_t)s * plane_units] = (uint32_t)lcur + b;
+                    const uint64_t u = (uint64_t)s * plane_units + half * wpr;
+                    W.pairs[u] = (uint16_t)((R == 1 || half ? npairs : before) - b);
+                    W.list[u] = lcur + b;
                 }
             }
             const uint32_t my_first = inc - m;
@@ -306,7 +315,7 @@ __global__ void __launch_bounds__(kManyThreads, 4)
                     const bool has = r0 + lane < nfill;
                     const uint32_t e = has ? W.buf[r0 + lane] : 0u;
                     const uint32_t h = R == 1 ? 0u : (e & 0xffu) / SEG, x = (e & 0xffu) & (SEG - 1), k = e >> 8;
-                    if (LIST && has && !lfull) pl.list[lcur + fill0 + r0 + lane] = (uint16_t)(x | (k << 8));
+                    if (LIST && has && !lfull) pl.list[(uint64_t)lcur + fill0 + r0 + lane] = (uint16_t)(x | (k << 8));
                     // corner code: bit r: row r's node x, bit 4 + r: its node x + 1
                     const uint16_t* a = W.mask[s & 1u][h] + x;
                     const uint16_t* b = W.mask[(s + 1) & 1u][h] + x;
@@ -346,13 +355,15 @@ __global__ void __launch_bounds__(kManyThreads, 4)
             }
             lcur += npairs;
             if (my_count) {
-                ucount[(uint64_t)s * plane_units * (uint32_t)niso] = (uint16_t)W.cnt[lane];
-                if (NODES && ncount) {
-                    ncount[s * plane_nodes] = W.cnt[lane] >> 16;
+                W.counts[((uint64_t)s * plane_units + ch * wpr) * (uint32_t)niso + ck] = (uint16_t)W.cnt[lane];
+                if (NODES && W.nodes) {
+                    const uint64_t plane_nodes = (uint64_t)G.vol.ny * wpr;
+                    uint32_t* n = W.nodes + ck * G.node_units + s * plane_nodes;
                     const uint32_t v = W.cnt[16 + lane];
-                    if (last_row) ncount[s * plane_nodes + wpr] = v & 0x3ffu;
-                    if (z + 1 == cz) ncount[(s + 1) * plane_nodes] = (v >> 10) & 0x3ffu;
-                    if (last_row && z + 1 == cz) ncount[(s + 1) * plane_nodes + wpr] = v >> 20;
+                    n[0] = W.cnt[lane] >> 16;
+                    if (last_row) n[wpr] = v & 0x3ffu;
+                    if (z + 1 == cz) n[plane_nodes] = (v >> 10) & 0x3ffu;
+                    if (last_row && z + 1 == cz) n[plane_nodes + wpr] = v >> 20;
                 }
             }
             __syncwarp();

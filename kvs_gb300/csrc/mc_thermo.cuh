@@ -131,19 +131,18 @@ __device__ __forceinline__ void load8(const int16_t* row, uint32_t x0, float* o)
     }
 }
 
-// Thermometer masks of the 9 nodes x0 .. x0+8 of a staged row (x0 a multiple of
-// 8): bit k set when the value is above isolevel k's threshold (v > t_k;
+// Thermometer masks of the N (8 or 9) nodes from x0 on of a staged row (x0 a
+// multiple of 8): bit k set when the value is above isolevel k's threshold (v > t_k;
 // thresholds sorted, so the set bits are 0 .. q-1), packed two nodes per word
 // (node 2m in the low half of word m, node 2m+1 in the high half; word 4 holds
 // node 8).
-template <typename T>
+template <typename T, int N = 9>
 __device__ __forceinline__ void row_masks(const T* row, uint32_t x0, const ThermoTables<T>& W, float bs, float bo,
                                           uint32_t* P)
 {
     uint32_t q[9];
     if constexpr (sizeof(T) == 1) {
         uint2 w = *reinterpret_cast<const uint2*>(row + x0);
-        const uint32_t last = (uint8_t)row[x0 + 8] ^ (kThermoFlip<T> & 0xffu);
         w.x ^= kThermoFlip<T>;
         w.y ^= kThermoFlip<T>;
 #pragma unroll
@@ -151,18 +150,18 @@ __device__ __forceinline__ void row_masks(const T* row, uint32_t x0, const Therm
             q[i] = W.lut[(w.x >> (8 * i)) & 255u];
             q[4 + i] = W.lut[(w.y >> (8 * i)) & 255u];
         }
-        q[8] = W.lut[last];
+        if (N == 9) q[8] = W.lut[(uint8_t)row[x0 + 8] ^ (kThermoFlip<T> & 0xffu)];
     } else {
         float v[9];
         load8(row, x0, v);
-        v[8] = (float)row[x0 + 8];
+        if (N == 9) v[8] = (float)row[x0 + 8];
 #pragma unroll
-        for (int i = 0; i < 9; ++i) q[i] = W.lut[bucket_index(v[i], bs, bo)];
+        for (int i = 0; i < N; ++i) q[i] = W.lut[bucket_index(v[i], bs, bo)];
 #pragma unroll
-        for (int i = 0; i < 9; ++i) q[i] += v[i] > W.thr[q[i]] ? 1u : 0u;
+        for (int i = 0; i < N; ++i) q[i] += v[i] > W.thr[q[i]] ? 1u : 0u;
         if (W.several) {
 #pragma unroll
-            for (int i = 0; i < 9; ++i)
+            for (int i = 0; i < N; ++i)
                 while (v[i] > W.thr[q[i]]) ++q[i];   // (ends at the +inf after the last one)
         }
     }
@@ -171,7 +170,7 @@ __device__ __forceinline__ void row_masks(const T* row, uint32_t x0, const Therm
 #pragma unroll
     for (int m = 0; m < 4; ++m)
         P[m] = (1u << q[2 * m]) + ((1u << q[2 * m + 1]) << 16) - 0x10001u;
-    P[4] = (1u << q[8]) - 1u;
+    if (N == 9) P[4] = (1u << q[8]) - 1u;
 }
 
 // The row word of cell i (0..7): node i in the low half, node i+1 in the high half.

@@ -31,8 +31,8 @@
 // task writes less than 2^16 triangles, so places are counted from the task's
 // start and the isolevels' 64-bit addresses are formed once per task), and an
 // edge's corners and axis are one byte of one table.  640x704x600 f32, 16
-// isolevels: 3810 -> 3635 us (40% of the 9 GB it writes at the copy rate);
-// 1024x768x640 u16, 4 isolevels: 2519 -> 2296 us.
+// isolevels: 3810 -> 3625 us (40% of the 9 GB it writes at the copy rate);
+// 1024x768x640 u16, 4 isolevels: 2519 -> 2280 us.
 #include <cuda_runtime.h>
 
 #include "mc_emit.cuh"
@@ -51,13 +51,26 @@ namespace {
 
 __device__ PairTables d_pair_tables = make_pair_tables();
 
+// An isolevel's constants: what a vertex needs is three 16-byte reads.  err is
+// infinite where the certificate does not apply (it then decides nothing).
+struct alignas(16) PairIso {
+    float ih, il, err, vmin;
+    float vmax, mc[3];
+    float sc[3], thr;
+    float* coords;
+    float* normals;
+    uint64_t cap_tris;
+    uint64_t pad;
+};
+static_assert(sizeof(PairIso) == 80, "lanes of different isolevels meet in different banks");
+
 struct alignas(16) PairOut {
     float* coords;
     float* normals;
 };
 
 template <typename V> struct alignas(16) PairWarp {
-    IsoConst ic[kStreamMaxIso];
+    PairIso ic[kStreamMaxIso];
     float4 pv[kPairVerts];     // vertex pool: x, y, z, unused (one 16-byte access per vertex)
     PairOut out[kStreamMaxIso];   // per isolevel: where the task's triangles go
     uint32_t room[kStreamMaxIso]; // and how many of them may be written
@@ -111,7 +124,21 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
         const int niso = G.niso, iso_begin = G.iso_begin;
         if (gi != gcur) {
             __syncwarp();
-            if (lane < (unsigned)niso) fill_iso(W.ic[lane], isos[iso_begin + lane], totals, iso_begin + (int)lane);
+            if (lane < (unsigned)niso) {
+                const StreamIso& I = isos[iso_begin + lane];
+                PairIso& c = W.ic[lane];
+                c.ih = I.f.ih;
+                c.il = I.f.il;
+                c.err = I.f.lean_ok ? I.f.iso_err : __int_as_float(0x7f800000);
+                c.vmin = I.f.vmin_f;
+                c.vmax = I.f.vmax_f;
+                c.thr = I.f.f_thr;
+                for (int a = 0; a < 3; ++a) { c.mc[a] = I.ip.min_coord[a]; c.sc[a] = I.ip.scale[a]; }
+                // a request that does not fit its outputs is not written at all
+                c.coords = totals && totals[iso_begin + (int)lane] > I.cap_tris ? nullptr : I.coords;
+                c.normals = I.normals;
+                c.cap_tris = I.cap_tris;
+            }
             live = __any_sync(FULL, lane < (unsigned)niso && W.ic[lane & 15u].coords != nullptr);
             gcur = gi;
         }
@@ -126,7 +153,7 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
             const uint64_t pi = isos[iso_begin + lane].plane_index;
             const uint64_t at = plane_base[pi + z] - plane_base[pi] +
                                 unit_offsets[G.unit_base + ((uint64_t)z * ((G.vol.ny - 1) * G.wpr) + u0) * niso + lane];
-            const IsoConst& c = W.ic[lane];
+            const PairIso& c = W.ic[lane];
             W.out[lane] = PairOut{c.coords + 9 * at, c.normals + 3 * at};
             W.room[lane] = !c.coords || c.cap_tris <= at ? 0u
                            : c.cap_tris - at < 0xffffu ? (uint32_t)(c.cap_tris - at) : 0xffffu;
@@ -148,10 +175,11 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
                 x += e & 0xffu;
                 k = e >> 8;
                 code = pair_corners<T, V>(vz + (uint64_t)y * pitch + x, pitch, slice, W.cv[lane], [&](T v) -> bool {
-                    if constexpr (kPairFast<T>) return (float)v > W.ic[k].f.f_thr;
+                    if constexpr (kPairFast<T>) return (float)v > W.ic[k].thr;
                     else return above(isos[iso_begin].cls, v);   // (one isolevel per group)
                 });
             }
+            const float fy = __uint2float_rn(y);   // (rows below 2^24: exact)
             const uint32_t cnt = has ? TB.counts[code] : 0u;
             const uint32_t ne0 = cnt >> 3;
             uint32_t vpre = 0;
@@ -196,28 +224,38 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
                 const uint32_t q = seen + (uint32_t)__popc(starts & (lt | (1u << lane))) - 1u;
                 seen += (uint32_t)__popc(starts);
                 const uint32_t qe = __shfl_sync(FULL, pe, q);
-                const uint32_t qy = __shfl_sync(FULL, y, q);
+                const float qy = __shfl_sync(FULL, fy, q);
                 const uint32_t ed = TB.edges[(qe >> 16) & 255u][hv ? j - (qe >> 24) : 0u];
                 const uint32_t c0 = ed & 7u, c1 = (ed >> 3) & 7u;
                 const int axis = (int)(ed >> 6);
                 const V va = W.cv[q][c0], vb = W.cv[q][c1];
                 const uint32_t qx = qe & 0xfffu, qk = (qe >> 12) & 15u;
                 // corner coordinates: integers below 2^24, exact as floats
-                const float ax = __uint2float_rn(qx + (c0 & 1u)), ay = __uint2float_rn(qy + ((c0 >> 1) & 1u));
+                const float ax = __uint2float_rn(qx + (c0 & 1u)), ay = __fadd_rn(qy, (c0 & 2u) ? 1.0f : 0.0f);
                 const float az = __fadd_rn(fz, (c0 & 4u) ? 1.0f : 0.0f);
                 const bool up = c1 > c0;
                 float3 v;
                 if constexpr (kPairFast<T>) {
                     const float a = axis == 0 ? ax : (axis == 1 ? ay : az);
-                    const IsoRegs I = load_iso(W.ic[qk]);
+                    const float4* ic = reinterpret_cast<const float4*>(&W.ic[qk]);
+                    const float4 i0 = ic[0], i1 = ic[1], i2 = ic[2];
+                    FastIso f;
+                    f.ih = i0.x;
+                    f.il = i0.y;
+                    f.iso_err = i0.z;
+                    f.vmin_f = i0.w;
+                    f.vmax_f = i1.x;
+                    f.lean_ok = 1;
                     float r;
-                    const bool good = fast_axis_lean<(sizeof(T) < 4)>(va, vb, a, up, I.f, r);
-                    v.x = __fmul_rn(__fadd_rn(axis == 0 ? r : ax, I.mc[0]), I.sc[0]);
-                    v.y = __fmul_rn(__fadd_rn(axis == 1 ? r : ay, I.mc[1]), I.sc[1]);
-                    v.z = __fmul_rn(__fadd_rn(axis == 2 ? r : az, I.mc[2]), I.sc[2]);
-                    if (hv && !good)   // (about one in 10^5) the exact FP64 sequence
-                        v = edge_vertex_axis(I.f, I.mc, I.sc, isos[iso_begin + qk].ip, va, vb, ax, ay, az, axis,
+                    const bool good = fast_axis_lean<(sizeof(T) < 4)>(va, vb, a, up, f, r);
+                    v.x = __fmul_rn(__fadd_rn(axis == 0 ? r : ax, i1.y), i2.x);
+                    v.y = __fmul_rn(__fadd_rn(axis == 1 ? r : ay, i1.z), i2.y);
+                    v.z = __fmul_rn(__fadd_rn(axis == 2 ? r : az, i1.w), i2.z);
+                    if (hv && !good) {   // (about one in 10^5) the exact FP64 sequence
+                        const StreamIso& I = isos[iso_begin + qk];
+                        v = edge_vertex_axis(I.f, I.ip.min_coord, I.ip.scale, I.ip, va, vb, ax, ay, az, axis,
                                              __fadd_rn(a, up ? 1.0f : -1.0f));
+                    }
                 } else {
                     const float d = up ? 1.0f : -1.0f;
                     v = interpolate_exact_axis(isos[iso_begin].ip, va, vb, ax, ay, az, axis == 0 ? __fadd_rn(ax, d) : ax,

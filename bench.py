@@ -980,8 +980,8 @@ def run_ours(args, rank, world, local):
         # however many isovalues share the launch, + the outputs: VertexNormal
         # 24 B per vertex (coords, normals) + 12 B per triangle (connections),
         # PolygonNormal 12 B per vertex + 24 B per triangle
-        readers = ("stream_count", "snode_count", "snode_emit", "snode_emit_multi", "sconnect", "sconnect_multi",
-                   "gather_cell_count", "gather_node_count", "gather_node_emit", "gather_connect")
+        readers = ("count_one", "count_many", "snode_count", "snode_emit", "snode_emit_multi", "sconnect",
+                   "sconnect_multi", "gather_cell_count", "gather_node_count", "gather_node_emit", "gather_connect")
         passes = sum(prof[k][0] for k in readers if k in prof) / args.steps
         outputs = 24 * nvert + 12 * ntri if mode == _abi.MODE_SHARED_VERTEX_NORMAL else 12 * nvert + 24 * ntri
         algo_bytes = int(nx * ny * nz * dt.itemsize * passes + outputs)
@@ -1367,7 +1367,7 @@ def run_batch(args, rank, world, local):
     hbm, peak_kind = peaks()
     algo = in_bytes + 48 * ntri
     emit_ms = sum(v[1] for k, v in prof.items() if k == "stream_emit")
-    count_ms = sum(v[1] for k, v in prof.items() if k == "stream_count")
+    count_ms = sum(v[1] for k, v in prof.items() if k in ("count_one", "count_many"))
     # the per-kind launches overlap, so the roofline is taken over the whole
     # replayed step (count + scans + emit): algorithmic bytes / step time
     roofline = {"kernel": "whole plan replay", "bound": "hbm", "achieved": round(algo / (ms_graph * 1e-3) / 1e9, 1),

@@ -114,11 +114,10 @@ kvsmc_status kvsmc_set_stream(kvsmc_context* ctx, void* cuda_stream);
 kvsmc_status kvsmc_synchronize(kvsmc_context* ctx);
 /* Number of kernels this context has launched since creation. */
 uint64_t kvsmc_kernel_launches(const kvsmc_context* ctx);
-/* Kernel family: 0 (default) = streaming kernels for requests on 8/16-bit and
- * float32 volumes (duplicated mode; in the shared-vertex modes the node and
- * connection passes), gather kernels for the rest; 1 = gather kernels for
- * everything.  Both give identical results.  No counterpart in the reference
- * (which has one CPU loop). */
+/* Kernel family: 0 (default) = streaming kernels for volumes of every value
+ * type up to 4097 nodes wide (finite isolevels), gather kernels for the rest;
+ * 1 = gather kernels for everything.  Both give identical results.  No
+ * counterpart in the reference (which has one CPU loop). */
 kvsmc_status kvsmc_set_kernel_path(kvsmc_context* ctx, int32_t path);
 
 /* ------------------------------------------------------------------ volumes */
@@ -575,9 +574,9 @@ kvsmc_status kvsmc_write_ply_host(kvsmc_context* ctx, const char* path, const fl
  * CPU loop and nothing to tune. */
 typedef struct kvsmc_tune_choice {
     int32_t rows;          /* cell rows per warp task: 1 (256-cell row segments) or 2 (two 128-cell rows) */
-    int32_t tasks_per_sm;  /* warp tasks per SM a launch is cut into (sets cell planes per task, 4..64) */
+    int32_t tasks_per_sm;  /* warp tasks per SM a launch is cut into (sets cell planes per task, 2 or 4..64) */
     int32_t ctas_per_sm;   /* resident CTAs per SM of the persistent launches (capped by what fits) */
-    int32_t scan_threads;  /* unit-scan tile: 64, 128 or 256 units per CTA pass */
+    int32_t scan_threads;  /* unit scan: 64, 128 or 256 threads per CTA */
 } kvsmc_tune_choice;
 
 /* One row of a tuning table. */

@@ -258,8 +258,6 @@ void StreamBatch::plan_tables()
             L.ntasks += stream_tasks(v, rows, g.wpr, g.zchunk);
             g.seg_elems = (uint32_t)kvsmc::stream_row_elems(dt, rows);
             g.seg_copy_bytes = g.seg_elems * (uint32_t)kvsmc::dtype_size(dt);
-            g.warp_smem_bytes = (uint32_t)kvsmc::stream_warp_smem_bytes(dt, rows);
-            g.warp_smem_offset = (uint32_t)kvsmc::stream_warp_smem_offset();
             // isolevels sorted by threshold
             std::vector<std::pair<float, Item*>> sorted;
             for (Item* it : l) sorted.push_back({make_fast(it->params.isolevel, it->vmin, it->vmax, dt).f_thr, it});

@@ -67,7 +67,7 @@ struct StreamBatch {
     std::vector<Launch1> launches;
     uint64_t unit_elems = 0;     // (unit, isolevel) counters
     uint32_t scan_blocks = 0;    // unit-scan blocks: one per (group, z)
-    int scan_threads = 256;      // unit-scan tile
+    int scan_threads = 256;      // unit-scan CTA
     uint64_t iso_planes = 0;     // (isolevel, z) planes
     // the count pass also counts the shared-vertex modes' vertices per
     // (isolevel, node unit) for the groups that take one row per task and

@@ -72,7 +72,6 @@ void vertex_normals_carve(Job& j, uint64_t ntri, uint64_t nvert, void* scratch);
 cudaError_t launch_vertex_normals(const Job& j, uint64_t ntri, uint64_t nvert, const Launch& L);
 
 // ---- streaming kernels (mc_stream.cu): duplicated mode, batched
-constexpr int kStreamThreads = 256;   // 8 independent warps per CTA
 constexpr int kStreamMaxIso = 16;     // isolevels of one volume per group
 constexpr int kStreamBuckets = 128;   // threshold lookup buckets
 constexpr int kStreamSegCells = 256;  // cells per warp step (one 256-cell row segment, or two of 128)
@@ -103,8 +102,6 @@ struct StreamGroup {
     uint32_t plane_begin;    // first unit-scan block of this group (one per z)
     uint32_t seg_elems;      // staged elements per node row (16-byte multiple)
     uint32_t seg_copy_bytes; // bytes copied per node row (last segment: fewer)
-    uint32_t warp_smem_bytes;
-    uint32_t warp_smem_offset;
     float bs, bo;            // bucket(v) = floor(kStreamBuckets * sat(v * bs + bo)), in [0, kStreamBuckets]
     const float2* bricks;    // the volume's brick min/max table, or null
     int32_t skip_emit;       // 1: no isolevel of the group is written by this emit launch
@@ -159,8 +156,6 @@ struct IngestOut {
 cudaError_t launch_ingest(const VolumeView& v, const void* src, float2* bricks, IngestOut* d_out, const Launch& L);
 
 size_t stream_shared_bytes(int dtype, int rows);
-size_t stream_warp_smem_bytes(int dtype, int rows);
-size_t stream_warp_smem_offset();
 size_t stream_row_elems(int dtype, int rows);
 // The emit that classifies the volume again.
 // d_next_task: a zeroed u64 per launch (the persistent warps' task counter).
@@ -201,7 +196,7 @@ cudaError_t launch_wide(int dtype, const StreamGroup* d_groups, int ngroups, uin
                         const StreamIso* d_isos, const uint16_t* d_unit_counts, const uint32_t* d_unit_offsets,
                         const uint64_t* d_plane_base, int* d_status, unsigned long long* d_next_task, const Launch& L,
                         uint64_t task0, const uint64_t* d_totals, const int* d_only_if);
-// scan_threads: units per CTA pass (64, 128 or 256; 0 = 256).
+// scan_threads: threads per CTA (64, 128 or 256; 0 = 256).
 cudaError_t launch_unit_scan(const StreamGroup* d_groups, int ngroups, uint32_t nplanes, const StreamIso* d_isos,
                              const uint16_t* d_unit_counts, uint32_t* d_unit_offsets, uint32_t* d_plane_totals,
                              const Launch& L, int scan_threads = 0);

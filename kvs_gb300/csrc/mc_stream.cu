@@ -817,14 +817,14 @@ size_t stream_row_elems(int dtype, int rows)
     return ((((size_t)kSegCells / rows + 1) * es + 15) / 16) * 16 / es;
 }
 
-size_t stream_warp_smem_bytes(int dtype, int rows)
+static size_t stream_warp_smem_bytes(int dtype, int rows)
 {
     const size_t plane = (size_t)(rows + 1) * stream_row_elems(dtype, rows) * dtype_size(dtype);
     const size_t state = dtype_size(dtype) == 1 ? sizeof(WarpState<uint8_t>) : sizeof(WarpState<float>);
     return align128(state) + align128(sizeof(WarpEmit)) + align128(3 * plane);
 }
 
-size_t stream_warp_smem_offset() { return align128(sizeof(Tables)); }
+static size_t stream_warp_smem_offset() { return align128(sizeof(Tables)); }
 
 size_t stream_shared_bytes(int dtype, int rows)
 {

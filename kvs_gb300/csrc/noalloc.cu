@@ -128,8 +128,6 @@ extern "C" kvsmc_status kvsmc_extract_noalloc(const void* d_values, kvsmc_dtype 
     g.plane_begin = 0;
     g.seg_elems = (uint32_t)stream_row_elems(dtype, rows);
     g.seg_copy_bytes = g.seg_elems * (uint32_t)es;
-    g.warp_smem_bytes = (uint32_t)stream_warp_smem_bytes(dtype, rows);
-    g.warp_smem_offset = (uint32_t)stream_warp_smem_offset();
 
     // carve the static array
     size_t off = 0;

@@ -22,7 +22,7 @@
 // word) with 24 warps an SM; 32 (64 registers, and less L1) take 771 us, 24
 // 745.  385x320x352 f32, 8 isolevels with vertex normals: classifying
 // connection pass 857 us, then lists by atomics 332 and sorted sums 303; now
-// 745 and 242.
+// 727 and 242 (745 before a round's list entries were read a round ahead).
 #include <cuda_runtime.h>
 
 #include "mc_device.cuh"
@@ -156,16 +156,22 @@ __global__ void __launch_bounds__(kPairThreads, 3)
         const T* vz = static_cast<const T*>(G.vol.data) + (uint64_t)z * slice;
         const float fz = __uint2float_rn(z);
         uint32_t taken = 0;
+        // the round's list entries, read a round ahead
+        uint32_t next_x, next_y, next_e = 0;
+        auto fetch = [&](uint32_t p0) {
+            const uint32_t at = pair_entry(B, p0 + lane, next_x, next_y);
+            if (p0 + lane < B.npairs) next_e = pl.list[at];
+        };
+        fetch(0);
         for (uint32_t r0 = 0; r0 < B.npairs; r0 += taken) {
             // ---- one pair per lane, as many as the vertex pool holds
             bool has = r0 + lane < B.npairs;
-            uint32_t x, y;
-            const uint32_t at = pair_entry(B, r0 + lane, x, y);
+            uint32_t x = next_x;
+            const uint32_t y = next_y;
             uint32_t k = 0, code = 0;
             if (has) {
-                const uint32_t e = pl.list[at];
-                x += e & 0xffu;
-                k = e >> 8;
+                x += next_e & 0xffu;
+                k = next_e >> 8;
                 code = pair_corners<T, V>(vz + (uint64_t)y * pitch + x, pitch, slice, W.cv[lane], [&](T v) -> bool {
                     if constexpr (kPairFast<T>) return (float)v > s_iso[k].f.f_thr;
                     else return above(isos[iso_begin].cls, v);   // (one isolevel per group)
@@ -181,6 +187,7 @@ __global__ void __launch_bounds__(kPairThreads, 3)
             has = has && vpre + ne0 <= (uint32_t)kPairVerts;   // a suffix of lanes waits
             taken = (uint32_t)__popc(__ballot_sync(FULL, has));
             const uint32_t nv = __shfl_sync(FULL, vpre + ne0, taken - 1);
+            if (r0 + taken < B.npairs) fetch(r0 + taken);
             const uint32_t nt = has ? cnt & 7u : 0u;
             const bool item = has && ne0 != 0;   // (a pair of a request that is not written has none)
             const uint32_t pe = x | (k << 12) | (code << 16) | (vpre << 24);   // (x < 4096; vpre < kPairVerts)
@@ -312,7 +319,7 @@ __global__ void __launch_bounds__(kPairThreads, 3)
 // 32-node word) collect the word's flags in shared memory; the first of them
 // stores the word, with its own first vertex as the word's; a word that goes on
 // in the next round gets the rest by atomics.
-// 385x320x352 f32, 8 isolevels: 711 us classifying every node again, 302 us.
+// 385x320x352 f32, 8 isolevels: 711 us classifying every node again, 291 us.
 struct __align__(16) NodeConst {
     FastIso f;
     float mc[3], sc[3];
@@ -387,16 +394,20 @@ __global__ void __launch_bounds__(kPairThreads, 4)
         uint32_t run = 0;   // lane k: the task's vertices of isolevel k so far
         const T* vz = static_cast<const T*>(G.vol.data) + (uint64_t)z * slice;
         const float fz = __uint2float_rn(zn);
+        uint32_t next_x, next_y, next_e = 0;
+        auto fetch = [&](uint32_t p0) {
+            const uint32_t at = pair_entry(B, p0 + lane, next_x, next_y);
+            if (p0 + lane < B.npairs) next_e = pl.list[at];
+        };
+        fetch(0);
         for (uint32_t r0 = 0; r0 < B.npairs; r0 += 32) {
             // ---- one pair per lane
             bool has = r0 + lane < B.npairs;
-            uint32_t x, y;
-            const uint32_t at = pair_entry(B, r0 + lane, x, y);
+            uint32_t x = next_x, y = next_y;
             uint32_t k = 0, cut = 0;
             if (has) {
-                const uint32_t ent = pl.list[at];
-                x += ent & 0xffu;
-                k = ent >> 8;
+                x += next_e & 0xffu;
+                k = next_e >> 8;
                 const uint32_t code = pair_corners<T, V>(vz + (uint64_t)y * pitch + x, pitch, slice, W.cv[lane],
                                                          [&](T v) -> bool {
                     if constexpr (kPairFast<T>) return (float)v > s_iso[k].f.f_thr;
@@ -414,6 +425,7 @@ __global__ void __launch_bounds__(kPairThreads, 4)
                 }
                 if (!has) cut = 0;
             }
+            if (r0 + 32 < B.npairs) fetch(r0 + 32);
             y += far_y ? 1u : 0u;   // the node's
             const uint32_t nv0 = (uint32_t)__popc(cut);
             const uint32_t kgrp = niso == 1 ? __ballot_sync(FULL, has) : __match_any_sync(FULL, has ? k : 32u + lane);

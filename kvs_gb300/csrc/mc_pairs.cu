@@ -31,8 +31,10 @@
 // task writes less than 2^16 triangles, so places are counted from the task's
 // start and the isolevels' 64-bit addresses are formed once per task), and an
 // edge's corners and axis are one byte of one table.  640x704x600 f32, 16
-// isolevels: 3810 -> 3625 us (40% of the 9 GB it writes at the copy rate);
-// 1024x768x640 u16, 4 isolevels: 2519 -> 2280 us.
+// isolevels: 3810 -> 3550 us (40% of the 9 GB it writes at the copy rate);
+// 1024x768x640 u16, 4 isolevels: 2519 -> 2255 us.  Of that, a round's list
+// entries read a round ahead: 3630 -> 3550 and 2276 -> 2255; 48 uneven volumes
+// 846 -> 805.
 #include <cuda_runtime.h>
 
 #include "mc_emit.cuh"
@@ -164,16 +166,22 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
         const T* vz = static_cast<const T*>(G.vol.data) + (uint64_t)z * slice;
         const float fz = __uint2float_rn(z);
         uint32_t taken = 0;
+        // the round's list entries, read a round ahead
+        uint32_t next_x, next_y, next_e = 0;
+        auto fetch = [&](uint32_t p0) {
+            const uint32_t at = pair_entry(B, p0 + lane, next_x, next_y);
+            if (p0 + lane < B.npairs) next_e = pl.list[at];
+        };
+        fetch(0);
         for (uint32_t r0 = 0; r0 < B.npairs; r0 += taken) {
             // ---- one pair per lane, as many as the vertex pool holds
             bool has = r0 + lane < B.npairs;
-            uint32_t x, y;
-            const uint32_t at = pair_entry(B, r0 + lane, x, y);
+            uint32_t x = next_x;
+            const uint32_t y = next_y;
             uint32_t k = 0, code = 0;
             if (has) {
-                const uint32_t e = pl.list[at];
-                x += e & 0xffu;
-                k = e >> 8;
+                x += next_e & 0xffu;
+                k = next_e >> 8;
                 code = pair_corners<T, V>(vz + (uint64_t)y * pitch + x, pitch, slice, W.cv[lane], [&](T v) -> bool {
                     if constexpr (kPairFast<T>) return (float)v > W.ic[k].thr;
                     else return above(isos[iso_begin].cls, v);   // (one isolevel per group)
@@ -189,6 +197,7 @@ __global__ void __launch_bounds__(kPairThreads, KVSMC_PAIRS_CTAS)
             has = has && vpre + ne0 <= (uint32_t)kPairVerts;   // a suffix of lanes waits
             taken = (uint32_t)__popc(__ballot_sync(FULL, has));
             const uint32_t nv = __shfl_sync(FULL, vpre + ne0, taken - 1);
+            if (r0 + taken < B.npairs) fetch(r0 + taken);
             const uint32_t nt = has ? cnt & 7u : 0u;
             const uint32_t pe = x | (k << 12) | (code << 16) | (vpre << 24);   // (x < 4096; vpre < kPairVerts)
             // output position of the pair's first triangle: its isolevel's running

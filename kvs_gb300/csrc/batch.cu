@@ -48,6 +48,13 @@ kvsmc::FastIso make_fast(double iso, double vmin, double vmax, int dtype)
                 std::fabs(vmin) <= lim && std::fabs(vmax) <= lim && (double)f.vmin_f == vmin &&
                 (double)f.vmax_f == vmax && std::isfinite(f.ih) && std::isfinite(f.il);
     f.lean_ok = f.fast_ok && f.vmin_f <= f.f_thr && f.f_thr < f.vmax_f;
+    switch (dtype) {   // (the wide types take no certificate)
+    case KVSMC_I8: f.lean_ok = f.lean_ok && kvsmc::lean_narrow_range(f.vmin_f, f.vmax_f, -128.0f, 127.0f); break;
+    case KVSMC_U8: f.lean_ok = f.lean_ok && kvsmc::lean_narrow_range(f.vmin_f, f.vmax_f, 0.0f, 255.0f); break;
+    case KVSMC_I16: f.lean_ok = f.lean_ok && kvsmc::lean_narrow_range(f.vmin_f, f.vmax_f, -32768.0f, 32767.0f); break;
+    case KVSMC_U16: f.lean_ok = f.lean_ok && kvsmc::lean_narrow_range(f.vmin_f, f.vmax_f, 0.0f, 65535.0f); break;
+    default: break;
+    }
     return f;
 }
 

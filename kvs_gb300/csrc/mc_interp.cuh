@@ -45,8 +45,15 @@ struct FastIso {
     float f_thr;         // largest float <= iso: v > f_thr <=> double(v) > iso
     float vmin_f, vmax_f;// the clamp range as floats (exact when fast_ok)
     int32_t fast_ok;     // 0: always take the FP64 sequence
-    int32_t lean_ok;     // fast_ok, and the clamp range spans the threshold (see fast_axis_lean)
+    int32_t lean_ok;     // fast_ok, and the clamp range is one that fast_axis_lean takes (see there)
 };
+
+// Whether values that are whole numbers in [lowest, highest] are whole numbers
+// after the clamp to [vmin, vmax] too: each end is one, or lies beyond them all.
+__host__ __device__ __forceinline__ bool lean_narrow_range(float vmin, float vmax, float lowest, float highest)
+{
+    return (vmin == floorf(vmin) || vmin <= lowest) && (vmax == floorf(vmax) || vmax >= highest);
+}
 
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e)
 {
@@ -187,13 +194,19 @@ __device__ __forceinline__ bool fast_axis_bf(float v0, float v1, float a, float 
 // above f_thr, as of every used edge of a case), in fewer operations: the
 // streaming emit's vertex, 58 instead of 95 instructions.  Same certificate:
 //  * lean_ok: vmin_f <= f_thr < vmax_f, so the clamped values lie on the same
-//    sides as the values themselves (a NaN, which is on neither, is refused),
-//    the ratio is in [0, 1] and |den| <= 2^61; fmin/fmax then clamp as
-//    clampf_ref does, up to the sign of a zero, which no step keeps;
+//    sides as the values themselves (a NaN, which is on neither, is refused)
+//    and |den| <= 2^61; fmin/fmax then clamp as clampf_ref does, up to the sign
+//    of a zero, which no step keeps;
+//  * the ratio is in [0, 1]: the isolevel is at least f_thr, so at least the
+//    lower value, and below the upper one: vmax_f is above f_thr and, as the
+//    next value of the type above f_thr is above the isolevel, so is vmax_f
+//    when it is a value of the type or beyond them all;
 //  * nh - q1 dh by one FMA: its exact value needs at most 26 bits (q1 is within
 //    4 ulps of nh / dh), so the rounding is below 2^-46 |q|; the bound
 //    1.5 * 2^-43 |R| of q1 + q2 holds with room;
-//  * EXACT_DEN (values that are integers below 2^17): v1 - v0 has no error;
+//  * EXACT_DEN (values that are whole numbers below 2^17 in magnitude, and stay
+//    so when clamped: lean_ok then includes lean_narrow_range, as an end like
+//    10.1f would make v1 - v0 round): v1 - v0 has no error;
 //  * yh + yl by Fast2Sum, valid for |ya| >= |yb2| (checked: it fails only for
 //    a vertex within a few 2^-24 of coordinate 0);
 //  * the error bound's terms by FMAs, each factor raised by 1.001 against

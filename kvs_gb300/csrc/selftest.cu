@@ -19,6 +19,34 @@ __device__ __forceinline__ uint64_t mix64(uint64_t x)
 
 __device__ __forceinline__ double unit(uint64_t h) { return (double)(h >> 11) * (1.0 / 9007199254740992.0); }
 
+// The same edge under a clamp range whose ends may cut its values off (whole
+// numbers, floats with all their bits, values beyond): every certified path
+// that the range's constants (make_fast) allow, against the FP64 sequence.
+__device__ bool clamped_edge_agrees(Interp j, FastIso f, int kind, uint64_t h4, uint64_t h5, float va, float vb, float ax,
+                                    float ay, float az, float bx, float by, float bz, int axis)
+{
+    const float lo = fminf(va, vb), hi = fmaxf(va, vb);
+    float cl = (float)((double)lo + (j.iso - (double)lo) * unit(h4)), ch = (float)(j.iso + ((double)hi - j.iso) * unit(h5));
+    cl = (h4 & 3) == 0 ? cl : ((h4 & 3) == 1 ? floorf(cl) : ((h4 & 3) == 2 ? lo : lo - 0.5f));
+    ch = (h5 & 3) == 0 ? ch : ((h5 & 3) == 1 ? ceilf(ch) : ((h5 & 3) == 2 ? hi : hi + 0.5f));
+    const bool narrow = kind == 2 || kind == 3 || kind == 7;   // integers from 0 to:
+    const float highest = kind == 2 ? 255.0f : (kind == 3 ? 65535.0f : 1024.0f);
+    if (narrow) f.f_thr = (float)floor(j.iso);
+    j.vmin = (double)cl;
+    j.vmax = (double)ch;
+    f.vmin_f = cl;
+    f.vmax_f = ch;
+    f.lean_ok = cl <= f.f_thr && f.f_thr < ch && (!narrow || lean_narrow_range(cl, ch, 0.0f, highest));
+    const float3 ex = interpolate_exact(j, (double)va, (double)vb, ax, ay, az, bx, by, bz);
+    const float3 fv = edge_vertex_fast(j, f, va, vb, ax, ay, az, bx, by, bz, axis);
+    const float want = axis == 0 ? ex.x : (axis == 1 ? ex.y : ex.z);
+    const float a = axis == 0 ? ax : (axis == 1 ? ay : az), b = axis == 0 ? bx : (axis == 1 ? by : bz);
+    float r;
+    const bool ok = narrow ? fast_axis_lean<true>(va, vb, a, b > a, f, r) : fast_axis_lean<false>(va, vb, a, b > a, f, r);
+    const int w = __float_as_int(want);
+    return (!ok || __float_as_int(r) == w) && __float_as_int(axis == 0 ? fv.x : (axis == 1 ? fv.y : fv.z)) == w;
+}
+
 // One random straddling edge per index; several value distributions.
 __global__ void k_selftest(uint64_t n, uint64_t seed, unsigned long long* counters)
 {
@@ -105,6 +133,8 @@ __global__ void k_selftest(uint64_t n, uint64_t seed, unsigned long long* counte
         else if (__float_as_int(ex.x) != __float_as_int(fv.x) || __float_as_int(ex.y) != __float_as_int(fv.y) ||
             __float_as_int(ex.z) != __float_as_int(fv.z) ||
             (ok && __float_as_int(r) != __float_as_int(want)) || (okb && __float_as_int(rb) != __float_as_int(want)))
+            ++mism;
+        else if (!clamped_edge_agrees(j, f, kind, mix64(h0 + 4), mix64(h0 + 5), va, vb, ax, ay, az, bx, by, bz, axis))
             ++mism;
     }
     atomicAdd(&counters[0], tested);

@@ -47,6 +47,11 @@ kvsmc::FastIso make_fast(double iso, double vmin, double vmax, int dtype)
     f.fast_ok = std::isfinite(iso) && std::fabs(iso) <= lim && std::isfinite(vmin) && std::isfinite(vmax) &&
                 std::fabs(vmin) <= lim && std::fabs(vmax) <= lim && (double)f.vmin_f == vmin &&
                 (double)f.vmax_f == vmax && std::isfinite(f.ih) && std::isfinite(f.il);
+    // The certificates take values on both sides of f_thr as values on both
+    // sides of the isolevel.  An upper end between the two (100.5 with isolevel
+    // 100.7 and integers) would be neither: its ratio is an absolute value of a
+    // negative quotient, which only the FP64 sequence forms.
+    if (dtype != KVSMC_F32 && f.f_thr < f.vmax_f && (double)f.vmax_f <= iso) f.fast_ok = 0;
     f.lean_ok = f.fast_ok && f.vmin_f <= f.f_thr && f.f_thr < f.vmax_f;
     switch (dtype) {   // (the wide types take no certificate)
     case KVSMC_I8: f.lean_ok = f.lean_ok && kvsmc::lean_narrow_range(f.vmin_f, f.vmax_f, -128.0f, 127.0f); break;

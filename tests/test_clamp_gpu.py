@@ -58,3 +58,26 @@ def test_a_range_that_cuts_the_data(kvsmc_ctx, oracle_lib, dtype, mode):
                     if mode:
                         assert np.array_equal(got["connections"], ref["connections"].view(np.uint32)), tag
             vol.free()
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("dtype,lo,hi,isos", [
+    (np.uint8, 0.0, 100.0625, (100.07, 100.5, 100.99)), (np.int8, -100.0, -3.75, (-3.7, -3.5, -3.01)),
+    (np.uint16, 0.0, 1000.5, (1000.51, 1000.75)), (np.int16, -30000.0, 0.25, (0.25, 0.3, 0.9)),
+])
+def test_an_isolevel_past_the_upper_end(kvsmc_ctx, oracle_lib, dtype, lo, hi, isos, mode):
+    """The upper end lies below the isolevel, with no value of the type between
+    them: an edge's clamped values are both below it, and the interpolation
+    ratio, an absolute value, starts from a negative quotient."""
+    info = np.iinfo(dtype)
+    v = np.random.default_rng(8).integers(info.min, info.max, (6, 13, 70), dtype=dtype, endpoint=True)
+    vol = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+    params = [_abi.make_params(x, mode, (lo, hi)) for x in isos]
+    together = extract_batch(kvsmc_ctx, [vol] * len(isos), params, _abi.PATH_AUTO)
+    for x, p, o in zip(isos, params, together):
+        ref = oracle_lib.extract(v, x, mode, lo, hi)
+        assert ref["coords"].size
+        for got in (o, extract_batch(kvsmc_ctx, [vol], [p], _abi.PATH_AUTO)[0]):
+            assert same_bits(got["coords"], ref["coords"]), (x, first_diff(got["coords"], ref["coords"]))
+            assert same_bits(got["normals"], ref["normals"]), (x, first_diff(got["normals"], ref["normals"]))
+    vol.free()

@@ -1065,6 +1065,10 @@ void kvsmc_destroy(kvsmc_context* ctx)
     cudaStreamSynchronize(ctx->stream);
     if (ctx->host_vol) { cudaFree(ctx->host_vol->dev); delete ctx->host_vol; }
     block_release(ctx);
+    if (ctx->dense_ev) {
+        cudaEventSynchronize(ctx->dense_ev);
+        cudaEventDestroy(ctx->dense_ev);
+    }
     if (ctx->dense) cudaFree(ctx->dense);
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->d_flag) cudaFree(ctx->d_flag);

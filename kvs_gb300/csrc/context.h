@@ -61,6 +61,7 @@ struct kvsmc_context {
     std::mutex spare_mutex;
     void* dense = nullptr;       // staging of host volumes whose rows are padded (at most kDenseStage)
     size_t dense_bytes = 0;
+    cudaEvent_t dense_ev = nullptr;   // behind the last pass that reads it, on whatever stream that was
     std::vector<kvsmc::KernelFit> fits;   // launch shapes of the kernels launched so far
     std::string last_error;
     // auxiliary streams for launches that may run side by side (created on first use)

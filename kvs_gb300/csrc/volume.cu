@@ -431,9 +431,12 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
     } else if (v->view.pitch != v->view.nx && dense <= kDenseStage) {
         // rows that are padded on the device: one dense copy into a staging
         // buffer, padded by the ingest pass (a row-by-row copy of 99-node rows
-        // of 16-bit values ran at 6 GB/s: 2.1 MB in 340 us)
+        // of 16-bit values ran at 6 GB/s: 2.1 MB in 340 us).  The last pass that
+        // reads the buffer may be on another stream (kvsmc_set_stream): the copy
+        // waits for it
+        if (!ctx->dense_ev) KVSMC_CUDA(ctx, cudaEventCreateWithFlags(&ctx->dense_ev, cudaEventDisableTiming));
         if (dense > ctx->dense_bytes) {
-            KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+            KVSMC_CUDA(ctx, cudaEventSynchronize(ctx->dense_ev));
             if (ctx->dense) cudaFree(ctx->dense);
             ctx->dense = nullptr;
             ctx->dense_bytes = 0;
@@ -441,6 +444,7 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
             KVSMC_CUDA(ctx, device_malloc(ctx, &ctx->dense, want));
             ctx->dense_bytes = want;
         }
+        KVSMC_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->dense_ev, 0));
         KVSMC_CUDA(ctx, cudaMemcpyAsync(ctx->dense, src, dense, cudaMemcpyHostToDevice, ctx->stream));
         from = ctx->dense;
     }
@@ -452,6 +456,7 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
             KVSMC_CUDA(ctx, cudaMemcpy2DAsync(v->dev, v->view.pitch * es, src, row, row, rows, kind, ctx->stream));
     }
     KVSMC_CUDA(ctx, kvsmc::launch_ingest(v->view, from, v->bricks, v->range, launch_of(ctx)));
+    if (from && from == ctx->dense) KVSMC_CUDA(ctx, cudaEventRecord(ctx->dense_ev, ctx->stream));
     v->bricks_valid = v->bricks != nullptr;
     v->range_ready = true;
     return KVSMC_OK;

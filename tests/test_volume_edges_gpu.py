@@ -1,0 +1,54 @@
+"""Resident volumes at the edges of the pass that lays them out: uploads on two
+streams.
+"""
+import numpy as np
+import pytest
+
+from kvs_gb300 import _abi
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("update", [False, True])
+def test_uploads_on_two_streams(kvsmc_ctx, update):
+    """Host volumes with padded rows go through one staging buffer of the
+    context: an upload on one stream must not overwrite what the pass of an
+    upload on another one still reads."""
+    shape = (60, 300, 301)
+    sizes = [shape, (60, 301, 299), (7, 9, 5), shape]   # (padded rows, the last ones smaller than the buffer)
+    hosts = []
+    for i, s in enumerate(sizes):
+        pinned = torch.empty(int(np.prod(s)) * 4, dtype=torch.uint8).pin_memory()
+        h = pinned.numpy().view(np.float32).reshape(s)
+        h[...] = np.arange(h.size, dtype=np.float32).reshape(s) % 997 + 1000 * i
+        hosts.append((pinned, h))
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    vols = [_abi.DeviceVolume.upload(kvsmc_ctx, h) for _, h in hosts] if update else [None] * len(hosts)
+    kvsmc_ctx.synchronize()
+    torch.cuda.synchronize()
+    try:
+        for turn in range(6):
+            order = range(len(hosts)) if turn % 2 == 0 else reversed(range(len(hosts)))
+            for j, i in enumerate(order):
+                kvsmc_ctx.set_stream(streams[j % 2].cuda_stream)
+                if j == 0:
+                    with torch.cuda.stream(streams[0]):
+                        torch.cuda._sleep(2_000_000)   # the first one starts behind other work
+                if update:
+                    kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_volume_update(kvsmc_ctx.handle, vols[i].handle,
+                                                                      hosts[i][1].ctypes.data), "update")
+                else:
+                    vols[i] = _abi.DeviceVolume.upload(kvsmc_ctx, hosts[i][1])
+            torch.cuda.synchronize()
+            for i, (_, h) in enumerate(hosts):
+                assert np.array_equal(vols[i].download(), h), (turn, i)
+                if not update:
+                    vols[i].free()
+    finally:
+        torch.cuda.synchronize()
+        kvsmc_ctx.set_stream(None)
+    if update:
+        for v in vols:
+            v.free()

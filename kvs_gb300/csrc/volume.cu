@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kIngestThreads)
     const uint64_t rp = COPY ? v.nx : v.pitch, sp = COPY ? (uint64_t)v.nx * v.ny : v.slice;
     const T* const from = COPY ? src : dst;
     T lo = Limits<T>::highest(), hi = Limits<T>::lowest();   // over this thread's values, NaN apart
-    unsigned long long zero = ~0ull;                          // (index << 1 | sign) of its first zero
+    unsigned long long zero = ~0ull;                          // (index << 1 | sign) of its zero of lowest index
     const uint64_t warps = (uint64_t)gridDim.x * (kIngestThreads / 32);
     for (uint64_t b = (uint64_t)blockIdx.x * (kIngestThreads / 32) + warp; b < nbricks; b += warps) {
         const uint32_t q = (uint32_t)(b / nbx), bx = (uint32_t)(b - (uint64_t)q * nbx);   // (below 2^32 brick rows)
@@ -137,8 +137,10 @@ __global__ void __launch_bounds__(kIngestThreads)
                     auto look = [&](T val, uint32_t y, uint32_t x) {
                         nan |= val != val;
                         // among equal values the scan keeps the first: only zeros' signs show it
-                        if (val == T(0) && zero == ~0ull)
-                            zero = ((((uint64_t)z * v.ny + y) * v.nx + x) << 1) | (raw_bits(val) != 0 ? 1u : 0u);
+                        // (a warp's bricks do not come in index order)
+                        if (val == T(0))
+                            zero = min(zero, ((((unsigned long long)z * v.ny + y) * v.nx + x) << 1) |
+                                                 (raw_bits(val) != 0 ? 1ull : 0ull));
                     };
 #pragma unroll
                     for (int r = 0; r < 3; ++r) {

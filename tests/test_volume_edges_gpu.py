@@ -1,10 +1,12 @@
 """Resident volumes at the edges of the pass that lays them out: uploads on two
-streams.
+streams, warps that go on to a second brick.
 """
 import numpy as np
 import pytest
 
 from kvs_gb300 import _abi
+
+from .helpers import same_bits
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +54,22 @@ def test_uploads_on_two_streams(kvsmc_ctx, update):
     if update:
         for v in vols:
             v.free()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("sign", [1, -1])
+def test_sign_of_a_zero_end_across_bricks(kvsmc_ctx, dtype, sign):
+    """The range keeps the first of equal values in index order.  With more
+    bricks in a plane than warps on the GPU, a warp meets a brick's high planes
+    before the low planes of a later brick."""
+    bricks = torch.cuda.get_device_properties(0).multi_processor_count * 64
+    base = np.full((9, 2 * bricks + 9, 2), 3.0 * sign, dtype)
+    for first, second in ((-0.0, 0.0), (0.0, -0.0)):
+        v = base.copy()
+        v[0, 2 * bricks + 1, 0] = first    # the lowest index, in no brick but the first warp's second one
+        v[7, 0, 0] = second                # in its first one
+        dv = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+        lo, hi = dv.minmax()
+        want = (first, 3.0) if sign > 0 else (-3.0, first)
+        assert same_bits(np.array([lo, hi]), np.array(want)), (lo, hi, want)
+        dv.free()

@@ -140,6 +140,7 @@ kvsmc_status prepare(kvsmc_context* ctx, Item& it)
 {
     if (!it.vol) return fail(ctx, KVSMC_ERR_INVALID_ARGUMENT, "null volume");
     if (it.params.mode < 0 || it.params.mode > 2) return fail(ctx, KVSMC_ERR_INVALID_ARGUMENT, "bad mode %d", it.params.mode);
+    volume_use(ctx, it.vol);
     if (it.params.has_minmax) {
         it.vmin = it.params.min_value;
         it.vmax = it.params.max_value;
@@ -1063,7 +1064,7 @@ void kvsmc_destroy(kvsmc_context* ctx)
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
-    if (ctx->host_vol) { cudaFree(ctx->host_vol->dev); delete ctx->host_vol; }
+    if (ctx->host_vol) volume_destroy(nullptr, ctx->host_vol);
     block_release(ctx);
     if (ctx->dense_ev) {
         cudaEventSynchronize(ctx->dense_ev);
@@ -1142,6 +1143,7 @@ kvsmc_status kvsmc_volume_upload(kvsmc_context* ctx, const void* host, kvsmc_dty
     if ((st = check_shape(ctx, dtype, nx, ny, nz))) return st;
     kvsmc_volume* v = new kvsmc_volume();
     if ((st = volume_alloc(ctx, dtype, nx, ny, nz, v)) || (st = volume_copy_in(ctx, v, host, false))) {
+        cudaStreamSynchronize(ctx->stream);
         volume_destroy(ctx, v);
         return st;
     }
@@ -1158,6 +1160,7 @@ kvsmc_status kvsmc_volume_from_device(kvsmc_context* ctx, const void* dev, kvsmc
     if ((st = check_shape(ctx, dtype, nx, ny, nz))) return st;
     kvsmc_volume* v = new kvsmc_volume();
     if ((st = volume_alloc(ctx, dtype, nx, ny, nz, v)) || (st = volume_copy_in(ctx, v, dev, true))) {
+        cudaStreamSynchronize(ctx->stream);
         volume_destroy(ctx, v);
         return st;
     }

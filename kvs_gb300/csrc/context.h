@@ -1,5 +1,6 @@
 // context.h -- host-side state of libkvsmc shared by api.cu and batch.cu.
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <functional>
 #include <mutex>
@@ -13,7 +14,12 @@ struct kvsmc_volume {
     kvsmc::VolumeView view;
     void* dev = nullptr;        // owned device allocation
     size_t bytes = 0;
+    cudaEvent_t ev = nullptr;   // comes with dev: behind the last copy or pass that a call left running on it
     int device = 0;             // the device it lies on
+    kvsmc_context* owner = nullptr;   // the context that allocated it
+    // read by work that no call of the owner's waits for (a plan's replays, a
+    // server's workers, another context): its block is not kept when it is freed
+    std::atomic<bool> lent{false};
     bool has_minmax = false;
     double vmin = 0.0, vmax = 0.0;
     // parts of the same allocation, written by the pass that every copy into a
@@ -56,7 +62,7 @@ struct kvsmc_context {
     // cudaFree of a new field's 83 MB a frame cost 350 us): at most
     // kSpareBlocks blocks of kSpareBytes in all, given back when an
     // allocation fails and with the context
-    struct Spare { void* p; size_t bytes; };
+    struct Spare { void* p; size_t bytes; cudaEvent_t ev; };
     std::vector<Spare> spare;
     std::mutex spare_mutex;
     void* dense = nullptr;       // staging of host volumes whose rows are padded (at most kDenseStage)
@@ -150,10 +156,15 @@ struct Item {
 // A volume's device block: from the context's spare blocks, or a new one.
 constexpr size_t kSpareBytes = (size_t)1 << 30;
 constexpr size_t kSpareBlocks = 4;
-kvsmc_status block_alloc(kvsmc_context* ctx, size_t bytes, void** p, size_t* got);
-// Give a block back: kept for the next volumes once nothing on the device
-// reads it any more, or freed (ctx null, or too large).
-void block_free(kvsmc_context* ctx, void* p, size_t bytes);
+kvsmc_status block_alloc(kvsmc_context* ctx, size_t bytes, kvsmc_volume* v);
+// Give a volume's block back: kept for the next volumes of ctx once nothing
+// reads it any more, or freed (ctx null, lent, or too large).
+void block_free(kvsmc_context* ctx, kvsmc_volume* v);
+// A call of ctx reads the volume.
+inline void volume_use(const kvsmc_context* ctx, kvsmc_volume* v)
+{
+    if (v->owner != ctx) v->lent = true;
+}
 // Free every spare block.
 void block_release(kvsmc_context* ctx);
 

@@ -104,6 +104,7 @@ kvsmc_status kvsmc_plan_create(kvsmc_context* ctx, const kvsmc_request* reqs, in
         if (st) { plan_free(p); return st; }
         p->base[i] = it.sizes;
         if (!it.extracted) continue;
+        it.vol->lent = true;   // (replays read it on any stream)
         if (!stream_eligible(ctx, it)) {
             plan_free(p);
             return fail(ctx, KVSMC_ERR_INVALID_ARGUMENT,

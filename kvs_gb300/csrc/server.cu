@@ -375,6 +375,7 @@ kvsmc_status kvsmc_server_submit(kvsmc_server* S, kvsmc_volume* vol, const kvsmc
             S->seen.insert(vol);
         }
     }
+    vol->lent = true;   // (the workers read it)
     std::lock_guard<std::mutex> lk(S->mu);
     *ticket = S->next_ticket++;
     S->pending.push_back(Pending{*ticket, vol, *p, S->now()});

@@ -450,6 +450,7 @@ kvsmc_status slice_count_enqueue(kvsmc_context* ctx, kvsmc_volume* v, const kvsm
     std::memset(&j, 0, sizeof j);
     if (!p || !p->tf_table || p->tf_resolution < 1)
         return fail(ctx, KVSMC_ERR_INVALID_ARGUMENT, "slice: bad parameters (colour table)");
+    volume_use(ctx, v);
     const kvsmc::VolumeView& vv = v->view;
     if (vv.nx < 2 || vv.ny < 2 || vv.nz < 2) return KVSMC_OK;   // no cells
     j.vol = vv;

@@ -315,7 +315,7 @@ size_t table_bytes(const kvsmc::VolumeView& v)
 
 }  // namespace
 
-kvsmc_status block_alloc(kvsmc_context* ctx, size_t bytes, void** p, size_t* got)
+kvsmc_status block_alloc(kvsmc_context* ctx, size_t bytes, kvsmc_volume* v)
 {
     {
         // a spare block at most a quarter larger than asked for
@@ -326,14 +326,23 @@ kvsmc_status block_alloc(kvsmc_context* ctx, size_t bytes, void** p, size_t* got
                 (best == ctx->spare.size() || ctx->spare[i].bytes < ctx->spare[best].bytes))
                 best = i;
         if (best < ctx->spare.size()) {
-            *p = ctx->spare[best].p;
-            *got = ctx->spare[best].bytes;
+            v->dev = ctx->spare[best].p;
+            v->bytes = ctx->spare[best].bytes;
+            v->ev = ctx->spare[best].ev;
             ctx->spare.erase(ctx->spare.begin() + (long)best);
             return KVSMC_OK;
         }
     }
-    KVSMC_CUDA(ctx, device_malloc(ctx, p, bytes));
-    *got = bytes;
+    cudaEvent_t ev = nullptr;
+    KVSMC_CUDA(ctx, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    const cudaError_t e = device_malloc(ctx, &v->dev, bytes);
+    if (e != cudaSuccess) {
+        cudaEventDestroy(ev);
+        v->dev = nullptr;
+        KVSMC_CUDA(ctx, e);
+    }
+    v->bytes = bytes;
+    v->ev = ev;
     return KVSMC_OK;
 }
 
@@ -351,28 +360,40 @@ cudaError_t device_malloc_bytes(kvsmc_context* ctx, void** p, size_t bytes)
 void block_release(kvsmc_context* ctx)
 {
     std::lock_guard<std::mutex> lock(ctx->spare_mutex);
-    for (const kvsmc_context::Spare& s : ctx->spare) cudaFree(s.p);
+    for (const kvsmc_context::Spare& s : ctx->spare) {
+        cudaFree(s.p);
+        cudaEventDestroy(s.ev);
+    }
     ctx->spare.clear();
 }
 
-void block_free(kvsmc_context* ctx, void* p, size_t bytes)
+void block_free(kvsmc_context* ctx, kvsmc_volume* v)
 {
-    if (!p) return;
-    // Other streams (a server's workers, a plan's) may still read the block:
-    // cudaFree waits for them, so a block that is kept waits for them here.
-    if (ctx && bytes <= kSpareBytes && cudaDeviceSynchronize() == cudaSuccess) {
+    if (!v->dev) return;
+    // cudaFree waits for all work on the device.  A block that is kept waits for
+    // the work that may still read it: calls wait for their own, the event stands
+    // behind what uploads and updates leave running, on whatever stream, and a
+    // block that other work reads is not kept.  (A wait for the whole device
+    // would do, but is refused while any thread captures a stream, and ends its
+    // capture.)
+    if (ctx && !v->lent && v->bytes <= kSpareBytes && cudaEventSynchronize(v->ev) == cudaSuccess) {
         std::lock_guard<std::mutex> lock(ctx->spare_mutex);
         size_t held = 0;
         for (const kvsmc_context::Spare& s : ctx->spare) held += s.bytes;
-        while (!ctx->spare.empty() && (held + bytes > kSpareBytes || ctx->spare.size() >= kSpareBlocks)) {
+        while (!ctx->spare.empty() && (held + v->bytes > kSpareBytes || ctx->spare.size() >= kSpareBlocks)) {
             held -= ctx->spare.front().bytes;   // the oldest leaves
             cudaFree(ctx->spare.front().p);
+            cudaEventDestroy(ctx->spare.front().ev);
             ctx->spare.erase(ctx->spare.begin());
         }
-        ctx->spare.push_back({p, bytes});
-        return;
+        ctx->spare.push_back({v->dev, v->bytes, v->ev});
+    } else {
+        cudaFree(v->dev);
+        cudaEventDestroy(v->ev);
     }
-    cudaFree(p);
+    v->dev = nullptr;
+    v->bytes = 0;
+    v->ev = nullptr;
 }
 
 kvsmc_status volume_alloc(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, uint32_t ny, uint32_t nz,
@@ -391,12 +412,11 @@ kvsmc_status volume_alloc(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, ui
     const size_t values = align_up((size_t)pitch * ny * nz * es + 256, 256);
     const size_t bytes = values + 256 + table_bytes(v->view);
     if (bytes > v->bytes) {
-        if (v->dev) block_free(ctx, v->dev, v->bytes);
-        v->dev = nullptr;
-        v->bytes = 0;
-        kvsmc_status st = block_alloc(ctx, bytes, &v->dev, &v->bytes);
+        block_free(ctx, v);
+        kvsmc_status st = block_alloc(ctx, bytes, v);
         if (st) return st;
         v->device = ctx->device;
+        v->owner = ctx;
     }
     v->view.data = v->dev;
     v->range = reinterpret_cast<kvsmc::IngestOut*>(static_cast<char*>(v->dev) + values);
@@ -407,6 +427,7 @@ kvsmc_status volume_alloc(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, ui
 kvsmc_status volume_bricks(kvsmc_context* ctx, kvsmc_volume* v)
 {
     KVSMC_CUDA(ctx, kvsmc::launch_ingest(v->view, nullptr, v->bricks, v->range, launch_of(ctx)));
+    KVSMC_CUDA(ctx, cudaEventRecord(v->ev, ctx->stream));
     v->bricks_valid = v->bricks != nullptr;
     v->range_ready = true;
     return KVSMC_OK;
@@ -420,6 +441,7 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
     const size_t dense = row * rows;
     v->has_minmax = false;
     v->range_ready = false;
+    KVSMC_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, v->ev, 0));   // (an update on another stream comes first)
     const void* from = nullptr;   // values the ingest pass copies (null: they are in place)
     if (on_device) {
         // read in place of a copy where the kernel can: device memory of this
@@ -458,6 +480,7 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
             KVSMC_CUDA(ctx, cudaMemcpy2DAsync(v->dev, v->view.pitch * es, src, row, row, rows, kind, ctx->stream));
     }
     KVSMC_CUDA(ctx, kvsmc::launch_ingest(v->view, from, v->bricks, v->range, launch_of(ctx)));
+    KVSMC_CUDA(ctx, cudaEventRecord(v->ev, ctx->stream));
     if (from && from == ctx->dense) KVSMC_CUDA(ctx, cudaEventRecord(ctx->dense_ev, ctx->stream));
     v->bricks_valid = v->bricks != nullptr;
     v->range_ready = true;
@@ -467,6 +490,7 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
 kvsmc_status volume_minmax(kvsmc_context* ctx, kvsmc_volume* v)
 {
     if (v->has_minmax) return KVSMC_OK;
+    volume_use(ctx, v);
     if (!v->range_ready)
         if (kvsmc_status st = volume_bricks(ctx, v)) return st;
     KVSMC_CUDA(ctx, cudaMemcpyAsync(ctx->h_small, v->range, sizeof(kvsmc::IngestOut), cudaMemcpyDeviceToHost,
@@ -481,7 +505,7 @@ kvsmc_status volume_minmax(kvsmc_context* ctx, kvsmc_volume* v)
 
 void volume_destroy(kvsmc_context* ctx, kvsmc_volume* v)
 {
-    if (v->dev) block_free(ctx && ctx->device == v->device ? ctx : nullptr, v->dev, v->bytes);
+    block_free(ctx && ctx->device == v->device ? ctx : nullptr, v);
     delete v;
 }
 

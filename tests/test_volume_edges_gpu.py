@@ -1,6 +1,9 @@
 """Resident volumes at the edges of the pass that lays them out: uploads on two
-streams, warps that go on to a second brick.
+streams, warps that go on to a second brick; volumes freed while other work is
+under way.
 """
+import threading
+
 import numpy as np
 import pytest
 
@@ -73,3 +76,84 @@ def test_sign_of_a_zero_end_across_bricks(kvsmc_ctx, dtype, sign):
         want = (first, 3.0) if sign > 0 else (-3.0, first)
         assert same_bits(np.array([lo, hi]), np.array(want)), (lo, hi, want)
         dv.free()
+
+
+def test_a_volume_freed_while_another_thread_captures(kvsmc_ctx):
+    """A wait for the whole device is refused during a capture and ends it:
+    giving a volume's block back must not need one."""
+    x = torch.zeros(1000, device="cuda")
+    vols = [_abi.DeviceVolume.upload(kvsmc_ctx, np.full((20, 30, 40), 5, np.uint8)) for _ in range(3)]
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="thread_local"):
+        x += 1
+        t = threading.Thread(target=lambda: [v.free() for v in vols])
+        t.start()
+        t.join()
+        x += 1
+    g.replay()
+    torch.cuda.synchronize()
+    assert x.eq(2).all()
+
+
+def test_a_volume_freed_behind_a_queued_upload(kvsmc_ctx):
+    """The upload waits on one stream while the volume is freed from another:
+    the next volume in its block must not get the late values."""
+    def host(value):
+        pinned = torch.empty(40 * 64 * 64 * 4, dtype=torch.uint8).pin_memory()
+        h = pinned.numpy().view(np.float32).reshape(40, 64, 64)
+        h[...] = value
+        return pinned, h
+
+    (p1, first), (p2, second) = host(1.0), host(2.0)
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    try:
+        for _ in range(4):
+            with torch.cuda.stream(a):
+                torch.cuda._sleep(5_000_000)
+            kvsmc_ctx.set_stream(a.cuda_stream)
+            v1 = _abi.DeviceVolume.upload(kvsmc_ctx, first)
+            kvsmc_ctx.set_stream(b.cuda_stream)
+            v1.free()
+            v2 = _abi.DeviceVolume.upload(kvsmc_ctx, second)
+            torch.cuda.synchronize()
+            assert np.array_equal(v2.download(), second) and v2.minmax() == (2.0, 2.0)
+            v2.free()
+    finally:
+        torch.cuda.synchronize()
+        kvsmc_ctx.set_stream(None)
+
+
+def test_a_volume_freed_behind_a_replay(kvsmc_ctx):
+    """A plan's replay is queued on a stream of the caller's when its volume is
+    freed and others are uploaded: it still reads the volume's own values."""
+    rng = np.random.default_rng(2)
+    v = rng.random((30, 32, 36)).astype(np.float32)
+    w = np.zeros_like(v)
+    vol = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+    params = _abi.make_params(0.5, 0)
+    s = _abi.Sizes()
+    kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_count(kvsmc_ctx.handle, vol.handle, params, s), "count")
+    want, got = [torch.zeros(s.ncoords, device="cuda") for _ in range(2)]
+    normals = torch.zeros(s.nnormals, device="cuda")
+    torch.cuda.synchronize()
+    reqs = (_abi.Request * 1)()
+    reqs[0].volume, reqs[0].params = vol.handle, params
+    reqs[0].d_normals, reqs[0].normals_capacity = normals.data_ptr(), normals.numel()
+    reqs[0].d_coords, reqs[0].coords_capacity = want.data_ptr(), want.numel()
+    kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_extract_batch(kvsmc_ctx.handle, reqs, 1), "extract")
+    reqs[0].d_coords = got.data_ptr()
+    plan = _abi.Plan(kvsmc_ctx, reqs)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(5_000_000)
+    plan.launch(stream.cuda_stream)
+    vol.free()
+    later = [_abi.DeviceVolume.upload(kvsmc_ctx, w) for _ in range(4)]
+    plan.wait()
+    torch.cuda.synchronize()
+    assert torch.equal(want, got)
+    plan.close()
+    for x in later:
+        x.free()

@@ -165,8 +165,8 @@ inline void volume_use(const kvsmc_context* ctx, kvsmc_volume* v)
 {
     if (v->owner != ctx) v->lent = true;
 }
-// Free every spare block.
-void block_release(kvsmc_context* ctx);
+// Free every spare block (whether there were any).
+bool block_release(kvsmc_context* ctx);
 
 // cudaMalloc that frees the spare blocks before it gives up.
 cudaError_t device_malloc_bytes(kvsmc_context* ctx, void** p, size_t bytes);

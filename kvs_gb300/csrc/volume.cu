@@ -349,22 +349,23 @@ kvsmc_status block_alloc(kvsmc_context* ctx, size_t bytes, kvsmc_volume* v)
 cudaError_t device_malloc_bytes(kvsmc_context* ctx, void** p, size_t bytes)
 {
     cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && ctx && !ctx->spare.empty()) {
+    if (e == cudaErrorMemoryAllocation && ctx && block_release(ctx)) {
         cudaGetLastError();
-        block_release(ctx);
         e = cudaMalloc(p, bytes);
     }
     return e;
 }
 
-void block_release(kvsmc_context* ctx)
+bool block_release(kvsmc_context* ctx)
 {
     std::lock_guard<std::mutex> lock(ctx->spare_mutex);
+    const bool any = !ctx->spare.empty();
     for (const kvsmc_context::Spare& s : ctx->spare) {
         cudaFree(s.p);
         cudaEventDestroy(s.ev);
     }
     ctx->spare.clear();
+    return any;
 }
 
 void block_free(kvsmc_context* ctx, kvsmc_volume* v)

@@ -23,7 +23,6 @@
 #include <mutex>
 #include <thread>
 #include <unordered_map>
-#include <unordered_set>
 #include <vector>
 
 #include "batch.h"
@@ -93,12 +92,11 @@ struct kvsmc_server {
     uint64_t arena_bytes = 0;
     FreeList free_list;                 // guarded by mu
     std::mutex mu;                      // queues, budget, counters
-    std::mutex mm_mu;                   // min/max passes and first-use waits on the owner context
+    std::mutex mm_mu;                   // min/max passes on the owner context
     std::condition_variable cv_work, cv_done, cv_budget;
     std::deque<Pending> pending;
     std::deque<kvsmc_completion> done;
     std::unordered_map<uint64_t, Held> held;
-    std::unordered_set<kvsmc_volume*> seen;   // volumes whose upload is known to be complete
     uint64_t next_ticket = 1;
     uint64_t in_use = 0, peak = 0, submitted = 0, completed = 0, batches = 0, budget_waits = 0;
     bool stop = false;
@@ -362,19 +360,15 @@ kvsmc_status kvsmc_server_submit(kvsmc_server* S, kvsmc_volume* vol, const kvsmc
                                 "<= 4097 are served");
     {
         std::lock_guard<std::mutex> lk(S->mm_mu);
-        if (!S->seen.count(vol) || (!p->has_minmax && !vol->has_minmax)) {
+        if (!p->has_minmax && !vol->has_minmax) {
             if (cudaSetDevice(S->ctx->device) != cudaSuccess) return KVSMC_ERR_CUDA;
-            if (!p->has_minmax) {
-                kvsmc_status st = kvsmc_host::volume_minmax(S->ctx, vol);
-                if (st) return st;
-            }
-            // the workers' streams read the volume (and its brick table): the
-            // owner stream's upload must be done
-            if (cudaStreamSynchronize(S->ctx->stream) != cudaSuccess)
-                return kvsmc_host::fail(S->ctx, KVSMC_ERR_CUDA, "server: synchronize");
-            S->seen.insert(vol);
+            if (kvsmc_status st = kvsmc_host::volume_minmax(S->ctx, vol)) return st;
         }
     }
+    // the workers' streams read the volume (and its brick table): its last
+    // upload or update, on whatever stream, must be done
+    if (cudaEventSynchronize(vol->ev) != cudaSuccess)
+        return kvsmc_host::fail(S->ctx, KVSMC_ERR_CUDA, "server: synchronize");
     vol->lent = true;   // (the workers read it)
     std::lock_guard<std::mutex> lk(S->mu);
     *ticket = S->next_ticket++;

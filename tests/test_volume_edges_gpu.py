@@ -157,3 +157,48 @@ def test_a_volume_freed_behind_a_replay(kvsmc_ctx):
     plan.close()
     for x in later:
         x.free()
+
+
+def test_a_request_behind_a_queued_update(kvsmc_ctx):
+    """A served volume is updated on a busy stream and asked for again: the
+    workers wait for the new values, whether they have seen the volume before
+    or not."""
+    def host(value):
+        pinned = torch.empty(32 * 32 * 32 * 4, dtype=torch.uint8).pin_memory()
+        h = pinned.numpy().view(np.float32).reshape(32, 32, 32)
+        h[...] = 0.0
+        h[8:8 + value, 8:20, 8:20] = 1.0
+        return pinned, h
+
+    hosts = [host(k) for k in (3, 7, 11, 2)]
+    params = _abi.make_params(0.5, 0, (0.0, 1.0))
+    want = []
+    for _, h in hosts:
+        v = _abi.DeviceVolume.upload(kvsmc_ctx, h)
+        s = _abi.Sizes()
+        kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_count(kvsmc_ctx.handle, v.handle, params, s), "count")
+        want.append(s.ntriangles)
+        v.free()
+    assert len(set(want)) == len(want)
+    vol = _abi.DeviceVolume.upload(kvsmc_ctx, hosts[-1][1])
+    stream = torch.cuda.Stream()
+    srv = _abi.Server(kvsmc_ctx, budget_bytes=1 << 26, max_batch=4, workers=2)
+    try:
+        for turn in range(3):
+            for (_, h), n in zip(hosts, want):
+                with torch.cuda.stream(stream):
+                    torch.cuda._sleep(3_000_000)
+                kvsmc_ctx.set_stream(stream.cuda_stream)
+                kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_volume_update(kvsmc_ctx.handle, vol.handle, h.ctypes.data), "update")
+                kvsmc_ctx.set_stream(None)
+                ticket, done = srv.submit(vol, params), []
+                while not done:
+                    done = srv.poll(timeout_ms=2000)
+                assert [c.ticket for c in done] == [ticket] and done[0].status == _abi.OK
+                assert done[0].sizes.ntriangles == n, (turn, n)
+                srv.release(ticket)
+    finally:
+        kvsmc_ctx.set_stream(None)
+        srv.close()
+        torch.cuda.synchronize()
+        vol.free()

@@ -326,7 +326,7 @@ void StreamBatch::plan_tables()
     list_cap = 0;
     list_sure = false;
     if (pair_units) {
-        const uint64_t tail = (uint64_t)ctx->num_sms * 32 * kvsmc::kPairRun * launches.size();   // (warps of each count)
+        const uint64_t tail = (uint64_t)ctx->num_sms * kvsmc::kListWarpsPerSm * kvsmc::kPairRun * launches.size();
         const uint64_t sure = 2 * pairs_most + tail;
         list_cap = std::min<uint64_t>(sure, std::max<uint64_t>((uint64_t)1 << 29, pairs_most / 8) + tail);
         list_cap = std::min<uint64_t>(list_cap, (uint64_t)1 << 31);

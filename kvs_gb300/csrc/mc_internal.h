@@ -132,9 +132,14 @@ struct PairList {
     unsigned long long* cursor;
     int* overflow;
 };
-// A count's warp takes entries in runs of this many (or one step's, if more).
+// A count's warp takes entries in runs of this many (or one step's, if more),
+// and a listing count runs at most kListWarpsPerSm warps on an SM (its launch
+// is capped to them), so what its last runs leave unused has a bound.
 constexpr uint32_t kPairRun = 1024;
-constexpr int kPairWarpsPerSm = 24;   // resident warps of the listing emit
+constexpr int kListWarpsPerSm = 32;
+// The emit's block size is chosen for two blocks a warp with this many warps an
+// SM (the kernel has 32 resident).
+constexpr int kPairWarpsPerSm = 24;
 
 // Brick min/max table of a volume: one float2 per (8 cell planes, 2 cell
 // rows, 128 cells) brick, the min and max of its node box ((-inf, +inf) when

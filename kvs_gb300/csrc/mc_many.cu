@@ -409,6 +409,7 @@ cudaError_t launch_count_many(int dtype, int rows, const StreamGroup* d_groups, 
         const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), kManyThreads, smem, &per_sm, true);
         if (e != cudaSuccess) return e;
         if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
+        if (list && per_sm > kListWarpsPerSm / kManyWarps) per_sm = kListWarpsPerSm / kManyWarps;
         const uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)L.num_sms;
         prof_begin(L, "count_many");
         kern<<<(unsigned)(need < resident ? need : resident), kManyThreads, smem, L.stream>>>(

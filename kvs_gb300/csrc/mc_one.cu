@@ -313,6 +313,7 @@ cudaError_t launch_count_one(int dtype, int rows, const StreamGroup* d_groups, i
         int per_sm = 0;
         const cudaError_t e = kernel_fit(L, reinterpret_cast<const void*>(kern), kOneThreads, smem, &per_sm, true);
         if (e != cudaSuccess) return e;
+        if (list && per_sm > kListWarpsPerSm / kOneWarps) per_sm = kListWarpsPerSm / kOneWarps;
         const uint64_t resident = (uint64_t)(per_sm > 0 ? per_sm : 1) * (uint64_t)L.num_sms;
         prof_begin(L, "count_one");
         kern<<<(unsigned)(need < resident ? need : resident), kOneThreads, smem, L.stream>>>(

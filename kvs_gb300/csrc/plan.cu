@@ -24,7 +24,8 @@ struct kvsmc_plan {
     std::vector<int32_t> iso_req;         // per planned isolevel: its request
     std::vector<uint64_t> cap;            // per planned isolevel: triangles its outputs hold
     void* d_mem = nullptr;
-    uint64_t* h_out = nullptr;            // pinned: [0] status word, [1 + i] total of isolevel i
+    uint64_t* h_out = nullptr;            // pinned: the status words' 256 bytes, then the isolevels' totals
+    bool listed = false;                  // the emit goes over listed pairs with no other one behind it
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     uint64_t kernels = 0;
@@ -69,9 +70,9 @@ cudaError_t record(kvsmc_host::StreamBatch& b, cudaStream_t s, int num_sms, uint
     if (e == cudaSuccess) e = per_kind(false);
     if (e == cudaSuccess) e = b.scans(L);
     if (e == cudaSuccess) e = per_kind(true);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_out, b.d_status, sizeof(int), cudaMemcpyDeviceToHost, s);
+    // (the totals lie 256 bytes behind the status words)
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(h_out + 1, b.d_totals, b.isos.size() * sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
+        e = cudaMemcpyAsync(h_out, b.d_status, 256 + b.isos.size() * sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
     return e;
 }
 
@@ -137,9 +138,10 @@ kvsmc_status kvsmc_plan_create(kvsmc_context* ctx, const kvsmc_request* reqs, in
         b.list_cap = 0;
         e = kvsmc_host::device_malloc(ctx, &p->d_mem, b.scratch_bytes());
     }
-    if (e == cudaSuccess) e = cudaMallocHost(&p->h_out, (b.isos.size() + 1) * sizeof(uint64_t));
+    p->listed = b.list_cap && b.list_sure;
+    if (e == cudaSuccess) e = cudaMallocHost(&p->h_out, 256 + b.isos.size() * sizeof(uint64_t));
     if (e == cudaSuccess) {
-        std::memset(p->h_out, 0, (b.isos.size() + 1) * sizeof(uint64_t));
+        std::memset(p->h_out, 0, 256 + b.isos.size() * sizeof(uint64_t));
         b.carve(static_cast<char*>(p->d_mem));
         e = cudaMemcpy(b.d_groups, b.groups.data(), b.groups.size() * sizeof(kvsmc::StreamGroup),
                        cudaMemcpyHostToDevice);
@@ -192,21 +194,27 @@ kvsmc_status kvsmc_plan_wait(kvsmc_plan* p, kvsmc_request* reqs, int32_t n)
         reqs[i].sizes = p->base[i];
         reqs[i].status = p->pre[i];
     }
-    int status = 0;
-    if (p->h_out) std::memcpy(&status, p->h_out, sizeof(int));
+    int status = 0, over = 0;
+    if (p->h_out) {
+        std::memcpy(&status, p->h_out, sizeof(int));
+        std::memcpy(&over, reinterpret_cast<const int*>(p->h_out) + 8, sizeof(int));   // the list's overflow word
+    }
+    over = over && p->listed;   // (never: the list has room for every pair; nothing would have been written)
     for (size_t k = 0; k < p->iso_req.size(); ++k) {
         kvsmc_request& r = reqs[p->iso_req[k]];
-        const uint64_t t = p->h_out[1 + k];
+        const uint64_t t = p->h_out[256 / sizeof(uint64_t) + k];
         r.sizes.ntriangles = t;
         r.sizes.nvertices = 3 * t;
         r.sizes.ncoords = 9 * t;
         r.sizes.nnormals = 3 * t;
         if (status) r.status = KVSMC_ERR_TIMEOUT;
+        else if (over) r.status = KVSMC_ERR_CUDA;
         else if (t > p->cap[k]) r.status = KVSMC_ERR_CAPACITY;
     }
     for (int32_t i = 0; i < n; ++i)
         if (reqs[i].status && !first) first = reqs[i].status;
     if (status) return kvsmc_host::fail(ctx, KVSMC_ERR_TIMEOUT, "plan: a shared-memory load did not complete");
+    if (over) return kvsmc_host::fail(ctx, KVSMC_ERR_CUDA, "plan: the pair list overflowed");
     if (first == KVSMC_ERR_CAPACITY) return kvsmc_host::fail(ctx, first, "plan: a result exceeds its output buffers");
     return first;
 }

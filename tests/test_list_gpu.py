@@ -1,0 +1,42 @@
+"""The list of crossed cells: its room, and what runs when it has none."""
+import numpy as np
+import pytest
+
+from kvs_gb300 import _abi
+
+from .helpers import same_bits
+from .test_stream_gpu import extract_batch
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("shape", [(600, 600, 2), (340, 900, 3), (90, 2100, 2), (2, 2, 2)])
+@pytest.mark.parametrize("dtype", [np.uint8, np.float32])
+def test_narrow_volumes_in_a_plan(kvsmc_ctx, dtype, shape):
+    """Few cells a task and many tasks: every counting warp holds a run of list
+    entries that it leaves nearly unused, beyond the cells there are.  A plan
+    whose list has room for all of them records no other emit."""
+    rng = np.random.default_rng(5)
+    v = (rng.random(shape) * 200).astype(dtype)
+    vol = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+    params = [_abi.make_params(x, 0) for x in (60.5, 100.5, 140.5)]
+    want = extract_batch(kvsmc_ctx, [vol] * 3, params, _abi.PATH_GATHER)
+    for group in ([0], [1], [0, 1, 2]):
+        reqs = (_abi.Request * len(group))()
+        outs = []
+        for r, i in zip(reqs, group):
+            c, n = torch.zeros(want[i]["coords"].size + 1, device="cuda"), torch.zeros(want[i]["normals"].size + 1, device="cuda")
+            outs.append((c, n))
+            r.volume, r.params = vol.handle, params[i]
+            r.d_coords, r.coords_capacity, r.d_normals, r.normals_capacity = c.data_ptr(), c.numel(), n.data_ptr(), n.numel()
+        torch.cuda.synchronize()
+        plan = _abi.Plan(kvsmc_ctx, reqs)
+        for _ in range(2):
+            plan.launch()
+            plan.wait()
+        for (c, n), i in zip(outs, group):
+            assert same_bits(c[:-1].cpu().numpy(), want[i]["coords"]) and same_bits(n[:-1].cpu().numpy(), want[i]["normals"])
+        plan.close()
+    vol.free()

@@ -89,9 +89,10 @@ __global__ void __launch_bounds__(kIngestThreads)
     for (uint64_t b = (uint64_t)blockIdx.x * (kIngestThreads / 32) + warp; b < nbricks; b += warps) {
         const uint32_t q = (uint32_t)(b / nbx), bx = (uint32_t)(b - (uint64_t)q * nbx);   // (below 2^32 brick rows)
         const uint32_t bz = q / nby, by = q - bz * nby;
-        const uint32_t x0 = bx * kBrickCells, x1 = min(x0 + kBrickCells, cx);
-        const uint32_t y0 = 2 * by, y1 = min(y0 + 2, cy);
-        const uint32_t z0 = bz * kBrickPlanes, z1 = min(z0 + kBrickPlanes, cz);
+        // (ends as a start and a length: a row may have 2^32 - 1 nodes)
+        const uint32_t x0 = bx * kBrickCells, x1 = x0 + min(kBrickCells, cx - x0);
+        const uint32_t y0 = 2 * by, y1 = y0 + min(2u, cy - y0);
+        const uint32_t z0 = bz * kBrickPlanes, z1 = z0 + min((uint32_t)kBrickPlanes, cz - z0);
         // this lane's nodes of a row: x0 + lane + 32 i, and lane r < 3 the one past
         // the brick's 128 cells in row r (its own only at the end of the row).
         // Columns and rows past the last are the last one again: the same values
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(kIngestThreads)
                     }
                 }
             }
-            if (COPY && (z < z0 + kBrickPlanes || z == cz)) {
+            if (COPY && (z - z0 < kBrickPlanes || z == cz)) {
                 T* const to_row[3] = {to, to + to1, to + to2};
 #pragma unroll
                 for (int r = 0; r < 3; ++r) {
@@ -228,9 +229,10 @@ __global__ void __launch_bounds__(kIngestThreads)
 
 cudaError_t launch_ingest(const VolumeView& v, const void* src, float2* bricks, IngestOut* d_out, const Launch& L)
 {
-    const uint32_t nbx = std::max(1u, (v.nx - 1 + kBrickCells - 1) / kBrickCells);
-    const uint32_t nby = std::max(1u, v.ny / 2);
-    const uint64_t nbz = std::max(1u, (v.nz - 1 + kBrickPlanes - 1) / kBrickPlanes);
+    // bricks of `per` cells along an axis of n nodes (at least one; n may be 2^32 - 1)
+    auto bricks_of = [](uint32_t n, uint32_t per) { return n < 2 ? 1u : (n - 2) / per + 1; };
+    const uint32_t nbx = bricks_of(v.nx, kBrickCells), nby = bricks_of(v.ny, 2);
+    const uint64_t nbz = bricks_of(v.nz, (uint32_t)kBrickPlanes);
     const uint64_t n = (uint64_t)nbx * nby * nbz;
     cudaError_t e = cudaMemsetAsync(d_out, 0xff, sizeof *d_out, L.stream);
     if (e != cudaSuccess) return e;

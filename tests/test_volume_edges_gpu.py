@@ -202,3 +202,14 @@ def test_a_request_behind_a_queued_update(kvsmc_ctx):
         srv.close()
         torch.cuda.synchronize()
         vol.free()
+
+
+def test_the_longest_row(kvsmc_ctx):
+    """2^32 - 1 nodes: the last brick's end is not a 32-bit number."""
+    n = (1 << 32) - 1
+    src = torch.full((n,), 100, dtype=torch.uint8, device="cuda")
+    src[-1], src[n - 200] = 7, 201
+    torch.cuda.synchronize()
+    vol = _abi.DeviceVolume.from_device(kvsmc_ctx, src.data_ptr(), np.uint8, (1, 1, n))
+    assert vol.minmax() == (7.0, 201.0)
+    vol.free()

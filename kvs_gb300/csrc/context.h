@@ -22,10 +22,11 @@ struct kvsmc_volume {
     std::atomic<bool> lent{false};
     bool has_minmax = false;
     double vmin = 0.0, vmax = 0.0;
-    // parts of the same allocation, written by the pass that every copy into a
-    // resident volume ends with: the values' range (range_ready; read back
-    // when it is first asked for) and the brick min/max table (the streaming
-    // kernels' empty-space skip; null for volumes that they do not take)
+    // parts of the same allocation: the brick min/max table (the streaming
+    // kernels' empty-space skip; null for volumes that they do not take), written
+    // by the pass that every copy into such a volume ends with, and the values'
+    // range (range_ready), by that pass or by one of its own when it is first
+    // asked for; it is read back then
     kvsmc::IngestOut* range = nullptr;
     bool range_ready = false;
     float2* bricks = nullptr;
@@ -191,8 +192,8 @@ void volume_destroy(kvsmc_context* ctx, kvsmc_volume* v);
 kvsmc_status volume_create(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, uint32_t ny, uint32_t nz,
                            kvsmc_volume** out);
 
-// (Re)build a resident volume's brick min/max table and its range from its
-// values on the context's stream.
+// (Re)build a resident volume's brick min/max table, if it has one, and with it
+// its range from its values on the context's stream.
 kvsmc_status volume_bricks(kvsmc_context* ctx, kvsmc_volume* v);
 
 // Run fn(i, stream) for i < n side by side on the context's auxiliary streams,

@@ -56,12 +56,46 @@ KVSMC_LIMITS(double, __longlong_as_double((long long)0xfff0000000000000ull), __l
 
 constexpr int kIngestThreads = 256;
 
+// A CTA's share of the range: the smallest of its threads' keys (all ones: none)
+// into `out`, and the volume's first value.
+template <bool FLOAT, typename T>
+__device__ __forceinline__ void range_out(unsigned long long klo, unsigned long long knhi, unsigned long long zero,
+                                          const T* values, IngestOut* out)
+{
+    __shared__ unsigned long long s_lo[kIngestThreads / 32], s_nhi[kIngestThreads / 32], s_zero[kIngestThreads / 32];
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        klo = min(klo, __shfl_xor_sync(0xffffffffu, klo, o));
+        knhi = min(knhi, __shfl_xor_sync(0xffffffffu, knhi, o));
+        if (FLOAT) zero = min(zero, __shfl_xor_sync(0xffffffffu, zero, o));
+    }
+    if (lane == 0) {
+        s_lo[warp] = klo;
+        s_nhi[warp] = knhi;
+        s_zero[warp] = zero;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < kIngestThreads / 32; ++k) {
+            klo = min(klo, s_lo[k]);
+            knhi = min(knhi, s_nhi[k]);
+            zero = min(zero, s_zero[k]);
+        }
+        // (most CTAs change nothing: a look saves their turns at the same word)
+        if (klo < __ldcg(&out->lo)) atomicMin(&out->lo, klo);
+        if (knhi < __ldcg(&out->nhi)) atomicMin(&out->nhi, knhi);
+        if (FLOAT && zero != ~0ull) atomicMin(&out->zero, zero);
+        if (blockIdx.x == 0) out->first = raw_bits(values[0]);
+    }
+}
+
 // One warp per brick of 8 cell planes x 2 cell rows x 128 cells (9 x 3 x 129
 // nodes; bricks share their border nodes), persistent over the bricks.  src
 // (may be null): the values, dense; every node is written once into the
 // padded layout by the brick that owns it.  Without src the values are read
-// in place.  Each brick's min and max go to `bricks` (null: no table), the
-// range of all values to `out`.
+// in place.  Each brick's min and max go to `bricks`, the range of all values to
+// `out`.
 //
 // Each value is read once from HBM (a brick's border nodes again from L1/L2,
 // 1.7 loads a node in all) and written once; a warp's 13 loads of one plane are
@@ -70,14 +104,15 @@ constexpr int kIngestThreads = 256;
 // only where one comparison a value has found some: branches for every value
 // made 73 instructions a value and 78 us.  83 MB of floats (301 x 256 x 270):
 // now 48 us, 3.4 TB/s read and written together (a copy, a brick pass and a
-// min/max scan took 72, 137 us and more).
-template <typename T, bool BRICKS, bool COPY>
+// min/max scan took 72, 137 us and more).  Looking at every zero of a background
+// made the pass up to a fifth slower than without zeros; only a brick's first
+// one is looked at.
+template <typename T, bool COPY>
 __global__ void __launch_bounds__(kIngestThreads)
     k_ingest(VolumeView v, const T* __restrict__ src, uint32_t nbx, uint32_t nby, uint64_t nbricks,
              float2* __restrict__ bricks, IngestOut* __restrict__ out)
 {
     constexpr bool kFloat = T(0.5) != T(0);
-    __shared__ unsigned long long s_lo[kIngestThreads / 32], s_nhi[kIngestThreads / 32], s_zero[kIngestThreads / 32];
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     T* const dst = static_cast<T*>(const_cast<void*>(v.data));
     const uint32_t cx = v.nx - 1, cy = v.ny - 1, cz = v.nz - 1;
@@ -104,7 +139,7 @@ __global__ void __launch_bounds__(kIngestThreads)
         for (int i = 0; i < 4; ++i) off[i] = min(lane + 32 * i, wx);
         const uint32_t r4 = min(lane, wy);   // (lanes 0 .. 2)
         T blo = Limits<T>::highest(), bhi = Limits<T>::lowest();   // NaN apart
-        bool nan = false;
+        bool nan = false, met = false;   // (met: a zero)
         const T* in = from + (uint64_t)z0 * sp + (uint64_t)y0 * rp + x0;
         T* to = dst + (uint64_t)z0 * v.slice + (uint64_t)y0 * v.pitch + x0;
         const uint64_t in1 = wy ? rp : 0, in2 = wy == 2 ? 2 * rp : in1;
@@ -119,7 +154,7 @@ __global__ void __launch_bounds__(kIngestThreads)
             if (lane < 3) e = (in + r4 * rp)[wx];
             bool special = false;   // a zero or a NaN among this lane's values
             auto take = [&](T val) {
-                if constexpr (BRICKS && kFloat) {
+                if constexpr (kFloat) {
                     blo = fminf(blo, val);
                     bhi = fmaxf(bhi, val);
                 } else {
@@ -134,20 +169,28 @@ __global__ void __launch_bounds__(kIngestThreads)
                 for (int i = 0; i < 4; ++i) take(w[r][i]);
             if (lane < 3) take(e);
             if constexpr (kFloat) {
-                if (special) {   // (a background of zeros pays for it, others do not)
-                    auto look = [&](T val, uint32_t y, uint32_t x) {
-                        nan |= val != val;
-                        // among equal values the scan keeps the first: only zeros' signs show it
-                        // (a warp's bricks do not come in index order)
-                        if (val == T(0))
+                if (special) {
+#pragma unroll
+                    for (int r = 0; r < 3; ++r)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) nan |= w[r][i] != w[r][i];
+                    nan |= e != e;
+                    // among equal values the scan keeps the first: only zeros' signs
+                    // show it.  A thread meets a brick's values in index order, so the
+                    // brick's first zero will do (a warp's bricks do not come in order)
+                    if (!met) {
+                        auto look = [&](T val, uint32_t y, uint32_t x) {
+                            if (met || val != T(0)) return;
+                            met = true;
                             zero = min(zero, ((((unsigned long long)z * v.ny + y) * v.nx + x) << 1) |
                                                  (raw_bits(val) != 0 ? 1ull : 0ull));
-                    };
+                        };
 #pragma unroll
-                    for (int r = 0; r < 3; ++r) {
+                        for (int r = 0; r < 3; ++r) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) look(w[r][i], y0 + ((uint32_t)r < wy ? (uint32_t)r : wy), x0 + off[i]);
-                        if ((int)lane == r) look(e, y0 + r4, x1);
+                            for (int i = 0; i < 4; ++i) look(w[r][i], y0 + ((uint32_t)r < wy ? (uint32_t)r : wy), x0 + off[i]);
+                            if ((int)lane == r) look(e, y0 + r4, x1);
+                        }
                     }
                 }
             }
@@ -167,85 +210,147 @@ __global__ void __launch_bounds__(kIngestThreads)
         }
         if (blo < lo) lo = blo;
         if (bhi > hi) hi = bhi;
-        if constexpr (BRICKS) {
-            if (bricks) {   // (values of these types are floats exactly)
-                float a = (float)blo, c = (float)bhi;
+        // (values of these types are floats exactly)
+        float a = (float)blo, c = (float)bhi;
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    a = fminf(a, __shfl_xor_sync(0xffffffffu, a, o));
-                    c = fmaxf(c, __shfl_xor_sync(0xffffffffu, c, o));
-                }
-                nan = __any_sync(0xffffffffu, nan);
-                // a brick holding a NaN is never skipped
-                if (lane == 0)
-                    bricks[b] = nan ? make_float2(__int_as_float(0xff800000), __int_as_float(0x7f800000))
-                                    : make_float2(a, c);
-            }
+        for (int o = 16; o > 0; o >>= 1) {
+            a = fminf(a, __shfl_xor_sync(0xffffffffu, a, o));
+            c = fmaxf(c, __shfl_xor_sync(0xffffffffu, c, o));
         }
+        nan = __any_sync(0xffffffffu, nan);
+        // a brick holding a NaN is never skipped
+        if (lane == 0)
+            bricks[b] = nan ? make_float2(__int_as_float(0xff800000), __int_as_float(0x7f800000)) : make_float2(a, c);
     }
     const bool any = lo <= hi;
-    unsigned long long klo = any ? value_key(lo) : ~0ull, knhi = any ? ~value_key(hi) : ~0ull;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        klo = min(klo, __shfl_xor_sync(0xffffffffu, klo, o));
-        knhi = min(knhi, __shfl_xor_sync(0xffffffffu, knhi, o));
-        zero = min(zero, __shfl_xor_sync(0xffffffffu, zero, o));
-    }
-    if (lane == 0) {
-        s_lo[warp] = klo;
-        s_nhi[warp] = knhi;
-        s_zero[warp] = zero;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 1; k < kIngestThreads / 32; ++k) {
-            klo = min(klo, s_lo[k]);
-            knhi = min(knhi, s_nhi[k]);
-            zero = min(zero, s_zero[k]);
+    range_out<kFloat>(any ? value_key(lo) : ~0ull, any ? ~value_key(hi) : ~0ull, zero, from, out);
+}
+
+// One value of the range of a thread's values (see k_flat).  8-byte values by
+// their keys: doubles compare at 1/58 of the integer rate.
+template <typename T> struct RangeTake {
+    static constexpr bool kFloat = T(0.5) != T(0);
+    unsigned long long klo = ~0ull, knhi = ~0ull, zero = ~0ull;
+    T lo = Limits<T>::highest(), hi = Limits<T>::lowest();
+    __device__ __forceinline__ void take(T val, uint64_t index)
+    {
+        if constexpr (sizeof(T) == 8) {
+            unsigned long long k = value_key(val);
+            if constexpr (kFloat) {
+                const unsigned long long u = raw_bits(val) << 1;
+                if (u - 1 >= 0xffe0000000000000ull) {   // a zero or a NaN
+                    if (u != 0) return;
+                    zero = min(zero, (index << 1) | (raw_bits(val) != 0 ? 1ull : 0ull));
+                }
+            }
+            klo = min(klo, k);
+            knhi = min(knhi, ~k);
+        } else {
+            if (val < lo) lo = val;   // (false for a NaN)
+            if (val > hi) hi = val;
+            if constexpr (kFloat)
+                if (val == T(0)) zero = min(zero, (index << 1) | (raw_bits(val) != 0 ? 1ull : 0ull));
         }
-        atomicMin(&out->lo, klo);
-        atomicMin(&out->nhi, knhi);
-        if (kFloat) atomicMin(&out->zero, zero);
-        if (blockIdx.x == 0) out->first = raw_bits(from[0]);
     }
+    __device__ __forceinline__ void keys()
+    {
+        if (sizeof(T) < 8 && lo <= hi) {
+            klo = value_key(lo);
+            knhi = ~value_key(hi);
+        }
+    }
+};
+
+// The same for volumes without a brick table (32/64-bit integers, doubles, and
+// shapes that the streaming kernels do not take: one node thick, or rows wider
+// than theirs): their values in index order, a warp 256 at a time with its eight
+// loads in flight, so that it does not matter how the volume is shaped.  By
+// bricks, an update of 262144 rows of one double took 985 us and one of
+// 256x256x512 doubles 1789; now 42, and 1290 (the copy: nobody asked for the
+// range).  A kvsmc_volume_from_device of the latter and its range: 183 us.
+constexpr uint32_t kFlatTile = 256;
+
+template <typename T, bool COPY>
+__global__ void __launch_bounds__(kIngestThreads)
+    k_flat(VolumeView v, const T* __restrict__ src, uint64_t n, IngestOut* __restrict__ out)
+{
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    T* const dst = static_cast<T*>(const_cast<void*>(v.data));
+    const bool padded = v.pitch != v.nx;
+    RangeTake<T> r;
+    const uint64_t tiles = (n + kFlatTile - 1) / kFlatTile, warps = (uint64_t)gridDim.x * (kIngestThreads / 32);
+    for (uint64_t t = (uint64_t)blockIdx.x * (kIngestThreads / 32) + warp; t < tiles; t += warps) {
+        const uint64_t i0 = t * kFlatTile, row0 = padded ? i0 / v.nx : 0;
+        const uint32_t left = v.nx - (uint32_t)(i0 - row0 * v.nx);   // of the tile's first row
+        uint64_t at[kFlatTile / 32];
+        T w[kFlatTile / 32];
+#pragma unroll
+        for (uint32_t k = 0; k < kFlatTile / 32; ++k) {
+            const uint32_t j = lane + 32 * k;
+            uint64_t row = row0;
+            uint32_t col = v.nx - left + j;
+            if (padded && j >= left) {   // of a later row
+                const uint32_t q = (j - left) / v.nx;
+                row += 1 + q;
+                col = (j - left) - q * v.nx;
+            }
+            at[k] = padded ? row * v.pitch + col : i0 + j;
+            if (i0 + j < n) w[k] = COPY ? src[i0 + j] : dst[at[k]];
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kFlatTile / 32; ++k) {
+            const uint64_t i = i0 + lane + 32 * k;
+            if (i >= n) continue;
+            if (COPY) dst[at[k]] = w[k];
+            r.take(w[k], i);
+        }
+    }
+    r.keys();
+    range_out<RangeTake<T>::kFloat>(r.klo, r.knhi, r.zero, COPY ? src : dst, out);
 }
 
 }  // namespace
 
-#define KVSMC_INGEST_SWITCH(DT, ...)                                                  \
-    switch (DT) {                                                                     \
-    case 0: { using T = int8_t; constexpr bool B = true; __VA_ARGS__; } break;        \
-    case 1: { using T = int16_t; constexpr bool B = true; __VA_ARGS__; } break;       \
-    case 2: { using T = int32_t; constexpr bool B = false; __VA_ARGS__; } break;      \
-    case 3: { using T = long long; constexpr bool B = false; __VA_ARGS__; } break;    \
-    case 4: { using T = uint8_t; constexpr bool B = true; __VA_ARGS__; } break;       \
-    case 5: { using T = uint16_t; constexpr bool B = true; __VA_ARGS__; } break;      \
-    case 6: { using T = uint32_t; constexpr bool B = false; __VA_ARGS__; } break;     \
-    case 7: { using T = unsigned long long; constexpr bool B = false; __VA_ARGS__; } break; \
-    case 8: { using T = float; constexpr bool B = true; __VA_ARGS__; } break;         \
-    case 9: { using T = double; constexpr bool B = false; __VA_ARGS__; } break;       \
-    default: return cudaErrorInvalidValue;                                            \
-    }
-
 cudaError_t launch_ingest(const VolumeView& v, const void* src, float2* bricks, IngestOut* d_out, const Launch& L)
 {
+    cudaError_t e = cudaMemsetAsync(d_out, 0xff, sizeof *d_out, L.stream);
+    if (e != cudaSuccess) return e;
     // bricks of `per` cells along an axis of n nodes (at least one; n may be 2^32 - 1)
     auto bricks_of = [](uint32_t n, uint32_t per) { return n < 2 ? 1u : (n - 2) / per + 1; };
     const uint32_t nbx = bricks_of(v.nx, kBrickCells), nby = bricks_of(v.ny, 2);
-    const uint64_t nbz = bricks_of(v.nz, (uint32_t)kBrickPlanes);
-    const uint64_t n = (uint64_t)nbx * nby * nbz;
-    cudaError_t e = cudaMemsetAsync(d_out, 0xff, sizeof *d_out, L.stream);
-    if (e != cudaSuccess) return e;
-    const uint64_t need = (n + kIngestThreads / 32 - 1) / (kIngestThreads / 32), cap = (uint64_t)L.num_sms * 8;
+    const uint64_t nbricks = (uint64_t)nbx * nby * bricks_of(v.nz, (uint32_t)kBrickPlanes);
+    const uint64_t n = (uint64_t)v.nx * v.ny * v.nz;
+    const uint64_t warps = bricks ? nbricks : (n + kFlatTile - 1) / kFlatTile;   // one each, if they fit
+    const uint64_t need = (warps + kIngestThreads / 32 - 1) / (kIngestThreads / 32), cap = (uint64_t)L.num_sms * 8;
+    const unsigned grid = (unsigned)(need < cap ? need : cap);
+#define KVSMC_FLAT(T)                                                                                    \
+    if (src) k_flat<T, true><<<grid, kIngestThreads, 0, L.stream>>>(v, static_cast<const T*>(src), n, d_out); \
+    else k_flat<T, false><<<grid, kIngestThreads, 0, L.stream>>>(v, nullptr, n, d_out);                  \
+    break;
+#define KVSMC_TABLE(T)                                                                                        \
+    if (!bricks) { KVSMC_FLAT(T) }                                                                            \
+    if (src)                                                                                                  \
+        k_ingest<T, true><<<grid, kIngestThreads, 0, L.stream>>>(v, static_cast<const T*>(src), nbx, nby, nbricks, \
+                                                                 bricks, d_out);                              \
+    else                                                                                                      \
+        k_ingest<T, false><<<grid, kIngestThreads, 0, L.stream>>>(v, nullptr, nbx, nby, nbricks, bricks, d_out);   \
+    break;
     prof_begin(L, "ingest");
-    KVSMC_INGEST_SWITCH(v.dtype, {
-        const unsigned grid = (unsigned)(need < cap ? need : cap);
-        if (src)
-            k_ingest<T, B, true><<<grid, kIngestThreads, 0, L.stream>>>(v, static_cast<const T*>(src), nbx, nby, n,
-                                                                         bricks, d_out);
-        else
-            k_ingest<T, B, false><<<grid, kIngestThreads, 0, L.stream>>>(v, nullptr, nbx, nby, n, bricks, d_out);
-    });
+    switch (v.dtype) {
+    case 0: KVSMC_TABLE(int8_t)
+    case 1: KVSMC_TABLE(int16_t)
+    case 2: KVSMC_FLAT(int32_t)
+    case 3: KVSMC_FLAT(long long)
+    case 4: KVSMC_TABLE(uint8_t)
+    case 5: KVSMC_TABLE(uint16_t)
+    case 6: KVSMC_FLAT(uint32_t)
+    case 7: KVSMC_FLAT(unsigned long long)
+    case 8: KVSMC_TABLE(float)
+    case 9: KVSMC_FLAT(double)
+    default: return cudaErrorInvalidValue;
+    }
+#undef KVSMC_TABLE
+#undef KVSMC_FLAT
     prof_end(L);
     *L.counter += 1;
     return cudaGetLastError();
@@ -427,7 +532,10 @@ kvsmc_status volume_alloc(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, ui
     return KVSMC_OK;
 }
 
-kvsmc_status volume_bricks(kvsmc_context* ctx, kvsmc_volume* v)
+namespace {
+
+// The pass over values that are in place.
+kvsmc_status ingest_in_place(kvsmc_context* ctx, kvsmc_volume* v)
 {
     KVSMC_CUDA(ctx, kvsmc::launch_ingest(v->view, nullptr, v->bricks, v->range, launch_of(ctx)));
     KVSMC_CUDA(ctx, cudaEventRecord(v->ev, ctx->stream));
@@ -435,6 +543,10 @@ kvsmc_status volume_bricks(kvsmc_context* ctx, kvsmc_volume* v)
     v->range_ready = true;
     return KVSMC_OK;
 }
+
+}  // namespace
+
+kvsmc_status volume_bricks(kvsmc_context* ctx, kvsmc_volume* v) { return v->bricks ? ingest_in_place(ctx, v) : KVSMC_OK; }
 
 kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src, bool on_device)
 {
@@ -482,11 +594,16 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
         else
             KVSMC_CUDA(ctx, cudaMemcpy2DAsync(v->dev, v->view.pitch * es, src, row, row, rows, kind, ctx->stream));
     }
-    KVSMC_CUDA(ctx, kvsmc::launch_ingest(v->view, from, v->bricks, v->range, launch_of(ctx)));
+    // values that are in place already and need no table: their range is taken
+    // when it is first asked for (an update with a preset one never does)
+    v->bricks_valid = false;
+    if (from || v->bricks) {
+        KVSMC_CUDA(ctx, kvsmc::launch_ingest(v->view, from, v->bricks, v->range, launch_of(ctx)));
+        v->bricks_valid = v->bricks != nullptr;
+        v->range_ready = true;
+    }
     KVSMC_CUDA(ctx, cudaEventRecord(v->ev, ctx->stream));
     if (from && from == ctx->dense) KVSMC_CUDA(ctx, cudaEventRecord(ctx->dense_ev, ctx->stream));
-    v->bricks_valid = v->bricks != nullptr;
-    v->range_ready = true;
     return KVSMC_OK;
 }
 
@@ -495,7 +612,7 @@ kvsmc_status volume_minmax(kvsmc_context* ctx, kvsmc_volume* v)
     if (v->has_minmax) return KVSMC_OK;
     volume_use(ctx, v);
     if (!v->range_ready)
-        if (kvsmc_status st = volume_bricks(ctx, v)) return st;
+        if (kvsmc_status st = ingest_in_place(ctx, v)) return st;
     KVSMC_CUDA(ctx, cudaMemcpyAsync(ctx->h_small, v->range, sizeof(kvsmc::IngestOut), cudaMemcpyDeviceToHost,
                                     ctx->stream));
     KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

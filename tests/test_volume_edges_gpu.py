@@ -10,6 +10,7 @@ import pytest
 from kvs_gb300 import _abi
 
 from .helpers import same_bits
+from .test_volume_gpu import _check, _values
 
 pytestmark = pytest.mark.gpu
 
@@ -213,3 +214,37 @@ def test_the_longest_row(kvsmc_ctx):
     vol = _abi.DeviceVolume.from_device(kvsmc_ctx, src.data_ptr(), np.uint8, (1, 1, n))
     assert vol.minmax() == (7.0, 201.0)
     vol.free()
+
+
+@pytest.mark.parametrize("dtype", _abi.DTYPES)
+def test_volumes_without_a_brick_table(kvsmc_ctx, dtype):
+    """One node thick, rows wider than the streaming kernels', and the wide
+    types: values in index order, 256 at a time, rows longer and much shorter
+    than that; the range is taken when it is asked for."""
+    for i, shape in enumerate([(1, 700, 3), (5, 3, 257), (2, 2, 4100), (300, 1, 2), (257, 1, 1), (1, 1, 256), (3, 5, 64)]):
+        v = _values(shape, dtype, i)
+        if np.dtype(dtype).kind == "f":
+            v.reshape(-1)[[1, 300 % v.size, v.size - 1]] = (-np.inf, np.nan, np.inf)
+        dv = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+        _check(dv, v)
+        w = _values(shape, dtype, 50 + i)
+        kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_volume_update(kvsmc_ctx.handle, dv.handle, w.ctypes.data), "update")
+        _check(dv, w)
+        dv.free()
+        raw = torch.from_numpy(v.reshape(-1).view(np.uint8).copy()).cuda()
+        torch.cuda.synchronize()
+        dv = _abi.DeviceVolume.from_device(kvsmc_ctx, raw.data_ptr(), dtype, shape)
+        _check(dv, v)
+        dv.free()
+
+
+def test_zero_signs_of_doubles(kvsmc_ctx):
+    base = np.full((4, 9, 301), 2.0)
+    for at, want in (([3, 700], -0.0), ([700, 3], 0.0), ([5000, 9], 0.0), ([0, 4], -0.0)):
+        for sign in (1.0, -1.0):
+            v = base * sign
+            v.put(at, [-0.0, 0.0])
+            dv = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+            lo, hi = dv.minmax()
+            assert same_bits(np.array([lo, hi]), np.array([want, 2.0] if sign > 0 else [-2.0, want])), (at, sign, lo, hi)
+            dv.free()

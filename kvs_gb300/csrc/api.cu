@@ -69,45 +69,58 @@ bool equal_ref(double a, double b)
     return ((d < 0) ? -d : d) < 1.e-6;
 }
 
+// The thresholds of float and up-to-32-bit integer values (see Classifier).
+void narrow_thresholds(double iso, float& f_thr, long long& i_thr)
+{
+    float f = (float)iso;
+    if (!std::isnan(iso) && (double)f > iso) f = std::nextafter(f, -INFINITY);
+    f_thr = f;
+    if (std::isnan(iso) || iso >= 4.0e18) i_thr = 0x7fffffffffffffffLL;
+    else if (iso < -4.0e18) i_thr = (long long)(-0x7fffffffffffffffLL - 1);
+    else i_thr = (long long)std::floor(iso);
+}
+
+namespace {
+
+// The largest of [lo, hi] whose nearest double is at most iso: the conversion is
+// monotone.  ((double)lo is, (double)hi is not.)
+template <typename I> I last_at_most(double iso, I lo, I hi)
+{
+    while (hi - lo > 1) {
+        const I mid = lo + (hi - lo) / 2;
+        if ((double)mid > iso) hi = mid; else lo = mid;
+    }
+    return lo;
+}
+
+}  // namespace
+
 // Exact classification thresholds (see Classifier).
 Classifier make_classifier(double iso)
 {
     Classifier c;
     c.iso = iso;
     c.all64 = 0;
-    // 64-bit integers: the conversion to double is monotone, so the values with
-    // (double)v > iso are the ones above the last value without
+    narrow_thresholds(iso, c.f_thr, c.i_thr);
+    // 64-bit integers: the values with (double)v > iso are the ones above the last
+    // value without: floor(iso) where doubles tell integers apart, by a search
+    // where they do not (one for every isolevel took 0.3 us of each: 64 small
+    // volumes in a batch 180 -> 160 us)
     constexpr long long kMin = (-0x7fffffffffffffffLL - 1), kMax = 0x7fffffffffffffffLL;
-    c.l_thr = kMax;
-    if ((double)kMax > iso) {   // (never for a NaN)
-        long long lo = kMin, hi = kMax;
-        while (lo < hi) {   // the smallest such value
-            const long long mid = (lo >> 1) + (hi >> 1) + (lo & hi & 1);   // floor((lo + hi) / 2)
-            if ((double)mid > iso) hi = mid; else lo = mid + 1;
-        }
-        if (lo == kMin) c.all64 |= 1;
-        c.l_thr = lo == kMin ? kMin : lo - 1;
-    }
-    c.u_thr = ~0ull;
-    if ((double)~0ull > iso) {
-        unsigned long long lo = 0, hi = ~0ull;
-        while (lo < hi) {
-            const unsigned long long mid = lo + (hi - lo) / 2;
-            if ((double)mid > iso) hi = mid; else lo = mid + 1;
-        }
-        if (lo == 0) c.all64 |= 2;
-        c.u_thr = lo == 0 ? 0 : lo - 1;
-    }
+    constexpr double k53 = 9007199254740992.0, k63 = 9223372036854775808.0, k64 = 2.0 * k63;
+    if (!(iso < k63)) c.l_thr = kMax;   // (a NaN too)
+    else if (iso < -k63) c.l_thr = kMin, c.all64 |= 1;
+    else if (std::fabs(iso) < k53) c.l_thr = (long long)std::floor(iso);
+    else if (iso > 0.0) c.l_thr = last_at_most<long long>(iso, 0, kMax);
+    else c.l_thr = last_at_most<long long>(iso, kMin, -1);
+    if (!(iso < k64)) c.u_thr = ~0ull;
+    else if (iso < 0.0) c.u_thr = 0, c.all64 |= 2;
+    else if (iso < k53) c.u_thr = (unsigned long long)std::floor(iso);
+    else c.u_thr = last_at_most<unsigned long long>(iso, 0, ~0ull);
     const double z = iso == 0.0 ? 0.0 : iso;
     long long bits;
     std::memcpy(&bits, &z, sizeof bits);
     c.d_key = std::isnan(iso) ? kMax : double_key(bits);
-    float f = (float)iso;
-    if (!std::isnan(iso) && (double)f > iso) f = std::nextafter(f, -INFINITY);
-    c.f_thr = f;
-    if (std::isnan(iso) || iso >= 4.0e18) c.i_thr = 0x7fffffffffffffffLL;
-    else if (iso < -4.0e18) c.i_thr = (long long)(-0x7fffffffffffffffLL - 1);
-    else c.i_thr = (long long)std::floor(iso);
     return c;
 }
 

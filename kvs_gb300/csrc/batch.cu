@@ -25,12 +25,10 @@ kvsmc::FastIso make_fast(double iso, double vmin, double vmax, int dtype)
 {
     kvsmc::FastIso f;
     std::memset(&f, 0, sizeof f);
-    const kvsmc::Classifier c = make_classifier(iso);
-    if (dtype == KVSMC_F32) {
-        f.f_thr = c.f_thr;
-    } else {
+    long long t;
+    narrow_thresholds(iso, f.f_thr, t);
+    if (dtype != KVSMC_F32) {
         // integer data: v > floor(iso) <=> float(v) > float(floor(iso)), |v| < 2^16
-        long long t = c.i_thr;
         if (t > (1LL << 24)) t = 1LL << 24;
         if (t < -(1LL << 24)) t = -(1LL << 24);
         f.f_thr = (float)t;

@@ -121,6 +121,7 @@ kvsmc_status ensure_stage(kvsmc_context* ctx, size_t bytes);
 kvsmc_status volume_minmax(kvsmc_context* ctx, kvsmc_volume* v);
 bool equal_ref(double a, double b);
 kvsmc::Classifier make_classifier(double iso);
+void narrow_thresholds(double iso, float& f_thr, long long& i_thr);
 
 // Bump allocator over an arena (256-byte aligned pieces).
 struct Carve {

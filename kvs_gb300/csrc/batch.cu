@@ -324,7 +324,14 @@ void StreamBatch::plan_tables()
     list_cap = 0;
     list_sure = false;
     if (pair_units) {
-        const uint64_t tail = (uint64_t)ctx->num_sms * kvsmc::kListWarpsPerSm * kvsmc::kPairRun * launches.size();
+        // (a warp that left a run unfinished had a task; with runs of 1024 for every
+        // warp, the list of a batch of small volumes was mostly room for those: 32 MB
+        // for 39 volumes of 9000 cells, now 1.8)
+        uint64_t warps = 0;
+        for (const Launch1& L : launches)
+            warps += std::min<uint64_t>(L.ntasks, (uint64_t)ctx->num_sms * kvsmc::kListWarpsPerSm);
+        list_run = (uint32_t)std::min<uint64_t>(kvsmc::kPairRun, std::max<uint64_t>(64, pairs_most / warps));
+        const uint64_t tail = warps * list_run;
         const uint64_t sure = 2 * pairs_most + tail;
         list_cap = std::min<uint64_t>(sure, std::max<uint64_t>((uint64_t)1 << 29, pairs_most / 8) + tail);
         list_cap = std::min<uint64_t>(list_cap, (uint64_t)1 << 31);
@@ -370,6 +377,7 @@ void StreamBatch::carve(char* base)
         list.unit_list = cv.take<uint32_t>(pair_units * 4);
         list.list = cv.take<uint16_t>(list_cap * 2);
         list.cap = list_cap;
+        list.run = list_run;
         list.cursor = reinterpret_cast<unsigned long long*>(d_status) + 16;
         list.overflow = d_status + 8;
     }

@@ -83,6 +83,7 @@ struct StreamBatch {
     // overflowed: the last count did, its emit classifies again
     bool want_list = false;
     uint64_t list_cap = 0;
+    uint32_t list_run = 0;   // entries that a warp of the count takes at a time
     bool list_sure = false;
     bool overflowed = false;
     uint64_t pair_units = 0;

@@ -131,10 +131,11 @@ struct PairList {
     uint64_t cap;
     unsigned long long* cursor;
     int* overflow;
+    uint32_t run;
 };
-// A count's warp takes entries in runs of this many (or one step's, if more),
-// and a listing count runs at most kListWarpsPerSm warps on an SM (its launch
-// is capped to them), so what its last runs leave unused has a bound.
+// A count's warp takes entries in runs of `run` (or one step's, if more), at
+// most kPairRun, and a listing count runs at most kListWarpsPerSm warps on an SM
+// (its launch is capped to them), so what its last runs leave unused has a bound.
 constexpr uint32_t kPairRun = 1024;
 constexpr int kListWarpsPerSm = 32;
 // The emit's block size is chosen for two blocks a warp with this many warps an

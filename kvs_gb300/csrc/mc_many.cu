@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(kManyThreads, 3)
             if (npairs == 0) continue;
             if (LIST) {
                 if (lcur + npairs > lend) {
-                    const uint32_t want = npairs > kPairRun ? npairs : kPairRun;
+                    const uint32_t want = npairs > pl.run ? npairs : pl.run;
                     unsigned long long at = 0;
                     if (lane == 0) at = atomicAdd(pl.cursor, (unsigned long long)want);
                     at = __shfl_sync(FULL, at, 0);

@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kOneThreads)
                         }
                         const uint32_t npairs = __shfl_sync(FULL, inc, 31);
                         if (lcur + npairs > lend) {
-                            const uint32_t want = npairs > kPairRun ? npairs : kPairRun;
+                            const uint32_t want = npairs > pl.run ? npairs : pl.run;
                             unsigned long long at = 0;
                             if (lane == 0) at = atomicAdd(pl.cursor, (unsigned long long)want);
                             lcur = __shfl_sync(FULL, at, 0);

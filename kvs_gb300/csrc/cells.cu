@@ -778,6 +778,10 @@ __global__ void __launch_bounds__(kCellThreads) k_cells_sweep_count(CellJob j)
         if ((int)lane + 32 * h < j.niso) j.block_counts[(lane + 32 * h) * blocks + blk] = sum[h];
 }
 
+// A warp takes 2^emit_shift groups of one isolevel: a sweep has isolevels times
+// blocks of work, so its blocks can be larger than the count's (whose triangles
+// are consecutive).  2e5 tetrahedra, 64 isolevels, most groups cut by none: with
+// the count's blocks of one group 205 us a call (emit 31), with blocks of 32 109 (16).
 template <int CT, typename T>
 __global__ void __launch_bounds__(kCellThreads) k_cells_sweep_emit(CellJob j)
 {
@@ -788,15 +792,16 @@ __global__ void __launch_bounds__(kCellThreads) k_cells_sweep_emit(CellJob j)
     __syncthreads();
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint64_t groups = (j.ncells + 31) / 32, blocks = (groups + (1ull << j.block_shift) - 1) >> j.block_shift;
-    const uint64_t it = (uint64_t)blockIdx.x * (kCellThreads / 32) + warp;   // (isolevel, block)
-    const uint64_t k = it / blocks, blk = it - k * blocks;
+    const uint64_t eblocks = (groups + (1ull << j.emit_shift) - 1) >> j.emit_shift;
+    const uint64_t it = (uint64_t)blockIdx.x * (kCellThreads / 32) + warp;   // (isolevel, emit block)
+    const uint64_t k = it / eblocks, eb = it - k * eblocks;
     if (k >= (uint64_t)j.niso) return;
-    const uint64_t g0 = blk << j.block_shift;
-    const uint32_t ng = (uint32_t)(groups - g0 < (1ull << j.block_shift) ? groups - g0 : 1ull << j.block_shift);
+    const uint64_t g0 = eb << j.emit_shift;
+    const uint32_t ng = (uint32_t)(groups - g0 < (1ull << j.emit_shift) ? groups - g0 : 1ull << j.emit_shift);
     const CellIso& I = j.isos[k];
     emit_block<CT, T, false>(j, I.cls, I.iso, I.f, I.out_coords, I.out_normals, I.cap_tris, TB, sw[warp], nullptr,
                              lane < ng ? j.cut_words[k * groups + g0 + lane] : 0u, g0,
-                             j.block_offsets[k * blocks + blk] - I.base, lane);
+                             j.block_offsets[k * blocks + (g0 >> j.block_shift)] - I.base, lane);
 }
 
 // base[k] = the first scanned offset of isolevel k, base[niso] = the total.
@@ -899,7 +904,7 @@ cudaError_t launch_cells_sweep_emit(const CellJob& j, const Launch& L)
     if (j.ncells == 0 || j.niso <= 0) return cudaSuccess;
     prof_begin(L, "cells_sweep_emit");
     KVSMC_CELL_SWITCH(j.cell_type, j.dtype, {
-        k_cells_sweep_emit<CT, T><<<cell_grid(cells_blocks(j.ncells, j.block_shift) * (uint64_t)j.niso), kCellThreads, 0, L.stream>>>(j);
+        k_cells_sweep_emit<CT, T><<<cell_grid(cells_blocks(j.ncells, j.emit_shift) * (uint64_t)j.niso), kCellThreads, 0, L.stream>>>(j);
     });
     prof_end(L);
     *L.counter += 1;
@@ -967,10 +972,10 @@ uint64_t cells_blocks(uint64_t ncells, int block_shift)
 // blocks fill the emit's rounds and shorten the scan; fewer of them would leave
 // warps idle: a mesh of 1e4 cells in blocks of one group takes 37 us a call,
 // where one warp to 32 groups in turn took 90.
-int cells_block_shift(uint64_t ncells, int num_sms)
+int cells_block_shift(uint64_t groups, int num_sms)
 {
     int s = 0;
-    while (s < 5 && (cells_groups(ncells) >> (s + 1)) >= (uint64_t)num_sms * 64) ++s;
+    while (s < 5 && (groups >> (s + 1)) >= (uint64_t)num_sms * 64) ++s;
     return s;
 }
 
@@ -1023,7 +1028,8 @@ kvsmc_status cells_prepare(kvsmc_context* ctx, kvsmc::CellJob& j, CellsScratch* 
     if (!ctx->d_flag) KVSMC_CUDA(ctx, kvsmc_host::device_malloc(ctx, &ctx->d_flag, sizeof(int)));
     j.bad_index = ctx->d_flag;
     KVSMC_CUDA(ctx, cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream));
-    j.block_shift = kvsmc::cells_block_shift(j.ncells, ctx->num_sms);
+    j.block_shift = kvsmc::cells_block_shift(kvsmc::cells_groups(j.ncells), ctx->num_sms);
+    j.emit_shift = kvsmc::cells_block_shift(kvsmc::cells_groups(j.ncells) * (uint64_t)niso, ctx->num_sms);
     sc->blocks = kvsmc::cells_blocks(j.ncells, j.block_shift);
     sc->nscan = sc->blocks * (uint64_t)niso;
     const size_t bw = align_up(kvsmc::cells_groups(j.ncells) * (uint64_t)niso * 4, 256),

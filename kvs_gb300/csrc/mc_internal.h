@@ -371,7 +371,8 @@ struct CellJob {
     Classifier cls;           // exact thresholds of the isolevel (no FP64 for float / 32-bit values)
     FastIso f;                // constants of the FP32 vertex certificate (emit pass)
     int32_t conn_vec16;       // connections 16-byte aligned: vector loads for tetrahedra / hexahedra
-    int32_t block_shift;      // 2^block_shift 32-cell groups per block
+    int32_t block_shift;      // 2^block_shift 32-cell groups per block of the count and its scan
+    int32_t emit_shift;       // sweep: per warp of the emit (at least block_shift)
     uint32_t* cut_words;      // per group: which of its cells have triangles
     uint32_t* block_counts;   // per block: its triangles
     uint64_t* block_offsets;  // and their exclusive scan
@@ -395,7 +396,7 @@ cudaError_t launch_cells_count(const CellJob& j, const Launch& L);
 cudaError_t launch_cells_emit(const CellJob& j, const Launch& L);
 uint64_t cells_groups(uint64_t ncells);
 uint64_t cells_blocks(uint64_t ncells, int block_shift);
-int cells_block_shift(uint64_t ncells, int num_sms);
+int cells_block_shift(uint64_t groups, int num_sms);
 cudaError_t launch_cells_sweep_count(const CellJob& j, const Launch& L);
 cudaError_t launch_cells_sweep_emit(const CellJob& j, const Launch& L);
 cudaError_t launch_sweep_bases(const uint64_t* offsets, uint64_t blocks, int niso, const uint64_t* total,

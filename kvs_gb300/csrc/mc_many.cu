@@ -13,7 +13,8 @@
 //   * the lanes only list their pairs (cell, isolevel) in a per-warp buffer;
 //     the pairs are then taken 32 at a time, one per lane: the eight mask bits,
 //     the triangle count, and one addition per distinct (row, isolevel) of the
-//     round (__match_any_sync and bit-sliced ballots), no atomics;
+//     round (__match_any_sync and bit-sliced ballots), no atomics; only steps
+//     where all lanes have many pairs keep the lanes' loops;
 //   * the same 32 entries go to the global list as one coalesced store;
 //   * a staged plane's values are not needed once its masks are formed, so two
 //     buffers a warp suffice, and the next copies start before the pairs are
@@ -22,8 +23,8 @@
 // it must not spill: 32 warps an SM at 64 registers took 1500 and 2312 us below,
 // 24 at 80 take 1220 and 1884, with the lower plane's masks read back from
 // shared memory and the task's addresses kept there.  640x704x600 f32, 16
-// isolevels: 1532 us with the lanes' loops, 1220 us; 1024x768x640 u16, 4
-// isolevels: 2735 -> 1884 us.
+// isolevels: 1532 us with the lanes' loops, 1210 us; 1024x768x640 u16, 4
+// isolevels: 2735 -> 1887 us.
 //
 // NODES: the shared-vertex modes' vertices per node unit too (plane, node row,
 // 256-node segment; those whose node segments are their cell segments).  A
@@ -43,7 +44,12 @@ namespace {
 
 constexpr int kManyThreads = 256;
 constexpr int kManyWarps = kManyThreads / 32;
-constexpr uint32_t kManyBuf = 128;   // listed pairs per warp at a time
+// Listed pairs per warp at a time.  A lane's pairs lie side by side, so where
+// every cell has several a short buffer is filled by one or two lanes at a time:
+// 16 isolevels of noise, 150^3: 6910 us a call with 128 entries, 5820 with 1024.
+constexpr uint32_t kManyBuf = 1024;
+// Pairs a step from which the lanes' own loops are looked at.
+constexpr uint32_t kManyCrowd = 512;
 constexpr unsigned FULL = 0xffffffffu;
 
 __device__ uint8_t d_many_ntri[256] = MC_NTRI_INIT;   // per reference case
@@ -294,21 +300,73 @@ __global__ void __launch_bounds__(kManyThreads, 3)
                 }
             }
             const uint32_t my_first = inc - m;
-            for (uint32_t fill0 = 0; fill0 < npairs; fill0 += kManyBuf) {
-                // this lane's pairs (cell order, then isolevel) that fall into the buffer
-                if (m && my_first < fill0 + kManyBuf && my_first + m > fill0) {
-                    uint32_t slot = my_first - fill0;   // (wraps below the window)
+            // the vertices of a pair's nodes behind the last row and plane
+            auto far_nodes = [&](uint32_t code, uint32_t k, bool last) {
+                auto cut = [&](int i, int j) -> uint32_t { return ((code >> i) ^ (code >> j)) & 1u; };
+                uint32_t v = 0;
+                if (last_row) v += cut(1, 5) + cut(1, 3) + (last ? cut(5, 7) : 0u);
+                if (z + 1 == cz) v += (cut(2, 6) + cut(2, 3) + (last ? cut(6, 7) : 0u)) << 10;
+                if (last_row && z + 1 == cz) v += cut(3, 7) << 20;
+                if (v) atomicAdd(&W.cnt[16 + k], v);
+            };
+            // this lane's pairs (cell order, then isolevel) that fall into the buffer
+            auto fill = [&](uint32_t fill0) {
+                if (!m || my_first >= fill0 + kManyBuf || my_first + m <= fill0) return;
+                uint32_t slot = my_first - fill0;   // (wraps below the window)
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        uint32_t am = (act[i >> 1] >> (16 * (i & 1))) & 0xffffu;
-                        while (am) {
-                            const uint32_t k = __ffs(am) - 1;
-                            am &= am - 1;
-                            if (slot < kManyBuf) W.buf[slot] = (uint16_t)((lane * 8 + i) | (k << 8));
-                            ++slot;
-                        }
+                for (int i = 0; i < 8; ++i) {
+                    uint32_t am = (act[i >> 1] >> (16 * (i & 1))) & 0xffffu;
+                    while (am) {
+                        const uint32_t k = __ffs(am) - 1;
+                        am &= am - 1;
+                        if (slot < kManyBuf) W.buf[slot] = (uint16_t)((lane * 8 + i) | (k << 8));
+                        ++slot;
                     }
                 }
+            };
+            // crowded, and evenly: the lanes' own loops with a shared atomic a pair (14
+            // instructions an iteration) take less than rounds of 32 pairs (60 each).
+            // The noise's count alone: 1430 us by rounds, 288
+            const bool crowded = npairs >= kManyCrowd && __reduce_max_sync(FULL, m) < npairs / 10;
+            if (crowded) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    uint32_t am = (act[i >> 1] >> (16 * (i & 1))) & 0xffffu;
+                    if (!am) continue;
+                    const uint32_t x = xl + i;
+                    const uint16_t* a = W.mask[s & 1u][half] + x;
+                    const uint16_t* b = W.mask[(s + 1) & 1u][half] + x;
+                    const uint32_t w0 = a[0] | ((uint32_t)a[1] << 16), w2 = b[0] | ((uint32_t)b[1] << 16);
+                    a += kMaskRow<R>;
+                    b += kMaskRow<R>;
+                    const uint32_t w1 = a[0] | ((uint32_t)a[1] << 16), w3 = b[0] | ((uint32_t)b[1] << 16);
+                    const bool last = NODES && xoff + x == cx - 1;
+                    do {
+                        const uint32_t k = __ffs(am) - 1;
+                        am &= am - 1;
+                        const uint32_t code = case_code(w0, w1, w2, w3, k), tab = s_tab[code];
+                        uint32_t v = tab & 7u;
+                        if (NODES) {
+                            v += (tab >> 3) << 16;
+                            if (last) v += ((((code >> 4) ^ (code >> 5)) & 1u) + (((code >> 4) ^ (code >> 6)) & 1u)) << 16;
+                            if (last_row || z + 1 == cz) far_nodes(code, k, last);
+                        }
+                        atomicAdd(&W.cnt[half * 16 + k], v);
+                    } while (am);
+                }
+                __syncwarp();
+                for (uint32_t fill0 = 0; LIST && fill0 < npairs; fill0 += kManyBuf) {
+                    fill(fill0);
+                    __syncwarp();
+                    for (uint32_t e = lane; e < kManyBuf && fill0 + e < npairs && !lfull; e += 32) {
+                        const uint32_t v = W.buf[e];
+                        pl.list[(uint64_t)lcur + fill0 + e] = (uint16_t)(((v & 0xffu) & (SEG - 1)) | (v & 0xff00u));
+                    }
+                    __syncwarp();
+                }
+            }
+            for (uint32_t fill0 = 0; !crowded && fill0 < npairs; fill0 += kManyBuf) {
+                fill(fill0);
                 __syncwarp();
                 const uint32_t nfill = npairs - fill0 < kManyBuf ? npairs - fill0 : kManyBuf;
                 for (uint32_t r0 = 0; r0 < nfill; r0 += 32) {
@@ -340,14 +398,7 @@ __global__ void __launch_bounds__(kManyThreads, 3)
 #pragma unroll
                         for (int bit = 0; bit < 3; ++bit)
                             sum += (uint32_t)__popc(__ballot_sync(FULL, (nv >> bit) & 1u) & grp) << (16 + bit);
-                        if (has && (last_row || z + 1 == cz)) {
-                            auto cut = [&](int i, int j) -> uint32_t { return ((code >> i) ^ (code >> j)) & 1u; };
-                            uint32_t v = 0;
-                            if (last_row) v += cut(1, 5) + cut(1, 3) + (last ? cut(5, 7) : 0u);
-                            if (z + 1 == cz) v += (cut(2, 6) + cut(2, 3) + (last ? cut(6, 7) : 0u)) << 10;
-                            if (last_row && z + 1 == cz) v += cut(3, 7) << 20;
-                            if (v) atomicAdd(&W.cnt[16 + k], v);
-                        }
+                        if (has && (last_row || z + 1 == cz)) far_nodes(code, k, last);
                     }
                     if (has && (grp & lt) == 0) W.cnt[key] += sum;   // one lane per distinct key
                     __syncwarp();

@@ -40,3 +40,26 @@ def test_narrow_volumes_in_a_plan(kvsmc_ctx, dtype, shape):
             assert same_bits(c[:-1].cpu().numpy(), want[i]["coords"]) and same_bits(n[:-1].cpu().numpy(), want[i]["normals"])
         plan.close()
     vol.free()
+
+
+@pytest.mark.parametrize("dtype", [np.uint16, np.float32])
+@pytest.mark.parametrize("noisy", [9, 70, 130, 257, 600])
+def test_crowded_steps(kvsmc_ctx, dtype, noisy):
+    """16 isolevels, noise in the first columns of rows that are smooth behind
+    them: steps whose pairs are few, many in a few lanes, and many in all (more
+    than the count's buffer holds); triangles and shared vertices."""
+    rng = np.random.default_rng(noisy)
+    v = np.broadcast_to(np.linspace(0.1, 0.9, 600), (5, 6, 600)).copy()
+    v[:, :, :noisy] = rng.random((5, 6, noisy))
+    v = (v * 60000).astype(dtype)
+    vol = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+    isos = [20000.5 + 1300 * k for k in range(16)]
+    for mode in (0, 2):
+        params = [_abi.make_params(x, mode) for x in isos]
+        want = extract_batch(kvsmc_ctx, [vol] * 16, params, _abi.PATH_GATHER)
+        got = extract_batch(kvsmc_ctx, [vol] * 16, params, _abi.PATH_AUTO)
+        for w, g in zip(want, got):
+            assert g["status"] == _abi.OK and g["ntri"] == w["ntri"]
+            assert same_bits(g["coords"], w["coords"]) and same_bits(g["normals"], w["normals"])
+            assert np.array_equal(g["connections"], w["connections"])
+    vol.free()

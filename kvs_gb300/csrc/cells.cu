@@ -781,7 +781,9 @@ __global__ void __launch_bounds__(kCellThreads) k_cells_sweep_count(CellJob j)
 // A warp takes 2^emit_shift groups of one isolevel: a sweep has isolevels times
 // blocks of work, so its blocks can be larger than the count's (whose triangles
 // are consecutive).  2e5 tetrahedra, 64 isolevels, most groups cut by none: with
-// the count's blocks of one group 205 us a call (emit 31), with blocks of 32 109 (16).
+// the count's blocks of one group 205 us a call (emit 31), with blocks of 16 110
+// (16).  Twice the count's blocks an SM: a warp's rounds over crowded blocks (every
+// cell cut) would leave the last wave half empty.
 template <int CT, typename T>
 __global__ void __launch_bounds__(kCellThreads) k_cells_sweep_emit(CellJob j)
 {
@@ -1029,7 +1031,7 @@ kvsmc_status cells_prepare(kvsmc_context* ctx, kvsmc::CellJob& j, CellsScratch* 
     j.bad_index = ctx->d_flag;
     KVSMC_CUDA(ctx, cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream));
     j.block_shift = kvsmc::cells_block_shift(kvsmc::cells_groups(j.ncells), ctx->num_sms);
-    j.emit_shift = kvsmc::cells_block_shift(kvsmc::cells_groups(j.ncells) * (uint64_t)niso, ctx->num_sms);
+    j.emit_shift = kvsmc::cells_block_shift(kvsmc::cells_groups(j.ncells) * (uint64_t)niso / 2, ctx->num_sms);
     sc->blocks = kvsmc::cells_blocks(j.ncells, j.block_shift);
     sc->nscan = sc->blocks * (uint64_t)niso;
     const size_t bw = align_up(kvsmc::cells_groups(j.ncells) * (uint64_t)niso * 4, 256),

@@ -268,7 +268,7 @@ void gather_setup(kvsmc_context* ctx, Plan& pl)
     pl.ntri = pl.nvert = 0;
     Job& j = pl.job;
     const int dt = j.vol.dtype;
-    pl.snode = pl.shared && ctx->path == 0;
+    pl.snode = pl.shared && ctx->path == 0 && (pl.want_list || !wide_count_by_cells(j.vol, j.mode, 1));
     if (pl.snode) {
         // node units replace the node tiles: (plane, row, 256-node segment)
         pl.wprn = (j.vol.nx + 255) / 256;
@@ -931,10 +931,15 @@ bool capacity_ok(const Item& it)
 kvsmc_status run_items(kvsmc_context* ctx, std::vector<Item*>& items, bool emit)
 {
     std::vector<Item*> stream_items, gather_items;
+    auto streams = [&](Item* it) { return !it->status && it->extracted && dup_stream_eligible(ctx, *it); };
+    size_t wide = 0;
+    if (!emit)
+        for (Item* it : items) wide += streams(it) && !stream_eligible(ctx, *it);
     for (Item* it : items) {
         if (it->status) continue;
         if (!it->extracted) continue;
-        (dup_stream_eligible(ctx, *it) ? stream_items : gather_items).push_back(it);
+        const bool s = streams(it) && (emit || !wide_count_by_cells(it->vol->view, it->params.mode, wide));
+        (s ? stream_items : gather_items).push_back(it);
     }
     kvsmc_status first = KVSMC_OK;
     if (!stream_items.empty()) {

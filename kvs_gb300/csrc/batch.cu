@@ -139,6 +139,17 @@ bool any_stream_eligible(const kvsmc_context* ctx, const Item& it)
            (double)(v.nx - 1) * (double)(v.ny - 1) * 5.0 < 4294967295.0 && std::isfinite(it.params.isolevel);
 }
 
+bool wide_count_by_cells(const kvsmc::VolumeView& v, int mode, size_t together)
+{
+    if (stream_dtype(v.dtype)) return false;
+    const size_t es = kvsmc::dtype_size(v.dtype);
+    const bool int64 = es == 8 && v.dtype != KVSMC_F64;
+    const double cells = (double)(v.nx - 1) * (v.ny - 1) * (v.nz - 1);
+    if (v.nx - 1 <= (es == 8 ? 32u : 2u)) return true;
+    if (mode != KVSMC_DUP_POLYGON_NORMAL) return int64 || cells < 3.0e7;
+    return together == 1 && (int64 || cells < 5.0e6);
+}
+
 bool stream_volume_eligible(const kvsmc_context* ctx, const Item& it)
 {
     if (ctx->path != 0 || !it.vol) return false;

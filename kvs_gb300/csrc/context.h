@@ -221,6 +221,18 @@ bool stream_volume_eligible(const kvsmc_context* ctx, const Item& it);
 // and the server take the narrow types only.)
 bool any_stream_eligible(const kvsmc_context* ctx, const Item& it);
 bool dup_stream_eligible(const kvsmc_context* ctx, const Item& it);
+// Whether a count alone (nothing is emitted) of a 32/64-bit integer or double
+// volume goes by cells through the gather kernels; `together`: the call's
+// duplicated-mode requests on such volumes.  The streaming count costs 48 us
+// before it reads anything, 34 by cells, and its vertices a pass of their own;
+// it reads a volume once and counts several requests in one launch.  Measured
+// (us by cells / streaming): 128^3 doubles 48 / 63, 200^3 95 / 82, 512^3 927 /
+// 475; 128^3 32-bit 46 / 54, 200^3 70 / 65; 64-bit integers 46 / 63 and at 512^3
+// 446 / 450; two requests at 128^3 85 / 65; with vertices 128^3 67 / 106 and
+// 55 / 88, 300^3 372 / 378, 420^3 928 / 723 (64-bit integers 773 / 807 at 512^3).
+// Rows of few cells leave most lanes idle: 17 x 400 x 400 doubles 107 / 165,
+// 2 x 1000 x 1000 406 / 717.
+bool wide_count_by_cells(const kvsmc::VolumeView& v, int mode, size_t together);
 // Count (and, for items with emit set, emit) all eligible items together.
 kvsmc_status stream_run(kvsmc_context* ctx, std::vector<Item*>& items);
 

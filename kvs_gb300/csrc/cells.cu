@@ -1031,7 +1031,9 @@ kvsmc_status cells_prepare(kvsmc_context* ctx, kvsmc::CellJob& j, CellsScratch* 
     j.bad_index = ctx->d_flag;
     KVSMC_CUDA(ctx, cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream));
     j.block_shift = kvsmc::cells_block_shift(kvsmc::cells_groups(j.ncells), ctx->num_sms);
-    j.emit_shift = kvsmc::cells_block_shift(kvsmc::cells_groups(j.ncells) * (uint64_t)niso / 2, ctx->num_sms);
+    // (whole blocks of the count: half of one isolevel's groups asks for less)
+    j.emit_shift = std::max(j.block_shift, kvsmc::cells_block_shift(kvsmc::cells_groups(j.ncells) * (uint64_t)niso / 2,
+                                                                    ctx->num_sms));
     sc->blocks = kvsmc::cells_blocks(j.ncells, j.block_shift);
     sc->nscan = sc->blocks * (uint64_t)niso;
     const size_t bw = align_up(kvsmc::cells_groups(j.ncells) * (uint64_t)niso * 4, 256),

@@ -51,3 +51,9 @@ def test_blocks_of_a_sweep(kvsmc_ctx, ct, ncells, niso):
     for i in (0, niso // 2, niso - 1):
         w = ocells.marching_cells(ct, v, xyz, conn, isos[i], (0.0, 1.0))
         assert same_bits(oc[i][:9 * t[i]].cpu().numpy(), w["coords"]) and same_bits(on[i][:3 * t[i]].cpu().numpy(), w["normals"])
+
+
+@pytest.mark.parametrize("ncells", [640033, 1300001])
+def test_a_sweep_of_one_isolevel(kvsmc_ctx, ncells):
+    """Where the count's blocks are of several groups, the emit's are no smaller."""
+    test_blocks_of_a_sweep(kvsmc_ctx, 0, ncells, 1)

@@ -25,8 +25,8 @@ struct kvsmc_volume {
     // parts of the same allocation: the brick min/max table (the streaming
     // kernels' empty-space skip; null for volumes that they do not take), written
     // by the pass that every copy into such a volume ends with, and the values'
-    // range (range_ready), by that pass or by one of its own when it is first
-    // asked for; it is read back then
+    // range, where that pass has run (range_ready); otherwise the range is taken
+    // when it is first asked for, into the asking context's memory
     kvsmc::IngestOut* range = nullptr;
     bool range_ready = false;
     float2* bricks = nullptr;

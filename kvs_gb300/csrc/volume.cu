@@ -532,21 +532,15 @@ kvsmc_status volume_alloc(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, ui
     return KVSMC_OK;
 }
 
-namespace {
-
-// The pass over values that are in place.
-kvsmc_status ingest_in_place(kvsmc_context* ctx, kvsmc_volume* v)
+kvsmc_status volume_bricks(kvsmc_context* ctx, kvsmc_volume* v)
 {
+    if (!v->bricks) return KVSMC_OK;
     KVSMC_CUDA(ctx, kvsmc::launch_ingest(v->view, nullptr, v->bricks, v->range, launch_of(ctx)));
     KVSMC_CUDA(ctx, cudaEventRecord(v->ev, ctx->stream));
-    v->bricks_valid = v->bricks != nullptr;
+    v->bricks_valid = true;
     v->range_ready = true;
     return KVSMC_OK;
 }
-
-}  // namespace
-
-kvsmc_status volume_bricks(kvsmc_context* ctx, kvsmc_volume* v) { return v->bricks ? ingest_in_place(ctx, v) : KVSMC_OK; }
 
 kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src, bool on_device)
 {
@@ -611,10 +605,15 @@ kvsmc_status volume_minmax(kvsmc_context* ctx, kvsmc_volume* v)
 {
     if (v->has_minmax) return KVSMC_OK;
     volume_use(ctx, v);
-    if (!v->range_ready)
-        if (kvsmc_status st = ingest_in_place(ctx, v)) return st;
-    KVSMC_CUDA(ctx, cudaMemcpyAsync(ctx->h_small, v->range, sizeof(kvsmc::IngestOut), cudaMemcpyDeviceToHost,
-                                    ctx->stream));
+    kvsmc::IngestOut* range = v->range;
+    if (!v->range_ready) {
+        // a pass of its own, into the context's memory: another context may ask for
+        // the same volume's range at the same time
+        if (kvsmc_status st = ensure_scratch(ctx, sizeof(kvsmc::IngestOut))) return st;
+        range = static_cast<kvsmc::IngestOut*>(ctx->scratch);
+        KVSMC_CUDA(ctx, kvsmc::launch_ingest(v->view, nullptr, nullptr, range, launch_of(ctx)));
+    }
+    KVSMC_CUDA(ctx, cudaMemcpyAsync(ctx->h_small, range, sizeof(kvsmc::IngestOut), cudaMemcpyDeviceToHost, ctx->stream));
     KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     kvsmc::IngestOut o;
     std::memcpy(&o, ctx->h_small, sizeof o);

@@ -2,7 +2,9 @@
 streams, warps that go on to a second brick; volumes freed while other work is
 under way.
 """
+import ctypes as C
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -248,3 +250,35 @@ def test_zero_signs_of_doubles(kvsmc_ctx):
             lo, hi = dv.minmax()
             assert same_bits(np.array([lo, hi]), np.array([want, 2.0] if sign > 0 else [-2.0, want])), (at, sign, lo, hi)
             dv.free()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.uint64, np.int32])
+def test_the_range_asked_for_by_two_contexts(kvsmc_ctx, dtype):
+    """One context's pass for a volume's range waits on a busy stream: another
+    context that asks for it meanwhile takes its own."""
+    v = _values((40, 50, 64), dtype, 5)   # (no padding: the upload leaves the range to whoever asks)
+    dv = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+    kvsmc_ctx.synchronize()
+    other = _abi.Context(0)
+    stream = torch.cuda.Stream()
+    got = {}
+
+    def ask(ctx, name):
+        lo, hi = C.c_double(), C.c_double()
+        ctx.check(ctx.lib.kvsmc_volume_minmax(ctx.handle, dv.handle, C.byref(lo), C.byref(hi)), "minmax")
+        got[name] = (lo.value, hi.value)
+
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(200_000_000)
+    other.set_stream(stream.cuda_stream)
+    t = threading.Thread(target=ask, args=(other, "other"))
+    t.start()
+    time.sleep(0.02)
+    ask(kvsmc_ctx, "first")
+    t.join()
+    torch.cuda.synchronize()
+    other.set_stream(None)
+    other.close()
+    want = (float(v.min()), float(v.max()))
+    assert got == {"first": want, "other": want}
+    dv.free()

@@ -17,8 +17,9 @@ struct kvsmc_volume {
     cudaEvent_t ev = nullptr;   // comes with dev: behind the last copy or pass that a call left running on it
     int device = 0;             // the device it lies on
     kvsmc_context* owner = nullptr;   // the context that allocated it
-    // read by work that no call of the owner's waits for (a plan's replays, a
-    // server's workers, another context): its block is not kept when it is freed
+    // read or written by work that no call of the owner's waits for (a plan's
+    // replays, a captured update's, a server's workers, another context): its block
+    // is not kept when it is freed
     std::atomic<bool> lent{false};
     bool has_minmax = false;
     double vmin = 0.0, vmax = 0.0;

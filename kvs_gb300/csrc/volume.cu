@@ -550,7 +550,14 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
     const size_t dense = row * rows;
     v->has_minmax = false;
     v->range_ready = false;
-    KVSMC_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, v->ev, 0));   // (an update on another stream comes first)
+    // An update may be captured into a caller's graph: its replays come when the
+    // caller likes, so it takes no part in the events, reads no buffer of the
+    // context's, and the block is not kept when the volume is freed.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess) cudaGetLastError();
+    const bool captured = cap != cudaStreamCaptureStatusNone;
+    if (captured) v->lent = true;
+    else KVSMC_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, v->ev, 0));   // (an update on another stream comes first)
     const void* from = nullptr;   // values the ingest pass copies (null: they are in place)
     if (on_device) {
         // read in place of a copy where the kernel can: device memory of this
@@ -561,7 +568,7 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
             from = src;
         else
             cudaGetLastError();
-    } else if (v->view.pitch != v->view.nx && dense <= kDenseStage) {
+    } else if (v->view.pitch != v->view.nx && dense <= kDenseStage && !captured) {
         // rows that are padded on the device: one dense copy into a staging
         // buffer, padded by the ingest pass (a row-by-row copy of 99-node rows
         // of 16-bit values ran at 6 GB/s: 2.1 MB in 340 us).  The last pass that
@@ -596,6 +603,7 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
         v->bricks_valid = v->bricks != nullptr;
         v->range_ready = true;
     }
+    if (captured) return KVSMC_OK;
     KVSMC_CUDA(ctx, cudaEventRecord(v->ev, ctx->stream));
     if (from && from == ctx->dense) KVSMC_CUDA(ctx, cudaEventRecord(ctx->dense_ev, ctx->stream));
     return KVSMC_OK;

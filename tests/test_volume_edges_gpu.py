@@ -282,3 +282,45 @@ def test_the_range_asked_for_by_two_contexts(kvsmc_ctx, dtype):
     want = (float(v.min()), float(v.max()))
     assert got == {"first": want, "other": want}
     dv.free()
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.float32, np.float64])
+@pytest.mark.parametrize("nx", [64, 61])
+def test_a_captured_update(kvsmc_ctx, dtype, nx):
+    """An update from pinned memory captured into a graph: each replay brings the
+    buffer's present values, whatever the context uploaded in between."""
+    shape = (20, 30, nx)
+    n = int(np.prod(shape)) * np.dtype(dtype).itemsize
+    pinned = torch.empty(n, dtype=torch.uint8).pin_memory()
+    h = pinned.numpy().view(dtype).reshape(shape)
+    h[...] = _values(shape, dtype, 1)
+    dv = _abi.DeviceVolume.upload(kvsmc_ctx, h)
+    kvsmc_ctx.synchronize()
+    torch.cuda.synchronize()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    try:
+        with torch.cuda.graph(graph, stream=stream):
+            kvsmc_ctx.set_stream(stream.cuda_stream)
+            st = kvsmc_ctx.lib.kvsmc_volume_update(kvsmc_ctx.handle, dv.handle, h.ctypes.data)
+    finally:
+        kvsmc_ctx.set_stream(None)
+    assert st == _abi.OK
+    for turn in (2, 3):
+        h[...] = v = _values(shape, dtype, turn)
+        later = _abi.DeviceVolume.upload(kvsmc_ctx, _values((30, 40, nx), dtype, 7))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(dv.download(), v)
+        params = _abi.make_params(float(np.median(v)), 0, (float(v.min()), float(v.max())))
+        s, w = _abi.Sizes(), _abi.Sizes()
+        kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_count(kvsmc_ctx.handle, dv.handle, params, s), "count")
+        fresh = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+        kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_count(kvsmc_ctx.handle, fresh.handle, params, w), "count")
+        assert s.ntriangles == w.ntriangles > 0
+        later.free()
+        fresh.free()
+    # an update outside the graph still works, and so does freeing
+    v = _values(shape, dtype, 9)
+    kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_volume_update(kvsmc_ctx.handle, dv.handle, v.ctypes.data), "update")
+    _check(dv, v)
+    dv.free()

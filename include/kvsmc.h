@@ -673,6 +673,14 @@ kvsmc_status kvsmc_checksum_words(kvsmc_context* ctx, const void* d_words, uint6
  * (MarchingCubes.cpp:50-67). */
 kvsmc_status kvsmc_set_wait_limit(kvsmc_context* ctx, int64_t count_polls, int64_t emit_polls);
 
+/* Test hook: cap the entries of the lists of crossed cells that an extraction's
+ * count leaves for its emit (negative = the built-in room, for every cell of
+ * any but very large volumes).  A list that does not suffice, or one of no
+ * entries, makes the emit classify the volume again, as it does where memory
+ * is short; results are the same.  Plans keep the limit they were made under.
+ * No counterpart in the reference. */
+kvsmc_status kvsmc_set_list_limit(kvsmc_context* ctx, int64_t entries);
+
 #ifdef __cplusplus
 }
 #endif

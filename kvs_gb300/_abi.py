@@ -51,7 +51,7 @@ EXPORTS = [
     "kvsmc_slice_count", "kvsmc_slice_extract_device", "kvsmc_slice_plane",
     "kvsmc_marching_cells_host", "kvsmc_marching_cells_device", "kvsmc_selftest_cells", "kvsmc_slice_cells_host",
     "kvsmc_cells_bounds", "kvsmc_marching_cells_sweep_device", "kvsmc_ply_record_bytes", "kvsmc_ply_header", "kvsmc_ply_records", "kvsmc_write_ply", "kvsmc_write_ply_host",
-    "kvsmc_checksum_words", "kvsmc_set_wait_limit", "kvsmc_write_stl_ascii", "kvsmc_write_stl_ascii_host",
+    "kvsmc_checksum_words", "kvsmc_set_wait_limit", "kvsmc_set_list_limit", "kvsmc_write_stl_ascii", "kvsmc_write_stl_ascii_host",
     "kvsmc_write_kvsml_polygon",
 ]
 
@@ -235,6 +235,7 @@ def load(path=LIB_PATH):
         "kvsmc_profile_read": (i32, [vp, i32, C.POINTER(C.c_char_p), C.POINTER(u64), C.POINTER(C.c_double)]),
         "kvsmc_checksum_words": (C.c_int, [vp, vp, u64, u64, C.POINTER(u64), u64]),
         "kvsmc_set_wait_limit": (C.c_int, [vp, C.c_int64, C.c_int64]),
+        "kvsmc_set_list_limit": (C.c_int, [vp, C.c_int64]),
     }
     for name, (res, args) in sig.items():
         f = getattr(lib, name)
@@ -306,6 +307,9 @@ class Context:
     def set_wait_limit(self, count_polls=-1, emit_polls=-1):
         self.check(self.lib.kvsmc_set_wait_limit(self.handle, int(count_polls), int(emit_polls)),
                    "kvsmc_set_wait_limit")
+
+    def set_list_limit(self, entries=-1):
+        self.check(self.lib.kvsmc_set_list_limit(self.handle, int(entries)), "kvsmc_set_list_limit")
 
     def selftest_interpolation(self, n, seed=1):
         t, m, f = C.c_uint64(), C.c_uint64(), C.c_uint64()

@@ -346,6 +346,7 @@ void StreamBatch::plan_tables()
         const uint64_t sure = 2 * pairs_most + tail;
         list_cap = std::min<uint64_t>(sure, std::max<uint64_t>((uint64_t)1 << 29, pairs_most / 8) + tail);
         list_cap = std::min<uint64_t>(list_cap, (uint64_t)1 << 31);
+        list_cap = std::min(list_cap, ctx->list_limit);
         list_sure = list_cap >= sure;
     }
 }

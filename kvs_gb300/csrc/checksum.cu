@@ -99,4 +99,11 @@ kvsmc_status kvsmc_set_wait_limit(kvsmc_context* ctx, int64_t count_polls, int64
     return KVSMC_OK;
 }
 
+kvsmc_status kvsmc_set_list_limit(kvsmc_context* ctx, int64_t entries)
+{
+    if (!ctx) return KVSMC_ERR_INVALID_ARGUMENT;
+    ctx->list_limit = entries < 0 ? ~0ull : (uint64_t)entries;
+    return KVSMC_OK;
+}
+
 }  // extern "C"

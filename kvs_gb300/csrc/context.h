@@ -59,6 +59,7 @@ struct kvsmc_context {
     int path = 0;                // 0: streaming kernels where eligible, 1: gather kernels only
     // plane-wait poll limits of the streaming count / emit kernels (kvsmc_set_wait_limit)
     uint32_t wait_polls[2] = {kvsmc::kStreamWaitPolls, kvsmc::kStreamWaitPolls};
+    uint64_t list_limit = ~0ull;   // entries that a pair list may have (kvsmc_set_list_limit)
     kvsmc::Profiler* prof = nullptr;
     // freed volumes' device blocks, kept for the next volumes (cudaMalloc and
     // cudaFree of a new field's 83 MB a frame cost 350 us): at most

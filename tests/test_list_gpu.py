@@ -63,3 +63,53 @@ def test_crowded_steps(kvsmc_ctx, dtype, noisy):
             assert same_bits(g["coords"], w["coords"]) and same_bits(g["normals"], w["normals"])
             assert np.array_equal(g["connections"], w["connections"])
     vol.free()
+
+
+@pytest.mark.parametrize("entries", [0, 40])
+@pytest.mark.parametrize("dtype", _abi.DTYPES)
+def test_no_room_for_the_list(kvsmc_ctx, dtype, entries):
+    """Without a list, or with one that overflows, the emit classifies the volume
+    again: every mode, one request and several, device and host calls, a plan."""
+    rng = np.random.default_rng(3)
+    v = (rng.random((7, 20, 270)) * 100).astype(dtype)
+    vol = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+    isos = (30.5, 50.25, 70.75)
+
+    def calls():
+        out = []
+        for n in (1, 3):
+            for mode in (0, 1, 2):
+                res = extract_batch(kvsmc_ctx, [vol] * n, [_abi.make_params(x, mode) for x in isos[:n]], _abi.PATH_AUTO)
+                assert all(r["status"] == _abi.OK and r["ntri"] > 0 for r in res)
+                out += [a for r in res for a in (r["coords"], r["normals"], r["connections"])]
+        for mode in (0, 1, 2):
+            out += list(_abi.marching_cubes_host(kvsmc_ctx, v, _abi.make_params(isos[0], mode))[:3])
+        for n in (1, 3):
+            res = _abi.extract_batch_host(kvsmc_ctx, v, [_abi.make_params(x, k % 3) for k, x in enumerate(isos[:n])])
+            out += [r[a] for r in res for a in ("coords", "normals", "connections")]
+        if v.itemsize <= 2 or dtype == np.float32:
+            reqs, outs = (_abi.Request * 3)(), []
+            for r, x in zip(reqs, isos):
+                c, m = torch.zeros(v.size * 45, device="cuda"), torch.zeros(v.size * 15, device="cuda")
+                outs += [c, m]
+                r.volume, r.params = vol.handle, _abi.make_params(x, 0)
+                r.d_coords, r.coords_capacity, r.d_normals, r.normals_capacity = c.data_ptr(), c.numel(), m.data_ptr(), m.numel()
+            torch.cuda.synchronize()
+            plan = _abi.Plan(kvsmc_ctx, reqs)
+            for _ in range(2):
+                plan.launch()
+                plan.wait()
+            out += [t.cpu().numpy() for t in outs]
+            plan.close()
+        return out
+
+    want = calls()
+    kvsmc_ctx.set_list_limit(entries)
+    try:
+        got = calls()
+    finally:
+        kvsmc_ctx.set_list_limit()
+    assert len(want) == len(got)
+    for a, b in zip(want, got):
+        assert np.array_equal(np.asarray(a).view(np.uint8), np.asarray(b).view(np.uint8))
+    vol.free()

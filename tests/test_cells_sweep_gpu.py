@@ -54,6 +54,29 @@ def test_blocks_of_a_sweep(kvsmc_ctx, ct, ncells, niso):
 
 
 @pytest.mark.parametrize("ncells", [640033, 1300001])
-def test_a_sweep_of_one_isolevel(kvsmc_ctx, ncells):
-    """Where the count's blocks are of several groups, the emit's are no smaller."""
-    test_blocks_of_a_sweep(kvsmc_ctx, 0, ncells, 1)
+@pytest.mark.parametrize("niso", [1, 2])
+def test_few_isolevels_of_noise(kvsmc_ctx, ncells, niso):
+    """Nearly every cell cut: where the count's blocks are of several groups, the
+    emit's are no smaller."""
+    rng = np.random.default_rng(ncells)
+    nodes = ncells // 4
+    xyz = rng.uniform(-4, 4, (nodes, 3)).astype(np.float32)
+    conn = rng.integers(0, nodes, (ncells, 4)).astype(np.uint32)
+    dv, dx, dk = (torch.from_numpy(a).cuda() for a in (rng.random(nodes).astype(np.float32), xyz, conn.view(np.int32)))
+    mesh = (kvsmc_ctx.handle, 0, dv.data_ptr(), 8, nodes, dx.data_ptr(), dk.data_ptr(), ncells)
+    want, isos = [], [0.4, 0.7][:niso]
+    for iso in isos:
+        c, n, s = torch.zeros(18 * ncells, device="cuda"), torch.zeros(6 * ncells, device="cuda"), _abi.Sizes()
+        torch.cuda.synchronize()
+        kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_marching_cells_device(*mesh, iso, 1, 0.0, 1.0, c.data_ptr(), c.numel(),
+                                                                  n.data_ptr(), n.numel(), C.byref(s)), "cells")
+        want.append((c, n, s.ntriangles))
+    got = [(torch.zeros_like(c), torch.zeros_like(n)) for c, n, _ in want]
+    torch.cuda.synchronize()
+    sizes = (_abi.Sizes * niso)()
+    kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_marching_cells_sweep_device(
+        *mesh, (C.c_double * niso)(*isos), niso, 1, 0.0, 1.0, (C.c_void_p * niso)(*[c.data_ptr() for c, _ in got]),
+        (C.c_uint64 * niso)(*[c.numel() for c, _ in got]), (C.c_void_p * niso)(*[n.data_ptr() for _, n in got]),
+        (C.c_uint64 * niso)(*[n.numel() for _, n in got]), sizes), "sweep")
+    for (c, n, t), (gc, gn), s in zip(want, got, sizes):
+        assert s.ntriangles == t > ncells // 2 and torch.equal(c, gc) and torch.equal(n, gn)

@@ -15,6 +15,7 @@ struct kvsmc_volume {
     void* dev = nullptr;        // owned device allocation
     size_t bytes = 0;
     cudaEvent_t ev = nullptr;   // comes with dev: behind the last copy or pass that a call left running on it
+    bool ev_own = true;         // ev stands on the owner's own stream, or on none
     int device = 0;             // the device it lies on
     kvsmc_context* owner = nullptr;   // the context that allocated it
     // read or written by work that no call of the owner's waits for (a plan's
@@ -70,7 +71,9 @@ struct kvsmc_context {
     std::mutex spare_mutex;
     void* dense = nullptr;       // staging of host volumes whose rows are padded (at most kDenseStage)
     size_t dense_bytes = 0;
-    cudaEvent_t dense_ev = nullptr;   // behind the last pass that reads it, on whatever stream that was
+    // the last pass that reads it: on own_stream, or behind dense_ev
+    bool dense_own = true;
+    cudaEvent_t dense_ev = nullptr;
     std::vector<kvsmc::KernelFit> fits;   // launch shapes of the kernels launched so far
     std::string last_error;
     // auxiliary streams for launches that may run side by side (created on first use)

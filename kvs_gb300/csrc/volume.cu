@@ -502,6 +502,7 @@ void block_free(kvsmc_context* ctx, kvsmc_volume* v)
     v->dev = nullptr;
     v->bytes = 0;
     v->ev = nullptr;
+    v->ev_own = true;
 }
 
 kvsmc_status volume_alloc(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, uint32_t ny, uint32_t nz,
@@ -536,6 +537,7 @@ kvsmc_status volume_bricks(kvsmc_context* ctx, kvsmc_volume* v)
 {
     if (!v->bricks) return KVSMC_OK;
     KVSMC_CUDA(ctx, kvsmc::launch_ingest(v->view, nullptr, v->bricks, v->range, launch_of(ctx)));
+    v->ev_own = v->owner == ctx && ctx->stream == ctx->own_stream;
     KVSMC_CUDA(ctx, cudaEventRecord(v->ev, ctx->stream));
     v->bricks_valid = true;
     v->range_ready = true;
@@ -556,8 +558,11 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess) cudaGetLastError();
     const bool captured = cap != cudaStreamCaptureStatusNone;
+    // what the context's own stream ran comes first there without an event
+    const bool own = ctx->stream == ctx->own_stream;
     if (captured) v->lent = true;
-    else KVSMC_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, v->ev, 0));   // (an update on another stream comes first)
+    else if (!(own && v->ev_own && v->owner == ctx))   // (an update on another stream comes first)
+        KVSMC_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, v->ev, 0));
     const void* from = nullptr;   // values the ingest pass copies (null: they are in place)
     if (on_device) {
         // read in place of a copy where the kernel can: device memory of this
@@ -575,8 +580,10 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
         // reads the buffer may be on another stream (kvsmc_set_stream): the copy
         // waits for it
         if (!ctx->dense_ev) KVSMC_CUDA(ctx, cudaEventCreateWithFlags(&ctx->dense_ev, cudaEventDisableTiming));
+        if (!own && ctx->dense_own) KVSMC_CUDA(ctx, cudaEventRecord(ctx->dense_ev, ctx->own_stream));
         if (dense > ctx->dense_bytes) {
-            KVSMC_CUDA(ctx, cudaEventSynchronize(ctx->dense_ev));
+            if (own && ctx->dense_own) KVSMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+            else KVSMC_CUDA(ctx, cudaEventSynchronize(ctx->dense_ev));
             if (ctx->dense) cudaFree(ctx->dense);
             ctx->dense = nullptr;
             ctx->dense_bytes = 0;
@@ -584,7 +591,7 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
             KVSMC_CUDA(ctx, device_malloc(ctx, &ctx->dense, want));
             ctx->dense_bytes = want;
         }
-        KVSMC_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->dense_ev, 0));
+        if (!(own && ctx->dense_own)) KVSMC_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->dense_ev, 0));
         KVSMC_CUDA(ctx, cudaMemcpyAsync(ctx->dense, src, dense, cudaMemcpyHostToDevice, ctx->stream));
         from = ctx->dense;
     }
@@ -604,8 +611,12 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
         v->range_ready = true;
     }
     if (captured) return KVSMC_OK;
+    v->ev_own = own && v->owner == ctx;
     KVSMC_CUDA(ctx, cudaEventRecord(v->ev, ctx->stream));
-    if (from && from == ctx->dense) KVSMC_CUDA(ctx, cudaEventRecord(ctx->dense_ev, ctx->stream));
+    if (from && from == ctx->dense) {
+        ctx->dense_own = own;
+        if (!own) KVSMC_CUDA(ctx, cudaEventRecord(ctx->dense_ev, ctx->stream));
+    }
     return KVSMC_OK;
 }
 

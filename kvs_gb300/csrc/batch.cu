@@ -145,7 +145,10 @@ bool wide_count_by_cells(const kvsmc::VolumeView& v, int mode, size_t together)
     const size_t es = kvsmc::dtype_size(v.dtype);
     const bool int64 = es == 8 && v.dtype != KVSMC_F64;
     const double cells = (double)(v.nx - 1) * (v.ny - 1) * (v.nz - 1);
-    if (v.nx - 1 <= (es == 8 ? 32u : 2u)) return true;
+    const bool short_rows = v.nx - 1 <= (es == 8 ? 32u : 2u);
+    if (short_rows && mode == KVSMC_DUP_POLYGON_NORMAL && together > 1)
+        return (double)(v.ny - 1) * (v.nz - 1) * (11.0 + v.nx) >= (es == 8 ? 3.6e6 : 8.4e6);
+    if (short_rows) return true;
     if (mode != KVSMC_DUP_POLYGON_NORMAL) return int64 || cells < 3.0e7;
     return together == 1 && (int64 || cells < 5.0e6);
 }

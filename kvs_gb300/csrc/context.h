@@ -236,7 +236,11 @@ bool dup_stream_eligible(const kvsmc_context* ctx, const Item& it);
 // 446 / 450; two requests at 128^3 85 / 65; with vertices 128^3 67 / 106 and
 // 55 / 88, 300^3 372 / 378, 420^3 928 / 723 (64-bit integers 773 / 807 at 512^3).
 // Rows of few cells leave most lanes idle: 17 x 400 x 400 doubles 107 / 165,
-// 2 x 1000 x 1000 406 / 717.
+// 2 x 1000 x 1000 406 / 717.  Several requests on them are one launch all the
+// same, and one of them takes 0.7 us a thousand rows there, by cells 30 us and
+// more the shorter the rows: of 16 requests one takes (doubles) 33 x 100 x 100
+// 51 / 11, 33 x 300 x 300 64 / 64, 33 x 500 x 500 112 / 167, 2 x 300 x 300 123 /
+// 63, 2 x 500 x 500 186 / 165; 32-bit 2 x 500 x 500 165 / 83, 3 x 700 x 900 236 / 227.
 bool wide_count_by_cells(const kvsmc::VolumeView& v, int mode, size_t together);
 // Count (and, for items with emit set, emit) all eligible items together.
 kvsmc_status stream_run(kvsmc_context* ctx, std::vector<Item*>& items);

@@ -57,3 +57,17 @@ def test_sizes_around_the_rule(kvsmc_ctx, dtype, shape):
             params = [_abi.make_params(x, mode) for x in isos]
             assert _counts(kvsmc_ctx, vol, params, _abi.PATH_AUTO) == _counts(kvsmc_ctx, vol, params, _abi.PATH_GATHER)
     vol.free()
+
+
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64, torch.float64])
+@pytest.mark.parametrize("shape", [(260, 316, 33), (290, 300, 33), (500, 555, 2), (520, 560, 2), (700, 870, 3), (740, 850, 3)])
+def test_short_rows_together(kvsmc_ctx, dtype, shape):
+    """Several requests on rows of few cells, either side of the rule."""
+    gen = torch.Generator(device="cuda").manual_seed(shape[0])
+    t = torch.randint(0, 1000, shape, generator=gen, device="cuda").to(dtype)
+    torch.cuda.synchronize()
+    code = {torch.int32: np.int32, torch.int64: np.int64, torch.float64: np.float64}[dtype]
+    vol = _abi.DeviceVolume.from_device(kvsmc_ctx, t.data_ptr(), code, shape)
+    params = [_abi.make_params(x, 0) for x in (100.5, 500.5, 900.25)]
+    assert _counts(kvsmc_ctx, vol, params, _abi.PATH_AUTO) == _counts(kvsmc_ctx, vol, params, _abi.PATH_GATHER)
+    vol.free()

@@ -268,7 +268,7 @@ void gather_setup(kvsmc_context* ctx, Plan& pl)
     pl.ntri = pl.nvert = 0;
     Job& j = pl.job;
     const int dt = j.vol.dtype;
-    pl.snode = pl.shared && ctx->path == 0 && (pl.want_list || !wide_count_by_cells(j.vol, j.mode, 1));
+    pl.snode = pl.shared && ctx->path == 0 && (pl.want_list || pl.sb || !count_by_cells(j.vol, j.mode, 1));
     if (pl.snode) {
         // node units replace the node tiles: (plane, row, 256-node segment)
         pl.wprn = (j.vol.nx + 255) / 256;

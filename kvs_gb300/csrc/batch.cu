@@ -139,12 +139,13 @@ bool any_stream_eligible(const kvsmc_context* ctx, const Item& it)
            (double)(v.nx - 1) * (double)(v.ny - 1) * 5.0 < 4294967295.0 && std::isfinite(it.params.isolevel);
 }
 
-bool wide_count_by_cells(const kvsmc::VolumeView& v, int mode, size_t together)
+bool count_by_cells(const kvsmc::VolumeView& v, int mode, size_t together)
 {
-    if (stream_dtype(v.dtype)) return false;
+    const double cells = (double)(v.nx - 1) * (v.ny - 1) * (v.nz - 1);
+    if (stream_dtype(v.dtype))
+        return mode != KVSMC_DUP_POLYGON_NORMAL && v.nx - 1 >= 8 && cells >= 2.0e6 && cells < 1.0e7;
     const size_t es = kvsmc::dtype_size(v.dtype);
     const bool int64 = es == 8 && v.dtype != KVSMC_F64;
-    const double cells = (double)(v.nx - 1) * (v.ny - 1) * (v.nz - 1);
     const bool short_rows = v.nx - 1 <= (es == 8 ? 32u : 2u);
     if (short_rows && mode == KVSMC_DUP_POLYGON_NORMAL && together > 1)
         return (double)(v.ny - 1) * (v.nz - 1) * (11.0 + v.nx) >= (es == 8 ? 3.6e6 : 8.4e6);

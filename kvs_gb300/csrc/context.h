@@ -226,9 +226,14 @@ bool stream_volume_eligible(const kvsmc_context* ctx, const Item& it);
 // and the server take the narrow types only.)
 bool any_stream_eligible(const kvsmc_context* ctx, const Item& it);
 bool dup_stream_eligible(const kvsmc_context* ctx, const Item& it);
-// Whether a count alone (nothing is emitted) of a 32/64-bit integer or double
-// volume goes by cells through the gather kernels; `together`: the call's
-// duplicated-mode requests on such volumes.  The streaming count costs 48 us
+// Whether a count alone (nothing is emitted) goes by cells through the gather
+// kernels.  8/16-bit and float32 volumes: a shared-vertex request that is counted
+// by itself, where the streaming count, whose time is its crossed pairs' with
+// vertices, is slower on smooth and crowded volumes alike (us by cells / smooth /
+// every cell crossed, float32: 17 x 500 x 500 165 / 196 / 329, 129^3 54 / 71 / 84,
+// 200^3 81 / 91 / 139; smaller ones 17 x 100 x 100 96 / 60 / 72, larger ones 201 x
+// 300 x 300 142 / 116 / 228).  32/64-bit integers and doubles, with `together` the
+// call's duplicated-mode requests on such volumes: the streaming count costs 48 us
 // before it reads anything, 34 by cells, and its vertices a pass of their own;
 // it reads a volume once and counts several requests in one launch.  Measured
 // (us by cells / streaming): 128^3 doubles 48 / 63, 200^3 95 / 82, 512^3 927 /
@@ -241,7 +246,7 @@ bool dup_stream_eligible(const kvsmc_context* ctx, const Item& it);
 // more the shorter the rows: of 16 requests one takes (doubles) 33 x 100 x 100
 // 51 / 11, 33 x 300 x 300 64 / 64, 33 x 500 x 500 112 / 167, 2 x 300 x 300 123 /
 // 63, 2 x 500 x 500 186 / 165; 32-bit 2 x 500 x 500 165 / 83, 3 x 700 x 900 236 / 227.
-bool wide_count_by_cells(const kvsmc::VolumeView& v, int mode, size_t together);
+bool count_by_cells(const kvsmc::VolumeView& v, int mode, size_t together);
 // Count (and, for items with emit set, emit) all eligible items together.
 kvsmc_status stream_run(kvsmc_context* ctx, std::vector<Item*>& items);
 

@@ -71,3 +71,20 @@ def test_short_rows_together(kvsmc_ctx, dtype, shape):
     params = [_abi.make_params(x, 0) for x in (100.5, 500.5, 900.25)]
     assert _counts(kvsmc_ctx, vol, params, _abi.PATH_AUTO) == _counts(kvsmc_ctx, vol, params, _abi.PATH_GATHER)
     vol.free()
+
+
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.int16, torch.float32])
+@pytest.mark.parametrize("shape", [(500, 520, 9), (480, 520, 9), (520, 540, 8), (126, 126, 129), (215, 217, 217), (217, 217, 216)])
+def test_shared_counts_of_narrow_types(kvsmc_ctx, dtype, shape):
+    """One shared-vertex request, and two of one call, either side of 2 and 10
+    million cells and of 8 cells a row."""
+    gen = torch.Generator(device="cuda").manual_seed(shape[0])
+    t = torch.randint(0, 100, shape, generator=gen, device="cuda").to(dtype)
+    torch.cuda.synchronize()
+    code = {torch.uint8: np.uint8, torch.int16: np.int16, torch.float32: np.float32}[dtype]
+    vol = _abi.DeviceVolume.from_device(kvsmc_ctx, t.data_ptr(), code, shape)
+    for mode in (1, 2):
+        for isos in ([50.5], [30.0, 70.25]):
+            params = [_abi.make_params(x, mode) for x in isos]
+            assert _counts(kvsmc_ctx, vol, params, _abi.PATH_AUTO) == _counts(kvsmc_ctx, vol, params, _abi.PATH_GATHER)
+    vol.free()

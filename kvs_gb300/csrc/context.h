@@ -190,6 +190,7 @@ kvsmc_status volume_alloc(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, ui
                           kvsmc_volume* v);
 // Dense values into the volume's layout, with its brick table and range.
 constexpr size_t kDenseStage = (size_t)64 << 20;
+constexpr size_t kStageRow = 8192;   // bytes of a row up to which volumes without a table are staged
 kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src, bool on_device);
 void volume_destroy(kvsmc_context* ctx, kvsmc_volume* v);
 

@@ -573,10 +573,13 @@ kvsmc_status volume_copy_in(kvsmc_context* ctx, kvsmc_volume* v, const void* src
             from = src;
         else
             cudaGetLastError();
-    } else if (v->view.pitch != v->view.nx && dense <= kDenseStage && !captured) {
+    } else if (v->view.pitch != v->view.nx && dense <= kDenseStage && !captured &&
+               (v->bricks || row <= kStageRow)) {
         // rows that are padded on the device: one dense copy into a staging
         // buffer, padded by the ingest pass (a row-by-row copy of 99-node rows
-        // of 16-bit values ran at 6 GB/s: 2.1 MB in 340 us).  The last pass that
+        // of 16-bit values ran at 6 GB/s: 2.1 MB in 340 us; where no table asks for a
+        // pass anyway, long rows are faster by themselves: 512 rows of 4097 doubles
+        // 131 us staged, 105, of 1001 49, 50).  The last pass that
         // reads the buffer may be on another stream (kvsmc_set_stream): the copy
         // waits for it
         if (!ctx->dense_ev) KVSMC_CUDA(ctx, cudaEventCreateWithFlags(&ctx->dense_ev, cudaEventDisableTiming));

@@ -324,3 +324,22 @@ def test_a_captured_update(kvsmc_ctx, dtype, nx):
     kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_volume_update(kvsmc_ctx.handle, dv.handle, v.ctypes.data), "update")
     _check(dv, v)
     dv.free()
+
+
+@pytest.mark.parametrize("dtype,nx", [(np.float64, 1023), (np.float64, 1025), (np.uint64, 4097), (np.int32, 2047),
+                                      (np.int32, 2049), (np.uint8, 8191), (np.uint8, 8193), (np.float32, 4099)])
+def test_long_padded_rows(kvsmc_ctx, dtype, nx):
+    """Volumes without a table, either side of the row length that is staged: the
+    values, the range, and a count."""
+    v, w = _values((3, 5, nx), dtype, nx), _values((3, 5, nx), dtype, nx + 1)
+    dv = _abi.DeviceVolume.upload(kvsmc_ctx, v)
+    _check(dv, v)
+    kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_volume_update(kvsmc_ctx.handle, dv.handle, w.ctypes.data), "update")
+    _check(dv, w)
+    sizes = [_abi.Sizes(), _abi.Sizes()]
+    for path, s in zip((_abi.PATH_AUTO, _abi.PATH_GATHER), sizes):
+        kvsmc_ctx.set_kernel_path(path)
+        kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_count(kvsmc_ctx.handle, dv.handle, _abi.make_params(float(np.median(w)), 0), s), "count")
+    kvsmc_ctx.set_kernel_path(_abi.PATH_AUTO)
+    assert sizes[0].ntriangles == sizes[1].ntriangles > 0
+    dv.free()

@@ -101,7 +101,14 @@ typedef struct kvsmc_sizes {
 /* ------------------------------------------------------------------ context */
 
 /* One context per (host thread, device).  Owns a CUDA stream, the scratch
- * arena and the device-resident volumes.  device < 0 picks the current one. */
+ * arenas and the device-resident volumes.  device < 0 picks the current one.
+ * A context keeps device memory until it is destroyed: its arenas, which grow
+ * to the largest request so far (a list of crossed cells for duplicated and
+ * one for shared-vertex requests, each of 4 bytes a cell and isolevel up to
+ * 1 GiB and of at most 4 GiB beyond; counters; the host calls' outputs), the
+ * blocks of up to 4 freed volumes (1 GiB in all, given
+ * back when an allocation of the library fails) and 64 MiB of staging for host
+ * volumes.  An application's own allocations do not make it give these back. */
 kvsmc_status kvsmc_create(int device, kvsmc_context** ctx);
 void kvsmc_destroy(kvsmc_context* ctx);
 const char* kvsmc_status_string(kvsmc_status st);
@@ -268,11 +275,11 @@ typedef struct kvsmc_completion {
 } kvsmc_completion;
 
 /* The server runs on ctx's device; volumes must stay alive and unchanged
- * while requests on them are pending.  The first request on a volume waits
- * for ctx's stream (so an upload on ctx is complete); a volume uploaded on
- * another context must be complete before it is submitted. */
+ * while requests on them are pending.  A request waits for its volume's last
+ * upload or update, on whatever context and stream it was (an update that the
+ * caller captured into a graph must be complete before). */
 kvsmc_status kvsmc_server_create(kvsmc_context* ctx, const kvsmc_server_config* cfg, kvsmc_server** out);
-/* Queue one request; never blocks on the GPU beyond the first-use wait above
+/* Queue one request; never blocks on the GPU beyond the wait above
  * (the volume's min/max is filled first if not cached).  *ticket identifies
  * its completion. */
 kvsmc_status kvsmc_server_submit(kvsmc_server* s, kvsmc_volume* vol, const kvsmc_params* p, uint64_t* ticket);

@@ -1,7 +1,11 @@
 // api.cu -- the C ABI of libkvsmc (include/kvsmc.h): contexts, resident
-// volumes, and request pipelines.  Duplicated-mode requests on 8/16-bit and
-// float32 volumes run through the streaming kernels (batch.cu); the others
-// through the gather kernels (mc_gather.cu), one request at a time.
+// volumes, and request pipelines.  Duplicated-mode requests of every value type
+// run through the streaming kernels together (batch.cu), shared-vertex ones
+// through the streaming count and the node and connection passes, those of
+// 8/16-bit and float32 volumes in groups.  The gather kernels (mc_gather.cu),
+// one request at a time, take what is left: rows wider than the streaming
+// kernels', volumes one node thick, isolevels that are not finite, the counts
+// that are faster there (count_by_cells).
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
@@ -938,7 +942,7 @@ kvsmc_status run_items(kvsmc_context* ctx, std::vector<Item*>& items, bool emit)
     for (Item* it : items) {
         if (it->status) continue;
         if (!it->extracted) continue;
-        const bool s = streams(it) && (emit || !wide_count_by_cells(it->vol->view, it->params.mode, wide));
+        const bool s = streams(it) && (emit || !count_by_cells(it->vol->view, it->params.mode, wide));
         (s ? stream_items : gather_items).push_back(it);
     }
     kvsmc_status first = KVSMC_OK;

@@ -21,7 +21,7 @@
 //     worked on.
 // Bound by instruction issue (70% busy) and shared-memory latency, and above all
 // it must not spill: 32 warps an SM at 64 registers took 1500 and 2312 us below,
-// 24 at 80 take 1220 and 1884, with the lower plane's masks read back from
+// 24 at 80 take 1210 and 1887, with the lower plane's masks read back from
 // shared memory and the task's addresses kept there.  640x704x600 f32, 16
 // isolevels: 1532 us with the lanes' loops, 1210 us; 1024x768x640 u16, 4
 // isolevels: 2735 -> 1887 us.

@@ -113,6 +113,25 @@ def test_server_budget_holds_back_and_refuses(kvsmc_ctx):
     small.close()
 
 
+def test_server_results_of_later_rounds(kvsmc_ctx):
+    """A budget of about two results: a batch's requests are written in many
+    rounds from one count, each with the triangles that the request has alone."""
+    v = _volumes(kvsmc_ctx)[2]
+    lo, hi = v.minmax()
+    params = [_abi.make_params(lo + f * (hi - lo), 0) for f in np.linspace(0.25, 0.75, 12)]
+    want = [_alone(kvsmc_ctx, v, p) for p in params]
+    srv = _abi.Server(kvsmc_ctx, budget_bytes=2 * 48 * max(w[0] for w in want), max_batch=16, workers=1)
+    tickets = [srv.submit(v, p) for p in params * 3]
+    got = _collect(srv, len(tickets))
+    stats = srv.stats()
+    srv.close()
+    assert len(got) == len(tickets) and stats["batches"] < len(tickets) // 2
+    for t, w in zip(tickets, want * 3):
+        c, out = got[t]
+        assert c.status == 0 and c.sizes.ntriangles == w[0]
+        assert same_bits(out[0], w[1]) and same_bits(out[1], w[2])
+
+
 def test_server_refuses_unserved_requests(kvsmc_ctx):
     vols = _volumes(kvsmc_ctx)
     srv = _abi.Server(kvsmc_ctx)

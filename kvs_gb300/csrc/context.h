@@ -199,8 +199,8 @@ void volume_destroy(kvsmc_context* ctx, kvsmc_volume* v);
 kvsmc_status volume_create(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, uint32_t ny, uint32_t nz,
                            kvsmc_volume** out);
 
-// (Re)build a resident volume's brick min/max table, if it has one, and with it
-// its range from its values on the context's stream.
+// The values that a caller wrote into a volume on the context's stream are all
+// enqueued: its brick min/max table, if it has one, and with it its range.
 kvsmc_status volume_bricks(kvsmc_context* ctx, kvsmc_volume* v);
 
 // Run fn(i, stream) for i < n side by side on the context's auxiliary streams,

@@ -535,12 +535,14 @@ kvsmc_status volume_alloc(kvsmc_context* ctx, kvsmc_dtype dtype, uint32_t nx, ui
 
 kvsmc_status volume_bricks(kvsmc_context* ctx, kvsmc_volume* v)
 {
-    if (!v->bricks) return KVSMC_OK;
-    KVSMC_CUDA(ctx, kvsmc::launch_ingest(v->view, nullptr, v->bricks, v->range, launch_of(ctx)));
+    if (v->bricks) {
+        KVSMC_CUDA(ctx, kvsmc::launch_ingest(v->view, nullptr, v->bricks, v->range, launch_of(ctx)));
+        v->bricks_valid = true;
+        v->range_ready = true;
+    }
+    // (without a table too: the pass that turned a file's bytes may still run)
     v->ev_own = v->owner == ctx && ctx->stream == ctx->own_stream;
     KVSMC_CUDA(ctx, cudaEventRecord(v->ev, ctx->stream));
-    v->bricks_valid = true;
-    v->range_ready = true;
     return KVSMC_OK;
 }
 

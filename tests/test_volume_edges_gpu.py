@@ -9,7 +9,7 @@ import time
 import numpy as np
 import pytest
 
-from kvs_gb300 import _abi
+from kvs_gb300 import _abi, ingest
 
 from .helpers import same_bits
 from .test_volume_gpu import _check, _values
@@ -343,3 +343,36 @@ def test_long_padded_rows(kvsmc_ctx, dtype, nx):
     kvsmc_ctx.set_kernel_path(_abi.PATH_AUTO)
     assert sizes[0].ntriangles == sizes[1].ntriangles > 0
     dv.free()
+
+
+def test_an_update_behind_a_loaded_file(kvsmc_ctx, tmp_path):
+    """Doubles of the other byte order, whose range the header gives, are turned by
+    a pass that the load leaves running: an update on another stream waits for it."""
+    shape = (32, 64, 64)
+    v, w = _values(shape, np.float64, 1), _values(shape, np.float64, 2)
+    (tmp_path / "v.dat").write_bytes(v.astype(">f8").tobytes())
+    (tmp_path / "v.kvsml").write_text(
+        '<?xml version="1.0" ?><KVSML><Object type="StructuredVolumeObject"><StructuredVolumeObject grid_type="uniform" '
+        'resolution="64 64 32"><Node><Value veclen="1" min_value="-9" max_value="9"><DataArray type="double" '
+        'format="binary" file="v.dat" endian="big" /></Value></Node></StructuredVolumeObject></Object></KVSML>')
+    pinned = torch.from_numpy(w.copy()).pin_memory()
+    busy = torch.ones(1 << 28, device="cuda")
+    a, b, c = [torch.cuda.Stream() for _ in range(3)]
+    torch.cuda.synchronize()
+    try:
+        for turn in range(2):
+            with torch.cuda.stream(c):
+                for _ in range(300):
+                    busy.sin_()   # (the GPU's SMs are taken)
+            kvsmc_ctx.set_stream(a.cuda_stream)
+            dv, info = ingest.load_kvsml(kvsmc_ctx, tmp_path / "v.kvsml")
+            assert info["byte_swap"] and info["volume_max"] == 9.0
+            if turn == 1:
+                kvsmc_ctx.set_stream(b.cuda_stream)
+                kvsmc_ctx.check(kvsmc_ctx.lib.kvsmc_volume_update(kvsmc_ctx.handle, dv.handle, pinned.data_ptr()), "update")
+            torch.cuda.synchronize()
+            assert np.array_equal(dv.download(), w if turn == 1 else v)
+            dv.free()
+    finally:
+        torch.cuda.synchronize()
+        kvsmc_ctx.set_stream(None)
